@@ -99,6 +99,40 @@ def test_refine_normal_equations_match_oracle(tb, oracle):
         assert abs(st['chi2'][b] - c2o) <= 1e-9 * c2o, (b, st['chi2'][b], c2o)
 
 
+@pytest.mark.parametrize('n_src', [1, 2, 4, 5, 7, 8])
+def test_refine_crowded_tiles_match_oracle(tb, oracle, n_src):
+    """tb_fit_refine where n_src masks of odd sizes share tiles, cut by the
+    edges of an odd-sized image: up to four sources in one evaluation, more in
+    groups of three.  Tolerances as test_refine_normal_equations_match_oracle."""
+    w, datas, inverrs = _small_blobs(oracle, 11, n_blobs=1)
+    rng = np.random.default_rng(100 + n_src)
+    W, H = 45, 37
+    pick = rng.integers(0, len(w['truth']), n_src)
+    for k in ('truth', 'start'):
+        w[k] = w[k][pick].copy()
+        w[k][:, 0], w[k][:, 1] = np.linspace(9., W - 7.3, n_src), np.linspace(H - 6.2, 5., n_src)
+    w['start'] += rng.uniform(-0.02, 0.02, w['start'].shape)
+    src = np.zeros(n_src, w['sources'].dtype)
+    src['profile'] = w['sources']['profile'][0]
+    hw = rng.integers(9, 18, n_src)
+    src['x0'], src['y0'] = w['truth'][:, 0].astype(int) - hw, w['truth'][:, 1].astype(int) - hw
+    src['w'], src['h'] = 2 * hw + 1, 2 * hw
+    w.update(sources=src, blob_src=np.array([0, n_src]), sides=np.array([[W, H]]))
+    data = rng.normal(2., 1., (3, H, W)).astype(np.float32)
+    inv = rng.uniform(0.3, 1., (3, H, W)).astype(np.float32)
+    f = _fitter(w, [data], [inv])
+    f.reset(w['start'], 1e-9)
+    f._iteration(0.0, 100, precise=True)
+    _, _, _, _, rects = _blob_args(w, 0)
+    Ho, go, c2o = oracle.blob_normal_equations(w['start'], rects, W, H, w['psf'][0], 3,
+                                               data.astype(np.float64), inv.astype(np.float64))
+    Hg, gg = f.normal_equations(0)
+    d = np.sqrt(np.diag(Ho))
+    assert np.all(np.abs(Hg - Ho) <= 1e-6 * np.outer(d, d))
+    assert np.all(np.abs(gg - go) <= 1e-6 * d * np.sqrt(c2o) + 1e-9)
+    assert abs(f.states()['chi2'][0] - c2o) <= 1e-9 * c2o
+
+
 def test_fit_converges_to_fp64_optimum(tb, oracle):
     """From the same perturbed start, the batched FP32 fitter and the FP64
     oracle fitter reach the same optimum within 1e-3 sigma."""

@@ -804,9 +804,24 @@ __device__ double max_step(int off) {
 // the steps of an ill-conditioned blob to converge; the final iterations of
 // a fit take all of them in FP64.  Same units, slices and layout as
 // tb_fit_pass.
+//
+// Bound: FP64 issue in the component loop (a component costs 31 FP64
+// operations per pixel: exponent 3, exponential 10, value and C^-1 u 5,
+// moments 13).  So each warp stages, per pixel row, only the components that
+// reach its row of a source's mask; the trace terms are folded into the
+// second moments; and the products A^T A, A^T r go to the FP64 tensor core
+// (mma m8n8k4), accumulated in two registers per 8 x 8 block over a whole run
+// of tiles with the same sources, where 35 products per pixel and their
+// shuffle reductions took more instructions than the evaluation.  Measured on
+// 300 blobs (192-512 px, 3 bands): 52 passes 142 -> 58 ms, the first (all
+// blobs running) 3.5 ms; model + gradient of 100 blobs 3.4 -> 2.7 ms.
 // ---------------------------------------------------------------------------
 constexpr int kRefThreads = 256;       // one 32 x 8 tile, one pixel per thread
-constexpr int kRefChunks = 8;          // 16-value chunks staged before a flush
+constexpr int kRefWarps = kRefThreads / 32;
+constexpr int kRefSlots = 4;           // sources whose columns a warp holds at once
+constexpr int kRefLd = 36;             // doubles per column row (see ref_frag)
+constexpr int kRefXs = 8 * kRefLd;     // doubles per source: 7 columns and r
+constexpr double kRefFloor = -50.0 * TB_LOG2E;   // exponents below count as 0 (log2 units)
 
 struct RefSrc {
     int32_t x0, y0, x1, y1;
@@ -816,100 +831,25 @@ struct RefSrc {
     double dM[3][3];
 };
 
+// One component staged for one pixel row (dy = row - mean y) by the warp
+// that owns the row: exponent e(dx) = h00 dx^2 + bx dx + c0 in log2 units,
+// C^-1 u = (i00 dx + uxy, i01 dx + uyy).
+struct __align__(16) RefC {
+    double mx, h00, bx, c0;
+    double i00, i01, uxy, uyy;
+    double i11, s, sn, v;
+    double dv, pad;
+};
+
 struct RefSmem {
     RefSrc us[TB_FIT_MAX_SRC];
-    double red[kRefThreads / 32][kRefChunks * 16];
-    int dst[kRefChunks * 16];   // >= 0: H index; <= -2: g index -dst - 2; -1: none
+    RefC wc[kRefWarps][32];                         // a warp's staged components
+    double X[kRefWarps][kRefSlots * kRefXs];        // a warp's weighted columns and residuals
+    double exp_tab[tb::kExpTab];
+    double red[kRefWarps];
     int64_t slot;
     int skip;
 };
-
-// Sum over the warp of v[0 .. 16): afterwards lanes 2k and 2k + 1 hold the
-// sum of v[k] (a reduce-scatter: 16 shuffles instead of 16 x 5).
-__device__ __forceinline__ double warp_reduce_scatter16(double (&v)[16], int lane) {
-    {
-        const bool hi = lane & 16;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const double send = hi ? v[i] : v[i + 8];
-            const double keep = hi ? v[i + 8] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-        }
-    }
-    {
-        const bool hi = lane & 8;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const double send = hi ? v[i] : v[i + 4];
-            const double keep = hi ? v[i + 4] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-        }
-    }
-    {
-        const bool hi = lane & 4;
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const double send = hi ? v[i] : v[i + 2];
-            const double keep = hi ? v[i + 2] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-        }
-    }
-    {
-        const bool hi = lane & 2;
-        const double send = hi ? v[0] : v[1];
-        const double keep = hi ? v[1] : v[0];
-        v[0] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-    }
-    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
-
-// The staged chunks summed over the warps and added to their destinations
-// (each destination at most once per flush: a flush never spans two tiles).
-__device__ void ref_flush(RefSmem& sm, int& nc, double* H, double* g) {
-    __syncthreads();
-    for (int j = threadIdx.x; j < nc * 16; j += kRefThreads) {
-        const int d = sm.dst[j];
-        if (d == -1) continue;
-        double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < kRefThreads / 32; w++) s += sm.red[w][j];
-        if (d >= 0) H[d] += s;
-        else g[-d - 2] += s;
-    }
-    __syncthreads();
-    nc = 0;
-}
-
-// Stages NV values (value(q), q a compile-time index after unrolling) in
-// chunks of 16, their destinations dest(q) (run time, warp 0).
-template <int NV, class Val, class Dst>
-__device__ __forceinline__ void ref_emit(RefSmem& sm, int& nc, double* H, double* g, Val value,
-                                         Dst dest) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int c0 = 0; c0 < NV; c0 += 16) {
-        double v[16];
-#pragma unroll
-        for (int k = 0; k < 16; k++) v[k] = c0 + k < NV ? value(c0 + k) : 0.0;
-        const double s = warp_reduce_scatter16(v, lane);
-        const int k = lane >> 1;
-        if (!(lane & 1)) {
-            sm.red[warp][nc * 16 + k] = s;
-            if (warp == 0) sm.dst[nc * 16 + k] = c0 + k < NV ? dest(c0 + k) : -1;
-        }
-        if (++nc == kRefChunks) ref_flush(sm, nc, H, g);
-    }
-}
-
-// (i, j), i <= j < 7, of the q-th element of a 7 x 7 upper triangle
-// (row-major; rows start at 0, 7, 13, 18, 22, 25, 27).  Branch-free, so that
-// a compile-time q folds to constants.
-__host__ __device__ constexpr int tri_row(int q) {
-    return (q >= 7) + (q >= 13) + (q >= 18) + (q >= 22) + (q >= 25) + (q >= 27);
-}
-__host__ __device__ constexpr int tri_col(int q) {
-    return q - (tri_row(q) * 7 - tri_row(q) * (tri_row(q) - 1) / 2) + tri_row(q);
-}
 
 // Parameter slot of column i (x y flux(band) logre ee1 ee2 n) of source sI;
 // -1 where the profile has no such parameter.
@@ -920,108 +860,344 @@ __device__ __forceinline__ int ref_slot(int sI, int profile, int band, int i) {
     return i < 2 ? base + i : i == 2 ? base + 2 + band : base + 2 + i;
 }
 
-// Source R's model at (px, py) (counts x its unit-flux mixture), FP64.
-__device__ __forceinline__ double ref_model(const RefSrc& R, const FitC64* cs, int px, int py) {
-    if (!(px >= R.x0 && px < R.x1 && py >= R.y0 && py < R.y1)) return 0.0;
-    double val = 0.0;
-    for (int k = 0; k < R.K; k++) {
+// Stages, by one warp, those of the components cs[k0 .. min(k0 + 32, K)) that
+// reach pixels [x0, x1] (absolute, inclusive) of row y into wc[0 ..), in
+// their order; returns how many.  As stage_row: the exponent is a concave
+// quadratic along the row, so a component whose maximum over the segment
+// stays below the floor (FP32 with a margin of 1) is exactly zero there.
+__device__ __forceinline__ int ref_stage(RefC* wc, const FitC64* __restrict__ cs, int k0, int K,
+                                         int y, int x0, int x1) {
+    const int lane = threadIdx.x & 31;
+    const int k = k0 + lane;
+    bool keep = false;
+    double mx = 0.0, dy = 0.0, i00 = 0.0, i01 = 0.0, i11 = 0.0;
+    __syncwarp();   // the warp's previous components are no longer read
+    if (k < K) {
         const FitC64& c = cs[k];
-        const double dx = px - c.mx, dy = py - c.my;
-        const double ux = c.i00 * dx + c.i01 * dy, uy = c.i01 * dx + c.i11 * dy;
-        const double e = -0.5 * (dx * ux + dy * uy);
-        if (e >= -50.0) val += c.s * tb::exp_taylor(fmin(e, 0.0));
+        mx = c.mx;
+        dy = (double)y - c.my;
+        i00 = c.i00;
+        i01 = c.i01;
+        i11 = c.i11;
+        const float a = (float)i00, bb = (float)(i01 * dy), cc = (float)(i11 * dy * dy);
+        const float lo = (float)((double)x0 - mx), hi = (float)((double)x1 - mx);
+        const bool ok = isfinite(a) && isfinite(bb) && isfinite(cc) && isfinite(lo) && a > 0.f;
+        const float dx = fminf(fmaxf(-bb / a, lo), hi);
+        const float q = fmaf(dx, fmaf(a, dx, 2.f * bb), cc);   // Mahalanobis^2
+        keep = !ok || !(q > 102.f);
     }
-    return R.counts * val;
+    const unsigned bal = __ballot_sync(0xffffffffu, keep);
+    if (keep) {
+        const FitC64& c = cs[k];
+        double2* f = reinterpret_cast<double2*>(wc + __popc(bal & ((1u << lane) - 1u)));
+        f[0] = make_double2(mx, -0.5 * TB_LOG2E * i00);
+        f[1] = make_double2(-TB_LOG2E * i01 * dy, -0.5 * TB_LOG2E * i11 * dy * dy);
+        f[2] = make_double2(i00, i01);
+        f[3] = make_double2(i01 * dy, i11 * dy);
+        f[4] = make_double2(i11, c.s);
+        f[5] = make_double2(c.sn, c.v);
+        f[6] = make_double2(c.dv, 0.0);
+    }
+    __syncwarp();   // staged components visible to the whole warp
+    return __popc(bal);
 }
 
-// Source R's seven derivative columns at (px, py) (zero outside its
-// rectangle) and its model there, FP64: per component the moments of
-// C^-1 u (u = pixel - mean) that d/d(mean, C, amplitude) produce, combined
-// once per source with dM (shape) and M (index).
-__device__ __forceinline__ double ref_cols(const RefSrc& R, const FitC64* cs, int px, int py,
-                                           double (&J)[7]) {
-#pragma unroll
-    for (int j = 0; j < 7; j++) J[j] = 0.0;
-    if (!(px >= R.x0 && px < R.x1 && py >= R.y0 && py < R.y1)) return 0.0;
-    double S0 = 0, Sx = 0, Sy = 0, Axx = 0, Axy = 0, Ayy = 0, At0 = 0, At1 = 0, At2 = 0;
-    double Dxx = 0, Dxy = 0, Dyy = 0, Dt = 0, Sn = 0;
-    for (int k = 0; k < R.K; k++) {
-        const FitC64& c = cs[k];
-        const double dx = px - c.mx, dy = py - c.my;
-        const double ux = c.i00 * dx + c.i01 * dy, uy = c.i01 * dx + c.i11 * dy;
-        const double e = -0.5 * (dx * ux + dy * uy);
-        if (e < -50.0) continue;
-        const double E = tb::exp_taylor(fmin(e, 0.0));
-        const double val = c.s * E;
-        S0 += val;
-        Sx = fma(val, ux, Sx);
-        Sy = fma(val, uy, Sy);
-        const double vv = val * c.v;
-        Axx = fma(vv * ux, ux, Axx);
-        Axy = fma(vv * ux, uy, Axy);
-        Ayy = fma(vv * uy, uy, Ayy);
-        At0 = fma(vv, c.t[0], At0);
-        At1 = fma(vv, c.t[1], At1);
-        At2 = fma(vv, c.t[2], At2);
-        const double vd = val * c.dv;
-        Dxx = fma(vd * ux, ux, Dxx);
-        Dxy = fma(vd * ux, uy, Dxy);
-        Dyy = fma(vd * uy, uy, Dyy);
-        Dt = fma(vd, c.t[3], Dt);
-        Sn = fma(c.sn, E, Sn);
+// Source R's model at this thread's pixel of row py (counts x its unit-flux
+// mixture; 0 outside its rectangle), FP64.  Called by whole warps.
+__device__ __forceinline__ double ref_model(RefSmem& sm, const RefSrc& R,
+                                            const FitC64* __restrict__ cs, int ox, int py) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int xa = max(R.x0, ox), xb = min(R.x1, ox + kTileW);
+    if (py < R.y0 || py >= R.y1 || xa >= xb) return 0.0;   // warp-uniform
+    RefC* wc = sm.wc[warp];
+    const int px = ox + lane;
+    double val = 0.0;
+    for (int k0 = 0; k0 < R.K; k0 += 32) {
+        const int n = ref_stage(wc, cs, k0, R.K, py, xa, xb - 1);
+#pragma unroll 2
+        for (int g = 0; g < n; g++) {
+            const RefC& c = wc[g];
+            const double dx = (double)px - c.mx;
+            const double e = fma(dx, fma(c.h00, dx, c.bx), c.c0);
+            const double E = tb::exp2_tab(e, sm.exp_tab);
+            val = fma(e >= kRefFloor ? E : 0.0, c.s, val);
+        }
     }
-    const double cn = R.counts;
-    const double At[3] = {At0, At1, At2};
-    J[0] = cn * Sx;
-    J[1] = cn * Sy;
-    J[2] = S0;
+    return px >= xa && px < xb ? R.counts * val : 0.0;
+}
+
+// Source R's seven derivative columns, times w, at this thread's pixel of
+// row py into X[0 .. 7)[lane] (0 outside its rectangle); returns its model
+// there.  Per component the moments of C^-1 u (u = pixel - mean) that
+// d/d(mean, C, amplitude) produce, d/dC = 1/2 (C^-1 u u^T C^-1 - C^-1),
+// combined once per source with dM (shape) and M (index).  Called by whole
+// warps; no block barrier.
+__device__ __forceinline__ double ref_cols(RefSmem& sm, const RefSrc& R,
+                                           const FitC64* __restrict__ cs, int ox, int py,
+                                           double w, double* X) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int xa = max(R.x0, ox), xb = min(R.x1, ox + kTileW);
+    double S0 = 0, Sx = 0, Sy = 0, Axx = 0, Axy = 0, Ayy = 0, Dxx = 0, Dxy = 0, Dyy = 0, Sn = 0;
+    const int px = ox + lane;
+    const bool row = py >= R.y0 && py < R.y1 && xa < xb;   // warp-uniform
+    if (row) {
+        RefC* wc = sm.wc[warp];
+        for (int k0 = 0; k0 < R.K; k0 += 32) {
+            const int n = ref_stage(wc, cs, k0, R.K, py, xa, xb - 1);
+#pragma unroll 2
+            for (int g = 0; g < n; g++) {
+                const RefC& c = wc[g];
+                const double dx = (double)px - c.mx;
+                const double e = fma(dx, fma(c.h00, dx, c.bx), c.c0);
+                double E = tb::exp2_tab(e, sm.exp_tab);
+                if (!(e >= kRefFloor)) E = 0.0;
+                const double ux = fma(c.i00, dx, c.uxy), uy = fma(c.i01, dx, c.uyy);
+                const double val = c.s * E;
+                S0 += val;
+                Sx = fma(val, ux, Sx);
+                Sy = fma(val, uy, Sy);
+                const double pxx = fma(ux, ux, -c.i00), pxy = fma(ux, uy, -c.i01),
+                             pyy = fma(uy, uy, -c.i11);
+                const double vv = val * c.v, vd = val * c.dv;
+                Axx = fma(vv, pxx, Axx);
+                Axy = fma(vv, pxy, Axy);
+                Ayy = fma(vv, pyy, Ayy);
+                Dxx = fma(vd, pxx, Dxx);
+                Dxy = fma(vd, pxy, Dxy);
+                Dyy = fma(vd, pyy, Dyy);
+                Sn = fma(c.sn, E, Sn);
+            }
+        }
+    }
+    const bool in = row && px >= xa && px < xb;
+    const double cn = in ? R.counts : 0.0;
+    const double cw = cn * w, h = 0.5 * cw;
+    X[lane] = cw * Sx;
+    X[kRefLd + lane] = cw * Sy;
+    X[2 * kRefLd + lane] = in ? w * S0 : 0.0;
 #pragma unroll
     for (int j = 0; j < 3; j++)
-        J[3 + j] = cn * 0.5 * (R.dM[j][0] * Axx + 2.0 * R.dM[j][1] * Axy + R.dM[j][2] * Ayy - At[j]);
-    J[6] = cn * (0.5 * (R.M[0] * Dxx + 2.0 * R.M[1] * Dxy + R.M[2] * Dyy - Dt) + Sn);
+        X[(3 + j) * kRefLd + lane] =
+            h * (R.dM[j][0] * Axx + 2.0 * R.dM[j][1] * Axy + R.dM[j][2] * Ayy);
+    X[6 * kRefLd + lane] =
+        h * (R.M[0] * Dxx + 2.0 * R.M[1] * Dxy + R.M[2] * Dyy) + cw * Sn;
     return cn * S0;
 }
 
-// A source's own block: REFINE, its 28 A^T A products (upper triangle) and
-// 7 A^T r values; VJP, the 7 contracted columns.
-__device__ __forceinline__ void ref_emit_own(RefSmem& sm, int& nc, double* H, double* g,
-                                             const double (&Jw)[7], double rr, int sI,
-                                             const RefSrc& R, int band, int P, bool refine) {
-    if (refine) {
-        ref_emit<35>(sm, nc, H, g,
-            [&](int q) { return q < 28 ? Jw[tri_row(q)] * Jw[tri_col(q)] : Jw[q - 28] * rr; },
-            [&](int q) {
-                if (q >= 28) {
-                    const int s = ref_slot(sI, R.profile, band, q - 28);
-                    return s < 0 ? -1 : -s - 2;
-                }
-                const int a = ref_slot(sI, R.profile, band, tri_row(q));
-                const int c = ref_slot(sI, R.profile, band, tri_col(q));
-                return a < 0 || c < 0 ? -1 : a * P + c;
-            });
-    } else {
-        ref_emit<7>(sm, nc, H, g, [&](int q) { return Jw[q] * rr; },
-            [&](int q) {
-                const int s = ref_slot(sI, R.profile, band, q);
-                return s < 0 ? -1 : -s - 2;
-            });
+// A^T A and A^T r are contractions over pixels: with X_s the 8 x 32 matrix of
+// source s's seven weighted columns and the residual over a warp's 32
+// pixels, X_a X_b^T is a chain of eight FP64 m8n8k4 tensor-core products.
+// Their A and B fragments are the same element per lane,
+// X[lane / 4][4 step + lane % 4]; the row stride of 36 doubles puts the 16
+// lanes of each half warp in different banks.
+__device__ __forceinline__ double ref_frag(const double* X, int step) {
+    const int lane = threadIdx.x & 31;
+    return X[(lane >> 2) * kRefLd + 4 * step + (lane & 3)];
+}
+
+__device__ __forceinline__ void ref_mma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// The warps' NB 8 x 8 blocks summed (in warp order) and added to their
+// destinations: element (i, j) of block q, between sources sa(q) <= sb(q)
+// (-1: no such source), to H (upper triangle) or, in the residual's column, to g.
+// The blocks pass through the component staging area, kRefRound at a time.
+// Called by the whole block.
+constexpr int kRefRound = 5;
+static_assert(kRefRound * 64 * sizeof(double) <= 32 * sizeof(RefC), "blocks fit the staging area");
+
+template <int NB, class SA, class SB>
+__device__ __forceinline__ void ref_flush(RefSmem& sm, const double (&c)[NB][2], SA sa, SB sb,
+                                          double* H, double* g, int P, int band) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncwarp();   // the warp's staged components are read
+#pragma unroll
+    for (int q0 = 0; q0 < NB; q0 += kRefRound) {
+#pragma unroll
+        for (int q = q0; q < NB && q < q0 + kRefRound; q++)
+            reinterpret_cast<double2*>(sm.wc[warp])[(q - q0) * 32 + lane] =
+                make_double2(c[q][0], c[q][1]);
+        __syncthreads();
+        const int nb = NB - q0 < kRefRound ? NB - q0 : kRefRound;
+        for (int e = threadIdx.x; e < nb * 64; e += kRefThreads) {
+            const int q = q0 + (e >> 6), i = (e >> 3) & 7, j = e & 7;
+            const int a = sa(q), b = sb(q);
+            if (a < 0 || b < 0 || i == 7 || (j == 7 ? a != b || !g : !H || (a == b && j < i)))
+                continue;
+            const int di = ref_slot(a, sm.us[a].profile, band, i);
+            const int dj = j == 7 ? 0 : ref_slot(b, sm.us[b].profile, band, j);
+            if (di < 0 || dj < 0) continue;
+            double s = 0.0;
+#pragma unroll
+            for (int w = 0; w < kRefWarps; w++) s += reinterpret_cast<const double*>(sm.wc[w])[e];
+            if (j == 7) g[di] += s;
+            else H[(int64_t)di * P + dj] += s;
+        }
+        __syncthreads();
     }
 }
 
-// The A^T A block of two sources sA < sB (49 products).
-__device__ __forceinline__ void ref_emit_pair(RefSmem& sm, int& nc, double* H, double* g,
-                                              const double (&Ja)[7], const double (&Jb)[7],
-                                              int sA, int sB, int band, int P) {
-    const int pa = sm.us[sA].profile, pb = sm.us[sB].profile;
-    ref_emit<49>(sm, nc, H, g, [&](int q) { return Ja[q / 7] * Jb[q % 7]; },
-        [&](int q) {
-            const int a = ref_slot(sA, pa, band, q / 7);
-            const int c = ref_slot(sB, pb, band, q % 7);
-            return a < 0 || c < 0 ? -1 : a * P + c;
-        });
+// Block q of R sources: q < R a source's own block, then the pairs (0, 1),
+// (0, 2), .. (R - 2, R - 1).
+__host__ __device__ constexpr int ref_pair_a(int q, int R) {
+    if (q < R) return q;
+    int a = 0, n = q - R;
+    while (n >= R - 1 - a) { n -= R - 1 - a; a++; }
+    return a;
+}
+__host__ __device__ constexpr int ref_pair_b(int q, int R) {
+    if (q < R) return q;
+    int a = 0, n = q - R;
+    while (n >= R - 1 - a) { n -= R - 1 - a; a++; }
+    return a + 1 + n;
 }
 
-// CTAs per SM the refinement kernel is compiled for (2: 128 registers)
+// The unit a CTA works on.
+struct RefUnit {
+    const FitC64* comps;      // its band of source s: comps + s * cstride
+    int64_t cstride, pix_off;
+    const int32_t* tiles;
+    const float* data;        // data, or (VJP) the upstream gradient
+    const float* inverr;      // null: no weights (VJP)
+    double *H, *g;
+    int W, Hh, P, band;
+};
+
+// This thread's pixel of tile `code` (0 outside the image): its value and weight.
+__device__ __forceinline__ void ref_pixel(const RefUnit& u, int px, int py, double& d, double& w) {
+    d = w = 0.0;
+    if (px < u.W && py < u.Hh) {
+        const int64_t pix = u.pix_off + (int64_t)py * u.W + px;
+        d = u.data[pix];
+        w = u.inverr ? (double)u.inverr[pix] : 1.0;
+    }
+}
+
+// Tiles [t0, t1), all met by exactly the R sources `hit`: each warp adds its
+// rows' products into register blocks without a block barrier, then one
+// flush.  kResid: r = (data - model) inverr, every pair's block, chi^2;
+// otherwise (one source) r = data.
+template <int R, bool kResid>
+__device__ void ref_run(RefSmem& sm, const RefUnit& u, unsigned hit, int t0, int t1,
+                        double& chi2) {
+    constexpr int NB = R * (R + 1) / 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double* X = sm.X[warp];
+    double c[NB][2];
+#pragma unroll
+    for (int q = 0; q < NB; q++) c[q][0] = c[q][1] = 0.0;
+    for (int t = t0; t < t1; t++) {
+        const int ox = (u.tiles[t] & 0x3ff) * kTileW;
+        const int py = ((u.tiles[t] >> 10) & 0x3ff) * kTileH + warp;
+        double d, w;
+        ref_pixel(u, ox + lane, py, d, w);
+        double m = 0.0;
+        bool any = false;
+        unsigned hm = hit;
+        __syncwarp();   // the previous tile's fragments are read
+#pragma unroll 1
+        for (int s = 0; s < R; s++, hm &= hm - 1) {
+            const int sI = __ffs(hm) - 1;
+            const RefSrc& S = sm.us[sI];
+            any = any || (py >= S.y0 && py < S.y1);
+            m += ref_cols(sm, S, u.comps + sI * u.cstride, ox, py, w, X + s * kRefXs);
+        }
+        const double r = kResid ? (d - m) * w : d;
+        if (kResid) chi2 += r * r;
+        if (!any) continue;   // warp-uniform: every column is 0 in this row
+#pragma unroll
+        for (int s = 0; s < R; s++) X[s * kRefXs + 7 * kRefLd + lane] = r;
+        __syncwarp();
+#pragma unroll
+        for (int step = 0; step < 8; step++) {
+            double f[R];
+#pragma unroll
+            for (int s = 0; s < R; s++) f[s] = ref_frag(X + s * kRefXs, step);
+#pragma unroll
+            for (int q = 0; q < NB; q++) ref_mma(c[q], f[ref_pair_a(q, R)], f[ref_pair_b(q, R)]);
+        }
+    }
+    auto src = [&](int i) { return nth_bit(hit, i); };
+    ref_flush(sm, c, [&](int q) { return src(ref_pair_a(q, R)); },
+              [&](int q) { return src(ref_pair_b(q, R)); }, u.H, u.g, u.P, u.band);
+}
+
+// A tile that more than kRefSlots sources meet: the model first, then groups
+// of three sources (their own and mutual blocks), each followed by its
+// blocks with every later source, whose columns are evaluated again.
+__device__ void ref_crowded(RefSmem& sm, const RefUnit& u, unsigned hit, int code, double& chi2) {
+    constexpr int kG3 = kRefSlots - 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int R = __popc(hit);
+    double* X = sm.X[warp];
+    const int ox = (code & 0x3ff) * kTileW, py = ((code >> 10) & 0x3ff) * kTileH + warp;
+    double d, w;
+    ref_pixel(u, ox + lane, py, d, w);
+    double m = 0.0;
+    for (unsigned hm = hit; hm; hm &= hm - 1) {
+        const int sI = __ffs(hm) - 1;
+        m += ref_model(sm, sm.us[sI], u.comps + sI * u.cstride, ox, py);
+    }
+    const double r = (d - m) * w;
+    chi2 += r * r;
+    for (int q0 = 0; q0 < R; q0 += kG3) {
+        __syncwarp();
+        for (int s = 0; s < kG3; s++) {
+            double* Xs = X + s * kRefXs;
+            if (q0 + s < R) {
+                const int sI = nth_bit(hit, q0 + s);
+                ref_cols(sm, sm.us[sI], u.comps + sI * u.cstride, ox, py, w, Xs);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 7; c++) Xs[c * kRefLd + lane] = 0.0;
+            }
+            Xs[7 * kRefLd + lane] = r;
+        }
+        __syncwarp();
+        auto src = [&](int i) { return q0 + i < R ? nth_bit(hit, q0 + i) : -1; };
+        {
+            constexpr int NB = kG3 * (kG3 + 1) / 2;
+            double c[NB][2];
+#pragma unroll
+            for (int q = 0; q < NB; q++) c[q][0] = c[q][1] = 0.0;
+#pragma unroll
+            for (int step = 0; step < 8; step++) {
+                double f[kG3];
+#pragma unroll
+                for (int s = 0; s < kG3; s++) f[s] = ref_frag(X + s * kRefXs, step);
+#pragma unroll
+                for (int q = 0; q < NB; q++)
+                    ref_mma(c[q], f[ref_pair_a(q, kG3)], f[ref_pair_b(q, kG3)]);
+            }
+            ref_flush(sm, c, [&](int q) { return src(ref_pair_a(q, kG3)); },
+                      [&](int q) { return src(ref_pair_b(q, kG3)); }, u.H, u.g, u.P, u.band);
+        }
+        for (int i = q0 + kG3; i < R; i++) {
+            const int sI = nth_bit(hit, i);
+            double* Xb = X + kG3 * kRefXs;
+            __syncwarp();
+            ref_cols(sm, sm.us[sI], u.comps + sI * u.cstride, ox, py, w, Xb);
+            Xb[7 * kRefLd + lane] = r;
+            __syncwarp();
+            double c[kG3][2];
+#pragma unroll
+            for (int q = 0; q < kG3; q++) c[q][0] = c[q][1] = 0.0;
+#pragma unroll
+            for (int step = 0; step < 8; step++) {
+                const double fb = ref_frag(Xb, step);
+#pragma unroll
+                for (int q = 0; q < kG3; q++) ref_mma(c[q], ref_frag(X + q * kRefXs, step), fb);
+            }
+            ref_flush(sm, c, src, [&](int) { return sI; }, u.H, u.g, u.P, u.band);
+        }
+    }
+}
+
+// CTAs per SM the refinement kernel is compiled for (2: 128 registers, and
+// twice its shared memory fits)
 #ifndef TB_REFINE_MINB
 #define TB_REFINE_MINB 2
 #endif
@@ -1039,10 +1215,12 @@ fit_refine_kernel(const tb_fit_unit* __restrict__ units, const int32_t* __restri
     // (data - model) inverr; TB_FIT_MODEL: the model into model_out (every
     // blob); TB_FIT_VJP: the columns contracted with data = an upstream
     // gradient, unweighted
-    __shared__ RefSmem sm;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    RefSmem& sm = *reinterpret_cast<RefSmem*>(smem_raw);
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const bool refine = mode == TB_FIT_REFINE;
+    tb::exp2_tab_init(sm.exp_tab);   // read after next_unit's barriers
     for (;;) {
         const int64_t oi = tb::next_unit(counter, &sm.slot);
         if (oi >= n_units) break;
@@ -1098,106 +1276,85 @@ fit_refine_kernel(const tb_fit_unit* __restrict__ units, const int32_t* __restri
             if (tid == 0 && chi2_out) chi2_out[b.unit0 + u.slice] = INFINITY;
             continue;
         }
-        const FitC64* band_comps = gcomps + ((int64_t)b.src0 * n_bands + u.band) * kCompStride;
-        const int64_t cstride = (int64_t)n_bands * kCompStride;
+        RefUnit ru;
+        ru.comps = gcomps + ((int64_t)b.src0 * n_bands + u.band) * kCompStride;
+        ru.cstride = (int64_t)n_bands * kCompStride;
+        ru.pix_off = u.pix_off;
+        ru.tiles = tiles + b.tile_off + u.t0;
+        ru.data = data;
+        ru.inverr = refine ? inverr : nullptr;
+        ru.H = H;
+        ru.g = g;
+        ru.W = u.W;
+        ru.Hh = u.H;
+        ru.P = P;
+        ru.band = u.band;
         const int n_t = u.t1 - u.t0;
-        const int32_t* tl = tiles + b.tile_off + u.t0;
-        double chi2 = 0.0;
-        int nc = 0;
-        for (int t = 0; t < n_t; t++) {
-            const int ox = (tl[t] & 0x3ff) * kTileW, oy = ((tl[t] >> 10) & 0x3ff) * kTileH;
-            const int px = ox + lane, py = oy + warp;
-            const bool in = px < u.W && py < u.H;
-            // the sources whose rectangles meet the tile (the same for every thread)
-            unsigned reach = 0u;
+        // the sources whose rectangles meet a tile (the same for every warp)
+        auto reach = [&](int t) -> unsigned {
+            const int ox = (ru.tiles[t] & 0x3ff) * kTileW, oy = ((ru.tiles[t] >> 10) & 0x3ff) * kTileH;
+            bool hit = false;
             if (lane < nsrc) {
                 const RefSrc& R = sm.us[lane];
-                reach = R.x1 > ox && R.x0 < ox + kTileW && R.y1 > oy && R.y0 < oy + kTileH;
+                hit = R.x1 > ox && R.x0 < ox + kTileW && R.y1 > oy && R.y0 < oy + kTileH;
             }
-            reach = __ballot_sync(0xffffffffu, reach);
-            const int nreach = __popc(reach);
-            double d = 0.0, w = 0.0;
-            const int64_t pix = u.pix_off + (int64_t)py * u.W + px;
-            // MODEL reads neither data nor inverr (both may be NULL); VJP
-            // reads the upstream gradient in `data` and no weights
-            if (in && mode != TB_FIT_MODEL) {
-                d = data[pix];
-                w = mode == TB_FIT_VJP ? 1.0 : inverr[pix];
-            }
+            return __ballot_sync(0xffffffffu, hit);
+        };
+        double chi2 = 0.0;
+        int t = 0;
+        while (t < n_t) {
+            // a run of tiles that the same sources meet
+            const unsigned hit = reach(t);
+            int t1 = t + 1;
+            while (t1 < n_t && reach(t1) == hit) t1++;
             if (mode == TB_FIT_MODEL) {
-                double m = 0.0;
-                for (unsigned rm = reach; rm && in; rm &= rm - 1) {
-                    const int sI = __ffs(rm) - 1;
-                    m += ref_model(sm.us[sI], band_comps + sI * cstride, px, py);
+                for (; t < t1; t++) {
+                    const int ox = (ru.tiles[t] & 0x3ff) * kTileW;
+                    const int py = ((ru.tiles[t] >> 10) & 0x3ff) * kTileH + warp;
+                    double m = 0.0;
+                    for (unsigned hm = hit; hm; hm &= hm - 1) {
+                        const int sI = __ffs(hm) - 1;
+                        m += ref_model(sm, sm.us[sI], ru.comps + sI * ru.cstride, ox, py);
+                    }
+                    if (ox + lane < u.W && py < u.H)
+                        model_out[u.pix_off + (int64_t)py * u.W + ox + lane] = (float)m;
                 }
-                if (in) model_out[pix] = (float)m;
-                continue;
-            }
-            if (nreach <= 2) {
-                // one or two sources: their columns and the model in one evaluation
-                const int s0 = nreach > 0 ? __ffs(reach) - 1 : -1;
-                const int s1 = nreach > 1 ? __ffs(reach & (reach - 1)) - 1 : -1;
-                double J0[7], J1[7];
-                double m = 0.0;
-                if (s0 >= 0) m += ref_cols(sm.us[s0], band_comps + s0 * cstride, px, py, J0);
-                if (s1 >= 0) m += ref_cols(sm.us[s1], band_comps + s1 * cstride, px, py, J1);
-                const double r = refine ? (d - m) * w : d;
-                if (refine) chi2 += r * r;
-                if (s0 >= 0) {
-#pragma unroll
-                    for (int j = 0; j < 7; j++) J0[j] *= w;
-                    ref_emit_own(sm, nc, H, g, J0, r, s0, sm.us[s0], u.band, P, refine);
-                }
-                if (s1 >= 0) {
-#pragma unroll
-                    for (int j = 0; j < 7; j++) J1[j] *= w;
-                    ref_emit_own(sm, nc, H, g, J1, r, s1, sm.us[s1], u.band, P, refine);
-                    if (refine) ref_emit_pair(sm, nc, H, g, J0, J1, s0, s1, u.band, P);
-                }
+            } else if (!refine) {
+                // the upstream gradient does not depend on the model: one source at a time
+                for (unsigned hm = hit; hm; hm &= hm - 1)
+                    ref_run<1, false>(sm, ru, hm & (0u - hm), t, t1, chi2);
             } else {
-                // three or more: the model first, then each source's columns
-                // (a pair's block re-evaluates the later source)
-                double m = 0.0;
-                if (refine)
-                    for (unsigned rm = reach; rm; rm &= rm - 1) {
-                        const int sI = __ffs(rm) - 1;
-                        m += ref_model(sm.us[sI], band_comps + sI * cstride, px, py);
-                    }
-                const double r = refine ? (d - m) * w : d;
-                if (refine) chi2 += r * r;
-                for (unsigned ra = reach; ra; ra &= ra - 1) {
-                    const int sA = __ffs(ra) - 1;
-                    double Ja[7];
-                    ref_cols(sm.us[sA], band_comps + sA * cstride, px, py, Ja);
-#pragma unroll
-                    for (int j = 0; j < 7; j++) Ja[j] *= w;
-                    ref_emit_own(sm, nc, H, g, Ja, r, sA, sm.us[sA], u.band, P, refine);
-                    if (!refine) continue;
-                    for (unsigned rb = ra & (ra - 1); rb; rb &= rb - 1) {
-                        const int sB = __ffs(rb) - 1;
-                        double Jb[7];
-                        ref_cols(sm.us[sB], band_comps + sB * cstride, px, py, Jb);
-#pragma unroll
-                        for (int j = 0; j < 7; j++) Jb[j] *= w;
-                        ref_emit_pair(sm, nc, H, g, Ja, Jb, sA, sB, u.band, P);
-                    }
+                switch (__popc(hit)) {
+                    case 0:
+                        for (int q = t; q < t1; q++) {
+                            double d, w;
+                            ref_pixel(ru, (ru.tiles[q] & 0x3ff) * kTileW + lane,
+                                      ((ru.tiles[q] >> 10) & 0x3ff) * kTileH + warp, d, w);
+                            chi2 += d * w * (d * w);
+                        }
+                        break;
+                    case 1: ref_run<1, true>(sm, ru, hit, t, t1, chi2); break;
+                    case 2: ref_run<2, true>(sm, ru, hit, t, t1, chi2); break;
+                    case 3: ref_run<3, true>(sm, ru, hit, t, t1, chi2); break;
+                    case 4: ref_run<4, true>(sm, ru, hit, t, t1, chi2); break;
+                    default:
+                        for (int q = t; q < t1; q++) ref_crowded(sm, ru, hit, ru.tiles[q], chi2);
                 }
             }
-            if (nc > 0) ref_flush(sm, nc, H, g);
+            t = t1;
         }
         if (mode == TB_FIT_MODEL) continue;
         // the unit's chi^2 (its active tiles; the constant part stays in chi2_const)
         for (int o = 16; o > 0; o >>= 1) chi2 += __shfl_xor_sync(0xffffffffu, chi2, o);
-        if (lane == 0) sm.red[warp][0] = chi2;
+        if (lane == 0) sm.red[warp] = chi2;
         __syncthreads();
         if (tid == 0 && chi2_out) {
             // the slice's chi^2 with its constant part (the tiles no mask
             // reaches), as tb_fit_pass writes it
             double c2 = chi2_const ? chi2_const[b.unit0 + u.slice] : 0.0;
-            for (int w2 = 0; w2 < kRefThreads / 32; w2++) c2 += sm.red[w2][0];
+            for (int w2 = 0; w2 < kRefWarps; w2++) c2 += sm.red[w2];
             chi2_out[b.unit0 + u.slice] = c2;
         }
-        __syncthreads();
     }
 }
 
@@ -1619,14 +1776,18 @@ extern "C" int tb_fit_refine(const tb_fit_unit* units, const int32_t* order, int
     if (cudaMemsetAsync(work_counter, 0, sizeof(int32_t), s) != cudaSuccess) return TB_ERR_LAUNCH;
     if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
         return TB_ERR_LAUNCH;
+    const int smem = (int)sizeof(RefSmem);
+    if (cudaFuncSetAttribute(fit_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             smem) != cudaSuccess)
+        return TB_ERR_LAUNCH;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fit_refine_kernel, kRefThreads,
-                                                      0) != cudaSuccess || per_sm < 1)
+                                                      smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
     const int64_t want = (int64_t)tb::num_sms() * per_sm;
     const int grid = (int)(n_units < want ? n_units : want);
     void* ws = const_cast<void*>(workspace);
-    fit_refine_kernel<<<grid, kRefThreads, 0, s>>>(
+    fit_refine_kernel<<<grid, kRefThreads, smem, s>>>(
         units, order, n_units, blobs, srcs, ws_tab(ws), ws_comps64(ws, n_src, n_bands), data,
         inverr, hbuf, gbuf, chi2_out, state, n_bands, tiles, work_counter, status, TB_FIT_REFINE,
         nullptr, chi2_const);
@@ -1649,14 +1810,18 @@ extern "C" int tb_fit_model_vjp(const tb_fit_unit* units, const int32_t* order, 
     if (cudaMemsetAsync(work_counter, 0, sizeof(int32_t), s) != cudaSuccess) return TB_ERR_LAUNCH;
     if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
         return TB_ERR_LAUNCH;
+    const int smem = (int)sizeof(RefSmem);
+    if (cudaFuncSetAttribute(fit_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             smem) != cudaSuccess)
+        return TB_ERR_LAUNCH;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fit_refine_kernel, kRefThreads,
-                                                      0) != cudaSuccess || per_sm < 1)
+                                                      smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
     const int64_t want = (int64_t)tb::num_sms() * per_sm;
     const int grid = (int)(n_units < want ? n_units : want);
     void* ws = const_cast<void*>(workspace);
-    fit_refine_kernel<<<grid, kRefThreads, 0, s>>>(
+    fit_refine_kernel<<<grid, kRefThreads, smem, s>>>(
         units, order, n_units, blobs, srcs, ws_tab(ws), ws_comps64(ws, n_src, n_bands), grad,
         nullptr, nullptr, gbuf, nullptr, nullptr, n_bands, tiles, work_counter, status, mode,
         model, nullptr);

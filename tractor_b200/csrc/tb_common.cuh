@@ -10,31 +10,37 @@
 
 namespace tb {
 
-// 2^x on the SFU (MUFU.EX2), flushing denormal results to zero.
-// exp(e) in FP64 for -50 <= e <= 0 (the Gaussian exponents of the model
-// evaluations), relative error below 3e-13: e = k ln 2 + g with k =
-// rint(e / ln 2) and |g| <= ln 2 / 2 (|k| <= 73, so k ln 2 rounds to within
-// 6e-15), exp(g) by its Taylor series to degree 10 (remainder below
-// 0.347^11 / 11! = 2.3e-13) in Horner form, and 2^k written into the
-// exponent field (a normal double for k >= -1022).
-__device__ __forceinline__ double exp_taylor(double e) {
-    const double k = rint(e * 1.4426950408889634);
-    const double g = fma(k, -0.6931471805599453, e);
-    double p = 1.0 / 3628800.0;
-    p = fma(p, g, 1.0 / 362880.0);
-    p = fma(p, g, 1.0 / 40320.0);
-    p = fma(p, g, 1.0 / 5040.0);
-    p = fma(p, g, 1.0 / 720.0);
-    p = fma(p, g, 1.0 / 120.0);
-    p = fma(p, g, 1.0 / 24.0);
-    p = fma(p, g, 1.0 / 6.0);
-    p = fma(p, g, 0.5);
-    p = fma(p, g, 1.0);
-    p = fma(p, g, 1.0);
-    const long long bits = (long long)((int)k + 1023) << 52;
-    return p * __longlong_as_double(bits);
+// 2^e in FP64 for |e| < 1000 by the table-driven scheme of Tang (ACM TOMS
+// 15(2), 1989): n = rint(16 e), r = e - n / 16 exactly (|r| <= 1/32),
+// 2^e = 2^(n div 16) T[n mod 16] 2^r with T[j] = 2^(j / 16) and 2^r by its
+// Taylor series to degree 6 (remainder below (ln 2 / 32)^7 / 7! = 5e-16);
+// relative error below 1e-15.  Ten FP64 operations.  The 16 table entries
+// lie in 16 different pairs of shared-memory banks, so the lookups of a warp
+// never conflict.
+constexpr int kExpTab = 16;
+
+__device__ __forceinline__ void exp2_tab_init(double* tab) {
+    if (threadIdx.x < kExpTab) tab[threadIdx.x] = exp2((double)threadIdx.x / kExpTab);
 }
 
+__device__ __forceinline__ double exp2_tab(double e, const double* tab) {
+    const double magic = 6755399441055744.0;   // 1.5 x 2^52: rounds to an integer in the low word
+    const double t = fma(e, (double)kExpTab, magic);
+    const int n = __double2loint(t);
+    const double r = fma(t - magic, -1.0 / kExpTab, e);
+    // (ln 2)^k / k!
+    double p = 1.5403530393381610e-04;
+    p = fma(p, r, 1.3333558146428443e-03);
+    p = fma(p, r, 9.6181291076284772e-03);
+    p = fma(p, r, 5.5504108664821580e-02);
+    p = fma(p, r, 2.4022650695910072e-01);
+    p = fma(p, r, 6.9314718055994531e-01);
+    const double T = tab[n & (kExpTab - 1)];
+    const double y = fma(T * r, p, T);
+    return __hiloint2double(__double2hiint(y) + ((n >> 4) << 20), __double2loint(y));
+}
+
+// 2^x on the SFU (MUFU.EX2), flushing denormal results to zero.
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
