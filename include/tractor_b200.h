@@ -612,7 +612,10 @@ typedef struct {
 /* Buffers of blob b: hbuf + h_off holds (n_slices + 2) P x P FP64 blocks
  * (per-slice partial A^T A, accepted A^T A, Cholesky factor); gbuf + g_off
  * holds (n_slices + 1) P-vectors (per-slice A^T r, accepted).  A slice is
- * one pass unit's share: a band's image, or a range of its active tiles. */
+ * one pass unit's share: a band's image, or a range of its active tiles; the
+ * passes fill the slices of A^T A and A^T r compactly, over the sources their
+ * tiles meet, for tb_fit_step to sum (tb_fit_model_vjp's gradient slices are
+ * plain P-vectors). */
 typedef struct {
     int32_t n_src;            /* sources (<= TB_FIT_MAX_SRC) */
     int32_t src0;             /* first source */

@@ -133,6 +133,38 @@ def test_refine_crowded_tiles_match_oracle(tb, oracle, n_src):
     assert abs(f.states()['chi2'][0] - c2o) <= 1e-9 * c2o
 
 
+@pytest.mark.parametrize('n_src', [1, 3, 14, 15, 32])
+def test_step_solves_the_damped_equations(tb, oracle, n_src):
+    """tb_fit_step against numpy on the H and g it assembled: 9 to 288
+    parameters (padded, in shared memory up to 128, in global memory above).
+    With damping 0.3 the scaled matrix's condition number is at most
+    P / 0.3, so FP64 leaves 1e3 x 1e-16 x P: 1e-10 of the largest step."""
+    from tractor_b200 import fit
+    w = fit.blob_workload(1, np.random.default_rng(31), side_range=(150, 150), mean_src=40,
+                          max_src=n_src)
+    assert len(w['truth']) == n_src
+    data, inv = fit.render_blobs(w, w['truth'], seed=3)
+    f = fit.BlobFitter(w['blob_src'], w['sides'], w['psf'], w['sources'], w['start'], data, inv)
+    f.reset(w['start'], 1.0)
+    f._iteration(0.0, 100, precise=True)
+    H, g = f.normal_equations(0)
+    assert np.array_equal(H, H.T) and f.states()['accepted'][0] == 1
+    lam = f.states()['lambda'][0]
+    assert lam == 0.3
+    p = w['start'].ravel()
+    d = np.sqrt(np.diag(H))
+    assert np.all(d > 0)
+    x = np.linalg.solve(H / np.outer(d, d) + lam * np.eye(len(d)), g / d) / d
+    most = np.tile([1., 1., 0., 0., 0., 1., 0.1, 0.1, 0.1], n_src)
+    big = (most > 0) & (np.abs(x) > most)
+    lim = min([1.] + list(most[big] / np.abs(x[big])))
+    for i in range(8, len(p), 9):
+        if not 0.29 <= p[i] + x[i] <= 6.3:
+            lim = min(lim, ((6.3 if x[i] > 0 else 0.29) - p[i]) / x[i])
+    got = f.trial.cpu().numpy() - p
+    assert np.all(np.abs(got - lim * x) * d <= 1e-10 * np.max(np.abs(lim * x) * d))
+
+
 def test_fit_converges_to_fp64_optimum(tb, oracle):
     """From the same perturbed start, the batched FP32 fitter and the FP64
     oracle fitter reach the same optimum within 1e-3 sigma."""

@@ -33,84 +33,45 @@ constexpr int kThreads = 256;          // pass CTA = one 32 x 8 tile, one pixel 
 constexpr int kTileW = 32;
 constexpr int kTileH = 8;
 constexpr int kCols = 7;               // columns per (source, band): x y flux logre ee1 ee2 n
-constexpr int kG = 4;                  // sources per shared-memory column group
-constexpr int kLd = kThreads + 1;      // padded column stride (floats)
-constexpr double kHn = 1e-5;           // central-difference step in n
-constexpr double kHs = 1e-6;           // central-difference step in shape parameters
 
 constexpr int kCompStride = kMaxGalK * TB_FIT_MAX_PSF;   // component slots per (source, band)
 
 // Per-source summary written by tb_fit_prep.
 struct SrcTab {
     double flux[TB_FIT_MAX_BANDS];
-    float M[3];                    // T T^T (xx, xy, yy)
-    float dM[3][3];                // d(T T^T) / d(logre, ee1, ee2)
+    double M[3];                   // T T^T (xx, xy, yy)
+    double dM[3][3];               // d(T T^T) / d(logre, ee1, ee2)
     int32_t K[TB_FIT_MAX_BANDS];   // components in each band (galaxy x PSF)
     int32_t ok;
-    double M64[3];                 // the same in FP64 (refinement pass)
-    double dM64[3][3];
 };
 
-// One PSF-convolved component of a (source, band), written by tb_fit_prep:
-// value, position and shape-derivative coefficients, the 1/2 of dN/dC
-// folded in.  The mean stays FP64 (absolute pixels); the pass makes it
-// tile-relative.
-// The shape derivative of component k is dC_k = v_k dM (dM per source), the
-// index derivative dC_k = dv_k M: the pass accumulates per source the
-// moments sum_k val_k v_k u u^T and sum_k val_k dv_k u u^T over components
-// and applies dM / M once per source and pixel.
-struct FitC {
+// One PSF-convolved component of a (source, band), written by tb_fit_prep in
+// both precisions (FP32 for tb_fit_pass, FP64 for tb_fit_refine and
+// tb_fit_model_vjp).  The mean stays FP64 (absolute pixels); a pass makes it
+// tile-relative.  The shape derivative of component k is dC_k = v_k dM (dM
+// per source), the index derivative dC_k = dv_k M: the passes accumulate per
+// source the moments sum_k val_k v_k (u u^T - C_k^-1) and sum_k val_k dv_k
+// (u u^T - C_k^-1), u = C_k^-1 (pixel - mean), over components and apply dM
+// / M once per source and pixel.
+template <class T>
+struct __align__(16) FitC {
     double mx, my;
-    float qxx, qxy, qyy;      // exponent, log2 units
-    float ixx, ixy, iyy;      // C^-1
-    float s;                  // unit-flux amplitude a / (2 pi sqrt det)
-    float sn;                 // d a / d n / (2 pi sqrt det)
-    float fl;                 // exponent floor, log2 units
-    float v, dv;              // the galaxy component's variance and d/dn
-    float t[4];               // tr(C^-1 dM_j) (j < 3), tr(C^-1 M)
-    int32_t pad[7];
-};
-
-// The same component in FP64 for the refinement pass (tb_fit_refine): the
-// model and its derivative columns evaluated in FP64 at the end of a fit.
-struct FitC64 {
-    double mx, my;
-    double i00, i01, i11;     // C^-1
-    double s, sn;             // a / (2 pi sqrt det), d a / d n / (2 pi sqrt det)
-    double v, dv;             // galaxy variance and d/dn
-    double t[4];              // tr(C^-1 dM_j) (j < 3), tr(C^-1 M)
-    double pad[3];
-};
-
-// One component staged for one pixel row y of a tile (origin (ox, oy)) by
-// the warp that owns the row: its FP32 tile-relative mean x, the exponent
-// along the row e(dx) = qxx dx^2 + bx dx + c0 (bx = qxy dy, c0 = qyy dy^2,
-// dy = y - my), C^-1 u = (ixx dx + uxy, ixy dx + uyy) (uxy = ixy dy,
-// uyy = iyy dy), and the per-component factors of FitC.
-struct __align__(16) FitR {
-    float mx, qxx, bx, c0;
-    float s, fl, ixx, ixy;
-    float uxy, uyy, sn, v;
-    float dv, t0, t1, t2;
-    float t3, pad[3];
+    T i00, i01, i11;          // C^-1
+    T s, sn;                  // a / (2 pi sqrt det), d a / d n / (2 pi sqrt det)
+    T v, dv;                  // the galaxy component's variance and d/dn
+    T pad;
 };
 
 // ---------------------------------------------------------------------------
 // prep
 // ---------------------------------------------------------------------------
 
-__device__ void shape_M(const double* cd, double s0, double s1, double s2, double M[3]) {
-    double G[4], re;
-    tb::shape_basis(TB_SHAPE_ELLIPSE_ESOFT, s0, s1, s2, G, re);
-    tb::pixel_factor(cd, G, M[0], M[1], M[2]);
-}
-
 __global__ void __launch_bounds__(kPrepThreads)
 fit_prep_kernel(const tb_fit_source* __restrict__ srcs, int n, const double* __restrict__ params,
                 int n_bands, const tb_fit_unit* __restrict__ units, int n_units,
                 tb_profile_tables Tg, double cd0, double cd1, double cd2, double cd3,
-                SrcTab* __restrict__ tab, FitC* __restrict__ comps,
-                FitC64* __restrict__ comps64, const tb_fit_state* __restrict__ state) {
+                SrcTab* __restrict__ tab, FitC<float>* __restrict__ comps,
+                FitC<double>* __restrict__ comps64, const tb_fit_state* __restrict__ state) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const tb_profile_tables T = tb::stage_tables(Tg, smem_raw);
     const int lane = threadIdx.x & 31;
@@ -127,28 +88,11 @@ fit_prep_kernel(const tb_fit_source* __restrict__ srcs, int n, const double* __r
     double a = 0.0, v = 0.0, da = 0.0, dv = 0.0;
     int K = 0;
     if (s.profile == TB_PROFILE_SERSIC) {
-        double nn = p[8];
-        const double lowest = T.range_lohi[0], highest = T.range_lohi[2 * T.n_ranges - 1];
-        int r = -1;
-        bool clamped = false;
-        if (nn <= lowest) { r = 0; nn = lowest; clamped = true; }
-        else if (nn >= highest) { r = T.n_ranges - 1; nn = highest; clamped = true; }
-        else {
-            for (int q = 0; q < T.n_ranges; q++)
-                if (T.range_lohi[2 * q] <= nn && nn < T.range_lohi[2 * q + 1]) { r = q; break; }
-        }
-        if (r < 0 || T.range_info[4 * r] + 1 > kMaxGalK) {
+        K = tb::sersic_with_slope(T, p[8], lane, kMaxGalK, a, v, da, dv);
+        if (K < 0) {
             ok = 0;
+            K = 0;
         } else {
-            const bool core = nn > 1.0;
-            K = tb::sersic_fixed(T, r, nn, core, lane, a, v);
-            if (!clamped) {
-                double ap, vp, am, vm;
-                tb::sersic_fixed(T, r, nn + kHn, core, lane, ap, vp);
-                tb::sersic_fixed(T, r, nn - kHn, core, lane, am, vm);
-                da = (ap - am) / (2.0 * kHn);
-                dv = (vp - vm) / (2.0 * kHn);
-            }
             // components sorted by variance (sersic.py:338-341); the sort is
             // a permutation of lanes, kept fixed for the derivative
             const int rank = tb::variance_rank(v, K, lane);
@@ -172,23 +116,11 @@ fit_prep_kernel(const tb_fit_source* __restrict__ srcs, int n, const double* __r
     } else {
         ok = 0;
     }
-    // shape factor and its derivatives (every lane, redundantly)
     double M[3] = {0.0, 0.0, 0.0};
     double dM[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
     if (s.profile != TB_PROFILE_POINT) {
-        const double* sh = p + 5;
-        shape_M(cd, sh[0], sh[1], sh[2], M);
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            double hp[3] = {sh[0], sh[1], sh[2]}, hm[3] = {sh[0], sh[1], sh[2]};
-            hp[j] += kHs;
-            hm[j] -= kHs;
-            double Mp[3], Mm[3];
-            shape_M(cd, hp[0], hp[1], hp[2], Mp);
-            shape_M(cd, hm[0], hm[1], hm[2], Mm);
-#pragma unroll
-            for (int q = 0; q < 3; q++) dM[j][q] = (Mp[q] - Mm[q]) / (2.0 * kHs);
-        }
+        double re;
+        tb::shape_with_slopes(cd, TB_SHAPE_ELLIPSE_ESOFT, p[5], p[6], p[7], lane, M, dM, re);
     }
     bool fin = isfinite(p[0]) && isfinite(p[1]);
     for (int q = 0; q < 3; q++) fin = fin && isfinite(M[q]);
@@ -197,12 +129,13 @@ fit_prep_kernel(const tb_fit_source* __restrict__ srcs, int n, const double* __r
     // (inner), mixture_profiles.py:158-172
     int Kb[TB_FIT_MAX_BANDS] = {0, 0, 0};
     for (int bd = 0; bd < n_bands; bd++) {
+        ok = __all_sync(0xffffffffu, ok);   // a lane may have met a bad component
         const tb_fit_unit* u = ok ? units + (int64_t)s.blob * n_bands + bd : units;
         const int Kp = u->psf_K;
         if (Kp < 1 || Kp > TB_FIT_MAX_PSF) ok = 0;
         const int Kt = ok ? K * Kp : 0;
         Kb[bd] = Kt;
-        for (int k0 = 0; k0 < kCompStride; k0 += 32) {
+        for (int k0 = 0; k0 < Kt; k0 += 32) {
             const int k = k0 + lane;
             const int gi = (Kt > 0 && k < Kt) ? k % K : 0;
             const int pp = (Kt > 0 && k < Kt) ? k / K : 0;
@@ -217,48 +150,23 @@ fit_prep_kernel(const tb_fit_source* __restrict__ srcs, int n, const double* __r
             const double det = C00 * C11 - C01 * C01;
             const double i00 = C11 / det, i01 = -C01 / det, i11 = C00 / det;
             const double norm = 1.0 / (2.0 * TB_PI * sqrt(det));
-            FitC c;
-            c.mx = p[0] + u->psf_mean[2 * pp];
-            c.my = p[1] + u->psf_mean[2 * pp + 1];
-            c.qxx = (float)(-0.5 * TB_LOG2E * i00);
-            c.qxy = (float)(-TB_LOG2E * i01);
-            c.qyy = (float)(-0.5 * TB_LOG2E * i11);
-            c.ixx = (float)i00;
-            c.ixy = (float)i01;
-            c.iyy = (float)i11;
-            c.s = (float)(ag * u->psf_amp[pp] * norm);
-            c.sn = (float)(dag * u->psf_amp[pp] * norm);
-            c.fl = (float)(-50.0 * TB_LOG2E);
-            c.v = (float)vg;
-            c.dv = (float)dvg;
-            // dC / d(logre, ee1, ee2) = v dM_j; dC / dn = dv M
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const double* d = j < 3 ? dM[j] : M;
-                c.t[j] = (float)(i00 * d[0] + 2.0 * i01 * d[1] + i11 * d[2]);
-            }
-#pragma unroll
-            for (int q = 0; q < 7; q++) c.pad[q] = 0;
             const bool good = det > 0.0 && isfinite(norm);
             if (!good) ok = 0;
-            comps[((int64_t)i * n_bands + bd) * kCompStride + k] = c;
-            FitC64 c6;
-            c6.mx = c.mx;
-            c6.my = c.my;
-            c6.i00 = i00;
-            c6.i01 = i01;
-            c6.i11 = i11;
-            c6.s = ag * u->psf_amp[pp] * norm;
-            c6.sn = dag * u->psf_amp[pp] * norm;
-            c6.v = vg;
-            c6.dv = dvg;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const double* d = j < 3 ? dM[j] : M;
-                c6.t[j] = i00 * d[0] + 2.0 * i01 * d[1] + i11 * d[2];
-            }
-            c6.pad[0] = c6.pad[1] = c6.pad[2] = 0.0;
-            comps64[((int64_t)i * n_bands + bd) * kCompStride + k] = c6;
+            FitC<double> c;
+            c.mx = p[0] + u->psf_mean[2 * pp];
+            c.my = p[1] + u->psf_mean[2 * pp + 1];
+            c.i00 = i00;
+            c.i01 = i01;
+            c.i11 = i11;
+            c.s = ag * u->psf_amp[pp] * norm;
+            c.sn = dag * u->psf_amp[pp] * norm;
+            c.v = vg;
+            c.dv = dvg;
+            c.pad = 0.0;
+            const int64_t at = ((int64_t)i * n_bands + bd) * kCompStride + k;
+            comps64[at] = c;
+            comps[at] = FitC<float>{c.mx, c.my, (float)i00, (float)i01, (float)i11, (float)c.s,
+                                    (float)c.sn, (float)vg, (float)dvg, 0.f};
         }
     }
     ok = __all_sync(0xffffffffu, ok);
@@ -270,159 +178,78 @@ fit_prep_kernel(const tb_fit_source* __restrict__ srcs, int n, const double* __r
         }
         t.ok = ok;
         for (int q = 0; q < 3; q++) {
-            t.M[q] = (float)M[q];
-            t.M64[q] = M[q];
-            for (int j = 0; j < 3; j++) {
-                t.dM[j][q] = (float)dM[j][q];
-                t.dM64[j][q] = dM[j][q];
-            }
+            t.M[q] = M[q];
+            for (int j = 0; j < 3; j++) t.dM[j][q] = dM[j][q];
         }
         tab[i] = t;
     }
 }
 
 // ---------------------------------------------------------------------------
-// pass
+// pass (tb_fit_pass, FP32) and refinement pass (tb_fit_refine and
+// tb_fit_model_vjp, FP64): one kernel, compiled for both precisions.
+//
+// Near the optimum the gradient is a sum of terms that cancel, FP32 chi^2
+// cannot verify gains below ~1e-4, and an FP32 A^T A (FP32 columns: the index
+// column is a difference of nearly equal sums) is too inexact for the steps
+// of an ill-conditioned blob to converge; the final iterations of a fit take
+// all of them in FP64.
+//
+// Bound: issue in the component loop (FP64: 31 operations per pixel and
+// component: exponent 3, exponential 10, value and C^-1 u 5, moments 13).  So
+// each warp stages, per pixel row, only the components that reach its row of
+// a source's mask; the trace terms are folded into the second moments; and
+// the products A^T A, A^T r go to the FP64 tensor core (mma m8n8k4),
+// accumulated in two registers per 8 x 8 block over a whole run of tiles with
+// the same sources: no block barrier inside a run, no reduction per pixel.
+// MEASURED
 // ---------------------------------------------------------------------------
+constexpr int kWarps = kThreads / 32;
+constexpr int kSlots = 4;              // sources whose columns a warp holds at once
+constexpr int kLd = 36;                // elements per column row (see frag)
+constexpr int kXs = 8 * kLd;           // elements per source: 7 columns and r
 
-// One source of the unit (its mask rectangle and shape factors in the
-// unit's band), copied to shared memory once per unit.
+// What a launch computes: the normal equations and chi^2 of the running
+// blobs; chi^2 of the tiles no mask reaches (FP32); the model (FP64); the
+// columns contracted with an upstream gradient (FP64).
+enum Mode { kEquations, kConstant, kModel, kVjp };
+
+// One source of the unit, copied to shared memory once per unit.
+template <class T>
 struct UnitSrc {
     int32_t x0, y0, x1, y1;   // mask [x0, x1) x [y0, y1), image pixels; an empty mask is all 0
-    float counts;             // flux in the unit's band
-    int32_t K;                // components (galaxy x PSF) in the unit's band
-    float M[3];               // T T^T (xx, xy, yy)
-    float dM[3][3];           // its shape derivatives
+    int32_t K, profile;       // components (galaxy x PSF) in the unit's band
+    T counts;                 // flux in the unit's band
+    T M[3];                   // T T^T (xx, xy, yy)
+    T dM[3][3];               // its shape derivatives
 };
 
+// One component staged for one pixel row of a tile (dy = row - mean y) by
+// the warp that owns the row: tile-relative mean x, exponent
+// e(dx) = h00 dx^2 + bx dx + c0 in log2 units, C^-1 u = (i00 dx + uxy,
+// i01 dx + uyy).
+template <class T>
+struct __align__(16) RowC {
+    T mx, h00, bx, c0;
+    T i00, i01, uxy, uyy;
+    T i11, s, sn, v;
+    T dv, pad[sizeof(T) == 8 ? 1 : 3];
+};
+
+template <class T>
 struct PassSmem {
-    float A[2][kG * kCols][kLd];            // two column groups (multi-source tiles)
-    float hstage[kG * kCols][kG * kCols];   // a block of A^T A before its global update
-    float gstage[kG * kCols];               // a group's A^T r before its global update
-    FitR wc[kThreads / 32][kCompStride];    // each warp's components staged for its pixel row
-    UnitSrc us[TB_FIT_MAX_SRC];
-    float r[kThreads];
-    float runred[kThreads / 32][36];
-    double red[kThreads / 32];
+    UnitSrc<T> us[TB_FIT_MAX_SRC];
+    RowC<T> wc[kWarps][32];                 // a warp's staged components
+    T X[kWarps][kSlots * kXs];              // a warp's weighted columns and residuals
+    double exp_tab[tb::kExpTab];
+    double red[kWarps];
     int64_t slot;
     int skip;
 };
 
-// Stages, by one warp, the components of one source (src_comps[0, K)) that
-// reach pixels [x0, x1] (tile-relative, inclusive) of row y of the tile at
-// (ox, oy) into wc[0 ..), in their order; returns how many.  Along a row
-// the exponent is a concave quadratic in dx whose maximum over the segment
-// is at its vertex clamped to the segment.  A component whose maximum
-// stays below its floor (minus a margin of 1, far above FP32 rounding)
-// contributes exactly zero to every pixel of the segment (E = 0, val = 0)
-// and is left out, so the sums over the staged components are the same.
-// Components with non-finite or non-concave coefficients are always staged.
-// The row terms are computed as the per-pixel expressions would compute
-// them, so every pixel's exponent and C^-1 u is bit-identical.
-__device__ __forceinline__ int stage_row(FitR* wc, const FitC* __restrict__ src_comps, int K,
-                                         int ox, int oy, int y, float x0, float x1) {
-    const int lane = threadIdx.x & 31;
-    int n = 0;
-    __syncwarp();   // the warp's previous components are no longer read
-    for (int k0 = 0; k0 < K; k0 += 32) {
-        const int k = k0 + lane;
-        bool keep = false;
-        float mx = 0.f, dy = 0.f, bx = 0.f, c0 = 0.f;
-        if (k < K) {
-            const FitC& c = src_comps[k];
-            mx = (float)(c.mx - (double)ox);
-            dy = (float)y - (float)(c.my - (double)oy);
-            bx = c.qxy * dy;
-            c0 = c.qyy * dy * dy;
-            const float qxx = c.qxx;
-            const bool ok = isfinite(mx) && isfinite(bx) && isfinite(c0) && qxx < 0.f;
-            float emax = 0.f;
-            if (ok) {
-                const float xs = fminf(fmaxf(mx - bx / (2.f * qxx), x0), x1);
-                const float dx = xs - mx;
-                emax = fmaf(dx, fmaf(qxx, dx, bx), c0);
-            }
-            keep = !ok || !(emax < c.fl - 1.f);
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, keep);
-        if (keep) {
-            const FitC& c = src_comps[k];
-            float4* f = reinterpret_cast<float4*>(wc + n + __popc(bal & ((1u << lane) - 1u)));
-            f[0] = make_float4(mx, c.qxx, bx, c0);
-            f[1] = make_float4(c.s, c.fl, c.ixx, c.ixy);
-            f[2] = make_float4(c.ixy * dy, c.iyy * dy, c.sn, c.v);
-            f[3] = make_float4(c.dv, c.t[0], c.t[1], c.t[2]);
-            f[4] = make_float4(c.t[3], 0.f, 0.f, 0.f);
-        }
-        n += __popc(bal);
-    }
-    __syncwarp();   // staged components visible to the whole warp
-    return n;
-}
-
-// One source at this thread's pixel (lane, warp) of the tile at (ox, oy):
-// returns its model (counts x its PSF-convolved mixture, 0 outside its
-// mask) and, with kDeriv, its 7 weighted derivative columns in J (0 outside
-// the mask), d/dtheta = 1/2 (dM : sum v val u u^T - sum v val tr(C^-1 dM))
-// for the shape and likewise (M, dv) for the index.  The warp stages the
-// components that reach its row of the mask; a row outside the mask
-// evaluates nothing.  No block barrier: each warp works on its own.
-template <bool kDeriv>
-__device__ __forceinline__ float eval_source(FitR* wc, const FitC* __restrict__ src_comps,
-                                             const UnitSrc& U, int ox, int oy, float w,
-                                             float* J) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int xa = max(U.x0 - ox, 0), xb = min(U.x1 - ox, kTileW);
-    const bool row = warp >= U.y0 - oy && warp < U.y1 - oy && xa < xb;   // warp-uniform
-    float m = 0.f, jx = 0.f, jy = 0.f, jn = 0.f;
-    float axx = 0.f, axy = 0.f, ayy = 0.f, t0 = 0.f, t1 = 0.f, t2 = 0.f;
-    float bxx = 0.f, bxy = 0.f, byy = 0.f, tn = 0.f;
-    if (row) {
-        const int K = stage_row(wc, src_comps, U.K, ox, oy, warp, (float)xa, (float)(xb - 1));
-        const float xf = (float)lane;
-#pragma unroll 2
-        for (int g = 0; g < K; g++) {
-            const FitR& c = wc[g];
-            const float dx = xf - c.mx;
-            const float e = fmaf(dx, fmaf(c.qxx, dx, c.bx), c.c0);
-            const float E = (e >= c.fl) ? tb::ex2(e) : 0.f;
-            const float val = c.s * E;
-            m += val;
-            if (kDeriv) {
-                const float ux = fmaf(c.ixx, dx, c.uxy);
-                const float uy = fmaf(c.ixy, dx, c.uyy);
-                jx = fmaf(val, ux, jx);
-                jy = fmaf(val, uy, jy);
-                const float pxx = ux * ux, pxy = ux * uy, pyy = uy * uy;
-                const float sv = val * c.v, wv = val * c.dv;
-                axx = fmaf(sv, pxx, axx);
-                axy = fmaf(sv, pxy, axy);
-                ayy = fmaf(sv, pyy, ayy);
-                t0 = fmaf(sv, c.t0, t0);
-                t1 = fmaf(sv, c.t1, t1);
-                t2 = fmaf(sv, c.t2, t2);
-                bxx = fmaf(wv, pxx, bxx);
-                bxy = fmaf(wv, pxy, bxy);
-                byy = fmaf(wv, pyy, byy);
-                tn = fmaf(wv, c.t3, tn);
-                jn = fmaf(c.sn, E, jn);
-            }
-        }
-    }
-    const bool in = row && lane >= xa && lane < xb;
-    const float cnt = U.counts;
-    if (kDeriv) {
-        const float cw = in ? cnt * w : 0.f;
-        const float h = 0.5f * cw;
-        J[0] = cw * jx;
-        J[1] = cw * jy;
-        J[2] = in ? w * m : 0.f;
-        J[3] = h * (fmaf(U.dM[0][0], axx, fmaf(2.f * U.dM[0][1], axy, U.dM[0][2] * ayy)) - t0);
-        J[4] = h * (fmaf(U.dM[1][0], axx, fmaf(2.f * U.dM[1][1], axy, U.dM[1][2] * ayy)) - t1);
-        J[5] = h * (fmaf(U.dM[2][0], axx, fmaf(2.f * U.dM[2][1], axy, U.dM[2][2] * ayy)) - t2);
-        J[6] = h * (fmaf(U.M[0], bxx, fmaf(2.f * U.M[1], bxy, U.M[2] * byy)) - tn) + cw * jn;
-    }
-    return in ? cnt * m : 0.f;
+__device__ __forceinline__ float exp2_of(float e, const double*) { return tb::ex2(e); }
+__device__ __forceinline__ double exp2_of(double e, const double* tab) {
+    return tb::exp2_tab(e, tab);
 }
 
 // Position of the (q+1)-th set bit of m (q < popc(m)).
@@ -431,173 +258,399 @@ __device__ __forceinline__ int nth_bit(unsigned m, int q) {
     return __ffs(m) - 1;
 }
 
-// Sources q0 .. q0 + nq - 1 of the tile's hit list (the set bits of `hit`,
-// in source order) at this thread's pixel: returns their model; with
-// kDeriv writes the 7 columns of source q at A[7 (q - q0) + c][thread].
-// No block barrier inside.
-template <bool kDeriv>
-__device__ float eval_group(PassSmem& sm, const FitC* __restrict__ band_comps, int n_bands,
-                            unsigned hit, int q0, int nq, int ox, int oy, float w,
-                            float (*A)[kLd]) {
-    const int tid = threadIdx.x, warp = tid >> 5;
-    unsigned mm = hit;
-    for (int i = 0; i < q0; i++) mm &= mm - 1u;
-    float model = 0.f;
-    for (int q = q0; q < q0 + nq; q++) {
-        const int s = __ffs(mm) - 1;
-        mm &= mm - 1u;
-        float J[kCols];
-        model += eval_source<kDeriv>(sm.wc[warp], band_comps + (int64_t)s * n_bands * kCompStride,
-                                     sm.us[s], ox, oy, w, J);
-        if (kDeriv) {
-            float* col = &A[(q - q0) * kCols][tid];
-#pragma unroll
-            for (int c = 0; c < kCols; c++) col[c * kLd] = J[c];
-        }
-    }
-    return model;
+// Parameter slot of column i (x y flux(band) logre ee1 ee2 n) of source sI;
+// -1 where the profile has no such parameter.
+__device__ __forceinline__ int param_slot(int sI, int profile, int band, int i) {
+    if (i >= 3 && profile == TB_PROFILE_POINT) return -1;
+    if (i == 6 && profile != TB_PROFILE_SERSIC) return -1;
+    const int base = sI * TB_FIT_NPAR;
+    return i < 2 ? base + i : i == 2 ? base + 2 + band : base + 2 + i;
 }
 
-__device__ __forceinline__ int col_of(int src, int c, int band) {
-    // parameter slots per source: x, y, flux[3], logre, ee1, ee2, n
-    const int off = c < 2 ? c : (c == 2 ? 2 + band : c + 2);
-    return src * TB_FIT_NPAR + off;
+// Stages, by one warp, those of the components cs[k0 .. min(k0 + 32, K)) that
+// reach pixels [xa, xb] (tile-relative, inclusive) of row py of the tile at
+// column ox into wc[0 ..), in their order; returns how many.  Along a row the
+// exponent is a concave quadratic in dx whose maximum over the segment is at
+// its vertex clamped to the segment: a component whose Mahalanobis^2 stays
+// above 100 there (FP32, with a margin of 2) is exactly zero at every pixel
+// (exponents below -50 count as 0) and is left out.  Components with
+// non-finite coefficients are always staged.
+template <class T>
+__device__ __forceinline__ int stage_row(RowC<T>* wc, const FitC<T>* __restrict__ cs, int k0,
+                                         int K, int ox, int py, int xa, int xb) {
+    const int lane = threadIdx.x & 31;
+    const int k = k0 + lane;
+    bool keep = false;
+    T mx = 0, dy = 0, i00 = 0, i01 = 0, i11 = 0;
+    __syncwarp();   // the warp's previous components are no longer read
+    if (k < K) {
+        const FitC<T>& c = cs[k];
+        mx = (T)(c.mx - (double)ox);
+        dy = (T)((double)py - c.my);
+        i00 = c.i00;
+        i01 = c.i01;
+        i11 = c.i11;
+        const float a = (float)i00, bb = (float)(i01 * dy), cc = (float)(i11 * dy * dy);
+        const float lo = (float)((T)xa - mx), hi = (float)((T)xb - mx);
+        const bool ok = isfinite(a) && isfinite(bb) && isfinite(cc) && isfinite(lo) && a > 0.f;
+        const float dx = fminf(fmaxf(__fdividef(-bb, a), lo), hi);
+        keep = !ok || !(fmaf(dx, fmaf(a, dx, 2.f * bb), cc) > 102.f);
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, keep);
+    if (keep) {
+        const FitC<T>& c = cs[k];
+        RowC<T>& f = wc[__popc(bal & ((1u << lane) - 1u))];
+        f.mx = mx;
+        f.h00 = (T)(-0.5 * TB_LOG2E) * i00;
+        f.bx = (T)-TB_LOG2E * i01 * dy;
+        f.c0 = (T)(-0.5 * TB_LOG2E) * i11 * dy * dy;
+        f.i00 = i00;
+        f.i01 = i01;
+        f.uxy = i01 * dy;
+        f.uyy = i11 * dy;
+        f.i11 = i11;
+        f.s = c.s;
+        f.sn = c.sn;
+        f.v = c.v;
+        f.dv = c.dv;
+    }
+    __syncwarp();   // staged components visible to the whole warp
+    return __popc(bal);
 }
 
-// Adds a single-source run's register accumulators (this thread's share of
-// the 7 x 7 block's upper triangle and of A^T r) into the owned H / g:
-// warp reductions, then a fixed-order sum over warps.
-__device__ void flush_run(PassSmem& sm, float* hacc, float* gacc, int src, double* H, double* g,
-                          int P, int band) {
-    const int tid = threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-    for (int v = 0; v < 35; v++) {
-        float x = v < 28 ? hacc[v] : gacc[v - 28];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (lane == 0) sm.runred[warp][v] = x;
-    }
-    __syncthreads();
-    if (tid < 35) {
-        double sum = 0.0;
-        for (int w2 = 0; w2 < kThreads / 32; w2++) sum += (double)sm.runred[w2][tid];
-        if (tid < 28) {
-            // upper-triangle index tid -> (c, c'), row-major over c <= c'
-            int c = 0, base = 0;
-            while (base + (kCols - c) <= tid) { base += kCols - c; c++; }
-            const int c2 = c + (tid - base);
-            const int r = col_of(src, c, band), cc = col_of(src, c2, band);
-            H[(int64_t)r * P + cc] += sum;
-        } else {
-            g[col_of(src, tid - 28, band)] += sum;
-        }
-    }
-    __syncthreads();
-}
-
-// A_a^T A_b of the column groups in Aa (na sources) and Ab (nb sources)
-// into hstage (upper triangle when diag) and, with grad, A_a^T r into
-// gstage.  Tasks of 2 x 2 column pairs (or 2 gradient columns) go to the
-// warps in turn; each task splits the tile's pixels over the lanes
-// (conflict-free consecutive shared-memory reads), then reduces.
-__device__ void stage_products(PassSmem& sm, float (*Aa)[kLd], int na, float (*Ab)[kLd], int nb,
-                               bool diag, bool grad) {
+// Source S's model at this thread's pixel (column lane of the tile at ox,
+// row py): counts x its unit-flux mixture; 0 outside its mask.  Called by
+// whole warps.
+template <class T>
+__device__ __forceinline__ T source_model(PassSmem<T>& sm, const UnitSrc<T>& S,
+                                          const FitC<T>* __restrict__ cs, int ox, int py) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ca = na * kCols, cb = nb * kCols;
-    const int ba = (ca + 1) / 2, bb = (cb + 1) / 2;
-    const int nblk = diag ? ba * (ba + 1) / 2 : ba * bb;
-    const int ntask = nblk + (grad ? ba : 0);
-    for (int e = warp; e < ntask; e += kThreads / 32) {
-        if (e < nblk) {
-            int bi, bj;
-            if (diag) {   // row-major over the upper triangle of 2 x 2 blocks
-                int t = e;
-                bi = 0;
-                while (t >= ba - bi) { t -= ba - bi; bi++; }
-                bj = bi + t;
+    const int xa = max(S.x0 - ox, 0), xb = min(S.x1 - ox, kTileW);
+    if (py < S.y0 || py >= S.y1 || xa >= xb) return 0;   // warp-uniform
+    RowC<T>* wc = sm.wc[warp];
+    T val = 0;
+    for (int k0 = 0; k0 < S.K; k0 += 32) {
+        const int n = stage_row<T>(wc, cs, k0, S.K, ox, py, xa, xb - 1);
+#pragma unroll 2
+        for (int g = 0; g < n; g++) {
+            const RowC<T>& c = wc[g];
+            const T dx = (T)lane - c.mx;
+            const T e = fma(dx, fma(c.h00, dx, c.bx), c.c0);
+            const T E = exp2_of(e, sm.exp_tab);
+            val = fma(e >= (T)(-50.0 * TB_LOG2E) ? E : (T)0, c.s, val);
+        }
+    }
+    return lane >= xa && lane < xb ? S.counts * val : (T)0;
+}
+
+// Source S's seven derivative columns, times w, at this thread's pixel of
+// row py into X[0 .. 7)[lane] (0 outside its mask); returns its model there.
+// Per component the moments of u that d/d(mean, C, amplitude) produce,
+// d/dC = 1/2 (u u^T - C^-1), combined once per source with dM (shape) and M
+// (index).  Called by whole warps; no block barrier.
+template <class T>
+__device__ __forceinline__ T source_columns(PassSmem<T>& sm, const UnitSrc<T>& S,
+                                            const FitC<T>* __restrict__ cs, int ox, int py, T w,
+                                            T* X) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int xa = max(S.x0 - ox, 0), xb = min(S.x1 - ox, kTileW);
+    T S0 = 0, Sx = 0, Sy = 0, Axx = 0, Axy = 0, Ayy = 0, Dxx = 0, Dxy = 0, Dyy = 0, Sn = 0;
+    const bool row = py >= S.y0 && py < S.y1 && xa < xb;   // warp-uniform
+    if (row) {
+        RowC<T>* wc = sm.wc[warp];
+        for (int k0 = 0; k0 < S.K; k0 += 32) {
+            const int n = stage_row<T>(wc, cs, k0, S.K, ox, py, xa, xb - 1);
+#pragma unroll 2
+            for (int g = 0; g < n; g++) {
+                const RowC<T>& c = wc[g];
+                const T dx = (T)lane - c.mx;
+                const T e = fma(dx, fma(c.h00, dx, c.bx), c.c0);
+                T E = exp2_of(e, sm.exp_tab);
+                if (!(e >= (T)(-50.0 * TB_LOG2E))) E = 0;
+                const T ux = fma(c.i00, dx, c.uxy), uy = fma(c.i01, dx, c.uyy);
+                const T val = c.s * E;
+                S0 += val;
+                Sx = fma(val, ux, Sx);
+                Sy = fma(val, uy, Sy);
+                const T pxx = fma(ux, ux, -c.i00), pxy = fma(ux, uy, -c.i01),
+                        pyy = fma(uy, uy, -c.i11);
+                const T vv = val * c.v, vd = val * c.dv;
+                Axx = fma(vv, pxx, Axx);
+                Axy = fma(vv, pxy, Axy);
+                Ayy = fma(vv, pyy, Ayy);
+                Dxx = fma(vd, pxx, Dxx);
+                Dxy = fma(vd, pxy, Dxy);
+                Dyy = fma(vd, pyy, Dyy);
+                Sn = fma(c.sn, E, Sn);
+            }
+        }
+    }
+    const bool in = row && lane >= xa && lane < xb;
+    const T cn = in ? S.counts : (T)0;
+    const T cw = cn * w, h = (T)0.5 * cw;
+    X[lane] = cw * Sx;
+    X[kLd + lane] = cw * Sy;
+    X[2 * kLd + lane] = in ? w * S0 : (T)0;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+        X[(3 + j) * kLd + lane] =
+            h * (S.dM[j][0] * Axx + (T)2 * S.dM[j][1] * Axy + S.dM[j][2] * Ayy);
+    X[6 * kLd + lane] =
+        h * (S.M[0] * Dxx + (T)2 * S.M[1] * Dxy + S.M[2] * Dyy) + cw * Sn;
+    return cn * S0;
+}
+
+// A^T A and A^T r are contractions over pixels: with X_s the 8 x 32 matrix of
+// source s's seven weighted columns and the residual over a warp's 32
+// pixels, X_a X_b^T is a chain of eight FP64 m8n8k4 tensor-core products
+// (FP32 columns are widened first).  Their A and B fragments are the same
+// element per lane, X[lane / 4][4 step + lane % 4]; the row stride of 36
+// elements puts the lanes of a (half, FP64) warp in different banks.
+template <class T>
+__device__ __forceinline__ double frag(const T* X, int step) {
+    const int lane = threadIdx.x & 31;
+    return (double)X[(lane >> 2) * kLd + 4 * step + (lane & 3)];
+}
+
+__device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// Where a unit adds its products.  kVjp: g alone, by parameter slot (P per
+// slice).  kEquations: compact slices that hold only the m sources whose masks
+// meet the unit (`mask`), seven columns each: a (7 m)^2 block of H (upper
+// triangle) and 7 m of g, so that a unit of a few tiles in a large blob neither
+// clears nor passes on a P x P block; the mask itself, and the band above it,
+// go to the slice's last g slot (7 m < 9 m <= P).
+struct SliceOut {
+    double *H, *g;
+    unsigned mask;
+    int ld;                   // 7 m
+    int P, band;
+};
+
+__device__ __forceinline__ int compact_row(unsigned mask, int src) {
+    return kCols * __popc(mask & ((1u << src) - 1u));
+}
+
+// The warps' NB 8 x 8 blocks summed (in warp order) and added to their
+// destinations: element (i, j) of block q, between sources sa(q) <= sb(q)
+// (-1: no such source), to H (upper triangle) or, in the residual's column,
+// to g.  The blocks pass through the component staging area, a round at a
+// time.  Called by the whole block.
+template <class T, int NB, class SA, class SB>
+__device__ __forceinline__ void flush(PassSmem<T>& sm, const double (&c)[NB][2], SA sa, SB sb,
+                                      const SliceOut& o) {
+    constexpr int kRound = (int)(32 * sizeof(RowC<T>) / (64 * sizeof(double)));
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncwarp();   // the warp's staged components are read
+#pragma unroll
+    for (int q0 = 0; q0 < NB; q0 += kRound) {
+#pragma unroll
+        for (int q = q0; q < NB && q < q0 + kRound; q++)
+            reinterpret_cast<double2*>(sm.wc[warp])[(q - q0) * 32 + lane] =
+                make_double2(c[q][0], c[q][1]);
+        __syncthreads();
+        const int nb = NB - q0 < kRound ? NB - q0 : kRound;
+        for (int e = threadIdx.x; e < nb * 64; e += kThreads) {
+            const int q = q0 + (e >> 6), i = (e >> 3) & 7, j = e & 7;
+            const int a = sa(q), b = sb(q);
+            if (a < 0 || b < 0 || i == 7 || (j == 7 ? a != b : !o.H || (a == b && j < i))) continue;
+            double s = 0.0;
+#pragma unroll
+            for (int w = 0; w < kWarps; w++) s += reinterpret_cast<const double*>(sm.wc[w])[e];
+            if (o.H) {
+                const int di = compact_row(o.mask, a) + i;
+                if (j == 7) o.g[di] += s;
+                else o.H[di * o.ld + compact_row(o.mask, b) + j] += s;
             } else {
-                bi = e / bb;
-                bj = e % bb;
+                const int di = param_slot(a, sm.us[a].profile, o.band, i);
+                if (di >= 0) o.g[di] += s;
             }
-            const int i = 2 * bi, j = 2 * bj;
-            const int i1 = min(i + 1, ca - 1), j1 = min(j + 1, cb - 1);
-            float s00 = 0.f, s01 = 0.f, s10 = 0.f, s11 = 0.f;
+        }
+        __syncthreads();
+    }
+}
+
+// Block q of R sources: q < R a source's own block, then the pairs (0, 1),
+// (0, 2), .. (R - 2, R - 1).
+__host__ __device__ constexpr int pair_a(int q, int R) {
+    if (q < R) return q;
+    int a = 0, n = q - R;
+    while (n >= R - 1 - a) { n -= R - 1 - a; a++; }
+    return a;
+}
+__host__ __device__ constexpr int pair_b(int q, int R) {
+    if (q < R) return q;
+    int a = 0, n = q - R;
+    while (n >= R - 1 - a) { n -= R - 1 - a; a++; }
+    return a + 1 + n;
+}
+
+// The unit a CTA works on.
+template <class T>
+struct PassUnit {
+    const FitC<T>* comps;     // its band of source s: comps + s * cstride
+    int64_t cstride, pix_off;
+    const int32_t* tiles;
+    const float* data;        // data, or (VJP) the upstream gradient
+    const float* inverr;      // null: no weights (VJP)
+    int W, Hh;
+    SliceOut out;
+};
+
+// This thread's pixel (0 outside the image): its value and weight.
+template <class T>
+__device__ __forceinline__ void load_pixel(const PassUnit<T>& u, int px, int py, T& d, T& w) {
+    d = w = 0;
+    if (px < u.W && py < u.Hh) {
+        const int64_t pix = u.pix_off + (int64_t)py * u.W + px;
+        d = (T)u.data[pix];
+        w = u.inverr ? (T)u.inverr[pix] : (T)1;
+    }
+}
+
+// Tiles [t0, t1), all met by exactly the R sources `hit`: each warp adds its
+// rows' products into register blocks without a block barrier, then one
+// flush.  kResid: r = (data - model) inverr, every pair's block, chi^2;
+// otherwise (one source) r = data.
+template <class T, int R, bool kResid>
+__device__ void run_tiles(PassSmem<T>& sm, const PassUnit<T>& u, unsigned hit, int t0, int t1,
+                          double& chi2) {
+    constexpr int NB = R * (R + 1) / 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T* X = sm.X[warp];
+    double c[NB][2];
 #pragma unroll
-            for (int p = lane; p < kThreads; p += 32) {
-                const float x0 = Aa[i][p], x1 = Aa[i1][p], y0 = Ab[j][p], y1 = Ab[j1][p];
-                s00 = fmaf(x0, y0, s00);
-                s01 = fmaf(x0, y1, s01);
-                s10 = fmaf(x1, y0, s10);
-                s11 = fmaf(x1, y1, s11);
-            }
+    for (int q = 0; q < NB; q++) c[q][0] = c[q][1] = 0.0;
+    for (int t = t0; t < t1; t++) {
+        const int ox = (u.tiles[t] & 0x3ff) * kTileW;
+        const int py = ((u.tiles[t] >> 10) & 0x3ff) * kTileH + warp;
+        T d, w;
+        load_pixel(u, ox + lane, py, d, w);
+        T m = 0;
+        bool any = false;
+        unsigned hm = hit;
+        __syncwarp();   // the previous tile's fragments are read
+#pragma unroll 1
+        for (int s = 0; s < R; s++, hm &= hm - 1) {
+            const int sI = __ffs(hm) - 1;
+            const UnitSrc<T>& S = sm.us[sI];
+            any = any || (py >= S.y0 && py < S.y1);
+            m += source_columns<T>(sm, S, u.comps + sI * u.cstride, ox, py, w, X + s * kXs);
+        }
+        const T r = kResid ? (d - m) * w : d;
+        if (kResid) chi2 += (double)(r * r);
+        if (!any) continue;   // warp-uniform: every column is 0 in this row
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                s00 += __shfl_xor_sync(0xffffffffu, s00, o);
-                s01 += __shfl_xor_sync(0xffffffffu, s01, o);
-                s10 += __shfl_xor_sync(0xffffffffu, s10, o);
-                s11 += __shfl_xor_sync(0xffffffffu, s11, o);
-            }
-            if (lane < 4) {
-                const int di = lane >> 1, dj = lane & 1;
-                const int ii = i + di, jj = j + dj;
-                if (ii < ca && jj < cb && !(diag && jj < ii))
-                    sm.hstage[ii][jj] = di == 0 ? (dj == 0 ? s00 : s01) : (dj == 0 ? s10 : s11);
-            }
-        } else {
-            const int i = 2 * (e - nblk), i1 = min(i + 1, ca - 1);
-            float s0 = 0.f, s1 = 0.f;
+        for (int s = 0; s < R; s++) X[s * kXs + 7 * kLd + lane] = r;
+        __syncwarp();
 #pragma unroll
-            for (int p = lane; p < kThreads; p += 32) {
-                const float rp = sm.r[p];
-                s0 = fmaf(Aa[i][p], rp, s0);
-                s1 = fmaf(Aa[i1][p], rp, s1);
-            }
+        for (int step = 0; step < 8; step++) {
+            double f[R];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-                s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+            for (int s = 0; s < R; s++) f[s] = frag(X + s * kXs, step);
+#pragma unroll
+            for (int q = 0; q < NB; q++) mma884(c[q], f[pair_a(q, R)], f[pair_b(q, R)]);
+        }
+    }
+    auto src = [&](int i) { return nth_bit(hit, i); };
+    flush<T, NB>(sm, c, [&](int q) { return src(pair_a(q, R)); },
+                 [&](int q) { return src(pair_b(q, R)); }, u.out);
+}
+
+// A tile that more than kSlots sources meet: the model first, then groups of
+// three sources (their own and mutual blocks), each followed by its blocks
+// with every later source, whose columns are evaluated again.
+template <class T>
+__device__ void crowded_tile(PassSmem<T>& sm, const PassUnit<T>& u, unsigned hit, int code,
+                             double& chi2) {
+    constexpr int kG3 = kSlots - 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int R = __popc(hit);
+    T* X = sm.X[warp];
+    const int ox = (code & 0x3ff) * kTileW, py = ((code >> 10) & 0x3ff) * kTileH + warp;
+    T d, w;
+    load_pixel(u, ox + lane, py, d, w);
+    T m = 0;
+    for (unsigned hm = hit; hm; hm &= hm - 1) {
+        const int sI = __ffs(hm) - 1;
+        m += source_model<T>(sm, sm.us[sI], u.comps + sI * u.cstride, ox, py);
+    }
+    const T r = (d - m) * w;
+    chi2 += (double)(r * r);
+    for (int q0 = 0; q0 < R; q0 += kG3) {
+        __syncwarp();
+        for (int s = 0; s < kG3; s++) {
+            T* Xs = X + s * kXs;
+            if (q0 + s < R) {
+                const int sI = nth_bit(hit, q0 + s);
+                source_columns<T>(sm, sm.us[sI], u.comps + sI * u.cstride, ox, py, w, Xs);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 7; c++) Xs[c * kLd + lane] = 0;
             }
-            if (lane == 0) sm.gstage[i] = s0;
-            if (lane == 1 && i + 1 < ca) sm.gstage[i + 1] = s1;
+            Xs[7 * kLd + lane] = r;
+        }
+        __syncwarp();
+        auto src = [&](int i) { return q0 + i < R ? nth_bit(hit, q0 + i) : -1; };
+        {
+            constexpr int NB = kG3 * (kG3 + 1) / 2;
+            double c[NB][2];
+#pragma unroll
+            for (int q = 0; q < NB; q++) c[q][0] = c[q][1] = 0.0;
+#pragma unroll
+            for (int step = 0; step < 8; step++) {
+                double f[kG3];
+#pragma unroll
+                for (int s = 0; s < kG3; s++) f[s] = frag(X + s * kXs, step);
+#pragma unroll
+                for (int q = 0; q < NB; q++) mma884(c[q], f[pair_a(q, kG3)], f[pair_b(q, kG3)]);
+            }
+            flush<T, NB>(sm, c, [&](int q) { return src(pair_a(q, kG3)); },
+                         [&](int q) { return src(pair_b(q, kG3)); }, u.out);
+        }
+        for (int i = q0 + kG3; i < R; i++) {
+            const int sI = nth_bit(hit, i);
+            T* Xb = X + kG3 * kXs;
+            __syncwarp();
+            source_columns<T>(sm, sm.us[sI], u.comps + sI * u.cstride, ox, py, w, Xb);
+            Xb[7 * kLd + lane] = r;
+            __syncwarp();
+            double c[kG3][2];
+#pragma unroll
+            for (int q = 0; q < kG3; q++) c[q][0] = c[q][1] = 0.0;
+#pragma unroll
+            for (int step = 0; step < 8; step++) {
+                const double fb = frag(Xb, step);
+#pragma unroll
+                for (int q = 0; q < kG3; q++) mma884(c[q], frag(X + q * kXs, step), fb);
+            }
+            flush<T, kG3>(sm, c, src, [&](int) { return sI; }, u.out);
         }
     }
 }
 
-// The staged products' global updates by all threads at once (each element
-// of the owned H / g once: independent read-modify-writes).  Column c of
-// group a belongs to hit source qa0 + c / 7 (likewise for b).
-__device__ void apply_products(PassSmem& sm, unsigned hit, int qa0, int na, int qb0, int nb,
-                               bool diag, bool grad, double* H, double* g, int P, int band) {
-    const int ca = na * kCols, cb = nb * kCols;
-    for (int e = threadIdx.x; e < ca * cb; e += kThreads) {
-        const int ii = e / cb, jj = e % cb;
-        if (diag && jj < ii) continue;
-        const int ga = col_of(nth_bit(hit, qa0 + ii / kCols), ii % kCols, band);
-        const int gb = col_of(nth_bit(hit, qb0 + jj / kCols), jj % kCols, band);
-        // upper triangle in global parameter order
-        const int r = min(ga, gb), c = max(ga, gb);
-        H[(int64_t)r * P + c] += (double)sm.hstage[ii][jj];
-    }
-    if (grad)
-        for (int c = threadIdx.x; c < ca; c += kThreads)
-            g[col_of(nth_bit(hit, qa0 + c / kCols), c % kCols, band)] += (double)sm.gstage[c];
-}
-
+// Two CTAs per SM: 128 registers hold the ten blocks of four sources without
+// spills in FP32 (three CTAs at 80 registers measured 8 % slower, four 17 %).
+template <class T>
 __global__ void __launch_bounds__(kThreads, 2)
 fit_pass_kernel(const tb_fit_unit* __restrict__ units, const int32_t* __restrict__ order,
                 int n_units, const tb_fit_blob* __restrict__ blobs,
                 const tb_fit_source* __restrict__ srcs, const SrcTab* __restrict__ tab,
-                const FitC* __restrict__ gcomps, const float* __restrict__ data,
+                const FitC<T>* __restrict__ gcomps, const float* __restrict__ data,
                 const float* __restrict__ inverr, double* __restrict__ hbuf,
                 double* __restrict__ gbuf, double* __restrict__ chi2_part,
                 const tb_fit_state* __restrict__ state, int n_bands,
-                const int32_t* __restrict__ tiles, double* __restrict__ chi2_const, int mode,
-                int32_t* counter, tb_status* st) {
+                const int32_t* __restrict__ tiles, double* chi2_const, Mode mode,
+                float* __restrict__ model_out, int32_t* counter, tb_status* st) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    PassSmem& sm = *reinterpret_cast<PassSmem*>(smem_raw);
+    PassSmem<T>& sm = *reinterpret_cast<PassSmem<T>*>(smem_raw);
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
+    if (sizeof(T) == 8) tb::exp2_tab_init(sm.exp_tab);   // read after next_unit's barriers
     for (;;) {
         const int64_t oi = tb::next_unit(counter, &sm.slot);   // barriers on both sides
         if (oi >= n_units) break;
@@ -608,15 +661,9 @@ fit_pass_kernel(const tb_fit_unit* __restrict__ units, const int32_t* __restrict
         }
         const tb_fit_unit& u = units[ui];
         const tb_fit_blob b = blobs[u.blob];
-        if (mode == 0 && state[u.blob].status != 0) continue;   // converged or stopped
+        if (mode == kEquations && state[u.blob].status != 0) continue;   // converged or stopped
         const int P = b.P;
         const int nsrc = b.n_src;
-        double* H = hbuf + b.h_off + (int64_t)u.slice * P * P;
-        double* g = gbuf + b.g_off + (int64_t)u.slice * P;
-        if (mode == 0) {
-            for (int e = tid; e < P * P; e += kThreads) H[e] = 0.0;
-            for (int e = tid; e < P; e += kThreads) g[e] = 0.0;
-        }
         // checks, and the unit's sources into shared memory (lane = source)
         if (warp == 0) {
             const bool unit_bad = nsrc < 0 || nsrc > TB_FIT_MAX_SRC || P != nsrc * TB_FIT_NPAR ||
@@ -630,18 +677,19 @@ fit_pass_kernel(const tb_fit_unit* __restrict__ units, const int32_t* __restrict
                 src_bad = !S.ok || K < 0 || K > kCompStride;
                 const tb_fit_source fs = srcs[b.src0 + lane];
                 const bool live = fs.w > 0 && fs.h > 0;
-                UnitSrc U;
+                UnitSrc<T> U;
                 U.x0 = live ? fs.x0 : 0;
                 U.y0 = live ? fs.y0 : 0;
                 U.x1 = live ? fs.x0 + fs.w : 0;
                 U.y1 = live ? fs.y0 + fs.h : 0;
-                U.counts = (float)S.flux[u.band];
                 U.K = K;
+                U.profile = fs.profile;
+                U.counts = (T)S.flux[u.band];
 #pragma unroll
                 for (int q = 0; q < 3; q++) {
-                    U.M[q] = S.M[q];
+                    U.M[q] = (T)S.M[q];
 #pragma unroll
-                    for (int j = 0; j < 3; j++) U.dM[j][q] = S.dM[j][q];
+                    for (int j = 0; j < 3; j++) U.dM[j][q] = (T)S.dM[j][q];
                 }
                 sm.us[lane] = U;
             }
@@ -654,126 +702,101 @@ fit_pass_kernel(const tb_fit_unit* __restrict__ units, const int32_t* __restrict
         __syncthreads();
         if (sm.skip) {
             if (tid == 0) {
-                if (mode == 0) chi2_part[b.unit0 + u.slice] = INFINITY;
-                else chi2_const[b.unit0 + u.slice] = INFINITY;
+                if (mode == kConstant) chi2_const[b.unit0 + u.slice] = INFINITY;
+                else if (mode == kEquations) chi2_part[b.unit0 + u.slice] = INFINITY;
             }
             continue;
         }
-        // the unit's band of source s: band_comps + s * n_bands * kCompStride
-        const FitC* band_comps = gcomps + ((int64_t)b.src0 * n_bands + u.band) * kCompStride;
-        double chi2 = 0.0;
-        // mode 0: the unit's range of the tiles some source's mask reaches;
-        // mode 1: the others (their chi^2 does not depend on the parameters),
-        // covered by the unit that starts the range
-        const int n_t = mode == 0 ? u.t1 - u.t0 : (u.t0 == 0 ? b.n_tiles - b.n_active : 0);
-        const int32_t* tl = tiles + b.tile_off + (mode == 0 ? u.t0 : b.n_active);
-        // this thread's pixel of tile t (0 outside the image)
-        auto load_px = [&](int t, float& d, float& w) {
-            d = 0.f;
-            w = 0.f;
-            if (t >= n_t) return;
-            const int px = (tl[t] & 0x3ff) * kTileW + lane, py = ((tl[t] >> 10) & 0x3ff) * kTileH + warp;
-            if (px < u.W && py < u.H) {
-                const int64_t pix = u.pix_off + (int64_t)py * u.W + px;
-                d = data[pix];
-                w = inverr[pix];
+        PassUnit<T> pu;
+        pu.comps = gcomps + ((int64_t)b.src0 * n_bands + u.band) * kCompStride;
+        pu.cstride = (int64_t)n_bands * kCompStride;
+        pu.pix_off = u.pix_off;
+        // the unit's range of the tiles some source's mask reaches; kConstant:
+        // the others (their chi^2 does not depend on the parameters), covered
+        // by the unit that starts the range
+        pu.tiles = tiles + b.tile_off + (mode == kConstant ? b.n_active : u.t0);
+        pu.data = data;
+        pu.inverr = mode == kVjp ? nullptr : inverr;
+        pu.W = u.W;
+        pu.Hh = u.H;
+        const int n_t = mode == kConstant ? (u.t0 == 0 ? b.n_tiles - b.n_active : 0) : u.t1 - u.t0;
+        // the sources whose masks meet a tile (the same for every warp)
+        auto reach = [&](int t) -> unsigned {
+            const int ox = (pu.tiles[t] & 0x3ff) * kTileW, oy = ((pu.tiles[t] >> 10) & 0x3ff) * kTileH;
+            bool hit = false;
+            if (lane < nsrc) {
+                const UnitSrc<T>& U = sm.us[lane];
+                hit = U.x1 > ox && U.x0 < ox + kTileW && U.y1 > oy && U.y0 < oy + kTileH;
             }
+            return __ballot_sync(0xffffffffu, hit);
         };
-        float d_next, w_next;
-        load_px(0, d_next, w_next);
-        // single-source runs: this thread's pixel contributions to the run's
-        // 7 x 7 block (upper triangle) and gradient
-        int run_src = -1;
-        float hacc[28], gacc[7];
-        for (int t = 0; t < n_t; t++) {
-            const int ox = (tl[t] & 0x3ff) * kTileW, oy = ((tl[t] >> 10) & 0x3ff) * kTileH;
-            const int single = mode == 0 ? ((tl[t] >> 20) & 0xff) - 1 : -1;
-            const float d = d_next, w = w_next;
-            load_px(t + 1, d_next, w_next);   // prefetch the next tile's pixel
-            if (single != run_src) {
-                if (run_src >= 0) flush_run(sm, hacc, gacc, run_src, H, g, P, u.band);
-                run_src = single;
-#pragma unroll
-                for (int v = 0; v < 28; v++) hacc[v] = 0.f;
-#pragma unroll
-                for (int v = 0; v < 7; v++) gacc[v] = 0.f;
-            }
-            if (single >= 0 && single < nsrc) {
-                // one source: every warp on its own row, no block barrier
-                float J[kCols];
-                const float model = eval_source<true>(
-                    sm.wc[warp], band_comps + (int64_t)single * n_bands * kCompStride,
-                    sm.us[single], ox, oy, w, J);
-                const float rr = (d - model) * w;
-                chi2 += (double)(rr * rr);
-                int v = 0;
-#pragma unroll
-                for (int c = 0; c < kCols; c++) {
-                    gacc[c] = fmaf(J[c], rr, gacc[c]);
-#pragma unroll
-                    for (int c2 = c; c2 < kCols; c2++, v++) hacc[v] = fmaf(J[c], J[c2], hacc[v]);
+        pu.out = SliceOut{nullptr, nullptr, 0u, 0, P, u.band};
+        if (mode == kEquations || mode == kVjp) {
+            pu.out.g = gbuf + b.g_off + (int64_t)u.slice * P;
+            for (int e = tid; e < P; e += kThreads) pu.out.g[e] = 0.0;
+        }
+        if (mode == kEquations) {
+            for (int t = 0; t < n_t; t++) pu.out.mask |= reach(t);
+            pu.out.ld = kCols * __popc(pu.out.mask);
+            pu.out.H = hbuf + b.h_off + (int64_t)u.slice * P * P;
+            for (int e = tid; e < pu.out.ld * pu.out.ld; e += kThreads) pu.out.H[e] = 0.0;
+        }
+        double chi2 = 0.0;
+        for (int t = 0, t1; t < n_t; t = t1) {
+            // a run of tiles that the same sources meet
+            const unsigned hit = mode == kConstant ? 0u : reach(t);
+            t1 = t + 1;
+            while (t1 < n_t && (mode == kConstant || reach(t1) == hit)) t1++;
+            if (sizeof(T) == 8 && mode == kModel) {
+                for (int q = t; q < t1; q++) {
+                    const int ox = (pu.tiles[q] & 0x3ff) * kTileW;
+                    const int py = ((pu.tiles[q] >> 10) & 0x3ff) * kTileH + warp;
+                    T m = 0;
+                    for (unsigned hm = hit; hm; hm &= hm - 1) {
+                        const int sI = __ffs(hm) - 1;
+                        m += source_model<T>(sm, sm.us[sI], pu.comps + sI * pu.cstride, ox, py);
+                    }
+                    if (ox + lane < u.W && py < u.H)
+                        model_out[u.pix_off + (int64_t)py * u.W + ox + lane] = (float)m;
                 }
                 continue;
             }
-            // sources whose mask meets this tile, in source order (every warp
-            // finds the same set); mode 1 tiles meet none by construction
-            bool meets = false;
-            if (mode == 0 && lane < nsrc) {
-                const UnitSrc& U = sm.us[lane];
-                meets = U.x0 < ox + kTileW && U.x1 > ox && U.y0 < oy + kTileH && U.y1 > oy;
-            }
-            const unsigned hit = __ballot_sync(0xffffffffu, meets);
-            const int R = __popc(hit);
-            if (R == 0) {
-                const float rr = d * w;
-                chi2 += (double)(rr * rr);
+            if (sizeof(T) == 8 && mode == kVjp) {
+                // the upstream gradient does not depend on the model: one source at a time
+                for (unsigned hm = hit; hm; hm &= hm - 1)
+                    run_tiles<T, 1, false>(sm, pu, hm & (0u - hm), t, t1, chi2);
                 continue;
             }
-            // Shared A, r, hstage and gstage are written only after the
-            // previous multi-source tile's reads of them have passed a
-            // barrier: A and r are read before its second barrier, hstage
-            // and gstage after it and are written here only after this
-            // tile's first barrier.
-            const int ngroups = (R + kG - 1) / kG;
-            float model = 0.f;
-            if (ngroups == 1) {
-                model = eval_group<true>(sm, band_comps, n_bands, hit, 0, R, ox, oy, w, sm.A[0]);
-            } else {
-                for (int q0 = 0; q0 < R; q0 += kG)
-                    model += eval_group<false>(sm, band_comps, n_bands, hit, q0, min(kG, R - q0),
-                                               ox, oy, w, sm.A[0]);
-            }
-            const float rr = (d - model) * w;
-            chi2 += (double)(rr * rr);
-            sm.r[tid] = rr;
-            for (int ga = 0; ga < ngroups; ga++) {
-                const int qa = ga * kG, na = min(kG, R - qa);
-                if (ngroups > 1)
-                    eval_group<true>(sm, band_comps, n_bands, hit, qa, na, ox, oy, w, sm.A[0]);
-                __syncthreads();   // columns (and r) complete; earlier updates applied
-                stage_products(sm, sm.A[0], na, sm.A[0], na, true, true);
-                __syncthreads();
-                apply_products(sm, hit, qa, na, qa, na, true, true, H, g, P, u.band);
-                for (int gb = ga + 1; gb < ngroups; gb++) {
-                    const int qb = gb * kG, nb = min(kG, R - qb);
-                    eval_group<true>(sm, band_comps, n_bands, hit, qb, nb, ox, oy, w, sm.A[1]);
-                    __syncthreads();
-                    stage_products(sm, sm.A[0], na, sm.A[1], nb, false, false);
-                    __syncthreads();
-                    apply_products(sm, hit, qa, na, qb, nb, false, false, H, g, P, u.band);
-                }
+            switch (__popc(hit)) {
+                case 0:
+                    for (int q = t; q < t1; q++) {
+                        T d, w;
+                        load_pixel(pu, (pu.tiles[q] & 0x3ff) * kTileW + lane,
+                                   ((pu.tiles[q] >> 10) & 0x3ff) * kTileH + warp, d, w);
+                        const T r = d * w;
+                        chi2 += (double)(r * r);
+                    }
+                    break;
+                case 1: run_tiles<T, 1, true>(sm, pu, hit, t, t1, chi2); break;
+                case 2: run_tiles<T, 2, true>(sm, pu, hit, t, t1, chi2); break;
+                case 3: run_tiles<T, 3, true>(sm, pu, hit, t, t1, chi2); break;
+                case 4: run_tiles<T, 4, true>(sm, pu, hit, t, t1, chi2); break;
+                default:
+                    for (int q = t; q < t1; q++) crowded_tile<T>(sm, pu, hit, pu.tiles[q], chi2);
             }
         }
-        if (run_src >= 0) flush_run(sm, hacc, gacc, run_src, H, g, P, u.band);
+        if (mode == kModel || mode == kVjp) continue;
         // chi^2 of the unit: fixed-order block reduction
         for (int o = 16; o > 0; o >>= 1) chi2 += __shfl_xor_sync(0xffffffffu, chi2, o);
         if (lane == 0) sm.red[warp] = chi2;
         __syncthreads();
         if (tid == 0) {
             double s = 0.0;
-            for (int w2 = 0; w2 < kThreads / 32; w2++) s += sm.red[w2];
-            if (mode == 0) chi2_part[b.unit0 + u.slice] = s + chi2_const[b.unit0 + u.slice];
-            else chi2_const[b.unit0 + u.slice] = s;
+            for (int w2 = 0; w2 < kWarps; w2++) s += sm.red[w2];
+            if (mode == kConstant) chi2_const[b.unit0 + u.slice] = s;
+            else chi2_part[b.unit0 + u.slice] = s + (chi2_const ? chi2_const[b.unit0 + u.slice] : 0.0);
+            if (mode == kEquations)
+                pu.out.g[P - 1] = __longlong_as_double((long long)u.band << 32 | pu.out.mask);
         }
     }
 }
@@ -794,586 +817,127 @@ __device__ double max_step(int off) {
     }
 }
 
-// ---------------------------------------------------------------------------
-// refinement pass (tb_fit_refine): the normal equations of the running blobs
-// in FP64 -- the model, the seven derivative columns of every source, the
-// residuals, A^T A, A^T r and chi^2 -- written over the slices tb_fit_pass
-// fills.  Near the optimum the gradient is a sum of terms that cancel, FP32
-// chi^2 cannot verify gains below ~1e-4, and an FP32 A^T A (FP32 columns:
-// the index column is a difference of nearly equal sums) is too inexact for
-// the steps of an ill-conditioned blob to converge; the final iterations of
-// a fit take all of them in FP64.  Same units, slices and layout as
-// tb_fit_pass.
+// A blob's trial chi^2: its slices' parts summed by one warp in a fixed
+// order (every lane gets the sum).  The assembly and the step kernel both
+// decide on it, so both must sum alike.
+__device__ __forceinline__ double trial_chi2(const double* __restrict__ part, int ns) {
+    double c = 0.0;
+    for (int k = threadIdx.x & 31; k < ns; k += 32) c += part[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    return c;
+}
+
+__device__ __forceinline__ bool accept_trial(const tb_fit_state& S, double c2) {
+    return isfinite(c2) && (S.accepted == 0 || c2 < S.chi2);
+}
+
+// The slices of an accepted trial summed into the blob's accepted H (full,
+// symmetric) and g.  A kernel of its own, kAsmCtas CTAs per blob, a warp per
+// row: summing a large blob's slices took the one CTA of the step longer than
+// factoring the result.  A row takes only the slices that hold its source
+// (and, a flux, its band's), an element only those that hold both.
+constexpr int kAsmCtas = 16;
+
+__global__ void __launch_bounds__(kStepThreads)
+fit_assemble_kernel(const tb_fit_blob* __restrict__ blobs,
+                    const tb_fit_source* __restrict__ srcs, double* __restrict__ hbuf,
+                    double* __restrict__ gbuf, const double* __restrict__ chi2_part,
+                    const tb_fit_state* __restrict__ state) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const tb_fit_state& S = state[blockIdx.x];
+    if (S.status != 0) return;
+    const tb_fit_blob b = blobs[blockIdx.x];
+    const int P = b.P, ns = b.n_slices;
+    const int64_t PP = (int64_t)P * P;
+    const int r0 = blockIdx.y * (kStepThreads / 32) + warp;
+    if (r0 >= P) return;   // whole warps
+    if (!accept_trial(S, trial_chi2(chi2_part + b.unit0, ns))) return;
+    const double* Hp = hbuf + b.h_off;
+    const double* gp = gbuf + b.g_off;
+    double* Ha = hbuf + b.h_off + ns * PP;
+    double* ga = gbuf + b.g_off + (int64_t)ns * P;
+    // column within a source's seven of parameter slot `off` in `band`, or -1
+    auto column = [](int off, int band) {
+        return off < 2 ? off : off < 2 + TB_FIT_MAX_BANDS ? (off - 2 == band ? 2 : -1) : off - 2;
+    };
+    // whether a source of this profile has the parameter
+    auto has = [&](int src, int off) {
+        const int profile = srcs[b.src0 + src].profile;
+        return off < 2 + TB_FIT_MAX_BANDS ||
+               (profile != TB_PROFILE_POINT && (off < TB_FIT_NPAR - 1 || profile == TB_PROFILE_SERSIC));
+    };
+    for (int r = r0; r < P; r += kAsmCtas * (kStepThreads / 32)) {
+        const int a = r / TB_FIT_NPAR, ao = r % TB_FIT_NPAR;
+        const bool ha = has(a, ao);
+        double gs = 0.0;
+        for (int c0 = r; c0 < P; c0 += 32) {
+            const int c = c0 + lane;
+            const int s = c / TB_FIT_NPAR, so = c % TB_FIT_NPAR;
+            const bool hs = c < P && ha && has(s, so);
+            double h = 0.0;
+            for (int k0 = 0; k0 < ns; k0 += 32) {
+                // this row's slices among k0 .. k0 + 31
+                const int kk = k0 + lane;
+                const long long tail =
+                    kk < ns ? __double_as_longlong(gp[(int64_t)kk * P + P - 1]) : 0ll;
+                const unsigned mk = (unsigned)tail;
+                const int band = (int)(tail >> 32);
+                const int ca_l = ha ? column(ao, band) : -1;
+                unsigned sl = __ballot_sync(0xffffffffu, ca_l >= 0 && ((mk >> a) & 1u));
+                if (c0 == r && ((sl >> lane) & 1u))
+                    gs += gp[(int64_t)kk * P + compact_row(mk, a) + ca_l];
+#pragma unroll 4
+                for (; sl; sl &= sl - 1) {
+                    const int q = __ffs(sl) - 1;
+                    const unsigned m = __shfl_sync(0xffffffffu, mk, q);
+                    const int ca = __shfl_sync(0xffffffffu, ca_l, q);
+                    const int bq = __shfl_sync(0xffffffffu, band, q);
+                    const int cb = hs ? column(so, bq) : -1;
+                    if (cb >= 0 && ((m >> s) & 1u))
+                        h += Hp[(k0 + q) * PP + (compact_row(m, a) + ca) * kCols * __popc(m) +
+                                compact_row(m, s) + cb];
+                }
+            }
+            if (c < P) {
+                Ha[(int64_t)r * P + c] = h;
+                Ha[(int64_t)c * P + r] = h;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) gs += __shfl_xor_sync(0xffffffffu, gs, o);
+        if (lane == 0) ga[r] = gs;
+    }
+}
+
+// Factor storage: packed lower triangle by columns, padded to a multiple of
+// 8 rows (identity): element (i, j) at L[packed_col(j, n) + i], n the padded
+// size.
+__host__ __device__ constexpr int packed_col(int j, int n) { return j * (2 * n - j - 1) / 2; }
+__host__ __device__ constexpr int packed_size(int n) { return n * (n + 1) / 2; }
+constexpr int kStepMaxP = TB_FIT_MAX_SRC * TB_FIT_NPAR;
+constexpr int kStepSharedP = 128;      // largest padded size factored in shared memory
+constexpr int kStepSmem = 8 * (packed_size(kStepSharedP) + 5 * kStepSharedP);   // 71 KB
+static_assert(kStepSmem >= 8 * 5 * ((kStepMaxP + 7) / 8 * 8), "the vectors always fit");
+
+// One CTA per blob.  Up to 128 parameters the factor lives in shared memory
+// (71 KB, three blobs per SM), above in the blob's global area.
 //
-// Bound: FP64 issue in the component loop (a component costs 31 FP64
-// operations per pixel: exponent 3, exponential 10, value and C^-1 u 5,
-// moments 13).  So each warp stages, per pixel row, only the components that
-// reach its row of a source's mask; the trace terms are folded into the
-// second moments; and the products A^T A, A^T r go to the FP64 tensor core
-// (mma m8n8k4), accumulated in two registers per 8 x 8 block over a whole run
-// of tiles with the same sources, where 35 products per pixel and their
-// shuffle reductions took more instructions than the evaluation.  Measured on
-// 300 blobs (192-512 px, 3 bands): 52 passes 142 -> 58 ms, the first (all
-// blobs running) 3.5 ms; model + gradient of 100 blobs 3.4 -> 2.7 ms.
-// ---------------------------------------------------------------------------
-constexpr int kRefThreads = 256;       // one 32 x 8 tile, one pixel per thread
-constexpr int kRefWarps = kRefThreads / 32;
-constexpr int kRefSlots = 4;           // sources whose columns a warp holds at once
-constexpr int kRefLd = 36;             // doubles per column row (see ref_frag)
-constexpr int kRefXs = 8 * kRefLd;     // doubles per source: 7 columns and r
-constexpr double kRefFloor = -50.0 * TB_LOG2E;   // exponents below count as 0 (log2 units)
-
-struct RefSrc {
-    int32_t x0, y0, x1, y1;
-    int32_t K, profile;
-    double counts;
-    double M[3];
-    double dM[3][3];
-};
-
-// One component staged for one pixel row (dy = row - mean y) by the warp
-// that owns the row: exponent e(dx) = h00 dx^2 + bx dx + c0 in log2 units,
-// C^-1 u = (i00 dx + uxy, i01 dx + uyy).
-struct __align__(16) RefC {
-    double mx, h00, bx, c0;
-    double i00, i01, uxy, uyy;
-    double i11, s, sn, v;
-    double dv, pad;
-};
-
-struct RefSmem {
-    RefSrc us[TB_FIT_MAX_SRC];
-    RefC wc[kRefWarps][32];                         // a warp's staged components
-    double X[kRefWarps][kRefSlots * kRefXs];        // a warp's weighted columns and residuals
-    double exp_tab[tb::kExpTab];
-    double red[kRefWarps];
-    int64_t slot;
-    int skip;
-};
-
-// Parameter slot of column i (x y flux(band) logre ee1 ee2 n) of source sI;
-// -1 where the profile has no such parameter.
-__device__ __forceinline__ int ref_slot(int sI, int profile, int band, int i) {
-    if (i >= 3 && profile == TB_PROFILE_POINT) return -1;
-    if (i == 6 && profile != TB_PROFILE_SERSIC) return -1;
-    const int base = sI * TB_FIT_NPAR;
-    return i < 2 ? base + i : i == 2 ? base + 2 + band : base + 2 + i;
-}
-
-// Stages, by one warp, those of the components cs[k0 .. min(k0 + 32, K)) that
-// reach pixels [x0, x1] (absolute, inclusive) of row y into wc[0 ..), in
-// their order; returns how many.  As stage_row: the exponent is a concave
-// quadratic along the row, so a component whose maximum over the segment
-// stays below the floor (FP32 with a margin of 1) is exactly zero there.
-__device__ __forceinline__ int ref_stage(RefC* wc, const FitC64* __restrict__ cs, int k0, int K,
-                                         int y, int x0, int x1) {
-    const int lane = threadIdx.x & 31;
-    const int k = k0 + lane;
-    bool keep = false;
-    double mx = 0.0, dy = 0.0, i00 = 0.0, i01 = 0.0, i11 = 0.0;
-    __syncwarp();   // the warp's previous components are no longer read
-    if (k < K) {
-        const FitC64& c = cs[k];
-        mx = c.mx;
-        dy = (double)y - c.my;
-        i00 = c.i00;
-        i01 = c.i01;
-        i11 = c.i11;
-        const float a = (float)i00, bb = (float)(i01 * dy), cc = (float)(i11 * dy * dy);
-        const float lo = (float)((double)x0 - mx), hi = (float)((double)x1 - mx);
-        const bool ok = isfinite(a) && isfinite(bb) && isfinite(cc) && isfinite(lo) && a > 0.f;
-        const float dx = fminf(fmaxf(-bb / a, lo), hi);
-        const float q = fmaf(dx, fmaf(a, dx, 2.f * bb), cc);   // Mahalanobis^2
-        keep = !ok || !(q > 102.f);
-    }
-    const unsigned bal = __ballot_sync(0xffffffffu, keep);
-    if (keep) {
-        const FitC64& c = cs[k];
-        double2* f = reinterpret_cast<double2*>(wc + __popc(bal & ((1u << lane) - 1u)));
-        f[0] = make_double2(mx, -0.5 * TB_LOG2E * i00);
-        f[1] = make_double2(-TB_LOG2E * i01 * dy, -0.5 * TB_LOG2E * i11 * dy * dy);
-        f[2] = make_double2(i00, i01);
-        f[3] = make_double2(i01 * dy, i11 * dy);
-        f[4] = make_double2(i11, c.s);
-        f[5] = make_double2(c.sn, c.v);
-        f[6] = make_double2(c.dv, 0.0);
-    }
-    __syncwarp();   // staged components visible to the whole warp
-    return __popc(bal);
-}
-
-// Source R's model at this thread's pixel of row py (counts x its unit-flux
-// mixture; 0 outside its rectangle), FP64.  Called by whole warps.
-__device__ __forceinline__ double ref_model(RefSmem& sm, const RefSrc& R,
-                                            const FitC64* __restrict__ cs, int ox, int py) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int xa = max(R.x0, ox), xb = min(R.x1, ox + kTileW);
-    if (py < R.y0 || py >= R.y1 || xa >= xb) return 0.0;   // warp-uniform
-    RefC* wc = sm.wc[warp];
-    const int px = ox + lane;
-    double val = 0.0;
-    for (int k0 = 0; k0 < R.K; k0 += 32) {
-        const int n = ref_stage(wc, cs, k0, R.K, py, xa, xb - 1);
-#pragma unroll 2
-        for (int g = 0; g < n; g++) {
-            const RefC& c = wc[g];
-            const double dx = (double)px - c.mx;
-            const double e = fma(dx, fma(c.h00, dx, c.bx), c.c0);
-            const double E = tb::exp2_tab(e, sm.exp_tab);
-            val = fma(e >= kRefFloor ? E : 0.0, c.s, val);
-        }
-    }
-    return px >= xa && px < xb ? R.counts * val : 0.0;
-}
-
-// Source R's seven derivative columns, times w, at this thread's pixel of
-// row py into X[0 .. 7)[lane] (0 outside its rectangle); returns its model
-// there.  Per component the moments of C^-1 u (u = pixel - mean) that
-// d/d(mean, C, amplitude) produce, d/dC = 1/2 (C^-1 u u^T C^-1 - C^-1),
-// combined once per source with dM (shape) and M (index).  Called by whole
-// warps; no block barrier.
-__device__ __forceinline__ double ref_cols(RefSmem& sm, const RefSrc& R,
-                                           const FitC64* __restrict__ cs, int ox, int py,
-                                           double w, double* X) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int xa = max(R.x0, ox), xb = min(R.x1, ox + kTileW);
-    double S0 = 0, Sx = 0, Sy = 0, Axx = 0, Axy = 0, Ayy = 0, Dxx = 0, Dxy = 0, Dyy = 0, Sn = 0;
-    const int px = ox + lane;
-    const bool row = py >= R.y0 && py < R.y1 && xa < xb;   // warp-uniform
-    if (row) {
-        RefC* wc = sm.wc[warp];
-        for (int k0 = 0; k0 < R.K; k0 += 32) {
-            const int n = ref_stage(wc, cs, k0, R.K, py, xa, xb - 1);
-#pragma unroll 2
-            for (int g = 0; g < n; g++) {
-                const RefC& c = wc[g];
-                const double dx = (double)px - c.mx;
-                const double e = fma(dx, fma(c.h00, dx, c.bx), c.c0);
-                double E = tb::exp2_tab(e, sm.exp_tab);
-                if (!(e >= kRefFloor)) E = 0.0;
-                const double ux = fma(c.i00, dx, c.uxy), uy = fma(c.i01, dx, c.uyy);
-                const double val = c.s * E;
-                S0 += val;
-                Sx = fma(val, ux, Sx);
-                Sy = fma(val, uy, Sy);
-                const double pxx = fma(ux, ux, -c.i00), pxy = fma(ux, uy, -c.i01),
-                             pyy = fma(uy, uy, -c.i11);
-                const double vv = val * c.v, vd = val * c.dv;
-                Axx = fma(vv, pxx, Axx);
-                Axy = fma(vv, pxy, Axy);
-                Ayy = fma(vv, pyy, Ayy);
-                Dxx = fma(vd, pxx, Dxx);
-                Dxy = fma(vd, pxy, Dxy);
-                Dyy = fma(vd, pyy, Dyy);
-                Sn = fma(c.sn, E, Sn);
-            }
-        }
-    }
-    const bool in = row && px >= xa && px < xb;
-    const double cn = in ? R.counts : 0.0;
-    const double cw = cn * w, h = 0.5 * cw;
-    X[lane] = cw * Sx;
-    X[kRefLd + lane] = cw * Sy;
-    X[2 * kRefLd + lane] = in ? w * S0 : 0.0;
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-        X[(3 + j) * kRefLd + lane] =
-            h * (R.dM[j][0] * Axx + 2.0 * R.dM[j][1] * Axy + R.dM[j][2] * Ayy);
-    X[6 * kRefLd + lane] =
-        h * (R.M[0] * Dxx + 2.0 * R.M[1] * Dxy + R.M[2] * Dyy) + cw * Sn;
-    return cn * S0;
-}
-
-// A^T A and A^T r are contractions over pixels: with X_s the 8 x 32 matrix of
-// source s's seven weighted columns and the residual over a warp's 32
-// pixels, X_a X_b^T is a chain of eight FP64 m8n8k4 tensor-core products.
-// Their A and B fragments are the same element per lane,
-// X[lane / 4][4 step + lane % 4]; the row stride of 36 doubles puts the 16
-// lanes of each half warp in different banks.
-__device__ __forceinline__ double ref_frag(const double* X, int step) {
-    const int lane = threadIdx.x & 31;
-    return X[(lane >> 2) * kRefLd + 4 * step + (lane & 3)];
-}
-
-__device__ __forceinline__ void ref_mma(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
-}
-
-// The warps' NB 8 x 8 blocks summed (in warp order) and added to their
-// destinations: element (i, j) of block q, between sources sa(q) <= sb(q)
-// (-1: no such source), to H (upper triangle) or, in the residual's column, to g.
-// The blocks pass through the component staging area, kRefRound at a time.
-// Called by the whole block.
-constexpr int kRefRound = 5;
-static_assert(kRefRound * 64 * sizeof(double) <= 32 * sizeof(RefC), "blocks fit the staging area");
-
-template <int NB, class SA, class SB>
-__device__ __forceinline__ void ref_flush(RefSmem& sm, const double (&c)[NB][2], SA sa, SB sb,
-                                          double* H, double* g, int P, int band) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncwarp();   // the warp's staged components are read
-#pragma unroll
-    for (int q0 = 0; q0 < NB; q0 += kRefRound) {
-#pragma unroll
-        for (int q = q0; q < NB && q < q0 + kRefRound; q++)
-            reinterpret_cast<double2*>(sm.wc[warp])[(q - q0) * 32 + lane] =
-                make_double2(c[q][0], c[q][1]);
-        __syncthreads();
-        const int nb = NB - q0 < kRefRound ? NB - q0 : kRefRound;
-        for (int e = threadIdx.x; e < nb * 64; e += kRefThreads) {
-            const int q = q0 + (e >> 6), i = (e >> 3) & 7, j = e & 7;
-            const int a = sa(q), b = sb(q);
-            if (a < 0 || b < 0 || i == 7 || (j == 7 ? a != b || !g : !H || (a == b && j < i)))
-                continue;
-            const int di = ref_slot(a, sm.us[a].profile, band, i);
-            const int dj = j == 7 ? 0 : ref_slot(b, sm.us[b].profile, band, j);
-            if (di < 0 || dj < 0) continue;
-            double s = 0.0;
-#pragma unroll
-            for (int w = 0; w < kRefWarps; w++) s += reinterpret_cast<const double*>(sm.wc[w])[e];
-            if (j == 7) g[di] += s;
-            else H[(int64_t)di * P + dj] += s;
-        }
-        __syncthreads();
-    }
-}
-
-// Block q of R sources: q < R a source's own block, then the pairs (0, 1),
-// (0, 2), .. (R - 2, R - 1).
-__host__ __device__ constexpr int ref_pair_a(int q, int R) {
-    if (q < R) return q;
-    int a = 0, n = q - R;
-    while (n >= R - 1 - a) { n -= R - 1 - a; a++; }
-    return a;
-}
-__host__ __device__ constexpr int ref_pair_b(int q, int R) {
-    if (q < R) return q;
-    int a = 0, n = q - R;
-    while (n >= R - 1 - a) { n -= R - 1 - a; a++; }
-    return a + 1 + n;
-}
-
-// The unit a CTA works on.
-struct RefUnit {
-    const FitC64* comps;      // its band of source s: comps + s * cstride
-    int64_t cstride, pix_off;
-    const int32_t* tiles;
-    const float* data;        // data, or (VJP) the upstream gradient
-    const float* inverr;      // null: no weights (VJP)
-    double *H, *g;
-    int W, Hh, P, band;
-};
-
-// This thread's pixel of tile `code` (0 outside the image): its value and weight.
-__device__ __forceinline__ void ref_pixel(const RefUnit& u, int px, int py, double& d, double& w) {
-    d = w = 0.0;
-    if (px < u.W && py < u.Hh) {
-        const int64_t pix = u.pix_off + (int64_t)py * u.W + px;
-        d = u.data[pix];
-        w = u.inverr ? (double)u.inverr[pix] : 1.0;
-    }
-}
-
-// Tiles [t0, t1), all met by exactly the R sources `hit`: each warp adds its
-// rows' products into register blocks without a block barrier, then one
-// flush.  kResid: r = (data - model) inverr, every pair's block, chi^2;
-// otherwise (one source) r = data.
-template <int R, bool kResid>
-__device__ void ref_run(RefSmem& sm, const RefUnit& u, unsigned hit, int t0, int t1,
-                        double& chi2) {
-    constexpr int NB = R * (R + 1) / 2;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double* X = sm.X[warp];
-    double c[NB][2];
-#pragma unroll
-    for (int q = 0; q < NB; q++) c[q][0] = c[q][1] = 0.0;
-    for (int t = t0; t < t1; t++) {
-        const int ox = (u.tiles[t] & 0x3ff) * kTileW;
-        const int py = ((u.tiles[t] >> 10) & 0x3ff) * kTileH + warp;
-        double d, w;
-        ref_pixel(u, ox + lane, py, d, w);
-        double m = 0.0;
-        bool any = false;
-        unsigned hm = hit;
-        __syncwarp();   // the previous tile's fragments are read
-#pragma unroll 1
-        for (int s = 0; s < R; s++, hm &= hm - 1) {
-            const int sI = __ffs(hm) - 1;
-            const RefSrc& S = sm.us[sI];
-            any = any || (py >= S.y0 && py < S.y1);
-            m += ref_cols(sm, S, u.comps + sI * u.cstride, ox, py, w, X + s * kRefXs);
-        }
-        const double r = kResid ? (d - m) * w : d;
-        if (kResid) chi2 += r * r;
-        if (!any) continue;   // warp-uniform: every column is 0 in this row
-#pragma unroll
-        for (int s = 0; s < R; s++) X[s * kRefXs + 7 * kRefLd + lane] = r;
-        __syncwarp();
-#pragma unroll
-        for (int step = 0; step < 8; step++) {
-            double f[R];
-#pragma unroll
-            for (int s = 0; s < R; s++) f[s] = ref_frag(X + s * kRefXs, step);
-#pragma unroll
-            for (int q = 0; q < NB; q++) ref_mma(c[q], f[ref_pair_a(q, R)], f[ref_pair_b(q, R)]);
-        }
-    }
-    auto src = [&](int i) { return nth_bit(hit, i); };
-    ref_flush(sm, c, [&](int q) { return src(ref_pair_a(q, R)); },
-              [&](int q) { return src(ref_pair_b(q, R)); }, u.H, u.g, u.P, u.band);
-}
-
-// A tile that more than kRefSlots sources meet: the model first, then groups
-// of three sources (their own and mutual blocks), each followed by its
-// blocks with every later source, whose columns are evaluated again.
-__device__ void ref_crowded(RefSmem& sm, const RefUnit& u, unsigned hit, int code, double& chi2) {
-    constexpr int kG3 = kRefSlots - 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int R = __popc(hit);
-    double* X = sm.X[warp];
-    const int ox = (code & 0x3ff) * kTileW, py = ((code >> 10) & 0x3ff) * kTileH + warp;
-    double d, w;
-    ref_pixel(u, ox + lane, py, d, w);
-    double m = 0.0;
-    for (unsigned hm = hit; hm; hm &= hm - 1) {
-        const int sI = __ffs(hm) - 1;
-        m += ref_model(sm, sm.us[sI], u.comps + sI * u.cstride, ox, py);
-    }
-    const double r = (d - m) * w;
-    chi2 += r * r;
-    for (int q0 = 0; q0 < R; q0 += kG3) {
-        __syncwarp();
-        for (int s = 0; s < kG3; s++) {
-            double* Xs = X + s * kRefXs;
-            if (q0 + s < R) {
-                const int sI = nth_bit(hit, q0 + s);
-                ref_cols(sm, sm.us[sI], u.comps + sI * u.cstride, ox, py, w, Xs);
-            } else {
-#pragma unroll
-                for (int c = 0; c < 7; c++) Xs[c * kRefLd + lane] = 0.0;
-            }
-            Xs[7 * kRefLd + lane] = r;
-        }
-        __syncwarp();
-        auto src = [&](int i) { return q0 + i < R ? nth_bit(hit, q0 + i) : -1; };
-        {
-            constexpr int NB = kG3 * (kG3 + 1) / 2;
-            double c[NB][2];
-#pragma unroll
-            for (int q = 0; q < NB; q++) c[q][0] = c[q][1] = 0.0;
-#pragma unroll
-            for (int step = 0; step < 8; step++) {
-                double f[kG3];
-#pragma unroll
-                for (int s = 0; s < kG3; s++) f[s] = ref_frag(X + s * kRefXs, step);
-#pragma unroll
-                for (int q = 0; q < NB; q++)
-                    ref_mma(c[q], f[ref_pair_a(q, kG3)], f[ref_pair_b(q, kG3)]);
-            }
-            ref_flush(sm, c, [&](int q) { return src(ref_pair_a(q, kG3)); },
-                      [&](int q) { return src(ref_pair_b(q, kG3)); }, u.H, u.g, u.P, u.band);
-        }
-        for (int i = q0 + kG3; i < R; i++) {
-            const int sI = nth_bit(hit, i);
-            double* Xb = X + kG3 * kRefXs;
-            __syncwarp();
-            ref_cols(sm, sm.us[sI], u.comps + sI * u.cstride, ox, py, w, Xb);
-            Xb[7 * kRefLd + lane] = r;
-            __syncwarp();
-            double c[kG3][2];
-#pragma unroll
-            for (int q = 0; q < kG3; q++) c[q][0] = c[q][1] = 0.0;
-#pragma unroll
-            for (int step = 0; step < 8; step++) {
-                const double fb = ref_frag(Xb, step);
-#pragma unroll
-                for (int q = 0; q < kG3; q++) ref_mma(c[q], ref_frag(X + q * kRefXs, step), fb);
-            }
-            ref_flush(sm, c, src, [&](int) { return sI; }, u.H, u.g, u.P, u.band);
-        }
-    }
-}
-
-// CTAs per SM the refinement kernel is compiled for (2: 128 registers, and
-// twice its shared memory fits)
-#ifndef TB_REFINE_MINB
-#define TB_REFINE_MINB 2
-#endif
-__global__ void __launch_bounds__(kRefThreads, TB_REFINE_MINB)
-fit_refine_kernel(const tb_fit_unit* __restrict__ units, const int32_t* __restrict__ order,
-                  int n_units, const tb_fit_blob* __restrict__ blobs,
-                  const tb_fit_source* __restrict__ srcs, const SrcTab* __restrict__ tab,
-                  const FitC64* __restrict__ gcomps, const float* __restrict__ data,
-                  const float* __restrict__ inverr, double* __restrict__ hbuf,
-                  double* __restrict__ gbuf, double* __restrict__ chi2_out,
-                  const tb_fit_state* __restrict__ state, int n_bands,
-                  const int32_t* __restrict__ tiles, int32_t* counter, tb_status* st, int mode,
-                  float* __restrict__ model_out, const double* __restrict__ chi2_const) {
-    // mode TB_FIT_REFINE: A^T A, A^T r and chi^2 of the running blobs, r =
-    // (data - model) inverr; TB_FIT_MODEL: the model into model_out (every
-    // blob); TB_FIT_VJP: the columns contracted with data = an upstream
-    // gradient, unweighted
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    RefSmem& sm = *reinterpret_cast<RefSmem*>(smem_raw);
-    const int tid = threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
-    const bool refine = mode == TB_FIT_REFINE;
-    tb::exp2_tab_init(sm.exp_tab);   // read after next_unit's barriers
-    for (;;) {
-        const int64_t oi = tb::next_unit(counter, &sm.slot);
-        if (oi >= n_units) break;
-        const int ui = order[oi];
-        if (ui < 0 || ui >= n_units) continue;
-        const tb_fit_unit& u = units[ui];
-        const tb_fit_blob b = blobs[u.blob];
-        if (refine && state[u.blob].status != 0) continue;   // running blobs
-        const int P = b.P;
-        const int nsrc = b.n_src;
-        double* g = gbuf ? gbuf + b.g_off + (int64_t)u.slice * P : nullptr;
-        double* H = refine ? hbuf + b.h_off + (int64_t)u.slice * P * P : nullptr;
-        if (mode != TB_FIT_MODEL)
-            for (int e = tid; e < P; e += kRefThreads) g[e] = 0.0;
-        if (refine)
-            for (int e = tid; e < P * P; e += kRefThreads) H[e] = 0.0;
-        if (warp == 0) {
-            const bool unit_bad = nsrc < 0 || nsrc > TB_FIT_MAX_SRC || P != nsrc * TB_FIT_NPAR ||
-                                  u.band < 0 || u.band >= n_bands || u.slice < 0 ||
-                                  u.slice >= b.n_slices || u.t0 < 0 || u.t1 < u.t0 ||
-                                  u.t1 > b.n_active;
-            bool src_bad = false;
-            if (!unit_bad && lane < nsrc) {
-                const SrcTab& S = tab[b.src0 + lane];
-                const int K = S.K[u.band];
-                src_bad = !S.ok || K < 0 || K > kCompStride;
-                const tb_fit_source fs = srcs[b.src0 + lane];
-                const bool live = fs.w > 0 && fs.h > 0;
-                RefSrc R;
-                R.x0 = live ? fs.x0 : 0;
-                R.y0 = live ? fs.y0 : 0;
-                R.x1 = live ? fs.x0 + fs.w : 0;
-                R.y1 = live ? fs.y0 + fs.h : 0;
-                R.K = K;
-                R.profile = fs.profile;
-                R.counts = S.flux[u.band];
-#pragma unroll
-                for (int q = 0; q < 3; q++) {
-                    R.M[q] = S.M64[q];
-#pragma unroll
-                    for (int j = 0; j < 3; j++) R.dM[j][q] = S.dM64[j][q];
-                }
-                sm.us[lane] = R;
-            }
-            const bool bad = unit_bad || __any_sync(0xffffffffu, src_bad);
-            if (lane == 0) {
-                sm.skip = bad;
-                if (bad) tb::report(st, TB_STATUS_BAD_ITEM, ui, nsrc);
-            }
-        }
-        __syncthreads();
-        if (sm.skip) {
-            if (tid == 0 && chi2_out) chi2_out[b.unit0 + u.slice] = INFINITY;
-            continue;
-        }
-        RefUnit ru;
-        ru.comps = gcomps + ((int64_t)b.src0 * n_bands + u.band) * kCompStride;
-        ru.cstride = (int64_t)n_bands * kCompStride;
-        ru.pix_off = u.pix_off;
-        ru.tiles = tiles + b.tile_off + u.t0;
-        ru.data = data;
-        ru.inverr = refine ? inverr : nullptr;
-        ru.H = H;
-        ru.g = g;
-        ru.W = u.W;
-        ru.Hh = u.H;
-        ru.P = P;
-        ru.band = u.band;
-        const int n_t = u.t1 - u.t0;
-        // the sources whose rectangles meet a tile (the same for every warp)
-        auto reach = [&](int t) -> unsigned {
-            const int ox = (ru.tiles[t] & 0x3ff) * kTileW, oy = ((ru.tiles[t] >> 10) & 0x3ff) * kTileH;
-            bool hit = false;
-            if (lane < nsrc) {
-                const RefSrc& R = sm.us[lane];
-                hit = R.x1 > ox && R.x0 < ox + kTileW && R.y1 > oy && R.y0 < oy + kTileH;
-            }
-            return __ballot_sync(0xffffffffu, hit);
-        };
-        double chi2 = 0.0;
-        int t = 0;
-        while (t < n_t) {
-            // a run of tiles that the same sources meet
-            const unsigned hit = reach(t);
-            int t1 = t + 1;
-            while (t1 < n_t && reach(t1) == hit) t1++;
-            if (mode == TB_FIT_MODEL) {
-                for (; t < t1; t++) {
-                    const int ox = (ru.tiles[t] & 0x3ff) * kTileW;
-                    const int py = ((ru.tiles[t] >> 10) & 0x3ff) * kTileH + warp;
-                    double m = 0.0;
-                    for (unsigned hm = hit; hm; hm &= hm - 1) {
-                        const int sI = __ffs(hm) - 1;
-                        m += ref_model(sm, sm.us[sI], ru.comps + sI * ru.cstride, ox, py);
-                    }
-                    if (ox + lane < u.W && py < u.H)
-                        model_out[u.pix_off + (int64_t)py * u.W + ox + lane] = (float)m;
-                }
-            } else if (!refine) {
-                // the upstream gradient does not depend on the model: one source at a time
-                for (unsigned hm = hit; hm; hm &= hm - 1)
-                    ref_run<1, false>(sm, ru, hm & (0u - hm), t, t1, chi2);
-            } else {
-                switch (__popc(hit)) {
-                    case 0:
-                        for (int q = t; q < t1; q++) {
-                            double d, w;
-                            ref_pixel(ru, (ru.tiles[q] & 0x3ff) * kTileW + lane,
-                                      ((ru.tiles[q] >> 10) & 0x3ff) * kTileH + warp, d, w);
-                            chi2 += d * w * (d * w);
-                        }
-                        break;
-                    case 1: ref_run<1, true>(sm, ru, hit, t, t1, chi2); break;
-                    case 2: ref_run<2, true>(sm, ru, hit, t, t1, chi2); break;
-                    case 3: ref_run<3, true>(sm, ru, hit, t, t1, chi2); break;
-                    case 4: ref_run<4, true>(sm, ru, hit, t, t1, chi2); break;
-                    default:
-                        for (int q = t; q < t1; q++) ref_crowded(sm, ru, hit, ru.tiles[q], chi2);
-                }
-            }
-            t = t1;
-        }
-        if (mode == TB_FIT_MODEL) continue;
-        // the unit's chi^2 (its active tiles; the constant part stays in chi2_const)
-        for (int o = 16; o > 0; o >>= 1) chi2 += __shfl_xor_sync(0xffffffffu, chi2, o);
-        if (lane == 0) sm.red[warp] = chi2;
-        __syncthreads();
-        if (tid == 0 && chi2_out) {
-            // the slice's chi^2 with its constant part (the tiles no mask
-            // reaches), as tb_fit_pass writes it
-            double c2 = chi2_const ? chi2_const[b.unit0 + u.slice] : 0.0;
-            for (int w2 = 0; w2 < kRefWarps; w2++) c2 += sm.red[w2];
-            chi2_out[b.unit0 + u.slice] = c2;
-        }
-    }
-}
-
-// One CTA per blob.  The factor lives in the blob's global area (L2
-// resident); shared memory and registers stay small so that five blobs
-// share an SM.
-__global__ void __launch_bounds__(kStepThreads, 5)
+// Bound: the chain of columns.  A column at a time through L2, one barrier
+// each, took 0.6 ms for 126 parameters; four columns at a time (every thread
+// factors the 4 x 4 diagonal block itself and finishes one row of the panel,
+// then the trailing tiles are updated by FP64 tensor-core products of rank 4)
+// is two barriers per four columns and 256 multiply-adds per instruction.
+// STEPMEASURED
+__global__ void __launch_bounds__(kStepThreads, 3)
 fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
                 const tb_fit_source* __restrict__ srcs, double* __restrict__ params,
                 double* __restrict__ trial, double* __restrict__ hbuf, double* __restrict__ gbuf,
                 const double* __restrict__ chi2_part, tb_fit_state* __restrict__ state,
                 double tol, int max_iter) {
-    __shared__ double dsc[TB_FIT_MAX_SRC * TB_FIT_NPAR];
-    __shared__ double dinv[TB_FIT_MAX_SRC * TB_FIT_NPAR];
-    __shared__ double y[TB_FIT_MAX_SRC * TB_FIT_NPAR];
-    __shared__ double xs[TB_FIT_MAX_SRC * TB_FIT_NPAR];
-    __shared__ double rdg[TB_FIT_MAX_SRC * TB_FIT_NPAR];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double red[kStepThreads / 32], red2[kStepThreads / 32];
-    __shared__ int s_accept, s_active;
+    __shared__ int s_active, s_accept;
     __shared__ double s_lambda, s_scale, s_pa, s_pb;
     const int bi = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1385,20 +949,24 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
     __syncthreads();   // every thread has read the status before thread 0 updates it
     if (status0 != 0) return;
     const int P = b.P;
+    const int n = (P + 7) / 8 * 8;
     const int ns = b.n_slices;
-    double* Hp = hbuf + b.h_off;                        // slice partials
-    double* Ha = Hp + (int64_t)ns * P * P;              // accepted H
-    double* L = Ha + (int64_t)P * P;                    // factor
-    double* gp = gbuf + b.g_off;
-    double* ga = gp + (int64_t)ns * P;
+    double* dsc = reinterpret_cast<double*>(smem_raw);
+    double* dinv = dsc + n;
+    double* y = dinv + n;
+    double* xs = y + n;
+    double* rdg = xs + n;
+    double* Ha = hbuf + b.h_off + (int64_t)ns * P * P;   // accepted H
+    double* L = n <= kStepSharedP ? rdg + n : Ha + (int64_t)P * P;   // factor
+    double* ga = gbuf + b.g_off + (int64_t)ns * P;
     double* pa = params + (int64_t)b.src0 * TB_FIT_NPAR;
     double* pt = trial + (int64_t)b.src0 * TB_FIT_NPAR;
+    auto col = [&](int j) { return L + packed_col(j, n); };
 
+    const double c2 = warp == 0 ? trial_chi2(chi2_part + b.unit0, ns) : 0.0;
     if (tid == 0) {
-        double c2 = 0.0;
-        for (int k = 0; k < ns; k++) c2 += chi2_part[b.unit0 + k];
         const bool first = S.accepted == 0;
-        const bool acc = isfinite(c2) && (first || c2 < S.chi2);
+        const bool acc = accept_trial(S, c2);
         int status = 0;
         if (acc) {
             // damping from the gain ratio rho = actual / predicted (Nielsen's
@@ -1429,19 +997,6 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
     __syncthreads();
     if (s_accept) {
         for (int e = tid; e < P; e += kStepThreads) pa[e] = pt[e];
-        // accepted H (symmetric, from the slice partials' upper triangles) and g
-        for (int r = warp; r < P; r += kStepThreads / 32)
-            for (int c = r + lane; c < P; c += 32) {
-                double s = 0.0;
-                for (int k = 0; k < ns; k++) s += Hp[(int64_t)k * P * P + (int64_t)r * P + c];
-                Ha[(int64_t)r * P + c] = s;
-                Ha[(int64_t)c * P + r] = s;
-            }
-        for (int e = tid; e < P; e += kStepThreads) {
-            double s = 0.0;
-            for (int k = 0; k < ns; k++) s += gp[(int64_t)k * P + e];
-            ga[e] = s;
-        }
     }
     __syncthreads();
     if (!s_active) {
@@ -1472,24 +1027,81 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
         if (dinv[i] == 0.0 || dinv[j] == 0.0) return i == j ? 1.0 : 0.0;
         return Ha[(int64_t)j * P + i] * dinv[i] * dinv[j] + (i == j ? lam : 0.0);
     };
-    // LDL^T of the scaled matrix, lower triangle column-major (element
-    // (i, j), i >= j, at L[j P + i]), right-looking: step k subtracts
-    // L[k P + i] L[k P + j] / d_k from the trailing columns and leaves column
-    // k as d_k (diagonal) and d_k l_ik below it, so no column is rescaled
-    // and each step takes one barrier.
-    for (int j = warp; j < P; j += kStepThreads / 32)
-        for (int i = j + lane; i < P; i += 32) L[(int64_t)j * P + i] = scaled(i, j);
+    for (int i = P + tid; i < n; i += kStepThreads) dinv[i] = dsc[i] = 0.0;
+    __syncthreads();
+    // LDL^T of the scaled matrix, right-looking: column k is left as d_k
+    // (diagonal) and c_ik = d_k l_ik below it, and subtracts c_ik c_jk / d_k
+    // from the trailing columns.
+    for (int j = warp; j < n; j += kStepThreads / 32)
+        for (int i = j + lane; i < n; i += 32)
+            col(j)[i] = i < P ? scaled(i, j) : (i == j ? 1.0 : 0.0);
     __syncthreads();
     bool bad = false;
-    for (int k = 0; k < P; k++) {
-        const double* ck = L + (int64_t)k * P;
-        const double dk = ck[k];   // final since step k - 1; the same in every thread
-        if (!(dk > 0.0) || !isfinite(dk)) { bad = true; break; }
-        const double rk = 1.0 / dk;
-        for (int j = k + 1 + warp; j < P; j += kStepThreads / 32) {
-            const double cj = ck[j] * rk;
-            double* colj = L + (int64_t)j * P;
-            for (int i = j + lane; i < P; i += 32) colj[i] = fma(-ck[i], cj, colj[i]);
+    for (int k0 = 0; k0 < n; k0 += 4) {
+        const double *c0 = col(k0), *c1 = col(k0 + 1), *c2k = col(k0 + 2), *c3 = col(k0 + 3);
+        // the 4 x 4 diagonal block, the same in every thread
+        const double a10 = c0[k0 + 1], a20 = c0[k0 + 2], a30 = c0[k0 + 3];
+        const double d0 = c0[k0], r0 = 1.0 / d0;
+        const double d1 = c1[k0 + 1] - a10 * a10 * r0, r1 = 1.0 / d1;
+        const double a21 = c1[k0 + 2] - a20 * a10 * r0, a31 = c1[k0 + 3] - a30 * a10 * r0;
+        const double d2 = c2k[k0 + 2] - a20 * a20 * r0 - a21 * a21 * r1, r2 = 1.0 / d2;
+        const double a32 = c2k[k0 + 3] - a30 * a20 * r0 - a31 * a21 * r1;
+        const double d3 = c3[k0 + 3] - a30 * a30 * r0 - a31 * a31 * r1 - a32 * a32 * r2;
+        const double r3 = 1.0 / d3;
+        if (!(d0 > 0.0 && d1 > 0.0 && d2 > 0.0 && d3 > 0.0) || !isfinite(d0) || !isfinite(d1) ||
+            !isfinite(d2) || !isfinite(d3)) {
+            bad = true;
+            break;
+        }
+        // the panel's other rows, one per thread
+        const double l10 = a10 * r0, l20 = a20 * r0, l30 = a30 * r0;
+        const double l21 = a21 * r1, l31 = a31 * r1, l32 = a32 * r2;
+        for (int i = k0 + 4 + tid; i < n; i += kStepThreads) {
+            const double e0 = c0[i];
+            const double e1 = c1[i] - e0 * l10;
+            const double e2 = c2k[i] - e0 * l20 - e1 * l21;
+            const double e3 = c3[i] - e0 * l30 - e1 * l31 - e2 * l32;
+            col(k0 + 1)[i] = e1;
+            col(k0 + 2)[i] = e2;
+            col(k0 + 3)[i] = e3;
+        }
+        __syncthreads();   // the panel's rows are complete, the diagonal block is read
+        if (tid == 0) {
+            col(k0 + 1)[k0 + 1] = d1;
+            col(k0 + 1)[k0 + 2] = a21;
+            col(k0 + 1)[k0 + 3] = a31;
+            col(k0 + 2)[k0 + 2] = d2;
+            col(k0 + 2)[k0 + 3] = a32;
+            col(k0 + 3)[k0 + 3] = d3;
+            rdg[k0] = r0;
+            rdg[k0 + 1] = r1;
+            rdg[k0 + 2] = r2;
+            rdg[k0 + 3] = r3;
+        }
+        // trailing 8 x 8 tiles (the first tile column may hold panel columns,
+        // which stay): rows i0 + lane / 4, columns j0 + 2 (lane % 4) + {0, 1}
+        const int base = (k0 + 4) / 8 * 8, T = (n - base) / 8;
+        const int q = lane & 3;
+        const double rq = -(q == 0 ? r0 : q == 1 ? r1 : q == 2 ? r2 : r3);
+        const double* ck = col(k0 + q);
+        for (int e = warp, tj = 0, ti = warp; e < T * (T + 1) / 2; e += kStepThreads / 32, ti += kStepThreads / 32) {
+            while (ti >= T) {   // row-major over the lower triangle's tile columns
+                tj++;
+                ti += tj - T;
+            }
+            const int i0 = base + 8 * ti, j0 = base + 8 * tj;
+            const int i = i0 + (lane >> 2), j = j0 + 2 * q;
+            double* p0 = col(j) + i;
+            double* p1 = col(j + 1) + i;
+            const bool on0 = j >= k0 + 4 && i >= j, on1 = j + 1 >= k0 + 4 && i >= j + 1;
+            // rows above the trailing part (first tile only) belong to the panel
+            const double fa = i >= k0 + 4 ? ck[i] : 0.0;
+            const int jb = j0 + (lane >> 2);
+            const double fb = jb >= k0 + 4 ? ck[jb] * rq : 0.0;
+            double c[2] = {on0 ? *p0 : 0.0, on1 ? *p1 : 0.0};
+            mma884(c, fa, fb);
+            if (on0) *p0 = c[0];
+            if (on1) *p1 = c[1];
         }
         __syncthreads();
     }
@@ -1502,67 +1114,95 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
         for (int e = tid; e < P; e += kStepThreads) pt[e] = pa[e];
         return;
     }
-    for (int i = tid; i < P; i += kStepThreads) {
-        rdg[i] = 1.0 / L[(int64_t)i * P + i];
+    for (int i = tid; i < n; i += kStepThreads) {
         xs[i] = 0.0;
-        y[i] = ga[i] * dinv[i];
+        y[i] = i < P ? ga[i] * dinv[i] : 0.0;
     }
     __syncthreads();
     // solution and one refinement step
     for (int pass = 0; pass < 2; pass++) {
         if (pass == 1) {
-            for (int i = tid; i < P; i += kStepThreads) {
-                double acc = ga[i] * dinv[i];
-                for (int j = 0; j < P; j++) acc -= scaled(i, j) * xs[j];
-                y[i] = acc;
+            // residual, a warp per row (Ha is symmetric)
+            for (int i = warp; i < P; i += kStepThreads / 32) {
+                double acc = 0.0;
+                if (dinv[i] != 0.0)
+                    for (int j = lane; j < P; j += 32)
+                        if (dinv[j] != 0.0)
+                            acc = fma(Ha[(int64_t)i * P + j] * dinv[j], xs[j], acc);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                if (lane == 0)
+                    y[i] = dinv[i] != 0.0 ? ga[i] * dinv[i] - (acc * dinv[i] + lam * xs[i])
+                                          : -xs[i];
             }
             __syncthreads();
         }
         if (warp == 0) {
-            // L z = y, w = D^-1 z, L^T x = w by columns, lane l holding rows
-            // l + 32 m in registers: l_ik = L[k P + i] / d_k
-            constexpr int kSlots = (TB_FIT_MAX_SRC * TB_FIT_NPAR + 31) / 32;
-            double v[kSlots];
+            // L z = y, w = D^-1 z, L^T x = w, four columns at a time, lane l
+            // holding rows l + 32 m in registers; l_ik = c_ik / d_k
+            constexpr int kSlots32 = (kStepMaxP + 31) / 32;
+            double v[kSlots32];
 #pragma unroll
-            for (int m = 0; m < kSlots; m++) {
-                const int i = lane + 32 * m;
-                v[m] = i < P ? y[i] : 0.0;
-            }
-            for (int k = 0; k < P; k++) {
-                double zk = 0.0;
+            for (int m = 0; m < kSlots32; m++) v[m] = lane + 32 * m < n ? y[lane + 32 * m] : 0.0;
+            auto row = [&](int k) {   // v at row k, in every lane
+                double z = 0.0;
 #pragma unroll
-                for (int m = 0; m < kSlots; m++)
-                    if (m == (k >> 5)) zk = v[m];
-                zk = __shfl_sync(0xffffffffu, zk, k & 31) * rdg[k];
-                const double* ck = L + (int64_t)k * P;
+                for (int m = 0; m < kSlots32; m++)
+                    if (m == (k >> 5)) z = v[m];
+                return __shfl_sync(0xffffffffu, z, k & 31);
+            };
+            for (int k = 0; k < n; k += 4) {
+                const double *c0 = col(k), *c1 = col(k + 1), *c2k = col(k + 2), *c3 = col(k + 3);
+                const double z0 = row(k) * rdg[k];
+                const double z1 = (row(k + 1) - c0[k + 1] * z0) * rdg[k + 1];
+                const double z2 = (row(k + 2) - c0[k + 2] * z0 - c1[k + 2] * z1) * rdg[k + 2];
+                const double z3 = (row(k + 3) - c0[k + 3] * z0 - c1[k + 3] * z1 -
+                                   c2k[k + 3] * z2) * rdg[k + 3];
 #pragma unroll
-                for (int m = 0; m < kSlots; m++) {
+                for (int m = 0; m < kSlots32; m++) {
                     const int i = lane + 32 * m;
-                    if (i > k && i < P) v[m] = fma(-ck[i], zk, v[m]);
+                    if (i >= k + 4 && i < n)
+                        v[m] -= c0[i] * z0 + c1[i] * z1 + c2k[i] * z2 + c3[i] * z3;
+                    else if (i >= k && i < k + 4)   // the solved rows, already times 1 / d
+                        v[m] = i == k ? z0 : i == k + 1 ? z1 : i == k + 2 ? z2 : z3;
+                }
+            }
+            for (int k = n - 4; k >= 0; k -= 4) {
+                // rows k .. k + 3 given every later one: x_k = w_k - sum_i c_ik / d_k x_i
+                const double *c0 = col(k), *c1 = col(k + 1), *c2k = col(k + 2), *c3 = col(k + 3);
+                double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+#pragma unroll
+                for (int m = 0; m < kSlots32; m++) {
+                    const int i = lane + 32 * m;
+                    if (i >= k + 4 && i < n) {
+                        s0 = fma(c0[i], v[m], s0);
+                        s1 = fma(c1[i], v[m], s1);
+                        s2 = fma(c2k[i], v[m], s2);
+                        s3 = fma(c3[i], v[m], s3);
+                    }
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+                    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+                    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+                    s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+                }
+                const double x3 = row(k + 3) - s3 * rdg[k + 3];
+                const double x2 = row(k + 2) - (s2 + c2k[k + 3] * x3) * rdg[k + 2];
+                const double x1 = row(k + 1) - (s1 + c1[k + 2] * x2 + c1[k + 3] * x3) * rdg[k + 1];
+                const double x0 = row(k) - (s0 + c0[k + 1] * x1 + c0[k + 2] * x2 +
+                                            c0[k + 3] * x3) * rdg[k];
+#pragma unroll
+                for (int m = 0; m < kSlots32; m++) {
+                    const int i = lane + 32 * m;
+                    if (i >= k && i < k + 4)
+                        v[m] = i == k ? x0 : i == k + 1 ? x1 : i == k + 2 ? x2 : x3;
                 }
             }
 #pragma unroll
-            for (int m = 0; m < kSlots; m++) {
-                const int i = lane + 32 * m;
-                if (i < P) v[m] *= rdg[i];
-            }
-            for (int k = P - 1; k > 0; k--) {
-                double xk = 0.0;
-#pragma unroll
-                for (int m = 0; m < kSlots; m++)
-                    if (m == (k >> 5)) xk = v[m];
-                xk = __shfl_sync(0xffffffffu, xk, k & 31);
-#pragma unroll
-                for (int m = 0; m < kSlots; m++) {
-                    const int j = lane + 32 * m;
-                    if (j < k) v[m] = fma(-L[(int64_t)j * P + k] * rdg[j], xk, v[m]);
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < kSlots; m++) {
-                const int i = lane + 32 * m;
-                if (i < P) y[i] = v[m];
-            }
+            for (int m = 0; m < kSlots32; m++)
+                if (lane + 32 * m < n) y[lane + 32 * m] = v[m];
         }
         __syncthreads();
         for (int i = tid; i < P; i += kStepThreads) xs[i] += y[i];
@@ -1667,19 +1307,55 @@ extern "C" int tb_fit_workspace(int32_t n_src, int32_t n_bands, int64_t* bytes) 
     if (n_src < 0 || n_bands < 1 || n_bands > TB_FIT_MAX_BANDS || !bytes) return TB_ERR_ARG;
     const int64_t tab = ((int64_t)n_src * (int64_t)sizeof(SrcTab) + 255) / 256 * 256;
     const int64_t nc = (int64_t)n_src * n_bands * kCompStride;
-    *bytes = tab + nc * (int64_t)sizeof(FitC) + nc * (int64_t)sizeof(FitC64);
+    *bytes = tab + nc * (int64_t)(sizeof(FitC<float>) + sizeof(FitC<double>));
     return TB_OK;
 }
 
 namespace {
 inline SrcTab* ws_tab(void* ws) { return static_cast<SrcTab*>(ws); }
-inline FitC* ws_comps(void* ws, int32_t n_src) {
+// component tables: FP64, then FP32
+inline FitC<double>* ws_comps64(void* ws, int32_t n_src) {
     const int64_t tab = ((int64_t)n_src * (int64_t)sizeof(SrcTab) + 255) / 256 * 256;
-    return reinterpret_cast<FitC*>(static_cast<char*>(ws) + tab);
+    return reinterpret_cast<FitC<double>*>(static_cast<char*>(ws) + tab);
 }
-inline FitC64* ws_comps64(void* ws, int32_t n_src, int32_t n_bands) {
-    return reinterpret_cast<FitC64*>(ws_comps(ws, n_src) +
-                                     (int64_t)n_src * n_bands * kCompStride);
+inline FitC<float>* ws_comps32(void* ws, int32_t n_src, int32_t n_bands) {
+    return reinterpret_cast<FitC<float>*>(ws_comps64(ws, n_src) +
+                                          (int64_t)n_src * n_bands * kCompStride);
+}
+inline const FitC<float>* ws_comps(void* ws, int32_t n_src, int32_t n_bands, float) {
+    return ws_comps32(ws, n_src, n_bands);
+}
+inline const FitC<double>* ws_comps(void* ws, int32_t n_src, int32_t, double) {
+    return ws_comps64(ws, n_src);
+}
+
+// One launch of the pass kernel in precision T over all units.
+template <class T>
+int launch_pass(const tb_fit_unit* units, const int32_t* order, int32_t n_units,
+                const tb_fit_blob* blobs, const tb_fit_source* srcs, int32_t n_src,
+                const void* workspace, const float* data, const float* inverr,
+                const int32_t* tiles, double* hbuf, double* gbuf, double* chi2_part,
+                double* chi2_const, const tb_fit_state* state, int32_t n_bands, Mode mode,
+                float* model, int32_t* work_counter, tb_status* status, cudaStream_t s) {
+    const int smem = (int)sizeof(PassSmem<T>);
+    if (cudaFuncSetAttribute(fit_pass_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             smem) != cudaSuccess)
+        return TB_ERR_LAUNCH;
+    if (cudaMemsetAsync(work_counter, 0, sizeof(int32_t), s) != cudaSuccess) return TB_ERR_LAUNCH;
+    if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
+        return TB_ERR_LAUNCH;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fit_pass_kernel<T>, kThreads,
+                                                      smem) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    const int64_t want = (int64_t)tb::num_sms() * per_sm;
+    const int grid = (int)(n_units < want ? n_units : want);
+    void* ws = const_cast<void*>(workspace);
+    fit_pass_kernel<T><<<grid, kThreads, smem, s>>>(
+        units, order, n_units, blobs, srcs, ws_tab(ws), ws_comps(ws, n_src, n_bands, T()), data,
+        inverr, hbuf, gbuf, chi2_part, state, n_bands, tiles, chi2_const, mode, model,
+        work_counter, status);
+    return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
 }
 }  // namespace
 
@@ -1708,8 +1384,9 @@ extern "C" int tb_fit_prep(const tb_fit_source* srcs, int32_t n_src, const doubl
     fit_prep_kernel<<<(n_src + per_block - 1) / per_block, kPrepThreads, smem,
                       (cudaStream_t)stream>>>(srcs, n_src, params, n_bands, units, n_units,
                                               *tables, cd_inv[0], cd_inv[1], cd_inv[2], cd_inv[3],
-                                              ws_tab(workspace), ws_comps(workspace, n_src),
-                                              ws_comps64(workspace, n_src, n_bands), state);
+                                              ws_tab(workspace),
+                                              ws_comps32(workspace, n_src, n_bands),
+                                              ws_comps64(workspace, n_src), state);
     return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
 }
 
@@ -1726,25 +1403,10 @@ extern "C" int tb_fit_pass(const tb_fit_unit* units, const int32_t* order, int32
     if (!units || !order || !blobs || !srcs || !workspace || !data || !inverr || !tiles ||
         !hbuf || !gbuf || !chi2_part || !chi2_const || !state || !work_counter)
         return TB_ERR_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    const int smem = (int)sizeof(PassSmem);
-    if (cudaFuncSetAttribute(fit_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-        cudaSuccess)
-        return TB_ERR_LAUNCH;
-    if (cudaMemsetAsync(work_counter, 0, sizeof(int32_t), s) != cudaSuccess) return TB_ERR_LAUNCH;
-    if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
-        return TB_ERR_LAUNCH;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fit_pass_kernel, kThreads, smem) !=
-            cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    const int64_t want = (int64_t)tb::num_sms() * per_sm;
-    const int grid = (int)(n_units < want ? n_units : want);
-    void* ws = const_cast<void*>(workspace);
-    fit_pass_kernel<<<grid, kThreads, smem, s>>>(
-        units, order, n_units, blobs, srcs, ws_tab(ws), ws_comps(ws, n_src), data, inverr, hbuf,
-        gbuf, chi2_part, state, n_bands, tiles, chi2_const, mode, work_counter, status);
-    return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
+    return launch_pass<float>(units, order, n_units, blobs, srcs, n_src, workspace, data, inverr,
+                              tiles, hbuf, gbuf, chi2_part, chi2_const, state, n_bands,
+                              mode == 0 ? kEquations : kConstant, nullptr, work_counter, status,
+                              (cudaStream_t)stream);
 }
 
 extern "C" int tb_fit_step(const tb_fit_blob* blobs, int32_t n_blobs, int32_t n_bands,
@@ -1755,7 +1417,12 @@ extern "C" int tb_fit_step(const tb_fit_blob* blobs, int32_t n_blobs, int32_t n_
     if (n_blobs == 0) return TB_OK;
     if (!blobs || !srcs || !params || !trial || !hbuf || !gbuf || !chi2_part || !state)
         return TB_ERR_ARG;
-    fit_step_kernel<<<n_blobs, kStepThreads, 0, (cudaStream_t)stream>>>(
+    if (cudaFuncSetAttribute(fit_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kStepSmem) != cudaSuccess)
+        return TB_ERR_LAUNCH;
+    fit_assemble_kernel<<<dim3(n_blobs, kAsmCtas), kStepThreads, 0, (cudaStream_t)stream>>>(
+        blobs, srcs, hbuf, gbuf, chi2_part, state);
+    fit_step_kernel<<<n_blobs, kStepThreads, kStepSmem, (cudaStream_t)stream>>>(
         blobs, n_blobs, n_bands, srcs, params, trial, hbuf, gbuf, chi2_part, state, tol, max_iter);
     return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
 }
@@ -1772,26 +1439,10 @@ extern "C" int tb_fit_refine(const tb_fit_unit* units, const int32_t* order, int
     if (!units || !order || !blobs || !srcs || !workspace || !data || !inverr || !tiles ||
         !hbuf || !gbuf || !chi2_out || !state || !work_counter)
         return TB_ERR_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    if (cudaMemsetAsync(work_counter, 0, sizeof(int32_t), s) != cudaSuccess) return TB_ERR_LAUNCH;
-    if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
-        return TB_ERR_LAUNCH;
-    const int smem = (int)sizeof(RefSmem);
-    if (cudaFuncSetAttribute(fit_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) != cudaSuccess)
-        return TB_ERR_LAUNCH;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fit_refine_kernel, kRefThreads,
-                                                      smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    const int64_t want = (int64_t)tb::num_sms() * per_sm;
-    const int grid = (int)(n_units < want ? n_units : want);
-    void* ws = const_cast<void*>(workspace);
-    fit_refine_kernel<<<grid, kRefThreads, smem, s>>>(
-        units, order, n_units, blobs, srcs, ws_tab(ws), ws_comps64(ws, n_src, n_bands), data,
-        inverr, hbuf, gbuf, chi2_out, state, n_bands, tiles, work_counter, status, TB_FIT_REFINE,
-        nullptr, chi2_const);
-    return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
+    return launch_pass<double>(units, order, n_units, blobs, srcs, n_src, workspace, data, inverr,
+                               tiles, hbuf, gbuf, chi2_out, const_cast<double*>(chi2_const), state,
+                               n_bands, kEquations, nullptr, work_counter, status,
+                               (cudaStream_t)stream);
 }
 
 extern "C" int tb_fit_model_vjp(const tb_fit_unit* units, const int32_t* order, int32_t n_units,
@@ -1806,25 +1457,9 @@ extern "C" int tb_fit_model_vjp(const tb_fit_unit* units, const int32_t* order, 
     if (!units || !order || !blobs || !srcs || !workspace || !tiles || !work_counter ||
         (mode == TB_FIT_MODEL && !model) || (mode == TB_FIT_VJP && (!grad || !gbuf)))
         return TB_ERR_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    if (cudaMemsetAsync(work_counter, 0, sizeof(int32_t), s) != cudaSuccess) return TB_ERR_LAUNCH;
-    if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
-        return TB_ERR_LAUNCH;
-    const int smem = (int)sizeof(RefSmem);
-    if (cudaFuncSetAttribute(fit_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) != cudaSuccess)
-        return TB_ERR_LAUNCH;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fit_refine_kernel, kRefThreads,
-                                                      smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    const int64_t want = (int64_t)tb::num_sms() * per_sm;
-    const int grid = (int)(n_units < want ? n_units : want);
-    void* ws = const_cast<void*>(workspace);
-    fit_refine_kernel<<<grid, kRefThreads, smem, s>>>(
-        units, order, n_units, blobs, srcs, ws_tab(ws), ws_comps64(ws, n_src, n_bands), grad,
-        nullptr, nullptr, gbuf, nullptr, nullptr, n_bands, tiles, work_counter, status, mode,
-        model, nullptr);
-    return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
+    return launch_pass<double>(units, order, n_units, blobs, srcs, n_src, workspace, grad, nullptr,
+                               tiles, nullptr, gbuf, nullptr, nullptr, nullptr, n_bands,
+                               mode == TB_FIT_MODEL ? kModel : kVjp, model, work_counter, status,
+                               (cudaStream_t)stream);
 }
 

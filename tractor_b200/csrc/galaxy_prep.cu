@@ -61,16 +61,6 @@ galaxy_fft_prep_kernel(const tb_galaxy_src* __restrict__ srcs, int n, tb_fft_ima
 }
 
 
-constexpr double kHn = 1e-5;   // central-difference step in the Sersic index
-constexpr double kHs = 1e-6;   // central-difference step in shape parameters
-
-__device__ void shape_factor(const tb_fft_image& img, int shape_type, double s0, double s1,
-                             double s2, double M[3], double& re) {
-    double G[4];
-    tb::shape_basis(shape_type, s0, s1, s2, G, re);
-    tb::pixel_factor(img.cd_inv, G, M[0], M[1], M[2]);
-}
-
 // Jacobian items: per source 7 items (x, y, counts, s0, s1, s2, n) on the
 // value item's geometry.  Position: the derivative Lanczos taps; counts: the
 // unit-flux render; shape and index: the spectrum's derivative with
@@ -93,29 +83,7 @@ galaxy_fft_jac_prep_kernel(const tb_galaxy_src* __restrict__ srcs, int n, tb_fft
     double a = 0.0, v = 0.0, da = 0.0, dv = 0.0;
     int K;
     if (s.profile == TB_PROFILE_SERSIC) {
-        double nn = s.sersic_n;
-        const double lowest = T.range_lohi[0], highest = T.range_lohi[2 * T.n_ranges - 1];
-        int r = -1;
-        bool clamped = false;
-        if (nn <= lowest) { r = 0; nn = lowest; clamped = true; }
-        else if (nn >= highest) { r = T.n_ranges - 1; nn = highest; clamped = true; }
-        else {
-            for (int q = 0; q < T.n_ranges; q++)
-                if (T.range_lohi[2 * q] <= nn && nn < T.range_lohi[2 * q + 1]) { r = q; break; }
-        }
-        if (r < 0 || T.range_info[4 * r] + 1 > kMaxComp) {
-            K = -1;
-        } else {
-            const bool core = nn > 1.0;
-            K = tb::sersic_fixed(T, r, nn, core, lane, a, v);
-            if (!clamped) {
-                double ap, vp, am, vm;
-                tb::sersic_fixed(T, r, nn + kHn, core, lane, ap, vp);
-                tb::sersic_fixed(T, r, nn - kHn, core, lane, am, vm);
-                da = (ap - am) / (2.0 * kHn);
-                dv = (vp - vm) / (2.0 * kHn);
-            }
-        }
+        K = tb::sersic_with_slope(T, s.sersic_n, lane, kMaxComp, a, v, da, dv);
     } else {
         K = tb::warp_profile(T, s.profile, s.sersic_n, lane, kMaxComp, a, v);
     }
@@ -123,21 +91,8 @@ galaxy_fft_jac_prep_kernel(const tb_galaxy_src* __restrict__ srcs, int n, tb_fft
     // derivative
     const int rank = tb::variance_rank(v, K, lane);
 
-    double M[3], re;
-    shape_factor(img, s.shape_type, s.s0, s.s1, s.s2, M, re);
-    double dM[3][3];
-    const double sp[3] = {s.s0, s.s1, s.s2};
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-        double hp[3] = {sp[0], sp[1], sp[2]}, hm[3] = {sp[0], sp[1], sp[2]};
-        hp[j] += kHs;
-        hm[j] -= kHs;
-        double Mp[3], Mm[3], rr;
-        shape_factor(img, s.shape_type, hp[0], hp[1], hp[2], Mp, rr);
-        shape_factor(img, s.shape_type, hm[0], hm[1], hm[2], Mm, rr);
-#pragma unroll
-        for (int q = 0; q < 3; q++) dM[j][q] = (Mp[q] - Mm[q]) / (2.0 * kHs);
-    }
+    double M[3], dM[3][3], re;
+    tb::shape_with_slopes(img.cd_inv, s.shape_type, s.s0, s.s1, s.s2, lane, M, dM, re);
 
     int flag, sz, si;
     prep_geometry(s, img, K, re, flag, sz, si);

@@ -223,26 +223,78 @@ __device__ inline int warp_profile(const tb_profile_tables& T, int profile, doub
     return K;
 }
 
-// Sersic mixture of range r at index nn with the core present or not, lane l
-// holding component l (the spline evaluation of warp_profile without the
-// range lookup, so that both sides of a central difference use the same
-// components).
+// Sum over K consecutive lanes from `first`, accumulated in lane order.
+__device__ __forceinline__ double lane_sum(double v, int K, int first) {
+    double s = 0.0;
+    for (int k = 0; k < K; k++) s += __shfl_sync(0xffffffffu, v, first + k);
+    return s;
+}
+
+// Sersic mixture of range r at index nn with the core present or not (the
+// spline evaluation of warp_profile without the range lookup, so that both
+// sides of a central difference use the same components).  Groups of lanes
+// may evaluate different nn at once: lane `first` + l of a group holds
+// component l; r and core_on are the same in every lane.
 __device__ inline int sersic_fixed(const tb_profile_tables& T, int r, double nn, bool core_on,
-                                   int lane, double& a, double& v) {
+                                   int l, int first, double& a, double& v) {
     const int Kr = T.range_info[4 * r], sa = T.range_info[4 * r + 1];
     const int sv = T.range_info[4 * r + 2];
     a = 0.0;
     v = 0.0;
-    if (lane < Kr) {
-        a = bspline(T, sa + lane, nn);
-        v = exp(bspline(T, sv + lane, nn));
+    if (l < Kr) {
+        a = bspline(T, sa + l, nn);
+        v = exp(bspline(T, sv + l, nn));
     }
-    a /= lane_sum(a, Kr);
+    a /= lane_sum(a, Kr, first);
     if (!core_on) return Kr;
     const double core = bspline(T, T.core_spline, nn);
-    a *= (1.0 - core) / lane_sum(a, Kr);
-    if (lane == Kr) { a = core; v = 0.0; }
+    a *= (1.0 - core) / lane_sum(a, Kr, first);
+    if (l == Kr) { a = core; v = 0.0; }
     return Kr + 1;
+}
+
+constexpr double kDiffN = 1e-5;    // central-difference step in the Sersic index
+constexpr double kDiffS = 1e-6;    // central-difference step in shape parameters
+constexpr int kDiffLanes = 10;     // lanes per difference point (components + core)
+
+// Sersic mixture at index n and its derivative in n by FP64 central
+// differences of the exact map with the range held fixed (zero where n is
+// clamped to the table): lane l < K holds component l's amplitude a, variance
+// v and their derivatives.  The index and its two difference points are
+// evaluated at once, ten lanes each.  Returns K, or -1 for more than max_k
+// components.  Whole warps.
+__device__ inline int sersic_with_slope(const tb_profile_tables& T, double n, int lane, int max_k,
+                                        double& a, double& v, double& da, double& dv) {
+    a = v = da = dv = 0.0;
+    double nn = n;
+    const double lowest = T.range_lohi[0], highest = T.range_lohi[2 * T.n_ranges - 1];
+    int r = -1;
+    bool clamped = false;
+    if (nn <= lowest) { r = 0; nn = lowest; clamped = true; }
+    else if (nn >= highest) { r = T.n_ranges - 1; nn = highest; clamped = true; }
+    else {
+        for (int q = 0; q < T.n_ranges; q++)
+            if (T.range_lohi[2 * q] <= nn && nn < T.range_lohi[2 * q + 1]) { r = q; break; }
+    }
+    if (r < 0 || T.range_info[4 * r] + 1 > max_k || T.range_info[4 * r] + 1 > kDiffLanes) return -1;
+    const int part = lane / kDiffLanes;
+    const double x = part == 1 ? nn + kDiffN : part == 2 ? nn - kDiffN : nn;
+    double a3, v3;
+    const int K = sersic_fixed(T, r, x, nn > 1.0, lane % kDiffLanes,
+                               part < 3 ? part * kDiffLanes : 0, a3, v3);
+    const double ap = __shfl_sync(0xffffffffu, a3, (lane + kDiffLanes) & 31);
+    const double vp = __shfl_sync(0xffffffffu, v3, (lane + kDiffLanes) & 31);
+    const double am = __shfl_sync(0xffffffffu, a3, (lane + 2 * kDiffLanes) & 31);
+    const double vm = __shfl_sync(0xffffffffu, v3, (lane + 2 * kDiffLanes) & 31);
+    if (lane < K) {
+        a = a3;
+        v = v3;
+        if (!clamped) {
+            da = (ap - am) / (2.0 * kDiffN);
+            dv = (vp - vm) / (2.0 * kDiffN);
+        }
+    }
+    return K;
 }
 
 // Stable rank of this lane's variance among lanes 0..K-1 (the argsort of
@@ -300,6 +352,31 @@ __device__ inline void pixel_factor(const double* C, const double G[4], double& 
     M00 = T0 * T0 + T1 * T1;
     M01 = T0 * T2 + T1 * T3;
     M11 = T2 * T2 + T3 * T3;
+}
+
+// A shape's pixel-space factor M = T T^T, its derivatives in the three shape
+// parameters by FP64 central differences, and r_e: lane 0 evaluates the shape,
+// lanes 1 + 2 j and 2 + 2 j its difference points in parameter j; every lane
+// receives the results.  Whole warps.
+__device__ inline void shape_with_slopes(const double* cd_inv, int shape_type, double s0, double s1,
+                                         double s2, int lane, double M[3], double dM[3][3],
+                                         double& re) {
+    double sh[3] = {s0, s1, s2};
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+        sh[j] += lane == 1 + 2 * j ? kDiffS : lane == 2 + 2 * j ? -kDiffS : 0.0;
+    double G[4], Ml[3];
+    shape_basis(shape_type, sh[0], sh[1], sh[2], G, re);
+    pixel_factor(cd_inv, G, Ml[0], Ml[1], Ml[2]);
+    re = __shfl_sync(0xffffffffu, re, 0);
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        M[q] = __shfl_sync(0xffffffffu, Ml[q], 0);
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+            dM[j][q] = (__shfl_sync(0xffffffffu, Ml[q], 1 + 2 * j) -
+                        __shfl_sync(0xffffffffu, Ml[q], 2 + 2 * j)) / (2.0 * kDiffS);
+    }
 }
 
 }  // namespace tb

@@ -25,7 +25,7 @@ import torch
 from . import _lib, batch, render
 
 NPAR = _lib.FIT_NPAR
-UNIT_TILES = 64      # active 32 x 8 tiles per pass unit (larger images are split)
+UNIT_TILES = 64      # active 32 x 8 tiles per pass unit at most (larger images are split)
 SERSIC_MIN, SERSIC_MAX = 0.29, 6.3
 
 
@@ -67,12 +67,13 @@ class BlobFitter(object):
         blobs['n_active'] = n_active
         blobs['n_tiles'] = n_tiles
         blobs['tile_off'] = np.concatenate([[0], np.cumsum(n_tiles)[:-1]])
-        # a band's active tiles go to ceil(n_active / UNIT_TILES) pass units,
-        # each with its own partial blocks (slices), so that no unit holds
-        # one CTA for long while few blobs are still running
+        # a band's active tiles go to pass units of a few tiles, each with its
+        # own partial blocks (slices), so that no unit holds one CTA for long
+        # while few blobs are still running
         unit_tiles = int(unit_tiles)
         if unit_tiles < 1:
             raise ValueError('unit_tiles must be positive')
+        unit_tiles = min(unit_tiles, pass_unit_tiles(n_active, P, self.n_bands))
         parts = np.maximum(1, -(-n_active // unit_tiles)).astype(np.int64)
         n_slices = self.n_bands * parts
         blobs['n_slices'] = n_slices
@@ -131,7 +132,8 @@ class BlobFitter(object):
         self.params = torch.from_numpy(np.ascontiguousarray(params0, np.float64).reshape(-1)).to(
             self.dev)
         self.trial = self.params.clone()
-        self.hbuf = torch.zeros(int(hsz.sum()), dtype=torch.float64, device=self.dev)
+        # (every unit clears what it uses of its slice)
+        self.hbuf = torch.empty(int(hsz.sum()), dtype=torch.float64, device=self.dev)
         self.gbuf = torch.zeros(int(gsz.sum()), dtype=torch.float64, device=self.dev)
         self.d_tiles = torch.from_numpy(tiles).to(self.dev)
         self.chi2_part = torch.zeros(int(n_slices.sum()), dtype=torch.float64,
@@ -313,6 +315,20 @@ class BlobFitter(object):
 
     def status(self):
         return self.misc[4:8]
+
+
+def pass_unit_tiles(n_active, P, n_bands):
+    """Active tiles per pass unit: about 2,400 units in all (16 per SM), so
+    that a few blobs still fill the GPU, but 4 tiles at least (a unit's start
+    costs about one tile) and 16 at most (on 300 blobs the late iterations,
+    with few blobs running, take 0.20 ms at 16 tiles and 0.45 ms at 64, and
+    smaller units slow the first ones), doubled while the partial blocks
+    would take more than 4 GB."""
+    n_active, P = np.asarray(n_active, np.int64), np.asarray(P, np.int64)
+    unit = int(min(16, max(4, n_bands * n_active.sum() // 2400)))
+    while unit < UNIT_TILES and 8 * int((n_bands * -(-n_active // unit) * P * P).sum()) > 4 << 30:
+        unit *= 2
+    return unit
 
 
 def blob_tiles(sides, sources, blob_src):
