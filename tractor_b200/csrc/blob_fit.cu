@@ -202,7 +202,10 @@ fit_prep_kernel(const tb_fit_source* __restrict__ srcs, int n, const double* __r
 // the products A^T A, A^T r go to the FP64 tensor core (mma m8n8k4),
 // accumulated in two registers per 8 x 8 block over a whole run of tiles with
 // the same sources: no block barrier inside a run, no reduction per pixel.
-// MEASURED
+// 300 blobs (192-512 px, 3 bands): first FP32 pass 2.5 -> 1.7 ms, first FP64
+// pass about 10 -> 3.1 ms; FP32 is latency-bound (2.3 instructions per cycle
+// and SM, FMA pipe 31 %, LSU 35 %, FP64 tensor 11 %), FP64 at 42 % of its pipe.
+// Model + gradient of 100 blobs 3.4 -> 1.8 ms of kernels.
 // ---------------------------------------------------------------------------
 constexpr int kWarps = kThreads / 32;
 constexpr int kSlots = 4;              // sources whose columns a warp holds at once
@@ -887,16 +890,22 @@ fit_assemble_kernel(const tb_fit_blob* __restrict__ blobs,
                 unsigned sl = __ballot_sync(0xffffffffu, ca_l >= 0 && ((mk >> a) & 1u));
                 if (c0 == r && ((sl >> lane) & 1u))
                     gs += gp[(int64_t)kk * P + compact_row(mk, a) + ca_l];
-#pragma unroll 4
-                for (; sl; sl &= sl - 1) {
-                    const int q = __ffs(sl) - 1;
-                    const unsigned m = __shfl_sync(0xffffffffu, mk, q);
-                    const int ca = __shfl_sync(0xffffffffu, ca_l, q);
-                    const int bq = __shfl_sync(0xffffffffu, band, q);
-                    const int cb = hs ? column(so, bq) : -1;
-                    if (cb >= 0 && ((m >> s) & 1u))
-                        h += Hp[(k0 + q) * PP + (compact_row(m, a) + ca) * kCols * __popc(m) +
-                                compact_row(m, s) + cb];
+                while (sl) {   // eight slices' loads in flight at a time
+                    double x[8];
+#pragma unroll
+                    for (int t = 0; t < 8; t++) {
+                        const int q = sl ? __ffs(sl) - 1 : 0;
+                        const unsigned m = __shfl_sync(0xffffffffu, mk, q);
+                        const int ca = __shfl_sync(0xffffffffu, ca_l, q);
+                        const int bq = __shfl_sync(0xffffffffu, band, q);
+                        const int cb = hs ? column(so, bq) : -1;
+                        x[t] = sl && cb >= 0 && ((m >> s) & 1u)
+                            ? Hp[(k0 + q) * PP + (compact_row(m, a) + ca) * kCols * __popc(m) +
+                                 compact_row(m, s) + cb] : 0.0;
+                        sl &= sl - 1;
+                    }
+#pragma unroll
+                    for (int t = 0; t < 8; t++) h += x[t];
                 }
             }
             if (c < P) {
@@ -908,6 +917,17 @@ fit_assemble_kernel(const tb_fit_blob* __restrict__ blobs,
         for (int o = 16; o > 0; o >>= 1) gs += __shfl_xor_sync(0xffffffffu, gs, o);
         if (lane == 0) ga[r] = gs;
     }
+}
+
+// 1 / d by Newton's iteration r <- r + r (1 - d r) from the hardware's
+// 20-bit estimate (twice: past FP64's precision): a shorter chain than an
+// IEEE division, and the refinement step covers its last bit.  A d that is
+// not a positive normal number is rejected by the caller.
+__device__ __forceinline__ double reciprocal(double d) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    r = fma(r, fma(-d, r, 1.0), r);
+    return fma(r, fma(-d, r, 1.0), r);
 }
 
 // Factor storage: packed lower triangle by columns, padded to a multiple of
@@ -928,7 +948,8 @@ static_assert(kStepSmem >= 8 * 5 * ((kStepMaxP + 7) / 8 * 8), "the vectors alway
 // factors the 4 x 4 diagonal block itself and finishes one row of the panel,
 // then the trailing tiles are updated by FP64 tensor-core products of rank 4)
 // is two barriers per four columns and 256 multiply-adds per instruction.
-// STEPMEASURED
+// Kernel time per step: 126 parameters 615 -> 175 us (with the assembly), 36
+// parameters 87 -> 29 us.
 __global__ void __launch_bounds__(kStepThreads, 3)
 fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
                 const tb_fit_source* __restrict__ srcs, double* __restrict__ params,
@@ -1021,33 +1042,35 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
         dsc[i] = d;
         dinv[i] = d == 0.0 ? 0.0 : 1.0 / d;
     }
-    __syncthreads();
-    // element (i, j) of the scaled matrix (H symmetric: read along i)
-    auto scaled = [&](int i, int j) -> double {
-        if (dinv[i] == 0.0 || dinv[j] == 0.0) return i == j ? 1.0 : 0.0;
-        return Ha[(int64_t)j * P + i] * dinv[i] * dinv[j] + (i == j ? lam : 0.0);
-    };
     for (int i = P + tid; i < n; i += kStepThreads) dinv[i] = dsc[i] = 0.0;
     __syncthreads();
     // LDL^T of the scaled matrix, right-looking: column k is left as d_k
     // (diagonal) and c_ik = d_k l_ik below it, and subtracts c_ik c_jk / d_k
     // from the trailing columns.
-    for (int j = warp; j < n; j += kStepThreads / 32)
-        for (int i = j + lane; i < n; i += 32)
-            col(j)[i] = i < P ? scaled(i, j) : (i == j ? 1.0 : 0.0);
+    for (int j0 = 0; j0 < n; j0 += kStepThreads / 32) {
+        const int j = j0 + warp;
+        const double dj = dinv[j];
+#pragma unroll 4
+        for (int i = j + lane; i < n; i += 32) {
+            const double h = i < P ? Ha[(int64_t)j * P + i] : 0.0;   // (j <= i)
+            const bool live = dinv[i] != 0.0 && dj != 0.0;
+            col(j)[i] = live ? h * dinv[i] * dj + (i == j ? lam : 0.0) : (i == j ? 1.0 : 0.0);
+        }
+    }
     __syncthreads();
     bool bad = false;
     for (int k0 = 0; k0 < n; k0 += 4) {
         const double *c0 = col(k0), *c1 = col(k0 + 1), *c2k = col(k0 + 2), *c3 = col(k0 + 3);
         // the 4 x 4 diagonal block, the same in every thread
         const double a10 = c0[k0 + 1], a20 = c0[k0 + 2], a30 = c0[k0 + 3];
-        const double d0 = c0[k0], r0 = 1.0 / d0;
-        const double d1 = c1[k0 + 1] - a10 * a10 * r0, r1 = 1.0 / d1;
+        const double d0 = c0[k0], r0 = reciprocal(d0);
+        const double d1 = c1[k0 + 1] - a10 * a10 * r0, r1 = reciprocal(d1);
         const double a21 = c1[k0 + 2] - a20 * a10 * r0, a31 = c1[k0 + 3] - a30 * a10 * r0;
-        const double d2 = c2k[k0 + 2] - a20 * a20 * r0 - a21 * a21 * r1, r2 = 1.0 / d2;
+        const double d2 = c2k[k0 + 2] - a20 * a20 * r0 - a21 * a21 * r1,
+                     r2 = reciprocal(d2);
         const double a32 = c2k[k0 + 3] - a30 * a20 * r0 - a31 * a21 * r1;
         const double d3 = c3[k0 + 3] - a30 * a30 * r0 - a31 * a31 * r1 - a32 * a32 * r2;
-        const double r3 = 1.0 / d3;
+        const double r3 = reciprocal(d3);
         if (!(d0 > 0.0 && d1 > 0.0 && d2 > 0.0 && d3 > 0.0) || !isfinite(d0) || !isfinite(d1) ||
             !isfinite(d2) || !isfinite(d3)) {
             bad = true;
@@ -1078,30 +1101,46 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
             rdg[k0 + 2] = r2;
             rdg[k0 + 3] = r3;
         }
-        // trailing 8 x 8 tiles (the first tile column may hold panel columns,
-        // which stay): rows i0 + lane / 4, columns j0 + 2 (lane % 4) + {0, 1}
+        // trailing 8 x 8 tiles: row lane / 4, columns 2 (lane % 4) + {0, 1}
         const int base = (k0 + 4) / 8 * 8, T = (n - base) / 8;
         const int q = lane & 3;
         const double rq = -(q == 0 ? r0 : q == 1 ? r1 : q == 2 ? r2 : r3);
         const double* ck = col(k0 + q);
-        for (int e = warp, tj = 0, ti = warp; e < T * (T + 1) / 2; e += kStepThreads / 32, ti += kStepThreads / 32) {
-            while (ti >= T) {   // row-major over the lower triangle's tile columns
-                tj++;
-                ti += tj - T;
+        int tj = 0, ti = warp;
+        for (int e = warp; e < T * (T + 1) / 2; e += 3 * (kStepThreads / 32)) {
+            // three tiles' loads before the first product
+            double *p0[3], *p1[3], fa[3], fb[3], c[3][2];
+            bool on0[3], on1[3];
+#pragma unroll
+            for (int t = 0; t < 3; t++) {
+                on0[t] = on1[t] = e + t * (kStepThreads / 32) < T * (T + 1) / 2;
+                fa[t] = fb[t] = c[t][0] = c[t][1] = 0.0;
+                if (!on0[t]) continue;
+                while (ti >= T) {   // the lower triangle's tile columns in turn
+                    tj++;
+                    ti += tj - T;
+                }
+                const int i = base + 8 * ti + (lane >> 2), j = base + 8 * tj + 2 * q;
+                const int jb = base + 8 * tj + (lane >> 2);
+                p0[t] = col(j) + i;
+                p1[t] = col(j + 1) + i;
+                // rows and columns above the trailing part (first tile only)
+                // belong to the panel
+                on0[t] = j >= k0 + 4 && i >= j;
+                on1[t] = j + 1 >= k0 + 4 && i >= j + 1;
+                if (i >= k0 + 4) fa[t] = ck[i];
+                if (jb >= k0 + 4) fb[t] = ck[jb] * rq;
+                if (on0[t]) c[t][0] = *p0[t];
+                if (on1[t]) c[t][1] = *p1[t];
+                ti += kStepThreads / 32;
             }
-            const int i0 = base + 8 * ti, j0 = base + 8 * tj;
-            const int i = i0 + (lane >> 2), j = j0 + 2 * q;
-            double* p0 = col(j) + i;
-            double* p1 = col(j + 1) + i;
-            const bool on0 = j >= k0 + 4 && i >= j, on1 = j + 1 >= k0 + 4 && i >= j + 1;
-            // rows above the trailing part (first tile only) belong to the panel
-            const double fa = i >= k0 + 4 ? ck[i] : 0.0;
-            const int jb = j0 + (lane >> 2);
-            const double fb = jb >= k0 + 4 ? ck[jb] * rq : 0.0;
-            double c[2] = {on0 ? *p0 : 0.0, on1 ? *p1 : 0.0};
-            mma884(c, fa, fb);
-            if (on0) *p0 = c[0];
-            if (on1) *p1 = c[1];
+#pragma unroll
+            for (int t = 0; t < 3; t++) mma884(c[t], fa[t], fb[t]);
+#pragma unroll
+            for (int t = 0; t < 3; t++) {
+                if (on0[t]) *p0[t] = c[t][0];
+                if (on1[t]) *p1[t] = c[t][1];
+            }
         }
         __syncthreads();
     }
@@ -1122,87 +1161,64 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
     // solution and one refinement step
     for (int pass = 0; pass < 2; pass++) {
         if (pass == 1) {
-            // residual, a warp per row (Ha is symmetric)
-            for (int i = warp; i < P; i += kStepThreads / 32) {
-                double acc = 0.0;
-                if (dinv[i] != 0.0)
-                    for (int j = lane; j < P; j += 32)
-                        if (dinv[j] != 0.0)
-                            acc = fma(Ha[(int64_t)i * P + j] * dinv[j], xs[j], acc);
+            // residual, four rows of a warp at a time (Ha is symmetric)
+            for (int i0 = 4 * warp; i0 < P; i0 += 4 * (kStepThreads / 32)) {
+                double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+                for (int j = lane; j < P; j += 32) {
+                    const bool live = dinv[j] != 0.0;
+                    const double xj = dinv[j] * xs[j];
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                if (lane == 0)
-                    y[i] = dinv[i] != 0.0 ? ga[i] * dinv[i] - (acc * dinv[i] + lam * xs[i])
-                                          : -xs[i];
+                    for (int t = 0; t < 4; t++) {
+                        const double h = i0 + t < P ? Ha[(int64_t)(i0 + t) * P + j] : 0.0;
+                        acc[t] = fma(live ? h : 0.0, xj, acc[t]);
+                    }
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int t = 0; t < 4; t++) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], o);
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    const int i = i0 + t;
+                    if (lane == t && i < P)
+                        y[i] = dinv[i] != 0.0 ? ga[i] * dinv[i] - (acc[t] * dinv[i] + lam * xs[i])
+                                              : -xs[i];
+                }
             }
             __syncthreads();
         }
         if (warp == 0) {
-            // L z = y, w = D^-1 z, L^T x = w, four columns at a time, lane l
-            // holding rows l + 32 m in registers; l_ik = c_ik / d_k
-            constexpr int kSlots32 = (kStepMaxP + 31) / 32;
-            double v[kSlots32];
-#pragma unroll
-            for (int m = 0; m < kSlots32; m++) v[m] = lane + 32 * m < n ? y[lane + 32 * m] : 0.0;
-            auto row = [&](int k) {   // v at row k, in every lane
-                double z = 0.0;
-#pragma unroll
-                for (int m = 0; m < kSlots32; m++)
-                    if (m == (k >> 5)) z = v[m];
-                return __shfl_sync(0xffffffffu, z, k & 31);
-            };
+            // L z = y, w = D^-1 z, L^T x = w in place in y, four columns at a
+            // time: every lane solves the 4 x 4 triangle, then the lanes
+            // update the remaining rows; l_ik = c_ik / d_k
             for (int k = 0; k < n; k += 4) {
                 const double *c0 = col(k), *c1 = col(k + 1), *c2k = col(k + 2), *c3 = col(k + 3);
-                const double z0 = row(k) * rdg[k];
-                const double z1 = (row(k + 1) - c0[k + 1] * z0) * rdg[k + 1];
-                const double z2 = (row(k + 2) - c0[k + 2] * z0 - c1[k + 2] * z1) * rdg[k + 2];
-                const double z3 = (row(k + 3) - c0[k + 3] * z0 - c1[k + 3] * z1 -
+                const double z0 = y[k] * rdg[k];
+                const double z1 = (y[k + 1] - c0[k + 1] * z0) * rdg[k + 1];
+                const double z2 = (y[k + 2] - c0[k + 2] * z0 - c1[k + 2] * z1) * rdg[k + 2];
+                const double z3 = (y[k + 3] - c0[k + 3] * z0 - c1[k + 3] * z1 -
                                    c2k[k + 3] * z2) * rdg[k + 3];
-#pragma unroll
-                for (int m = 0; m < kSlots32; m++) {
-                    const int i = lane + 32 * m;
-                    if (i >= k + 4 && i < n)
-                        v[m] -= c0[i] * z0 + c1[i] * z1 + c2k[i] * z2 + c3[i] * z3;
-                    else if (i >= k && i < k + 4)   // the solved rows, already times 1 / d
-                        v[m] = i == k ? z0 : i == k + 1 ? z1 : i == k + 2 ? z2 : z3;
-                }
+                for (int i = k + 4 + lane; i < n; i += 32)
+                    y[i] -= (c0[i] * z0 + c1[i] * z1) + (c2k[i] * z2 + c3[i] * z3);
+                __syncwarp();   // the triangle's rows are read
+                if (lane < 4) y[k + lane] = lane == 0 ? z0 : lane == 1 ? z1 : lane == 2 ? z2 : z3;
+                __syncwarp();
             }
             for (int k = n - 4; k >= 0; k -= 4) {
-                // rows k .. k + 3 given every later one: x_k = w_k - sum_i c_ik / d_k x_i
-                const double *c0 = col(k), *c1 = col(k + 1), *c2k = col(k + 2), *c3 = col(k + 3);
-                double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-#pragma unroll
-                for (int m = 0; m < kSlots32; m++) {
-                    const int i = lane + 32 * m;
-                    if (i >= k + 4 && i < n) {
-                        s0 = fma(c0[i], v[m], s0);
-                        s1 = fma(c1[i], v[m], s1);
-                        s2 = fma(c2k[i], v[m], s2);
-                        s3 = fma(c3[i], v[m], s3);
-                    }
+                const double *c0 = col(k), *c1 = col(k + 1), *c2k = col(k + 2);
+                const double x3 = y[k + 3];
+                const double x2 = y[k + 2] - c2k[k + 3] * rdg[k + 2] * x3;
+                const double x1 = y[k + 1] - (c1[k + 2] * x2 + c1[k + 3] * x3) * rdg[k + 1];
+                const double x0 = y[k] - (c0[k + 1] * x1 + c0[k + 2] * x2 + c0[k + 3] * x3) * rdg[k];
+                for (int j = lane; j < k; j += 32) {
+                    const double* cj = col(j) + k;
+                    y[j] -= ((cj[0] * x0 + cj[1] * x1) + (cj[2] * x2 + cj[3] * x3)) * rdg[j];
                 }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-                    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-                    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-                    s3 += __shfl_xor_sync(0xffffffffu, s3, o);
-                }
-                const double x3 = row(k + 3) - s3 * rdg[k + 3];
-                const double x2 = row(k + 2) - (s2 + c2k[k + 3] * x3) * rdg[k + 2];
-                const double x1 = row(k + 1) - (s1 + c1[k + 2] * x2 + c1[k + 3] * x3) * rdg[k + 1];
-                const double x0 = row(k) - (s0 + c0[k + 1] * x1 + c0[k + 2] * x2 +
-                                            c0[k + 3] * x3) * rdg[k];
-#pragma unroll
-                for (int m = 0; m < kSlots32; m++) {
-                    const int i = lane + 32 * m;
-                    if (i >= k && i < k + 4)
-                        v[m] = i == k ? x0 : i == k + 1 ? x1 : i == k + 2 ? x2 : x3;
-                }
+                __syncwarp();
+                if (lane < 3) y[k + lane] = lane == 0 ? x0 : lane == 1 ? x1 : x2;
+                __syncwarp();
             }
-#pragma unroll
-            for (int m = 0; m < kSlots32; m++)
-                if (lane + 32 * m < n) y[lane + 32 * m] = v[m];
         }
         __syncthreads();
         for (int i = tid; i < P; i += kStepThreads) xs[i] += y[i];
