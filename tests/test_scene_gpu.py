@@ -201,3 +201,26 @@ def test_full_size_scene_windows_match_oracle(tb, oracle):
             assert _peak_err(win, ref) < PEAK_TOL, (wx, wy)
         else:
             assert np.all(win == 0)
+
+
+@pytest.mark.parametrize('tile_h', [16, 32, 64])
+@pytest.mark.parametrize('sigma', [0.3, 0.7, 0.84, 0.86, 1.2, 40.])
+def test_sharp_and_wide_components_match_oracle(tb, oracle, tile_h, sigma):
+    """Around the curvature where the render leaves the exponential's row
+    recurrence (variance 0.72 px^2), far below and far above it, on odd
+    rectangles of an odd-sized image, sources off pixel centres.  Per pixel a
+    component's error is at most its exponentials' 2^-22 each, three of them
+    along a chain, plus FP32 rounding (a few 2^-24): 1.5e-6, of values up to
+    the peak."""
+    from tractor_b200 import batch
+    rng = np.random.default_rng(23)
+    W, H = 117, 131
+    s = batch.scene_sources(30, rng, W=W, H=H, hw_range=(3, 60))
+    rows = records_to_rows(s)
+    x0, y0 = np.maximum(rows[:, 4], 0), np.maximum(rows[:, 5], 0)
+    x1, y1 = np.minimum(rows[:, 4] + rows[:, 6], W), np.minimum(rows[:, 5] + rows[:, 7], H)
+    rows[:, 4], rows[:, 5], rows[:, 6], rows[:, 7] = x0, y0, x1 - x0, y1 - y0
+    r = batch.SceneRenderer([batch.SceneImage.circular(W, H, [sigma, 2 * sigma], [0.8, 0.2])])
+    got = r.image(r.render(s, tile_h=tile_h), 0).numpy()
+    ref = oracle.scene_model(rows, [0.8, 0.2], [sigma, 2 * sigma], H, W)
+    assert _peak_err(got, ref) < 1.5e-6

@@ -5,7 +5,7 @@
 // (tractor/engine.py:279-339, 455-473), with ConstrainedOptimizer's bounds and
 // maximum steps (tractor/constrained_optimizer.py:12-159).
 //
-// One iteration = three launches:
+// One iteration:
 //   tb_fit_prep  one warp per source: the profile mixture (exp / deV /
 //                Sersic) and its derivative with respect to the Sersic index,
 //                the pixel-space shape factor M = T T^T and its derivatives
@@ -15,10 +15,10 @@
 //   tb_fit_pass  one CTA per (blob, band) image, 32 x 8 pixel tiles: the
 //                model (every source's PSF-convolved mixture, as
 //                galaxy.py:307-326) and the analytic derivative columns
-//                (position, flux, shape, index), weighted by inverr, staged
-//                in shared memory; per tile A^T A, A^T r and r^T r added into
-//                buffers the CTA owns (no atomics);
-//   tb_fit_step  one CTA per blob: sums the band partials, accepts or
+//                (position, flux, shape, index), weighted by inverr; A^T A,
+//                A^T r and r^T r into the slice the CTA owns (no atomics);
+//   tb_fit_step  sums the slices (many CTAs per blob), then one CTA per blob:
+//                accepts or
 //                rejects the trial parameters, solves the Marquardt-damped
 //                normal equations by FP64 Cholesky with one refinement step,
 //                limits the step (bounds, maximum steps) and writes the next

@@ -22,8 +22,6 @@ namespace {
 
 constexpr int kPrepThreads = 128;   // 4 records (warps) per block
 constexpr int kMaxGal = 32;         // galaxy components of one source (one per lane)
-constexpr int kThreads = 256;       // render CTA
-constexpr int kSlots = kThreads;    // components staged per pass
 constexpr int kCap = 1024;          // items of one tile handled per chunk
 
 // ---------------------------------------------------------------------------
@@ -37,8 +35,8 @@ scene_prep_kernel(const tb_scene_src* __restrict__ srcs, int n,
                   const double* __restrict__ pvar, tb_profile_tables Tg,
                   tb_scene_item* __restrict__ items, double* __restrict__ camp,
                   double* __restrict__ cmean, double* __restrict__ cvar, int stride) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const tb_profile_tables T = tb::stage_tables(Tg, smem_raw);
+    // the tables are read where they lie (L1-cached), as in galaxy_fft_prep_kernel
+    const tb_profile_tables T = Tg;
     const int lane = threadIdx.x & 31;
     const int i = blockIdx.x * (kPrepThreads / 32) + (threadIdx.x >> 5);
     if (i >= n) return;   // whole warps leave together
@@ -172,36 +170,44 @@ __device__ __forceinline__ bool item_tiles(const tb_scene_item& it, const tb_sce
     return true;
 }
 
+// One warp per item, its lanes over the tiles the item's rectangle touches
+// (a thread per item waited for up to 81 returning atomics in turn: 23 us for
+// 150 items, 46 us for 20,000; now 3 and 9).  The count pass fills `counts`,
+// the fill pass takes list positions from the end of each tile's range by
+// counting it down (the render sorts each tile's items).
+constexpr int kBinThreads = 256;
+
 template <bool kFill>
-__global__ void scene_bin_kernel(const tb_scene_item* __restrict__ items, int n_items,
-                                 const tb_scene_image* __restrict__ images, int n_images,
-                                 int64_t n_tiles, int tile_h, int32_t* __restrict__ counts,
-                                 const int32_t* __restrict__ offsets, int32_t* __restrict__ list,
-                                 int64_t max_pairs, tb_status* st) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kBinThreads)
+scene_bin_kernel(const tb_scene_item* __restrict__ items, int n_items,
+                 const tb_scene_image* __restrict__ images, int n_images, int64_t n_tiles,
+                 int tile_h, int32_t* __restrict__ counts, const int32_t* __restrict__ offsets,
+                 int32_t* __restrict__ list, int64_t max_pairs, tb_status* st) {
+    const int lane = threadIdx.x & 31;
+    const int i = blockIdx.x * (kBinThreads / 32) + (threadIdx.x >> 5);
     if (i >= n_items) return;
     const tb_scene_item it = items[i];
     if (it.image < 0 || it.image >= n_images) {
-        if (!kFill && it.flag == 0) tb::report(st, TB_STATUS_BAD_ITEM, i, -1);
+        if (!kFill && it.flag == 0 && lane == 0) tb::report(st, TB_STATUS_BAD_ITEM, i, -1);
         return;
     }
     const tb_scene_image im = images[it.image];
     int tx0, tx1, ty0, ty1;
     if (!item_tiles(it, im, tile_h, tx0, tx1, ty0, ty1)) return;
     const int tiles_x = (im.W + TB_MOG_TILE - 1) / TB_MOG_TILE;
-    for (int ty = ty0; ty <= ty1; ty++) {
-        for (int tx = tx0; tx <= tx1; tx++) {
-            const int64_t t = im.tile0 + (int64_t)ty * tiles_x + tx;
-            if (t < 0 || t >= n_tiles) {
-                if (!kFill) tb::report(st, TB_STATUS_BAD_ITEM, i, -2);
-                continue;
-            }
-            const int pos = atomicAdd(&counts[t], 1);
-            if (kFill) {
-                const int64_t at = (int64_t)offsets[t] + pos;
-                if (at < max_pairs) list[at] = i;
-                else tb::report(st, TB_STATUS_BAD_ITEM, i, -3);
-            }
+    const int nx = tx1 - tx0 + 1, n = nx * (ty1 - ty0 + 1);
+    for (int q = lane; q < n; q += 32) {
+        const int64_t t = im.tile0 + (int64_t)(ty0 + q / nx) * tiles_x + tx0 + q % nx;
+        if (t < 0 || t >= n_tiles) {
+            if (!kFill) tb::report(st, TB_STATUS_BAD_ITEM, i, -2);
+            continue;
+        }
+        if (kFill) {
+            const int64_t at = (int64_t)offsets[t] + atomicSub(&counts[t], 1) - 1;
+            if (at < max_pairs) list[at] = i;
+            else tb::report(st, TB_STATUS_BAD_ITEM, i, -3);
+        } else {
+            atomicAdd(&counts[t], 1);
         }
     }
 }
@@ -240,13 +246,17 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_tot, int& t
 __global__ void __launch_bounds__(kScanThreads)
 scan_blocks_kernel(const int32_t* __restrict__ counts, int64_t n, int32_t* __restrict__ offsets,
                    int32_t* __restrict__ bsum) {
+    // (one block: the whole scan, its total included)
     __shared__ int warp_tot[32];
     const int64_t i = (int64_t)blockIdx.x * kScanThreads + threadIdx.x;
     const int v = i < n ? counts[i] : 0;
     int total;
     const int ex = block_exclusive_scan(v, warp_tot, total);
     if (i < n) offsets[i] = ex;
-    if (threadIdx.x == 0) bsum[blockIdx.x] = total;
+    if (threadIdx.x == 0) {
+        bsum[blockIdx.x] = total;
+        if (gridDim.x == 1) offsets[n] = total;
+    }
 }
 
 __global__ void __launch_bounds__(kScanThreads)
@@ -271,21 +281,87 @@ scan_add_kernel(int32_t* __restrict__ offsets, int64_t n, const int32_t* __restr
 }
 
 // ---------------------------------------------------------------------------
-// 3. tile renderer
+// 3. render
 // ---------------------------------------------------------------------------
 
-struct SceneC {
-    float mx, my;           // mean relative to the tile origin
-    float qxx, qxy, qyy;    // exponent (log2 units) = qxx dx^2 + qxy dx dy + qyy dy^2
-    float s;                // counts * amp / (2 pi sqrt(det))
-    float fl;               // exponent floor, log2 units
-    int32_t src;            // position of the source in the tile's sorted list
-    uint32_t rect;          // source rectangle in tile coordinates: x0 | x1<<8 | y0<<16 | y1<<24
-    int32_t pad;
-};
+// Two floats in one 64-bit register, for the packed FP32 instructions (two
+// multiply-adds per issue slot).
+using f32x2 = unsigned long long;
 
-template <int ROWS>
-__global__ void __launch_bounds__(kThreads)
+__device__ __forceinline__ f32x2 pack(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// A staged component: exponent qxx dx^2 + qxy dx dy + qyy dy^2 (log2 units),
+// its tile-relative centre as the nearest pixel plus a fraction (the centre
+// as one FP32 number was the largest error of the render: half an ulp of a
+// coordinate up to 64), Q = 2^(2 qyy), the amplitude s, the floor 2^fl, the
+// source it belongs to and the source's rectangle in the tile.
+struct __align__(16) SceneC {
+    float qxx[2], qxy[2];     // twice each: packed operands
+    float Q[2], s[2];
+    float ix, fx, iy, fy;
+    float qyy, thr;
+    int src;
+    uint32_t rect;            // x0 | x1 << 6 | y0 << 12 | y1 << 19, kInner, kDirect
+};
+constexpr uint32_t kInner = 1u << 30;    // no pixel of the rectangle is below the floor
+constexpr uint32_t kDirect = 1u << 31;   // every pixel's exponential by itself
+
+constexpr int kRows = 4;      // rows (and two columns) per thread
+constexpr float kMaxCurve = 1.0f;
+
+// Largest exponent of a component (a dx^2 + b dx dy + c dy^2, concave) over
+// the box [x0, x1] x [y0, y1] about its centre.
+__device__ __forceinline__ float max_exponent(float a, float b, float c, float x0, float x1,
+                                              float y0, float y1) {
+    if (x0 <= 0.f && x1 >= 0.f && y0 <= 0.f && y1 >= 0.f) return 0.f;
+    auto e = [&](float x, float y) { return fmaf(x, fmaf(a, x, b * y), c * y * y); };
+    const float ky = __fdividef(-0.5f * b, c), kx = __fdividef(-0.5f * b, a);
+    float m = e(x0, fminf(fmaxf(ky * x0, y0), y1));
+    m = fmaxf(m, e(x1, fminf(fmaxf(ky * x1, y0), y1)));
+    m = fmaxf(m, e(fminf(fmaxf(kx * y0, x0), x1), y0));
+    return fmaxf(m, e(fminf(fmaxf(kx * y1, x0), x1), y1));
+}
+
+// Persistent over tiles of 32 x TH pixels, 4 TH threads: a thread holds two
+// adjacent columns of four consecutive rows.
+//
+// Bound: issue slots and ex2.  Down a column the exponential follows
+//   E(y + 1) = E(y) R(y), R(y + 1) = R(y) Q, Q = 2^(2 qyy),
+// so eight pixels take four ex2 (E and R of the first row in two columns) and
+// five packed multiplies instead of eight ex2 and their exponents.  Three
+// steps from an anchor add about 3 ulp; with the centre split into pixel and
+// fraction the result is nearer to FP64 than eight separate ex2 from a
+// rounded centre.  The chain holds while |qyy| <= 1 (variance 0.72 px^2): a
+// first row so far out that E flushes to zero (2^-126) then has no row within
+// 2^-64 of the component's peak; sharper components take every pixel's ex2.
+// Exponents below the floor count as 0 (c_gauss_2d_grid skips Mahalanobis^2
+// >= 100), tested only where the component reaches it inside the rectangle.
+template <int TH>
+__global__ void __launch_bounds__(4 * TH, 256 / TH)
 scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
                     const tb_scene_image* __restrict__ images, int n_images, int64_t n_tiles,
                     int64_t max_pairs,
@@ -293,20 +369,21 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
                     const double* __restrict__ var, const int32_t* __restrict__ offsets,
                     const int32_t* __restrict__ list, float* __restrict__ out, int mode,
                     int32_t* counter, tb_status* st) {
-    constexpr int TH = 8 * ROWS;   // tile height (8 warps x ROWS rows)
-    __shared__ SceneC comps[kSlots];
+    constexpr int kThreads = 4 * TH;
+    constexpr int kWarps = kThreads / 32;
+    __shared__ SceneC comps[kThreads];
     __shared__ int ids[kCap];
     __shared__ int raw[kCap];
     __shared__ int prefK[kCap + 1];
     __shared__ int64_t slot;
     __shared__ int img_idx;
-    __shared__ int warp_count[kThreads / 32];
+    __shared__ int warp_count[kWarps];
     __shared__ int warp_tot[32];
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    const float xf = (float)lane;
+    const int x0 = 2 * (lane & 15), y0 = 8 * warp + kRows * (lane >> 4);
 
     // More overlaps than the list holds: the fill dropped some, so no tile
     // list can be trusted (tb_scene_render reports it from the fill pass).
@@ -336,9 +413,9 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
             continue;
         }
 
-        float acc[ROWS];
+        f32x2 acc[kRows], part[kRows];
 #pragma unroll
-        for (int j = 0; j < ROWS; j++) acc[j] = 0.f;
+        for (int j = 0; j < kRows; j++) acc[j] = part[j] = 0ull;
 
         const int beg = offsets[u];
         const int n = offsets[u + 1] - beg;
@@ -360,37 +437,44 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
                 ids[r] = v;
             }
             __syncthreads();
-            // exclusive prefix of component counts over the sorted items,
-            // 4 consecutive items per thread
+            // exclusive prefix of component counts over the sorted items, a
+            // few consecutive items per thread
             {
-                int k4[4], sum = 0;
-#pragma unroll
-                for (int z = 0; z < 4; z++) {
-                    const int q = 4 * tid + z;
-                    k4[z] = (q < m && ids[q] >= 0) ? items[ids[q]].K : 0;
-                    sum += k4[z];
+                constexpr int kPer = kCap / kThreads;
+                int sum = 0;
+                for (int z = 0; z < kPer; z++) {
+                    const int q = kPer * tid + z;
+                    if (q >= m) break;
+                    prefK[q] = sum;
+                    sum += ids[q] >= 0 ? items[ids[q]].K : 0;
                 }
                 int total;
-                int ex = block_exclusive_scan(sum, warp_tot, total);
-#pragma unroll
-                for (int z = 0; z < 4; z++) {
-                    const int q = 4 * tid + z;
-                    if (q < m) prefK[q] = ex;
-                    ex += k4[z];
+                const int ex = block_exclusive_scan(sum, warp_tot, total);
+                for (int z = 0; z < kPer; z++) {
+                    const int q = kPer * tid + z;
+                    if (q >= m) break;
+                    prefK[q] += ex;
                 }
                 if (tid == 0) prefK[m] = total;
             }
             __syncthreads();
             const int total = prefK[m];
 
-            float part[ROWS];
-#pragma unroll
-            for (int j = 0; j < ROWS; j++) part[j] = 0.f;
             int cur = -1;
-            bool colin = false;
-            unsigned rowmask = 0u;
+            bool rows = false;          // some row of this warp is in the source's rectangle
+            unsigned inside = 0u;       // bit 2 j + i: column i, row j of this thread is
+            // the finished source's patch, inside its rectangle
+            auto add_part = [&]() {
+#pragma unroll
+                for (int j = 0; j < kRows; j++) {
+                    const float2 p = unpack(part[j]);
+                    acc[j] = add2(acc[j], pack((inside >> (2 * j)) & 1u ? p.x : 0.f,
+                                               (inside >> (2 * j + 1)) & 1u ? p.y : 0.f));
+                    part[j] = 0ull;
+                }
+            };
 
-            for (int base = 0; base < total; base += kSlots) {
+            for (int base = 0; base < total; base += kThreads) {
                 const int g = base + tid;
                 bool keep = false;
                 SceneC c;
@@ -411,33 +495,42 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
                     const double v0 = var[4 * ci], v3 = var[4 * ci + 3];
                     const double vxy = 0.5 * (var[4 * ci + 1] + var[4 * ci + 2]);
                     const double det = v0 * v3 - vxy * vxy;
-                    const double sc = (double)it.scale * a / (2.0 * TB_PI * sqrt(det));
-                    const double f = -0.5 / det * TB_LOG2E;
-                    const double fl = (double)it.floor;
+                    const double ri = rsqrt(det);
+                    const double sc = (double)it.scale * a * (0.5 / TB_PI) * ri;
+                    const double f = (-0.5 * TB_LOG2E) * ri * ri;
+                    const float fl = (float)((double)it.floor * TB_LOG2E);
                     const double mx = (mean[2 * ci] + it.fx) - (double)ox;
                     const double my = (mean[2 * ci + 1] + it.fy) - (double)oy;
-                    c.qxx = (float)(v3 * f);
-                    c.qxy = (float)(-2.0 * vxy * f);
+                    const double mxi = rint(mx), myi = rint(my);
+                    c.qxx[0] = c.qxx[1] = (float)(v3 * f);
+                    c.qxy[0] = c.qxy[1] = (float)(-2.0 * vxy * f);
                     c.qyy = (float)(v0 * f);
-                    c.s = (float)sc;
-                    c.fl = (float)(fl * TB_LOG2E);
-                    c.mx = (float)mx;
-                    c.my = (float)my;
+                    c.Q[0] = c.Q[1] = exp2f((float)(2.0 * v0 * f));
+                    c.s[0] = c.s[1] = (float)sc;
+                    c.thr = exp2f(fl);
+                    c.ix = (float)mxi;
+                    c.fx = (float)(mx - mxi);
+                    c.iy = (float)myi;
+                    c.fy = (float)(my - myi);
                     c.src = lo;
-                    c.rect = (uint32_t)rx0 | ((uint32_t)rx1 << 8) | ((uint32_t)ry0 << 16) |
-                             ((uint32_t)ry1 << 24);
-                    c.pad = 0;
+                    c.rect = (uint32_t)rx0 | ((uint32_t)rx1 << 6) | ((uint32_t)ry0 << 12) |
+                             ((uint32_t)ry1 << 19);
                     const bool finite = det > 0.0 && isfinite(sc) && isfinite(f) &&
                                         isfinite(mx) && isfinite(my);
                     if (!finite) {
                         tb::report(st, TB_STATUS_NONFINITE, ii, k);
-                    } else if (a != 0.0 && rx0 < rx1 && ry0 < ry1) {
-                        // evaluated region (exponent >= floor) against the
-                        // part of the tile inside the rectangle
-                        const double r2 = -2.0 * fl;
-                        const double ex = sqrt(r2 * v0), ey = sqrt(r2 * v3);
-                        keep = (mx + ex >= rx0) && (mx - ex <= rx1 - 1) && (my + ey >= ry0) &&
-                               (my - ey <= ry1 - 1);
+                    } else if (a != 0.0 && rx0 < rx1 && ry0 < ry1 && v0 > 0.0) {
+                        // exponents over the part of the tile inside the
+                        // rectangle: all below the floor (with a margin), or none
+                        const float bx0 = (float)(rx0 - mx), bx1 = (float)(rx1 - 1 - mx);
+                        const float by0 = (float)(ry0 - my), by1 = (float)(ry1 - 1 - my);
+                        const float qa = c.qxx[0], qb = c.qxy[0], qc = c.qyy;
+                        keep = !(max_exponent(qa, qb, qc, bx0, bx1, by0, by1) < fl - 1.f);
+                        auto e = [&](float x, float y) { return fmaf(x, fmaf(qa, x, qb * y), qc * y * y); };
+                        const float lowest = fminf(fminf(e(bx0, by0), e(bx1, by0)),
+                                                   fminf(e(bx0, by1), e(bx1, by1)));
+                        if (lowest > fl + 1.f) c.rect |= kInner;
+                        if (!(fabsf(qc) <= kMaxCurve) || fl < -73.f) c.rect |= kDirect;
                     }
                 }
                 // order-preserving compaction of the kept components
@@ -446,7 +539,7 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
                 __syncthreads();
                 int wbase = 0, kept = 0;
 #pragma unroll
-                for (int w = 0; w < kThreads / 32; w++) {
+                for (int w = 0; w < kWarps; w++) {
                     wbase += (w < warp) ? warp_count[w] : 0;
                     kept += warp_count[w];
                 }
@@ -454,77 +547,103 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
                 __syncthreads();
 
                 for (int q = 0; q < kept; q++) {
-                    const SceneC g2 = comps[q];
+                    const SceneC& g2 = comps[q];
+                    const uint32_t rect = g2.rect;
                     if (g2.src != cur) {
-                        // previous source done: add its patch inside its rectangle
-#pragma unroll
-                        for (int j = 0; j < ROWS; j++) {
-                            acc[j] += colin ? part[j] : 0.f;
-                            part[j] = 0.f;
-                        }
+                        add_part();
                         cur = g2.src;
-                        const int rx0 = g2.rect & 0xff, rx1 = (g2.rect >> 8) & 0xff;
-                        const int ry0 = (g2.rect >> 16) & 0xff, ry1 = g2.rect >> 24;
-                        colin = lane >= rx0 && lane < rx1;
-                        rowmask = 0u;
+                        const int rx0 = rect & 63, rx1 = (rect >> 6) & 63;
+                        const int ry0 = (rect >> 12) & 127, ry1 = (rect >> 19) & 127;
+                        rows = 8 * warp < ry1 && 8 * warp + 8 > ry0;
+                        const unsigned cols = (x0 >= rx0 && x0 < rx1 ? 1u : 0u) |
+                                              (x0 + 1 >= rx0 && x0 + 1 < rx1 ? 2u : 0u);
+                        inside = 0u;
 #pragma unroll
-                        for (int j = 0; j < ROWS; j++) {
-                            const int y = warp + 8 * j;
-                            rowmask |= (y >= ry0 && y < ry1) ? (1u << j) : 0u;
-                        }
+                        for (int j = 0; j < kRows; j++)
+                            if (y0 + j >= ry0 && y0 + j < ry1) inside |= cols << (2 * j);
                     }
-                    const float dx = xf - g2.mx;
-                    const float A = g2.qxx * dx * dx;
-                    const float B = g2.qxy * dx;
+                    if (!rows) continue;
+                    const ulonglong2 pq = *reinterpret_cast<const ulonglong2*>(g2.qxx);
+                    const ulonglong2 ps = *reinterpret_cast<const ulonglong2*>(g2.Q);
+                    const float qyy = g2.qyy, thr = g2.thr;
+                    const float dx0 = ((float)x0 - g2.ix) - g2.fx;
+                    const float dy = ((float)y0 - g2.iy) - g2.fy;
+                    const f32x2 dx = pack(dx0, dx0 + 1.f);
+                    const f32x2 A = mul2(mul2(pq.x, dx), dx), B = mul2(pq.y, dx);
+                    if (rect & kDirect) {
+                        const float2 a2 = unpack(A), b2 = unpack(B);
 #pragma unroll
-                    for (int j = 0; j < ROWS; j++) {
-                        if (rowmask & (1u << j)) {
-                            const float dy = (float)(warp + 8 * j) - g2.my;
-                            const float e = fmaf(dy, fmaf(g2.qyy, dy, B), A);
-                            const float sv = (e >= g2.fl) ? g2.s : 0.f;
-                            part[j] = fmaf(sv, tb::ex2(e), part[j]);
+                        for (int j = 0; j < kRows; j++) {
+                            const float dj = dy + (float)j;
+                            const float ea = tb::ex2(fmaf(dj, fmaf(qyy, dj, b2.x), a2.x));
+                            const float eb = tb::ex2(fmaf(dj, fmaf(qyy, dj, b2.y), a2.y));
+                            part[j] = fma2(ps.y, pack(ea >= thr ? ea : 0.f, eb >= thr ? eb : 0.f),
+                                           part[j]);
+                        }
+                        continue;
+                    }
+                    // first row: E = 2^(A + dy (B + qyy dy)), R = 2^(B + qyy (2 dy + 1))
+                    const float u1 = qyy * dy, u2 = fmaf(2.f, u1, qyy);
+                    const float2 e0 = unpack(fma2(pack(dy, dy), add2(B, pack(u1, u1)), A));
+                    const float2 r0 = unpack(add2(B, pack(u2, u2)));
+                    f32x2 E = pack(tb::ex2(e0.x), tb::ex2(e0.y));
+                    // (a ratio above 2^126 starts from E = 0: kept finite)
+                    f32x2 R = pack(tb::ex2(fminf(r0.x, 126.f)), tb::ex2(fminf(r0.y, 126.f)));
+                    if (rect & kInner) {
+#pragma unroll
+                        for (int j = 0; j < kRows; j++) {
+                            part[j] = fma2(ps.y, E, part[j]);
+                            if (j + 1 < kRows) E = mul2(E, R);
+                            if (j + 2 < kRows) R = mul2(R, ps.x);
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < kRows; j++) {
+                            const float2 v = unpack(E);
+                            part[j] = fma2(ps.y, pack(v.x >= thr ? v.x : 0.f, v.y >= thr ? v.y : 0.f),
+                                           part[j]);
+                            if (j + 1 < kRows) E = mul2(E, R);
+                            if (j + 2 < kRows) R = mul2(R, ps.x);
                         }
                     }
                 }
                 __syncthreads();   // comps is overwritten by the next pass
             }
-#pragma unroll
-            for (int j = 0; j < ROWS; j++) acc[j] += colin ? part[j] : 0.f;
+            add_part();
         }
 
         const int64_t ldo = im.ldo > 0 ? im.ldo : im.W;
 #pragma unroll
-        for (int j = 0; j < ROWS; j++) {
-            const int y = warp + 8 * j;
-            if (lane < tw && y < th) {
-                float* p = out + im.out_off + (int64_t)(oy + y) * ldo + (ox + lane);
-                if (mode == TB_MOG_ACCUM) *p += acc[j];
-                else *p = acc[j];
-            }
+        for (int j = 0; j < kRows; j++) {
+            const float2 v = unpack(acc[j]);
+            if (y0 + j >= th) continue;
+            float* p = out + im.out_off + (int64_t)(oy + y0 + j) * ldo + (ox + x0);
+            if (x0 < tw) p[0] = mode == TB_MOG_ACCUM ? p[0] + v.x : v.x;
+            if (x0 + 1 < tw) p[1] = mode == TB_MOG_ACCUM ? p[1] + v.y : v.y;
         }
     }
 }
 
-template <int ROWS>
+template <int TH>
 int launch_render(const tb_scene_item* items, int n_items, const tb_scene_image* images,
                   int n_images, int64_t n_tiles, int64_t max_pairs, const double* a, const double* m, const double* v,
                   const int32_t* offsets, const int32_t* list, float* out, int mode,
                   int32_t* counter, tb_status* st, cudaStream_t s) {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scene_render_kernel<ROWS>, kThreads,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scene_render_kernel<TH>, 4 * TH,
                                                       0) != cudaSuccess || per_sm < 1)
         per_sm = 1;
     const int64_t want = (int64_t)tb::num_sms() * per_sm;
     const int grid = (int)(n_tiles < want ? n_tiles : want);
-    scene_render_kernel<ROWS><<<grid, kThreads, 0, s>>>(items, n_items, images, n_images, n_tiles,
+    scene_render_kernel<TH><<<grid, 4 * TH, 0, s>>>(items, n_items, images, n_images, n_tiles,
                                                         max_pairs, a, m, v, offsets, list, out,
                                                         mode, counter, st);
     return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
 }
 
-// Workspace layout (bytes, each section 256-aligned): counts[n_tiles] int32,
-// offsets[n_tiles + 1] int32, block sums int32, list[max_pairs] int32, the
-// work counter.
+// Workspace layout (bytes, each section 256-aligned): the work counter and
+// counts[n_tiles] int32 (cleared together), offsets[n_tiles + 1] int32, block
+// sums int32, list[max_pairs] int32.
 struct Workspace {
     int32_t* counts;
     int32_t* offsets;
@@ -541,16 +660,15 @@ Workspace carve(void* base, int64_t n_tiles, int64_t max_pairs) {
     const int64_t nb = (n_tiles + kScanThreads - 1) / kScanThreads;
     int64_t o = 0;
     char* b = static_cast<char*>(base);
-    w.counts = reinterpret_cast<int32_t*>(b + o);
-    o += align256(4 * n_tiles);
+    w.counter = reinterpret_cast<int32_t*>(b + o);
+    w.counts = w.counter + 1;
+    o += align256(4 * (n_tiles + 1));
     w.offsets = reinterpret_cast<int32_t*>(b + o);
     o += align256(4 * (n_tiles + 1));
     w.bsum = reinterpret_cast<int32_t*>(b + o);
     o += align256(4 * (nb > 0 ? nb : 1));
     w.list = reinterpret_cast<int32_t*>(b + o);
     o += align256(4 * (max_pairs > 0 ? max_pairs : 1));
-    w.counter = reinterpret_cast<int32_t*>(b + o);
-    o += 256;
     w.bytes = o;
     return w;
 }
@@ -568,14 +686,8 @@ extern "C" int tb_scene_prep(const tb_scene_src* srcs, int32_t n, const tb_scene
         !comp_amp || !comp_mean || !comp_var)
         return TB_ERR_ARG;
     if (comp_stride < 1 || comp_stride > TB_MOG_MAX_K) return TB_ERR_SIZE;
-    const int smem = tb::tables_smem_bytes(*tables);
-    if (smem > TB_PROFILE_SMEM_MAX) return TB_ERR_SIZE;
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(scene_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) != cudaSuccess)
-        return TB_ERR_LAUNCH;
     const int per_block = kPrepThreads / 32;
-    scene_prep_kernel<<<(n + per_block - 1) / per_block, kPrepThreads, smem,
+    scene_prep_kernel<<<(n + per_block - 1) / per_block, kPrepThreads, 0,
                         (cudaStream_t)stream>>>(srcs, n, images, n_images, psf_amp, psf_mean,
                                                 psf_var, *tables, items, comp_amp, comp_mean,
                                                 comp_var, comp_stride);
@@ -608,34 +720,35 @@ extern "C" int tb_scene_render(const tb_scene_item* items, int32_t n_items,
     cudaStream_t s = (cudaStream_t)stream;
     if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
         return TB_ERR_LAUNCH;
-    if (cudaMemsetAsync(w.counts, 0, 4 * n_tiles, s) != cudaSuccess) return TB_ERR_LAUNCH;
-    if (cudaMemsetAsync(w.counter, 0, 4, s) != cudaSuccess) return TB_ERR_LAUNCH;
-    const int nb_items = (n_items + 255) / 256;
+    if (cudaMemsetAsync(w.counter, 0, 4 * (n_tiles + 1), s) != cudaSuccess) return TB_ERR_LAUNCH;
+    const int per_bin = kBinThreads / 32;
+    const int nb_items = (n_items + per_bin - 1) / per_bin;
     if (n_items > 0) {
-        scene_bin_kernel<false><<<nb_items, 256, 0, s>>>(items, n_items, images, n_images, n_tiles,
-                                                         tile_h, w.counts, nullptr, nullptr,
-                                                         max_pairs, status);
+        scene_bin_kernel<false><<<nb_items, kBinThreads, 0, s>>>(
+            items, n_items, images, n_images, n_tiles, tile_h, w.counts, nullptr, nullptr,
+            max_pairs, status);
     }
     const int nb = (int)((n_tiles + kScanThreads - 1) / kScanThreads);
     scan_blocks_kernel<<<nb, kScanThreads, 0, s>>>(w.counts, n_tiles, w.offsets, w.bsum);
-    scan_sums_kernel<<<1, kScanThreads, 0, s>>>(w.bsum, nb, w.offsets, n_tiles);
-    scan_add_kernel<<<nb, kScanThreads, 0, s>>>(w.offsets, n_tiles, w.bsum);
+    if (nb > 1) {
+        scan_sums_kernel<<<1, kScanThreads, 0, s>>>(w.bsum, nb, w.offsets, n_tiles);
+        scan_add_kernel<<<nb, kScanThreads, 0, s>>>(w.offsets, n_tiles, w.bsum);
+    }
     if (n_items > 0) {
-        if (cudaMemsetAsync(w.counts, 0, 4 * n_tiles, s) != cudaSuccess) return TB_ERR_LAUNCH;
-        scene_bin_kernel<true><<<nb_items, 256, 0, s>>>(items, n_items, images, n_images, n_tiles,
-                                                        tile_h, w.counts, w.offsets, w.list,
-                                                        max_pairs, status);
+        scene_bin_kernel<true><<<nb_items, kBinThreads, 0, s>>>(
+            items, n_items, images, n_images, n_tiles, tile_h, w.counts, w.offsets, w.list,
+            max_pairs, status);
     }
     if (cudaGetLastError() != cudaSuccess) return TB_ERR_LAUNCH;
     switch (tile_h) {
         case 16:
-            return launch_render<2>(items, n_items, images, n_images, n_tiles, max_pairs, comp_amp, comp_mean, comp_var,
+            return launch_render<16>(items, n_items, images, n_images, n_tiles, max_pairs, comp_amp, comp_mean, comp_var,
                                     w.offsets, w.list, out, mode, w.counter, status, s);
         case 32:
-            return launch_render<4>(items, n_items, images, n_images, n_tiles, max_pairs, comp_amp, comp_mean, comp_var,
+            return launch_render<32>(items, n_items, images, n_images, n_tiles, max_pairs, comp_amp, comp_mean, comp_var,
                                     w.offsets, w.list, out, mode, w.counter, status, s);
         default:
-            return launch_render<8>(items, n_items, images, n_images, n_tiles, max_pairs, comp_amp, comp_mean, comp_var,
+            return launch_render<64>(items, n_items, images, n_images, n_tiles, max_pairs, comp_amp, comp_mean, comp_var,
                                     w.offsets, w.list, out, mode, w.counter, status, s);
     }
 }
