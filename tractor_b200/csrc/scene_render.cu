@@ -330,7 +330,6 @@ struct __align__(16) SceneC {
 constexpr uint32_t kInner = 1u << 30;    // no pixel of the rectangle is below the floor
 constexpr uint32_t kDirect = 1u << 31;   // every pixel's exponential by itself
 
-constexpr int kRows = 4;      // rows (and two columns) per thread
 constexpr float kMaxCurve = 1.0f;
 
 // Largest exponent of a component (a dx^2 + b dx dy + c dy^2, concave) over
@@ -346,8 +345,8 @@ __device__ __forceinline__ float max_exponent(float a, float b, float c, float x
     return fmaxf(m, e(fminf(fmaxf(kx * y1, x0), x1), y1));
 }
 
-// Persistent over tiles of 32 x TH pixels, 4 TH threads: a thread holds two
-// adjacent columns of four consecutive rows.
+// Persistent over tiles of 32 x TH pixels; a thread holds CP pairs of adjacent
+// columns of R consecutive rows.
 //
 // Bound: issue slots and ex2.  Down a column the exponential follows
 //   E(y + 1) = E(y) R(y), R(y + 1) = R(y) Q, Q = 2^(2 qyy),
@@ -360,8 +359,8 @@ __device__ __forceinline__ float max_exponent(float a, float b, float c, float x
 // 2^-64 of the component's peak; sharper components take every pixel's ex2.
 // Exponents below the floor count as 0 (c_gauss_2d_grid skips Mahalanobis^2
 // >= 100), tested only where the component reaches it inside the rectangle.
-template <int TH>
-__global__ void __launch_bounds__(4 * TH, 256 / TH)
+template <int TH, int CP, int R>
+__global__ void __launch_bounds__(16 * TH / (CP * R), (CP == 1 ? 1024 : 768) / (16 * TH / (CP * R)))
 scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
                     const tb_scene_image* __restrict__ images, int n_images, int64_t n_tiles,
                     int64_t max_pairs,
@@ -369,8 +368,9 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
                     const double* __restrict__ var, const int32_t* __restrict__ offsets,
                     const int32_t* __restrict__ list, float* __restrict__ out, int mode,
                     int32_t* counter, tb_status* st) {
-    constexpr int kThreads = 4 * TH;
+    constexpr int kThreads = 16 * TH / (CP * R);
     constexpr int kWarps = kThreads / 32;
+    constexpr int kWarpRows = 2 * CP * R;      // rows a warp covers, 32 columns wide
     __shared__ SceneC comps[kThreads];
     __shared__ int ids[kCap];
     __shared__ int raw[kCap];
@@ -383,7 +383,7 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    const int x0 = 2 * (lane & 15), y0 = 8 * warp + kRows * (lane >> 4);
+    const int x0 = 2 * CP * (lane % (16 / CP)), y0 = kWarpRows * warp + R * (lane / (16 / CP));
 
     // More overlaps than the list holds: the fill dropped some, so no tile
     // list can be trusted (tb_scene_render reports it from the fill pass).
@@ -413,9 +413,11 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
             continue;
         }
 
-        f32x2 acc[kRows], part[kRows];
+        f32x2 acc[R][CP], part[R][CP];
 #pragma unroll
-        for (int j = 0; j < kRows; j++) acc[j] = part[j] = 0ull;
+        for (int j = 0; j < R; j++)
+#pragma unroll
+            for (int p = 0; p < CP; p++) acc[j][p] = part[j][p] = 0ull;
 
         const int beg = offsets[u];
         const int n = offsets[u + 1] - beg;
@@ -462,16 +464,18 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
 
             int cur = -1;
             bool rows = false;          // some row of this warp is in the source's rectangle
-            unsigned inside = 0u;       // bit 2 j + i: column i, row j of this thread is
+            unsigned in_cols = 0u, in_rows = 0u;   // this thread's columns and rows that are
             // the finished source's patch, inside its rectangle
             auto add_part = [&]() {
 #pragma unroll
-                for (int j = 0; j < kRows; j++) {
-                    const float2 p = unpack(part[j]);
-                    acc[j] = add2(acc[j], pack((inside >> (2 * j)) & 1u ? p.x : 0.f,
-                                               (inside >> (2 * j + 1)) & 1u ? p.y : 0.f));
-                    part[j] = 0ull;
-                }
+                for (int j = 0; j < R; j++)
+#pragma unroll
+                    for (int p = 0; p < CP; p++) {
+                        const float2 v = unpack(part[j][p]);
+                        const unsigned in = (in_rows >> j) & 1u ? in_cols >> (2 * p) : 0u;
+                        acc[j][p] = add2(acc[j][p], pack(in & 1u ? v.x : 0.f, in & 2u ? v.y : 0.f));
+                        part[j][p] = 0ull;
+                    }
             };
 
             for (int base = 0; base < total; base += kThreads) {
@@ -548,97 +552,131 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
 
                 for (int q = 0; q < kept; q++) {
                     const SceneC& g2 = comps[q];
-                    const uint32_t rect = g2.rect;
-                    if (g2.src != cur) {
-                        add_part();
-                        cur = g2.src;
+                    const float4 head = *reinterpret_cast<const float4*>(&g2.qyy);
+                    const float qyy = head.x, thr = head.y;
+                    const int src = __float_as_int(head.z);
+                    const uint32_t rect = __float_as_uint(head.w);
+                    if (src != cur) {
+                        if (rows) add_part();
+                        cur = src;
                         const int rx0 = rect & 63, rx1 = (rect >> 6) & 63;
                         const int ry0 = (rect >> 12) & 127, ry1 = (rect >> 19) & 127;
-                        rows = 8 * warp < ry1 && 8 * warp + 8 > ry0;
-                        const unsigned cols = (x0 >= rx0 && x0 < rx1 ? 1u : 0u) |
-                                              (x0 + 1 >= rx0 && x0 + 1 < rx1 ? 2u : 0u);
-                        inside = 0u;
+                        rows = kWarpRows * warp < ry1 && kWarpRows * (warp + 1) > ry0;
+                        in_cols = in_rows = 0u;
 #pragma unroll
-                        for (int j = 0; j < kRows; j++)
-                            if (y0 + j >= ry0 && y0 + j < ry1) inside |= cols << (2 * j);
+                        for (int i = 0; i < 2 * CP; i++)
+                            if (x0 + i >= rx0 && x0 + i < rx1) in_cols |= 1u << i;
+#pragma unroll
+                        for (int j = 0; j < R; j++)
+                            if (y0 + j >= ry0 && y0 + j < ry1) in_rows |= 1u << j;
                     }
                     if (!rows) continue;
                     const ulonglong2 pq = *reinterpret_cast<const ulonglong2*>(g2.qxx);
                     const ulonglong2 ps = *reinterpret_cast<const ulonglong2*>(g2.Q);
-                    const float qyy = g2.qyy, thr = g2.thr;
-                    const float dx0 = ((float)x0 - g2.ix) - g2.fx;
-                    const float dy = ((float)y0 - g2.iy) - g2.fy;
-                    const f32x2 dx = pack(dx0, dx0 + 1.f);
-                    const f32x2 A = mul2(mul2(pq.x, dx), dx), B = mul2(pq.y, dx);
-                    if (rect & kDirect) {
-                        const float2 a2 = unpack(A), b2 = unpack(B);
+                    const float4 ctr = *reinterpret_cast<const float4*>(&g2.ix);
+                    const float dx0 = ((float)x0 - ctr.x) - ctr.y;
+                    const float dy = ((float)y0 - ctr.z) - ctr.w;
+                    f32x2 A[CP], B[CP];
 #pragma unroll
-                        for (int j = 0; j < kRows; j++) {
-                            const float dj = dy + (float)j;
-                            const float ea = tb::ex2(fmaf(dj, fmaf(qyy, dj, b2.x), a2.x));
-                            const float eb = tb::ex2(fmaf(dj, fmaf(qyy, dj, b2.y), a2.y));
-                            part[j] = fma2(ps.y, pack(ea >= thr ? ea : 0.f, eb >= thr ? eb : 0.f),
-                                           part[j]);
+                    for (int p = 0; p < CP; p++) {
+                        const f32x2 dx = pack(dx0 + (float)(2 * p), dx0 + (float)(2 * p + 1));
+                        A[p] = mul2(mul2(pq.x, dx), dx);
+                        B[p] = mul2(pq.y, dx);
+                    }
+                    if (rect & kDirect) {
+#pragma unroll
+                        for (int p = 0; p < CP; p++) {
+                            const float2 a2 = unpack(A[p]), b2 = unpack(B[p]);
+#pragma unroll
+                            for (int j = 0; j < R; j++) {
+                                const float dj = dy + (float)j;
+                                const float ea = tb::ex2(fmaf(dj, fmaf(qyy, dj, b2.x), a2.x));
+                                const float eb = tb::ex2(fmaf(dj, fmaf(qyy, dj, b2.y), a2.y));
+                                part[j][p] = fma2(ps.y, pack(ea >= thr ? ea : 0.f,
+                                                             eb >= thr ? eb : 0.f), part[j][p]);
+                            }
                         }
                         continue;
                     }
                     // first row: E = 2^(A + dy (B + qyy dy)), R = 2^(B + qyy (2 dy + 1))
                     const float u1 = qyy * dy, u2 = fmaf(2.f, u1, qyy);
-                    const float2 e0 = unpack(fma2(pack(dy, dy), add2(B, pack(u1, u1)), A));
-                    const float2 r0 = unpack(add2(B, pack(u2, u2)));
-                    f32x2 E = pack(tb::ex2(e0.x), tb::ex2(e0.y));
-                    // (a ratio above 2^126 starts from E = 0: kept finite)
-                    f32x2 R = pack(tb::ex2(fminf(r0.x, 126.f)), tb::ex2(fminf(r0.y, 126.f)));
+                    f32x2 E[CP], F[CP];
+#pragma unroll
+                    for (int p = 0; p < CP; p++) {
+                        const float2 e0 = unpack(fma2(pack(dy, dy), add2(B[p], pack(u1, u1)), A[p]));
+                        const float2 r0 = unpack(add2(B[p], pack(u2, u2)));
+                        E[p] = pack(tb::ex2(e0.x), tb::ex2(e0.y));
+                        // (a ratio above 2^126 starts from E = 0: kept finite)
+                        F[p] = pack(tb::ex2(fminf(r0.x, 126.f)), tb::ex2(fminf(r0.y, 126.f)));
+                    }
                     if (rect & kInner) {
 #pragma unroll
-                        for (int j = 0; j < kRows; j++) {
-                            part[j] = fma2(ps.y, E, part[j]);
-                            if (j + 1 < kRows) E = mul2(E, R);
-                            if (j + 2 < kRows) R = mul2(R, ps.x);
-                        }
+                        for (int j = 0; j < R; j++)
+#pragma unroll
+                            for (int p = 0; p < CP; p++) {
+                                part[j][p] = fma2(ps.y, E[p], part[j][p]);
+                                if (j + 1 < R) E[p] = mul2(E[p], F[p]);
+                                if (j + 2 < R) F[p] = mul2(F[p], ps.x);
+                            }
                     } else {
 #pragma unroll
-                        for (int j = 0; j < kRows; j++) {
-                            const float2 v = unpack(E);
-                            part[j] = fma2(ps.y, pack(v.x >= thr ? v.x : 0.f, v.y >= thr ? v.y : 0.f),
-                                           part[j]);
-                            if (j + 1 < kRows) E = mul2(E, R);
-                            if (j + 2 < kRows) R = mul2(R, ps.x);
-                        }
+                        for (int j = 0; j < R; j++)
+#pragma unroll
+                            for (int p = 0; p < CP; p++) {
+                                const float2 v = unpack(E[p]);
+                                part[j][p] = fma2(ps.y, pack(v.x >= thr ? v.x : 0.f,
+                                                             v.y >= thr ? v.y : 0.f), part[j][p]);
+                                if (j + 1 < R) E[p] = mul2(E[p], F[p]);
+                                if (j + 2 < R) F[p] = mul2(F[p], ps.x);
+                            }
                     }
                 }
                 __syncthreads();   // comps is overwritten by the next pass
             }
-            add_part();
+            if (rows) add_part();
         }
 
         const int64_t ldo = im.ldo > 0 ? im.ldo : im.W;
 #pragma unroll
-        for (int j = 0; j < kRows; j++) {
-            const float2 v = unpack(acc[j]);
+        for (int j = 0; j < R; j++) {
             if (y0 + j >= th) continue;
-            float* p = out + im.out_off + (int64_t)(oy + y0 + j) * ldo + (ox + x0);
-            if (x0 < tw) p[0] = mode == TB_MOG_ACCUM ? p[0] + v.x : v.x;
-            if (x0 + 1 < tw) p[1] = mode == TB_MOG_ACCUM ? p[1] + v.y : v.y;
+            float* o = out + im.out_off + (int64_t)(oy + y0 + j) * ldo + (ox + x0);
+#pragma unroll
+            for (int p = 0; p < CP; p++) {
+                const float2 v = unpack(acc[j][p]);
+                if (x0 + 2 * p < tw) o[2 * p] = mode == TB_MOG_ACCUM ? o[2 * p] + v.x : v.x;
+                if (x0 + 2 * p + 1 < tw)
+                    o[2 * p + 1] = mode == TB_MOG_ACCUM ? o[2 * p + 1] + v.y : v.y;
+            }
         }
     }
 }
 
-template <int TH>
+template <int TH, int CP, int R>
 int launch_render(const tb_scene_item* items, int n_items, const tb_scene_image* images,
-                  int n_images, int64_t n_tiles, int64_t max_pairs, const double* a, const double* m, const double* v,
-                  const int32_t* offsets, const int32_t* list, float* out, int mode,
+                  int n_images, int64_t n_tiles, int64_t max_pairs, const double* a, const double* m,
+                  const double* v, const int32_t* offsets, const int32_t* list, float* out, int mode,
                   int32_t* counter, tb_status* st, cudaStream_t s) {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scene_render_kernel<TH>, 4 * TH,
-                                                      0) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    const int64_t want = (int64_t)tb::num_sms() * per_sm;
+    constexpr int kThreads = 16 * TH / (CP * R);
+    // the CTAs per SM of the kernel's launch bounds
+    const int64_t want = (int64_t)tb::num_sms() * ((CP == 1 ? 1024 : 768) / kThreads);
     const int grid = (int)(n_tiles < want ? n_tiles : want);
-    scene_render_kernel<TH><<<grid, 4 * TH, 0, s>>>(items, n_items, images, n_images, n_tiles,
-                                                        max_pairs, a, m, v, offsets, list, out,
-                                                        mode, counter, st);
+    scene_render_kernel<TH, CP, R><<<grid, kThreads, 0, s>>>(
+        items, n_items, images, n_images, n_tiles, max_pairs, a, m, v, offsets, list, out, mode,
+        counter, st);
     return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
+}
+
+// Pixels per thread by the number of tiles: sixteen spend the fewest
+// instructions per pixel (16,384 tiles: 724 us, against 789 at eight and 1,089
+// at four; 2,820 tiles: 178, 179, 218), but a few tiles are rendered sooner by
+// more threads each (208 tiles: 70, 62, 57; 550 tiles: 78, 69, 69).
+template <int TH, class... Args>
+int dispatch_render(int64_t n_tiles, Args... args) {
+    const int64_t sms = tb::num_sms();
+    if (n_tiles >= 16 * sms) return launch_render<TH, 2, 4>(args...);
+    if (n_tiles >= 3 * sms) return launch_render<TH, 1, 4>(args...);
+    return launch_render<TH, 1, 2>(args...);
 }
 
 // Workspace layout (bytes, each section 256-aligned): the work counter and
@@ -740,15 +778,12 @@ extern "C" int tb_scene_render(const tb_scene_item* items, int32_t n_items,
             max_pairs, status);
     }
     if (cudaGetLastError() != cudaSuccess) return TB_ERR_LAUNCH;
-    switch (tile_h) {
-        case 16:
-            return launch_render<16>(items, n_items, images, n_images, n_tiles, max_pairs, comp_amp, comp_mean, comp_var,
-                                    w.offsets, w.list, out, mode, w.counter, status, s);
-        case 32:
-            return launch_render<32>(items, n_items, images, n_images, n_tiles, max_pairs, comp_amp, comp_mean, comp_var,
-                                    w.offsets, w.list, out, mode, w.counter, status, s);
-        default:
-            return launch_render<64>(items, n_items, images, n_images, n_tiles, max_pairs, comp_amp, comp_mean, comp_var,
-                                    w.offsets, w.list, out, mode, w.counter, status, s);
-    }
+    auto render = [&](auto... args) {
+        return tile_h == 16 ? dispatch_render<16>(n_tiles, args...)
+             : tile_h == 32 ? dispatch_render<32>(n_tiles, args...)
+                            : dispatch_render<64>(n_tiles, args...);
+    };
+    return render(items, n_items, images, n_images, n_tiles, max_pairs, comp_amp, comp_mean,
+                  comp_var, (const int32_t*)w.offsets, (const int32_t*)w.list, out, mode, w.counter,
+                  status, s);
 }
