@@ -12,8 +12,8 @@ device memory, by the fastest of three methods timed first on the workload:
 tb_galaxy_fft_render (each source's profile, shape and geometry prepared by
 one warp into shared memory, then spectrum, FFTs, Lanczos and crop by its
 block: one persistent launch), or tb_galaxy_fft_prep followed by the
-persistent tb_fourier_render or by tb_fourier_render_split (column and row
-kernels through an L2-resident scratch).  The metric
+persistent tb_fourier_render or by tb_fourier_render_split (items sorted by
+FFT size, packed transforms).  The metric
 is Mpix x components per second with Npix = sz^2 per source and the
 source's Gaussian component count (SersicGalaxy mixtures have 5-9), summed
 over sources.  L2 is flushed (a 256 MB write) before every timed step.
@@ -1475,10 +1475,9 @@ def main():
     clocks = ClockSampler(gpu_id)
     clocks.start()
     time.sleep(0.3)
-    # split: setup + column + row kernels per 256 items and the persistent
-    # kernel for the items outside the split path; persistent: one launch
+    # split: the sort and the render; persistent: one launch
     # after the prep; fused: one launch in all
-    launches_per_render = 3 * (-(-n // 256)) + 1 if method == 'split' else 1
+    launches_per_render = 2 if method == 'split' else 1
     ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True),
            torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
     for k in range(args.steps):
@@ -1594,7 +1593,7 @@ def main():
         'gpu_launches': gpu_launches,
         'fourier_method': {'chosen': method, 'ms': {k: _sig(v) for k, v in tune.items()}},
         'roofline': {'bound': 'sfu', 'kernel': {
-                         'split': 'tb_fourier_render_split (setup + column + row kernels)',
+                         'split': 'tb_fourier_render_split (sort + render by FFT size)',
                          'persistent': 'tb_fourier_render (persistent)',
                          'fused': 'tb_galaxy_fft_render (preparation + persistent render, '
                                   'one launch)'}[method],

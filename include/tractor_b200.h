@@ -264,18 +264,15 @@ int tb_fourier_render_deriv(const tb_fft_item* items, int32_t n_items,
                             double* dots, int32_t* work_counter, tb_status* status,
                             void* stream);
 
-/* The same renders (values, derivative items, TB_FFT_DOT) through the
- * split spectral path: a column kernel (units of 16 rfft columns of one
- * item: the mixture spectrum times the PSF spectrum and the y taps'
- * response, inverse FFT along y, the real parts only of the DC and Nyquist
- * columns) writes the kept rows of every column to `workspace`
- * (L2-resident: at most 256 items per column / row launch pair), and a row
- * kernel (units of 16 kept rows: times the x taps' response, inverse FFT
- * along x, two real rows per complex transform) writes the output.  Items
- * whose Lanczos-3 window reaches the FFT box edge, and TB_FFT_DOT items, go
- * to tb_fourier_render_deriv's kernel in a third launch.  Results equal
- * tb_fourier_render's up to FP32 rounding.  workspace: device, 256-byte
- * aligned, at least tb_fourier_workspace(n_items) bytes. */
+/* The same renders (values, derivative items, TB_FFT_DOT) with the items
+ * sorted by FFT size first and value items of up to 32 components whose
+ * Lanczos-3 window keeps 3 px from the FFT box's edges rendered on packed
+ * transforms, two columns or two row pairs at a time, by groups of warps (a
+ * CTA per item of size 256, two items per CTA at 128, seven at 64, sixteen at
+ * 32); the others as tb_fourier_render_deriv renders them.  Two launches.
+ * Results equal tb_fourier_render's up to FP32 rounding.  workspace: device,
+ * 256-byte aligned, at least tb_fourier_workspace(n_items) bytes, not shared
+ * by calls that may overlap. */
 int tb_fourier_workspace(int32_t n_items, int64_t* bytes);
 int tb_fourier_render_split(const tb_fft_item* items, int32_t n_items,
                             const double* comp_amp, const double* comp_var,

@@ -5,6 +5,8 @@ rendering); Lanczos bit-exact with the reference's float arithmetic; FFT-based
 spectra within 2e-6 relative to the largest element; least-squares solutions
 within 1e-9 relative of numpy's FP64 lstsq on well-conditioned problems.
 """
+from unittest import mock
+
 import numpy as np
 import pytest
 
@@ -291,6 +293,51 @@ def test_split_path_matches_persistent_kernel(tb, oracle):
                           specs.data_ptr(), out2.data_ptr(), misc.data_ptr() + 16,
                           dcoef_ptr=dcoef.data_ptr(), method='split')
     assert torch.equal(out1, out2)
+
+
+@pytest.mark.parametrize('sz, sides', [
+    (32, [(26, 26), (9, 24), (1, 5)]), (64, [(58, 58), (57, 31), (3, 2)]),
+    (128, [(122, 122), (61, 119), (7, 90)]),
+    (256, [(250, 250), (132, 131), (133, 128), (129, 134), (5, 249)])])
+def test_sorted_path_at_its_edges(tb, oracle, sz, sides):
+    """tb_fourier_render_split's packed transforms against plain FP64 transforms
+    at the largest windows they take (3 px from the box's edges), around the
+    rows one pass holds (132 at size 256), on rows and columns that leave
+    remainders, with 1 to 33 components (33: the general kernel), a point-like
+    core and a needle among them, stored and accumulated.  An FP32 transform
+    pair of size N rounds about 2 log2 N times: 16 x 2^-24 = 1e-6 of the peak
+    at 256, and as much for the spectrum: 2e-6."""
+    import torch
+    from tractor_b200 import render, plain
+    rng = np.random.default_rng(sz)
+    psf = _moffat({32: 15, 64: 31}.get(sz, 63))
+    spec, cx, cy = render.psf_spectra().get(('sorted-edges', sz), psf, sz)
+    spec64, cx64, cy64 = plain.psf_spectrum_fp64(psf, sz, torch.device('cuda'))
+    b, want = render.FftBatch(), []
+    for mw, mh in sides:
+        for K, mode in ((1, render.MOG_STORE), (9, render.MOG_STORE), (32, render.MOG_ACCUM),
+                        (33, render.MOG_STORE)):
+            amp, var = rng.uniform(.1, 1., K), np.zeros((K, 2, 2))
+            for k in range(K):
+                T = rng.normal(size=(2, 2)) * rng.uniform(0.3, sz / 40.)
+                var[k] = T @ T.T
+            if K > 1:
+                var[0] = 0.
+                var[1] = sz * np.array([[1., 0.999], [0.999, 1.]])
+            sx, sy = -((sz - mw) // 2), -((sz - mh) // 2)
+            px, py = cx + sx + rng.uniform(-.49, .49), cy + sy + rng.uniform(-.49, .49)
+            b.add(amp, var, sz, ('sorted-edges', sz), spec, mw, mh, sx, sy, px - cx - sx,
+                  py - cy - sy, scale=2., mode=mode)
+            want.append(plain.fourier_render_fp64(amp, var, spec64, cx64, cy64, sz, px, py, 0, 0,
+                                                  mw, mh, 2.).cpu().numpy())
+    out = torch.zeros(b.nout + 4, device='cuda')
+    with mock.patch.dict(render.fourier_method, {torch.cuda.current_device(): 'split'}):
+        b.run(out=out)
+    got, at = out.cpu().numpy(), 0
+    for w in want:
+        p = got[at:at + w.size].reshape(w.shape)
+        at += w.size
+        assert np.abs(p - w).max() <= 2e-6 * np.abs(w).max()
 
 
 @pytest.mark.parametrize('derivs', [False, True])

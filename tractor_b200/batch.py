@@ -4,8 +4,8 @@ FourierGalaxyRenderer renders thousands of galaxies through the
 pixelized-PSF Fourier path of ProfileGalaxy._realGetUnitFluxModelPatch
 (tractor/galaxy.py:336-519): tb_galaxy_fft_prep turns source parameters into
 work items and component tables on the device, and tb_fourier_render_split
-renders every item (column and row kernels, 256 items per pair, and the
-persistent kernel for the few items they do not cover).
+renders every item (sorted by FFT size); a few galaxies take one launch,
+tb_galaxy_fft_render.
 """
 import ctypes
 
@@ -127,10 +127,14 @@ class FourierGalaxyRenderer(object):
             cvar = torch.empty(n * COMP_STRIDE * 4, dtype=torch.float64, device=dev)
             flags = torch.empty(n, dtype=torch.int32, device=dev)
             misc = torch.zeros(8, dtype=torch.int32, device=dev)   # counter + status
-            self._scratch[n] = (items, camp, cvar, flags, misc)
+            ws = render.new_fourier_workspace(n, dev)
+            self._scratch[n] = (items, camp, cvar, flags, misc, ws)
         return self._scratch[n]
 
     METHODS = ('fused', 'persistent', 'split')
+    # one launch in place of three: 17 against 29 us for one 32-px patch; from
+    # about 30 patches of 100-200 px (77 us both) the sorted path is faster
+    FUSED_MAX = 24
 
     def render_device(self, srcs, n, out, stream=None, method=None):
         """Renders n sources whose GALAXY_SRC records are in device tensor
@@ -139,11 +143,13 @@ class FourierGalaxyRenderer(object):
         preparation and render in one persistent launch), 'persistent' or
         'split' (tb_galaxy_fft_prep, then tb_fourier_render /
         tb_fourier_render_split); None: the method autotune chose, else
-        'fused'.  Returns the flags tensor (see tb_galaxy_fft_prep)."""
+        'fused' for a few sources and 'split' for more (FUSED_MAX).  Returns
+        the flags tensor (see tb_galaxy_fft_prep)."""
         lib = _lib.load()
-        items, camp, cvar, flags, misc = self._work(n)
+        items, camp, cvar, flags, misc, ws = self._work(n)
         s = _lib.stream_ptr(stream)
-        method = method or getattr(self, 'method', None) or 'fused'
+        method = method or getattr(self, 'method', None) or (
+            'fused' if n <= self.FUSED_MAX else 'split')
         if method == 'fused':
             rc = lib.tb_galaxy_fft_render(srcs.data_ptr(), n, ctypes.addressof(self.image),
                                           ctypes.addressof(self.tables.struct),
@@ -159,7 +165,7 @@ class FourierGalaxyRenderer(object):
         _lib.check(rc, 'tb_galaxy_fft_prep')
         render.fourier_render(items.data_ptr(), n, camp.data_ptr(), cvar.data_ptr(),
                               self.spec.data_ptr(), out.data_ptr(), misc.data_ptr() + 16,
-                              stream=stream, method=method)
+                              stream=stream, method=method, workspace=ws)
         return flags
 
     def autotune(self, srcs, n, out):

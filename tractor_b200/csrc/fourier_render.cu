@@ -29,6 +29,7 @@
 // Windows taller than the row buffer are processed in row chunks (the column
 // pass is repeated per chunk).
 #include "fft16.cuh"
+#include "fft_pair.cuh"
 #include "galaxy_geom.cuh"
 
 namespace {
@@ -728,22 +729,21 @@ __device__ void render_staged_item(const tb_fft_item& it, int K,
     }
 }
 
+// Renders items[0 .. n_items), or the `n_list` of them that `list` names,
+// taken from `counter`.  The whole block.
 template <bool kDeriv>
-__global__ void __launch_bounds__(kThreads, 1)
-fourier_render_kernel(const tb_fft_item* __restrict__ items, int n_items,
-                      const double* __restrict__ amp, const double* __restrict__ var,
-                      const double* __restrict__ dcoef, const float* __restrict__ psf_spec,
-                      float* __restrict__ out, double* __restrict__ dots, int32_t* counter,
-                      tb_status* st, const int32_t* __restrict__ list = nullptr,
-                      const int32_t* __restrict__ list_count = nullptr) {
-    // `list` (optional): render only items list[0 .. *list_count)
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+__device__ void render_items(const tb_fft_item* __restrict__ items, int n_items,
+                             const double* __restrict__ amp, const double* __restrict__ var,
+                             const double* __restrict__ dcoef, const float* __restrict__ psf_spec,
+                             float* __restrict__ out, double* __restrict__ dots, int32_t* counter,
+                             tb_status* st, const int32_t* __restrict__ list, int n_list,
+                             unsigned char* smem_raw) {
     Shared sh = carve_shared(smem_raw);
     __shared__ int64_t slot;
     __shared__ int cur_n;
     if (threadIdx.x == 0) cur_n = 0;
 
-    const int64_t n_units = list ? (int64_t)*list_count : (int64_t)n_items;
+    const int64_t n_units = list ? n_list : n_items;
     for (;;) {
         const int64_t uu = tb::next_unit(counter, &slot);
         if (uu >= n_units) break;
@@ -785,6 +785,18 @@ fourier_render_kernel(const tb_fft_item* __restrict__ items, int n_items,
         }
         render_staged_item<kDeriv>(it, K, psf_spec, out, dots, sh, cur_n);
     }
+}
+
+template <bool kDeriv>
+__global__ void __launch_bounds__(kThreads, 1)
+fourier_render_kernel(const tb_fft_item* __restrict__ items, int n_items,
+                      const double* __restrict__ amp, const double* __restrict__ var,
+                      const double* __restrict__ dcoef, const float* __restrict__ psf_spec,
+                      float* __restrict__ out, double* __restrict__ dots, int32_t* counter,
+                      tb_status* st) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    render_items<kDeriv>(items, n_items, amp, var, dcoef, psf_spec, out, dots, counter, st,
+                         nullptr, 0, smem_raw);
 }
 
 // Fused preparation and render (tb_galaxy_fft_render): the persistent
@@ -834,42 +846,10 @@ galaxy_fft_render_kernel(const tb_galaxy_src* __restrict__ srcs, int n, tb_fft_i
 }
 
 // ---------------------------------------------------------------------------
-// Split spectral path (tb_fourier_render_split): a column kernel and a row
-// kernel joined by an L2-resident scratch, for every item whose Lanczos-3
-// shift is a spectral product (render_item's xin && yin) and whose output is
-// written or added (not TB_FFT_DOT).  Work units are small -- 16 rfft
-// columns or 16 kept rows of one item -- so every SM runs several CTAs of
-// 8 warps and the units of 256 galaxies spread evenly over the SMs; the
-// persistent kernel above holds one galaxy per SM and needs the whole
-// sz x (sz/2+1) transpose in its 180 KB of shared memory.
-//
-// Scratch: per item, column-major over the N/2 + 1 rfft columns, the kept
-// rows [gr0, gr1) of each column transform: S1[v * (gr1 - gr0) + (row -
-// gr0)] (the DC and Nyquist columns' real parts only, as irfftn).
-// Items that are not eligible are appended to a list for the persistent
-// kernel (third launch).
+// Main path of value items (tb_fourier_render_split).
 // ---------------------------------------------------------------------------
-// CTAs per SM the column and row kernels are compiled for (their register
-// budget: 3 -> 80, 4 -> 64 registers per thread)
-#ifndef TB_SPLIT_COL_MINB
-#define TB_SPLIT_COL_MINB 3
-#endif
-#ifndef TB_SPLIT_ROW_MINB
-#define TB_SPLIT_ROW_MINB 4
-#endif
-constexpr int kSplitThreads = 256;
-constexpr int kSplitWarps = kSplitThreads / 32;
-constexpr int kColBlock = 16;                 // rfft columns per column unit
-constexpr int kColUnits = (128 + 1 + kColBlock - 1) / kColBlock;   // per item at N = 256
-constexpr int kRowBlock = 16;                 // kept rows per row unit
-constexpr int kRowUnits = 256 / kRowBlock;
-constexpr int64_t kS1PerItem = 256 * 129;     // float2 per item (N x (N/2+1) at N = 256)
 
-struct SplitWs {
-    int32_t col_counter, row_counter, fb_counter, fb_count;
-    int32_t pad[60];
-};
-
+// Whether an item's zero-edged Lanczos-3 shift is a spectral product.
 __device__ __forceinline__ bool split_eligible(const tb_fft_item& it) {
     const int N = it.sz;
     const int gr0 = max(0, -it.sy), gr1 = min(N, it.mh - it.sy);
@@ -888,296 +868,7 @@ __device__ __forceinline__ bool item_ok(const tb_fft_item& it, const double* dco
            fabs(it.muy) <= 0.5;
 }
 
-struct SplitColShared {
-    float2 tw[256];
-    float4 comp[kMaxK];
-    float4 dcomp[kMaxK];
-    float taps[8];
-    float2 hy[256];
-    float2 xbuf[kSplitWarps * kXbufPerWarp];
-    int cur_n;
-    int64_t slot;
-};
-
-__device__ void stage_components(const tb_fft_item& it, const double* __restrict__ amp,
-                                 const double* __restrict__ var, const double* __restrict__ dcoef,
-                                 float4* comp, float4* dcomp) {
-    const double c2 = -2.0 * TB_PI * TB_PI * TB_LOG2E;
-    for (int k = threadIdx.x; k < it.K; k += kSplitThreads) {
-        const int c = it.c0 + k;
-        const double a = var[4 * c], bb = var[4 * c + 1], d = var[4 * c + 3];
-        comp[k] = make_float4((float)amp[c], (float)(c2 * a), (float)(c2 * 2.0 * bb),
-                              (float)(c2 * d));
-        if (it.dmode == TB_FFT_DSPEC) {
-            const double* dc = dcoef + 4 * ((int64_t)it.dc0 + k);
-            const double m2 = -2.0 * TB_PI * TB_PI * amp[c];
-            dcomp[k] = make_float4((float)dc[0], (float)(m2 * dc[1]), (float)(m2 * 2.0 * dc[2]),
-                                   (float)(m2 * dc[3]));
-        } else if (it.dmode == TB_FFT_DIFF) {
-            const double* dc = dcoef + 4 * ((int64_t)it.dc0 + k);
-            const double n2 = -2.0 * TB_PI * TB_PI;
-            dcomp[k] = make_float4((float)dc[0], (float)(n2 * dc[1]), (float)(n2 * 2.0 * dc[2]),
-                                   (float)(n2 * dc[3]));
-        }
-    }
-}
-
-// Spectrum of column v for the 8 rows of one thread, by item mode.
-__device__ __forceinline__ void spectrum_any(const tb_fft_item& it, const float4* comp,
-                                             const float4* dcomp, float vf, const float* wf,
-                                             float* acc) {
-    if (it.dmode == TB_FFT_DSPEC) dspectrum_rows<8>(comp, dcomp, it.K, vf, wf, acc);
-    else if (it.dmode == TB_FFT_DIFF) diffspectrum_rows<8>(comp, dcomp, it.K, vf, wf, acc);
-    else spectrum_rows<8>(comp, it.K, vf, wf, acc);
-}
-
-// Frequency response of the 7 Lanczos-3 taps at frequency index fr of an
-// N-point transform: sum_k taps[k] exp(2 pi i fr (k - 3) / N), from the
-// twiddle table.
-__device__ __forceinline__ float2 taps_response(const float* taps, const float2* tw, int fr,
-                                                int N) {
-    float2 r = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int k = 0; k < 7; k++) {
-        const float2 w = tw[(fr * (k - 3)) & (N - 1)];
-        r.x = fmaf(taps[k], w.x, r.x);
-        r.y = fmaf(taps[k], w.y, r.y);
-    }
-    return r;
-}
-
-template <int N>
-__device__ void split_col_unit(const tb_fft_item& it, int cb, const float* __restrict__ spec,
-                               float2* __restrict__ s1, SplitColShared& sh) {
-    constexpr int NH = N / 2 + 1;         // rfft columns
-    constexpr int T = N / 8;
-    constexpr int GPW = 32 / T;
-    constexpr int XB = tb::fft_xbuf_elems<N>();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t = lane % T;
-    float2* xb = sh.xbuf + warp * kXbufPerWarp + (lane / T) * XB;
-    const int gr0 = max(0, -it.sy), gr1 = min(N, it.mh - it.sy);
-    const int nr = gr1 - gr0;
-    const int cend = min(NH, (cb + 1) * kColBlock);
-    float wf[8];
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-        const int j = t + m * T;
-        wf[m] = (float)(j < N / 2 ? j : j - N) / (float)N;
-    }
-    for (int c0 = cb * kColBlock + warp * GPW; c0 < cend; c0 += kSplitWarps * GPW) {
-        const bool act = c0 + lane / T < cend;
-        const int c = act ? c0 + lane / T : cend - 1;
-        float2 x[8];
-        float acc[8];
-        spectrum_any(it, sh.comp, sh.dcomp, (float)c / (float)N, wf, acc);
-        const float2* P = reinterpret_cast<const float2*>(spec) + (int64_t)c * N;
-#pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const int j = t + m * T;
-            const float2 p = __ldg(P + j);
-            x[m] = cmulf(make_float2(acc[m] * p.x, acc[m] * p.y), sh.hy[j]);
-        }
-        // irfftn keeps only the real parts of the DC and Nyquist columns'
-        // transforms (the Nyquist column of the mixture spectrum is not
-        // Hermitian in w, so the two cannot share one complex transform)
-        const bool realcol = c == 0 || c == N / 2;
-        float2* col = s1 + (int64_t)c * nr;
-        tb::fft_run<N, +1>(x, t, xb, sh.tw, [&](int row, float2 z) {
-            if (act && row >= gr0 && row < gr1) col[row - gr0] = realcol ? make_float2(z.x, 0.f) : z;
-        });
-        __syncwarp();
-    }
-}
-
-__global__ void __launch_bounds__(kSplitThreads, TB_SPLIT_COL_MINB)
-fourier_split_col_kernel(const tb_fft_item* __restrict__ items, int i0, int n_items,
-                         const double* __restrict__ amp, const double* __restrict__ var,
-                         const double* __restrict__ dcoef, const float* __restrict__ psf_spec,
-                         float* __restrict__ out, SplitWs* ws, int32_t* fb_list,
-                         float2* __restrict__ s1_all, tb_status* st) {
-    __shared__ SplitColShared sh;
-    if (threadIdx.x == 0) sh.cur_n = 0;
-    const int64_t n_units = (int64_t)n_items * kColUnits;
-    for (;;) {
-        const int64_t u = tb::next_unit(&ws->col_counter, &sh.slot);
-        if (u >= n_units) break;
-        const int li = (int)(u / kColUnits), cb = (int)(u % kColUnits);
-        const int ii = i0 + li;
-        const tb_fft_item& it = items[ii];
-        const int N = it.sz;
-        if (cb == 0) {
-            if (!item_ok(it, dcoef)) {
-                if (threadIdx.x == 0) tb::report(st, TB_STATUS_BAD_ITEM, ii, N);
-                continue;
-            }
-            if (!split_eligible(it)) {
-                if (threadIdx.x == 0) fb_list[atomicAdd(&ws->fb_count, 1)] = ii;
-                continue;
-            }
-            // STORE: the mask's pixels outside the transform window are zero
-            const int gr0 = max(0, -it.sy), gr1 = min(N, it.mh - it.sy);
-            const int gc0 = max(0, -it.sx), gc1 = min(N, it.mw - it.sx);
-            if (it.mode == TB_MOG_STORE)
-                zero_outside(out + it.out_off, it.ldo > 0 ? it.ldo : it.mw, it.mw, it.mh, it.sx,
-                             it.sy, gr0, gr1, gc0, gc1, gr0 >= gr1 || gc0 >= gc1);
-        } else if (!item_ok(it, dcoef) || !split_eligible(it)) {
-            continue;
-        }
-        if (cb * kColBlock > N / 2) continue;
-        {
-            const int gr0 = max(0, -it.sy), gr1 = min(N, it.mh - it.sy);
-            const int gc0 = max(0, -it.sx), gc1 = min(N, it.mw - it.sx);
-            if (gr0 >= gr1 || gc0 >= gc1) continue;
-        }
-        // stage: components, y taps and their frequency response, twiddles
-        stage_components(it, amp, var, dcoef, sh.comp, sh.dcomp);
-        if (threadIdx.x < 32) taps_warp(it.muy, it.dmode == TB_FFT_DY, sh.taps);
-        if (sh.cur_n != N) {
-            __syncthreads();
-            switch (N) {
-                case 256: tb::build_twiddles<256>(sh.tw); break;
-                case 128: tb::build_twiddles<128>(sh.tw); break;
-                case 64: tb::build_twiddles<64>(sh.tw); break;
-                default: tb::build_twiddles<32>(sh.tw); break;
-            }
-            if (threadIdx.x == 0) sh.cur_n = N;
-        }
-        __syncthreads();
-        for (int j = threadIdx.x; j < N; j += kSplitThreads)
-            sh.hy[j] = taps_response(sh.taps, sh.tw, j, N);
-        __syncthreads();
-        float2* s1 = s1_all + (int64_t)li * kS1PerItem;
-        const float* spec = psf_spec + it.spec_off;
-        switch (N) {
-            case 256: split_col_unit<256>(it, cb, spec, s1, sh); break;
-            case 128: split_col_unit<128>(it, cb, spec, s1, sh); break;
-            case 64: split_col_unit<64>(it, cb, spec, s1, sh); break;
-            default: split_col_unit<32>(it, cb, spec, s1, sh); break;
-        }
-    }
-}
-
-struct SplitRowShared {
-    float2 tw[256];
-    float taps[8];
-    float2 hx[129];
-    float2 xbuf[kSplitWarps * kXbufPerWarp];
-    float2 rows[kRowBlock * 129];     // [r][v], the N/2 + 1 rfft columns
-    int cur_n;
-    int64_t slot;
-};
-
-template <int N>
-__device__ void split_row_unit(const tb_fft_item& it, int rb, const float2* __restrict__ s1,
-                               float* __restrict__ out, SplitRowShared& sh) {
-    constexpr int NH = N / 2 + 1;
-    constexpr int T = N / 8;
-    constexpr int GPW = 32 / T;
-    constexpr int XB = tb::fft_xbuf_elems<N>();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t = lane % T;
-    float2* xb = sh.xbuf + warp * kXbufPerWarp + (lane / T) * XB;
-    const int gr0 = max(0, -it.sy), gr1 = min(N, it.mh - it.sy);
-    const int gc0 = max(0, -it.sx), gc1 = min(N, it.mw - it.sx);
-    const int nr = gr1 - gr0;
-    const int r0 = rb * kRowBlock;
-    const int nrows = min(kRowBlock, nr - r0);
-    // this unit's rows of every rfft column, transposed into shared memory
-    // by asynchronous 8-byte copies (all of a thread's copies in flight at
-    // once, no registers held); rows >= nrows are not read below
-    constexpr int kLd = (NH * kRowBlock + kSplitThreads - 1) / kSplitThreads;
-#pragma unroll
-    for (int q = 0; q < kLd; q++) {
-        const int e = threadIdx.x + q * kSplitThreads;
-        const int c = e / kRowBlock, r = e % kRowBlock;
-        if (e < NH * kRowBlock && r < nrows) {
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sh.rows[r * 129 + c]);
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst),
-                         "l"(s1 + (int64_t)c * nr + r0 + r) : "memory");
-        }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    const float osc = it.scale / (float)(N * N);
-    float* O = out + it.out_off;
-    const int64_t ldo = it.ldo > 0 ? it.ldo : it.mw;
-    const int npairs = (nrows + 1) / 2;
-    for (int p0 = warp * GPW; p0 < npairs; p0 += kSplitWarps * GPW) {
-        const bool act = p0 + lane / T < npairs;
-        const int p = act ? p0 + lane / T : npairs - 1;
-        const int ia = 2 * p, ib = 2 * p + 1;
-        const bool hasb = ib < nrows;
-        const float2* H1 = sh.rows + ia * 129;
-        const float2* H2 = sh.rows + (hasb ? ib : ia) * 129;
-        float2 x[8];
-#pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const int n = t + m * T;
-            const int q = n <= N / 2 ? n : N - n;
-            const float2 g1 = H1[q], g2 = H2[q];
-            const float2 hx = sh.hx[q];
-            const float2 h1 = cmulf(g1, hx);
-            const float2 h2 = hasb ? cmulf(g2, hx) : make_float2(0.f, 0.f);
-            x[m] = n <= N / 2 ? make_float2(h1.x - h2.y, h1.y + h2.x)
-                              : make_float2(h1.x + h2.y, h2.x - h1.y);
-        }
-        float* oa = O + (int64_t)(gr0 + r0 + ia + it.sy) * ldo + it.sx;
-        float* ob = O + (int64_t)(gr0 + r0 + ib + it.sy) * ldo + it.sx;
-        float dummy = 0.f;
-        tb::fft_run<N, +1>(x, t, xb, sh.tw, [&](int col, float2 z) {
-            if (act && col >= gc0 && col < gc1) {
-                put<false>(oa + col, z.x * osc, it.mode, dummy);
-                if (hasb) put<false>(ob + col, z.y * osc, it.mode, dummy);
-            }
-        });
-        __syncwarp();
-    }
-}
-
-__global__ void __launch_bounds__(kSplitThreads, TB_SPLIT_ROW_MINB)
-fourier_split_row_kernel(const tb_fft_item* __restrict__ items, int i0, int n_items,
-                         const double* __restrict__ dcoef, float* __restrict__ out, SplitWs* ws,
-                         const float2* __restrict__ s1_all) {
-    __shared__ SplitRowShared sh;
-    if (threadIdx.x == 0) sh.cur_n = 0;
-    const int64_t n_units = (int64_t)n_items * kRowUnits;
-    for (;;) {
-        const int64_t u = tb::next_unit(&ws->row_counter, &sh.slot);
-        if (u >= n_units) break;
-        const int li = (int)(u / kRowUnits), rb = (int)(u % kRowUnits);
-        const tb_fft_item& it = items[i0 + li];
-        if (!item_ok(it, dcoef) || !split_eligible(it)) continue;
-        const int N = it.sz;
-        const int gr0 = max(0, -it.sy), gr1 = min(N, it.mh - it.sy);
-        const int gc0 = max(0, -it.sx), gc1 = min(N, it.mw - it.sx);
-        if (gr0 >= gr1 || gc0 >= gc1 || rb * kRowBlock >= gr1 - gr0) continue;
-        if (threadIdx.x < 32) taps_warp(it.mux, it.dmode == TB_FFT_DX, sh.taps);
-        if (sh.cur_n != N) {
-            __syncthreads();
-            switch (N) {
-                case 256: tb::build_twiddles<256>(sh.tw); break;
-                case 128: tb::build_twiddles<128>(sh.tw); break;
-                case 64: tb::build_twiddles<64>(sh.tw); break;
-                default: tb::build_twiddles<32>(sh.tw); break;
-            }
-            if (threadIdx.x == 0) sh.cur_n = N;
-        }
-        __syncthreads();
-        // the x taps' frequency response
-        for (int f = threadIdx.x; f <= N / 2; f += kSplitThreads)
-            sh.hx[f] = taps_response(sh.taps, sh.tw, f, N);
-        __syncthreads();
-        const float2* s1 = s1_all + (int64_t)li * kS1PerItem;
-        switch (N) {
-            case 256: split_row_unit<256>(it, rb, s1, out, sh); break;
-            case 128: split_row_unit<128>(it, rb, s1, out, sh); break;
-            case 64: split_row_unit<64>(it, rb, s1, out, sh); break;
-            default: split_row_unit<32>(it, rb, s1, out, sh); break;
-        }
-    }
-}
+#include "fourier_pair.cuh"
 
 }  // namespace
 
@@ -1248,29 +939,12 @@ extern "C" int tb_galaxy_fft_render(const tb_galaxy_src* srcs, int32_t n,
 }
 
 namespace {
-constexpr int kSplitChunk = 256;      // items per column/row launch pair (scratch bound)
-
-int64_t split_list_bytes(int32_t n_items) { return ((int64_t)n_items * 4 + 255) / 256 * 256; }
-
-int split_grid(const void* fn) {
-    static int cached[2] = {0, 0};
-    const int which = fn == (const void*)fourier_split_col_kernel ? 0 : 1;
-    if (cached[which] == 0) {
-        int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSplitThreads, 0) !=
-                cudaSuccess || per_sm < 1)
-            per_sm = 1;
-        cached[which] = per_sm;
-    }
-    return tb::num_sms() * cached[which];
-}
+int64_t list_bytes(int32_t n_items) { return ((int64_t)n_items * 4 * 5 + 255) / 256 * 256; }
 }  // namespace
 
 extern "C" int tb_fourier_workspace(int32_t n_items, int64_t* bytes) {
     if (n_items < 0 || !bytes) return TB_ERR_ARG;
-    const int64_t chunk = n_items < kSplitChunk ? n_items : kSplitChunk;
-    *bytes = (int64_t)sizeof(SplitWs) + split_list_bytes(n_items) +
-             chunk * kS1PerItem * (int64_t)sizeof(float2);
+    *bytes = (int64_t)sizeof(PairWs) + list_bytes(n_items);
     return TB_OK;
 }
 
@@ -1288,40 +962,24 @@ extern "C" int tb_fourier_render_split(const tb_fft_item* items, int32_t n_items
     tb_fourier_workspace(n_items, &need);
     if (workspace_bytes < need) return TB_ERR_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
-    SplitWs* ws = static_cast<SplitWs*>(workspace);
-    int32_t* fb_list = reinterpret_cast<int32_t*>(static_cast<char*>(workspace) + sizeof(SplitWs));
-    float2* s1 = reinterpret_cast<float2*>(static_cast<char*>(workspace) + sizeof(SplitWs) +
-                                           split_list_bytes(n_items));
-    if (cudaMemsetAsync(ws, 0, sizeof(SplitWs), s) != cudaSuccess) return TB_ERR_LAUNCH;
-    if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
+    PairWs* ws = static_cast<PairWs*>(workspace);
+    int32_t* lists = reinterpret_cast<int32_t*>(static_cast<char*>(workspace) + sizeof(PairWs));
+    if (cudaFuncSetAttribute(fourier_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kPairSmem) != cudaSuccess)
         return TB_ERR_LAUNCH;
-    const int gcol = split_grid((const void*)fourier_split_col_kernel);
-    const int grow = split_grid((const void*)fourier_split_row_kernel);
-    for (int32_t i0 = 0; i0 < n_items; i0 += kSplitChunk) {
-        const int32_t n = n_items - i0 < kSplitChunk ? n_items - i0 : kSplitChunk;
-        if (i0 > 0 && cudaMemsetAsync(ws, 0, 2 * sizeof(int32_t), s) != cudaSuccess)
+    const int grid = n_items < tb::num_sms() ? n_items : tb::num_sms();
+    if (n_items <= kSortItems) {
+        fourier_sort_kernel<<<1, kSortThreads, 0, s>>>(items, n_items, comp_dcoef, ws, lists, status,
+                                                       true);
+    } else {
+        if (cudaMemsetAsync(ws, 0, sizeof(PairWs), s) != cudaSuccess) return TB_ERR_LAUNCH;
+        if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
             return TB_ERR_LAUNCH;
-        const int64_t cu = (int64_t)n * kColUnits, ru = (int64_t)n * kRowUnits;
-        fourier_split_col_kernel<<<(int)(cu < gcol ? cu : gcol), kSplitThreads, 0, s>>>(
-            items, i0, n, comp_amp, comp_var, comp_dcoef, psf_spec, out, ws, fb_list, s1,
-            status);
-        fourier_split_row_kernel<<<(int)(ru < grow ? ru : grow), kSplitThreads, 0, s>>>(
-            items, i0, n, comp_dcoef, out, ws, s1);
+        fourier_sort_kernel<<<(n_items + kSortThreads - 1) / kSortThreads, kSortThreads, 0, s>>>(
+            items, n_items, comp_dcoef, ws, lists, status, false);
     }
-    // items outside the split path (Lanczos-3 reaching the box edge, TB_FFT_DOT)
-    const bool deriv = comp_dcoef != nullptr || dots != nullptr;
-    if (cudaFuncSetAttribute(deriv ? fourier_render_kernel<true> : fourier_render_kernel<false>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
-        return TB_ERR_LAUNCH;
-    const int gfb = tb::num_sms() < n_items ? tb::num_sms() : n_items;
-    if (deriv)
-        fourier_render_kernel<true><<<gfb, kThreads, kSmemBytes, s>>>(
-            items, n_items, comp_amp, comp_var, comp_dcoef, psf_spec, out, dots, &ws->fb_counter,
-            status, fb_list, &ws->fb_count);
-    else
-        fourier_render_kernel<false><<<gfb, kThreads, kSmemBytes, s>>>(
-            items, n_items, comp_amp, comp_var, nullptr, psf_spec, out, nullptr, &ws->fb_counter,
-            status, fb_list, &ws->fb_count);
+    fourier_pair_kernel<<<grid, kPairThreads, kPairSmem, s>>>(
+        items, n_items, comp_amp, comp_var, comp_dcoef, psf_spec, out, dots, ws, lists, status);
     return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
 }
 

@@ -16,6 +16,7 @@
 //    per-source partial (the reference's patch), adds the partial inside the
 //    rectangle to the tile accumulator, and writes every tile pixel once.
 //    No float atomics; the result does not depend on scheduling.
+#include "f32x2.cuh"
 #include "profile_eval.cuh"
 
 namespace {
@@ -284,35 +285,12 @@ scan_add_kernel(int32_t* __restrict__ offsets, int64_t n, const int32_t* __restr
 // 3. render
 // ---------------------------------------------------------------------------
 
-// Two floats in one 64-bit register, for the packed FP32 instructions (two
-// multiply-adds per issue slot).
-using f32x2 = unsigned long long;
-
-__device__ __forceinline__ f32x2 pack(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 unpack(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
+using tb::f32x2;
+using tb::pack;
+using tb::unpack;
+using tb::fma2;
+using tb::mul2;
+using tb::add2;
 
 // A staged component: exponent qxx dx^2 + qxy dx dy + qyy dy^2 (log2 units),
 // its tile-relative centre as the nearest pixel plus a fraction (the centre

@@ -588,18 +588,26 @@ LARGE_FFT_MAX = 8192     # the reference warns above a half-size of 4096 (galaxy
 _fourier_ws = {}
 
 
-def fourier_workspace(n_items, dev=None):
-    """Device scratch of tb_fourier_render_split for n_items items (one
-    buffer per device, grown when needed and reused: launches on one stream
-    use it one after another)."""
+def new_fourier_workspace(n_items, dev):
+    """Device scratch of tb_fourier_render_split for n_items items."""
     lib = _lib.load()
+    nb = ctypes.c_int64()
+    _lib.check(lib.tb_fourier_workspace(int(n_items), ctypes.byref(nb)), 'tb_fourier_workspace')
+    return torch.empty(max(nb.value, 256), dtype=torch.uint8, device=dev)
+
+
+def fourier_workspace(n_items, dev=None):
+    """The device's shared scratch of tb_fourier_render_split, for callers
+    that keep none of their own (one buffer per device, grown when needed and
+    reused: launches on one stream use it one after another)."""
     dev = dev or device()
+    lib = _lib.load()
     nb = ctypes.c_int64()
     _lib.check(lib.tb_fourier_workspace(int(n_items), ctypes.byref(nb)), 'tb_fourier_workspace')
     ws = _fourier_ws.get(dev.index)
     if ws is None or ws.numel() < nb.value:
-        ws = torch.empty(max(nb.value, 1 << 20), dtype=torch.uint8, device=dev)
-        _fourier_ws[dev.index] = ws
+        ws = _fourier_ws[dev.index] = torch.empty(max(nb.value, 1 << 20), dtype=torch.uint8,
+                                                  device=dev)
     return ws
 
 
@@ -608,19 +616,20 @@ fourier_method = {'default': 'persistent'}   # per device index, set by autotune
 
 
 def fourier_render(items_ptr, n_items, amp_ptr, var_ptr, spec_ptr, out_ptr, status_ptr,
-                   dcoef_ptr=None, dots_ptr=None, stream=None, method=None):
+                   dcoef_ptr=None, dots_ptr=None, stream=None, method=None, workspace=None):
     """Renders device Fourier items: 'persistent' -- tb_fourier_render(_deriv),
-    one CTA per galaxy holding its whole transpose in shared memory -- or
-    'split' -- tb_fourier_render_split, column and row kernels through an
-    L2-resident scratch.  The default is the device's autotuned choice
-    (autotune_fourier), else 'persistent'."""
+    one CTA per item -- or 'split' -- tb_fourier_render_split, the items sorted
+    by FFT size and rendered by groups of warps on packed transforms.  The
+    default is the device's autotuned choice (autotune_fourier), else
+    'persistent'.  `workspace`: the caller's new_fourier_workspace (the
+    device's shared one if None)."""
     lib = _lib.load()
     if method is None:
         dev = device()
         method = fourier_method.get(dev.index, fourier_method['default'])
     s = _lib.stream_ptr(stream)
     if method == 'split':
-        ws = fourier_workspace(n_items)
+        ws = fourier_workspace(n_items) if workspace is None else workspace
         rc = lib.tb_fourier_render_split(items_ptr, int(n_items), amp_ptr, var_ptr, dcoef_ptr,
                                          spec_ptr, out_ptr, dots_ptr, ws.data_ptr(), ws.numel(),
                                          status_ptr, s)
