@@ -403,6 +403,23 @@ int tb_galaxy_fft_jac_prep(const tb_galaxy_src* srcs, int32_t n, const tb_fft_im
                            int32_t comp_stride, int32_t mode, int64_t col_stride,
                            int32_t* flags, void* stream);
 
+/* The vector-Jacobian product of n galaxies (TB_FFT_DOT of their seven
+ * Jacobian items each, items as tb_galaxy_fft_jac_prep writes them with mode
+ * TB_FFT_DOT and col_stride 0): dots[dot_off] of each item = its derivative
+ * patch contracted with the upstream gradient `grad` (at the items' out_off),
+ * by one adjoint transform per galaxy instead of seven renders; galaxies whose
+ * window does not keep 3 px from the FFT box's edges as
+ * tb_fourier_render_deriv.  Equal to it up to FP32 rounding.  The gradient
+ * that replaces Galaxy.getParamDerivatives' finite differences
+ * (tractor/galaxy.py:137-223, tractor/sersic.py:402-445).  workspace: device,
+ * 256-byte aligned, at least tb_galaxy_fft_vjp_workspace(n) bytes, not shared
+ * by calls that may overlap. */
+int tb_galaxy_fft_vjp_workspace(int32_t n, int64_t* bytes);
+int tb_galaxy_fft_vjp(const tb_fft_item* items, int32_t n, const double* comp_amp,
+                      const double* comp_var, const double* comp_dcoef, const float* psf_spec,
+                      const float* grad, double* dots, void* workspace,
+                      int64_t workspace_bytes, tb_status* status, void* stream);
+
 /* Forward real FFT of n zero-padded sz x sz float32 PSF images (prepared by
  * the caller, image i at pad + i*sz*sz) into complex64 spectra
  * sz x (sz/2+1) (interleaved, column-major as tb_fourier_render reads them),

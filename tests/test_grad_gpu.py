@@ -101,6 +101,45 @@ def test_vjp_matches_jacobian_contraction(tb):
     assert np.all(np.abs(dots.cpu().numpy() - want) <= 1e-5 * scale + 1e-12)
 
 
+@pytest.mark.parametrize('psf, sides', [
+    (15, [(26, 26), (24, 7), (29, 29)]), (31, [(58, 58), (57, 30), (61, 61)]),
+    (63, [(122, 122), (63, 119), (125, 90)]),
+    (63, [(250, 250), (131, 132), (129, 133), (134, 128), (253, 253), (253, 131)])])
+def test_vjp_at_its_edges(tb, psf, sides):
+    """tb_galaxy_fft_vjp against the Jacobian's contraction at the FFT sizes
+    32 to 256: the largest windows of the adjoint transform and of the general
+    path beyond them (windows that reach the box's edge), rows around what one
+    pass holds (132 at size 256), remainders, all profiles, a galaxy without
+    a patch (no counts).  Tolerance as test_vjp_matches_jacobian_contraction."""
+    import torch
+    from tractor_b200 import batch, grad, _lib
+    rng = np.random.default_rng(psf)
+    n = 3 * len(sides)
+    w = np.repeat([a for a, _ in sides], 3)
+    h = np.repeat([b for _, b in sides], 3)
+    srcs = batch.sersic_sources(n, rng, mask=64)
+    srcs['profile'][::3], srcs['profile'][1::3] = _lib.PROFILE_EXP, _lib.PROFILE_DEV
+    srcs['px'], srcs['py'] = w / 2 + rng.uniform(-.5, .5, n), h / 2 + rng.uniform(-.5, .5, n)
+    srcs['mw'], srcs['mh'] = w, h
+    srcs['out_off'] = np.concatenate([[0], np.cumsum(w * h)[:-1]])
+    srcs['counts'][-1] = 0.
+    npix = int((w * h).sum())
+    r = batch.FourierGalaxyRenderer(batch.moffat_psf(psf))
+    jac = grad.FourierJacobian(r)
+    d = torch.from_numpy(srcs.view(np.uint8).copy()).cuda()
+    J, flags, st = jac.jacobian(d, n, npix)
+    assert not st.any() and flags.cpu().tolist() == [0] * (n - 1) + [1]
+    v = torch.randn(npix, generator=torch.Generator().manual_seed(3)).cuda()
+    dots, _, st = jac.vjp(d, n, v)
+    assert not st.any()
+    Jn, vn = J.cpu().numpy().astype(np.float64), v.cpu().numpy().astype(np.float64)
+    for i in range(n - 1):
+        o = slice(int(srcs['out_off'][i]), int(srcs['out_off'][i] + w[i] * h[i]))
+        want, scale = Jn[:, o] @ vn[o], np.abs(Jn[:, o]) @ np.abs(vn[o])
+        assert np.all(np.abs(dots[i].cpu().numpy() - want) <= 1e-5 * scale + 1e-12), i
+    assert not dots[-1].any()
+
+
 def test_autograd_backward_is_the_analytic_vjp(tb, oracle):
     import torch
     from tractor_b200 import batch, grad

@@ -278,23 +278,29 @@ __device__ __forceinline__ void pair_rows(const tb_fft_item& it, const PairGroup
     }
 }
 
+// Frequency response of seven taps at index fr of an N-point transform: sum_k
+// tap_k exp(2 pi i fr (k - 3) / N).
+template <int N>
+__device__ __forceinline__ float2 tap_response(const float* tap, int fr) {
+    float c = tap[3], s = 0.f;
+#pragma unroll
+    for (int k = 1; k <= 3; k++) {
+        float sk, ck;
+        sincospif(2.f * (float)((fr * k) & (N - 1)) / (float)N, &sk, &ck);
+        c = fmaf(tap[3 + k] + tap[3 - k], ck, c);
+        s = fmaf(tap[3 + k] - tap[3 - k], sk, s);
+    }
+    return make_float2(c, s);
+}
+
 // Tap responses of an item, twice each, for the packed products.
 template <int N>
 __device__ __forceinline__ void pair_responses(const PairGroup& sh) {
     for (int f = sh.tid; f < PairPlan<N>::NH + N; f += PairPlan<N>::kThreads) {
         const bool isx = f < PairPlan<N>::NH;
         const int fr = isx ? f : f - PairPlan<N>::NH;
-        const float* tp = isx ? sh.taps : sh.taps + 8;
-        float c = tp[3], s = 0.f;
-        // sum_k tap_k exp(2 pi i fr (k - 3) / N)
-#pragma unroll
-        for (int k = 1; k <= 3; k++) {
-            float sk, ck;
-            sincospif(2.f * (float)((fr * k) & (N - 1)) / (float)N, &sk, &ck);
-            c = fmaf(tp[3 + k] + tp[3 - k], ck, c);
-            s = fmaf(tp[3 + k] - tp[3 - k], sk, s);
-        }
-        (isx ? sh.hx : sh.hy)[fr] = make_float4(c, c, s, s);
+        const float2 r = tap_response<N>(isx ? sh.taps : sh.taps + 8, fr);
+        (isx ? sh.hx : sh.hy)[fr] = make_float4(r.x, r.x, r.y, r.y);
     }
 }
 

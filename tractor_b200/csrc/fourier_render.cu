@@ -869,6 +869,7 @@ __device__ __forceinline__ bool item_ok(const tb_fft_item& it, const double* dco
 }
 
 #include "fourier_pair.cuh"
+#include "fourier_vjp.cuh"
 
 }  // namespace
 
@@ -980,6 +981,43 @@ extern "C" int tb_fourier_render_split(const tb_fft_item* items, int32_t n_items
     }
     fourier_pair_kernel<<<grid, kPairThreads, kPairSmem, s>>>(
         items, n_items, comp_amp, comp_var, comp_dcoef, psf_spec, out, dots, ws, lists, status);
+    return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
+}
+
+extern "C" int tb_galaxy_fft_vjp_workspace(int32_t n, int64_t* bytes) {
+    if (n < 0 || !bytes) return TB_ERR_ARG;
+    *bytes = (int64_t)sizeof(PairWs) + ((int64_t)n * 4 * 11 + 255) / 256 * 256;   // lists 4 n + 7 n
+    return TB_OK;
+}
+
+extern "C" int tb_galaxy_fft_vjp(const tb_fft_item* items, int32_t n, const double* comp_amp,
+                                 const double* comp_var, const double* comp_dcoef,
+                                 const float* psf_spec, const float* grad, double* dots,
+                                 void* workspace, int64_t workspace_bytes, tb_status* status,
+                                 void* stream) {
+    if (n < 0) return TB_ERR_ARG;
+    if (n == 0) return TB_OK;
+    if (!items || !comp_amp || !comp_var || !comp_dcoef || !psf_spec || !grad || !dots || !workspace)
+        return TB_ERR_ARG;
+    if ((reinterpret_cast<uintptr_t>(workspace) & 255) != 0) return TB_ERR_ARG;
+    int64_t need = 0;
+    tb_galaxy_fft_vjp_workspace(n, &need);
+    if (workspace_bytes < need) return TB_ERR_SIZE;
+    cudaStream_t s = (cudaStream_t)stream;
+    PairWs* ws = static_cast<PairWs*>(workspace);
+    int32_t* lists = reinterpret_cast<int32_t*>(static_cast<char*>(workspace) + sizeof(PairWs));
+    if (cudaFuncSetAttribute(fourier_vjp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kVjpSmem) != cudaSuccess)
+        return TB_ERR_LAUNCH;
+    if (cudaMemsetAsync(ws, 0, sizeof(PairWs), s) != cudaSuccess) return TB_ERR_LAUNCH;
+    if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
+        return TB_ERR_LAUNCH;
+    const int grid = n < tb::num_sms() ? n : tb::num_sms();
+    fourier_vjp_sort_kernel<<<(n + 127) / 128, 128, 0, s>>>(items, n, comp_dcoef, ws, lists, dots,
+                                                            status);
+    fourier_vjp_kernel<<<grid, kPairThreads, kVjpSmem, s>>>(
+        items, n, comp_amp, comp_var, comp_dcoef, psf_spec, const_cast<float*>(grad), dots, ws,
+        lists, status);
     return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
 }
 

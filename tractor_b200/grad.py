@@ -8,10 +8,10 @@ Lanczos-3 taps, counts (the unit-flux render), the three shape parameters and
 the Sersic index through the derivative of the Gaussian-mixture spectrum,
 d/dtheta sum_k a_k exp(-2 pi^2 f^T C_k f) = sum_k (da_k - 2 pi^2 a_k
 f^T dC_k f) exp(...) -- and tb_fourier_render_deriv renders them through the
-same FFT / Lanczos / crop pipeline as the model.  In TB_FFT_DOT mode the
-kernel contracts each derivative item with an upstream gradient instead of
-writing it (the vector-Jacobian product), so backward never materialises
-the Jacobian.
+same FFT / Lanczos / crop pipeline as the model.  The vector-Jacobian product
+(tb_galaxy_fft_vjp) transforms the upstream gradient instead and contracts all
+seven derivative spectra with it in frequency space, so backward neither
+renders nor stores the Jacobian.
 
 These replace the finite-difference derivatives of Galaxy.getParamDerivatives
 and SersicGalaxy.getParamDerivatives (tractor/galaxy.py:137-223,
@@ -37,6 +37,7 @@ class FourierJacobian(object):
     def __init__(self, renderer):
         self.r = renderer
         self._scratch = {}
+        self._vjp_scratch = {}
 
     def _work(self, n):
         if n not in self._scratch:
@@ -51,37 +52,52 @@ class FourierJacobian(object):
             self._scratch[n] = (items, camp, cvar, dcoef, flags, misc)
         return self._scratch[n]
 
-    def _run(self, srcs, n, out, mode, col_stride, dots=None, stream=None):
+    def _vjp_workspace(self, n):
+        if n not in self._vjp_scratch:
+            nb = ctypes.c_int64()
+            _lib.check(_lib.load().tb_galaxy_fft_vjp_workspace(n, ctypes.byref(nb)),
+                       'tb_galaxy_fft_vjp_workspace')
+            self._vjp_scratch[n] = torch.empty(nb.value, dtype=torch.uint8,
+                                               device=render.device())
+        return self._vjp_scratch[n]
+
+    def _prep(self, srcs, n, mode, col_stride, s):
         lib = _lib.load()
         items, camp, cvar, dcoef, flags, misc = self._work(n)
-        s = _lib.stream_ptr(stream)
         rc = lib.tb_galaxy_fft_jac_prep(srcs.data_ptr(), n, ctypes.addressof(self.r.image),
                                         ctypes.addressof(self.r.tables.struct), items.data_ptr(),
                                         camp.data_ptr(), cvar.data_ptr(), dcoef.data_ptr(),
                                         batch.COMP_STRIDE, mode, col_stride, flags.data_ptr(), s)
         _lib.check(rc, 'tb_galaxy_fft_jac_prep')
-        render.fourier_render(items.data_ptr(), 7 * n, camp.data_ptr(), cvar.data_ptr(),
-                              self.r.spec.data_ptr(), out.data_ptr(), misc.data_ptr() + 16,
-                              dcoef_ptr=dcoef.data_ptr(),
-                              dots_ptr=None if dots is None else dots.data_ptr(), stream=stream)
-        return flags, misc[4:8]
+        return items, camp, cvar, dcoef, flags, misc
 
     def jacobian(self, srcs, n, npix, stream=None):
         """float32 (7, npix) device tensor: row j holds d(model)/d(param j)
         of every galaxy, each at its record's out_off (the layout of the
         value patches).  Also returns the prep flags."""
         out = torch.empty(7 * npix, dtype=torch.float32, device=render.device())
-        flags, st = self._run(srcs, n, out, _lib.MOG_STORE, npix, stream=stream)
-        return out.view(7, npix), flags, st
+        items, camp, cvar, dcoef, flags, misc = self._prep(srcs, n, _lib.MOG_STORE, npix,
+                                                           _lib.stream_ptr(stream))
+        render.fourier_render(items.data_ptr(), 7 * n, camp.data_ptr(), cvar.data_ptr(),
+                              self.r.spec.data_ptr(), out.data_ptr(), misc.data_ptr() + 16,
+                              dcoef_ptr=dcoef.data_ptr(), stream=stream)
+        return out.view(7, npix), flags, misc[4:8]
 
     def vjp(self, srcs, n, grad, stream=None):
         """float64 (n, 7): sum over each galaxy's patch of grad * d(model)/
-        d(param), grad laid out like the value patches (one kernel: the
-        derivative renders are contracted as they are produced)."""
+        d(param), grad laid out like the value patches (tb_galaxy_fft_vjp:
+        one adjoint transform per galaxy)."""
+        s = _lib.stream_ptr(stream)
         dots = torch.zeros(7 * n, dtype=torch.float64, device=render.device())
-        flags, st = self._run(srcs, n, grad.contiguous(), _lib.FFT_DOT, 0, dots=dots,
-                              stream=stream)
-        return dots.view(n, 7), flags, st
+        grad = grad.contiguous()
+        items, camp, cvar, dcoef, flags, misc = self._prep(srcs, n, _lib.FFT_DOT, 0, s)
+        ws = self._vjp_workspace(n)
+        rc = _lib.load().tb_galaxy_fft_vjp(items.data_ptr(), n, camp.data_ptr(), cvar.data_ptr(),
+                                           dcoef.data_ptr(), self.r.spec.data_ptr(),
+                                           grad.data_ptr(), dots.data_ptr(), ws.data_ptr(),
+                                           ws.numel(), misc.data_ptr() + 16, s)
+        _lib.check(rc, 'tb_galaxy_fft_vjp')
+        return dots.view(n, 7), flags, misc[4:8]
 
 
 def records_with_params(template, theta):
