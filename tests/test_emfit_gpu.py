@@ -120,3 +120,44 @@ def test_em_sky_all_component_counts_match_oracle(tb, oracle):
         r, s1 = emfit.em_fit_2d_reg2(imgs[i], -11, -10, a1, m1, v1, 0.1, 80, 1e-30)
         assert r == 0 and s1 == sky[i]
         assert np.array_equal(a[i], a1) and np.array_equal(m[i], m1) and np.array_equal(v[i], v1)
+
+
+@pytest.mark.parametrize('shape', [(1, 9), (70, 1), (9, 7), (25, 33), (2, 63), (31, 64), (7, 65),
+                                   (5, 130)])
+def test_em_run_cuts_match_oracle(tb, oracle, shape):
+    """Stamps narrower and wider than a block's 64 threads, whose columns are
+    cut into different runs of rows."""
+    from tractor_b200 import emfit
+    h, w = shape
+    rng = np.random.default_rng(h * 1000 + w)
+    img = _stamp(rng, h, w, 2)
+    amp, mean, var = emfit.em_init_params(2, None, None, None)
+    a1, m1, v1 = amp.copy(), mean.copy(), var.copy()
+    a2, m2, v2 = amp.copy(), mean.copy(), var.copy()
+    args = (-(w // 2), -(h // 2))
+    r1 = emfit.em_fit_2d_reg(img, *args, a1, m1, v1, 0.3, 40)
+    r2 = oracle.em_fit_2d_reg(img, *args, a2, m2, v2, 0.3, 40)
+    assert r1 == r2
+    np.testing.assert_allclose(a1, a2, rtol=1e-9, atol=1e-13)
+    np.testing.assert_allclose(m1, m2, rtol=0, atol=1e-9)
+    np.testing.assert_allclose(v1, v2, rtol=1e-9, atol=1e-12)
+
+
+def test_em_indefinite_covariance_matches_oracle(tb, oracle):
+    """A first covariance of positive determinant whose quadratic form is not
+    positive: exponents above 0, outside the table-driven exponential's range."""
+    from tractor_b200 import emfit
+    rng = np.random.default_rng(3)
+    img = _stamp(rng, 12, 13, 2)
+    amp, mean, var = emfit.em_init_params(2, None, None, None)
+    for V in ([[-9., 0.], [0., -7.]], [[1., 4.], [-3., 1.]]):
+        var = var.copy()
+        var[1] = V
+        a1, m1, v1 = amp.copy(), mean.copy(), var.copy()
+        a2, m2, v2 = amp.copy(), mean.copy(), var.copy()
+        r1 = emfit.em_fit_2d_reg(img, -6, -6, a1, m1, v1, 0.3, 1)
+        r2 = oracle.em_fit_2d_reg(img, -6, -6, a2, m2, v2, 0.3, 1)
+        assert r1 == r2
+        np.testing.assert_allclose(a1, a2, rtol=1e-9, atol=1e-13)
+        np.testing.assert_allclose(m1, m2, rtol=0, atol=1e-9)
+        np.testing.assert_allclose(v1, v2, rtol=1e-9, atol=1e-12)

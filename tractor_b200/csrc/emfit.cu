@@ -11,14 +11,30 @@
 //     z_k = scale_k exp(-dsq_k / 2), 0 for dsq >= 100 (z itself where the
 //     sum is 0, as the reference leaves it);
 //   * M step from the weighted moments w = img z_k / sum z (sum w, sum w x,
-//     sum w y, sum w x^2, sum w x y, sum w y^2), summed per thread over a
-//     fixed pixel stride and then over the block in a fixed order (every
-//     launch gives the same result): mean = (sum w x, sum w y) / sum w,
-//     covariance = (alpha I + sum w (x - mean)(x - mean)^T) / (sum w + alpha)
-//     with sum w (x - m)^2 = sum w x^2 - m sum w x, amplitude = sum w.
+//     sum w y, sum w x^2, sum w x y, sum w y^2), summed per thread, then over
+//     the block in a fixed order (every launch gives the same result):
+//     mean = (sum w x, sum w y) / sum w, covariance = (alpha I + sum w
+//     (x - mean)(x - mean)^T) / (sum w + alpha) with sum w (x - m)^2 =
+//     sum w x^2 - m sum w x, amplitude = sum w.
 // The reference sums the second moments about the new mean in a second pass
 // over the pixels; the expansion above is the same sum in one pass (the
 // difference is FP64 rounding).
+//
+// Bound: FP64 issue and latency (60 % of the issue slots, 37 % of the FP64 pipe;
+// the rest waits on the chain of a pixel's exponentials, their sum and its
+// reciprocal).  A thread keeps one column of pixels, so a component's exponent
+// is a quadratic in y alone, its moments three sums (w, w y, w y^2) and the x
+// moments follow once per column; the exponential is exp2_tab; each warp takes
+// the M step and the next iteration's parameters itself, so an iteration has
+// one block barrier.  100 iterations, 1024 stamps of 25 x 25 (against a pixel
+// stride per thread with exp(), divisions and a butterfly per moment): 1
+// component 487 -> 394 us, 3 components 1045 -> 743, 8 components 4657 -> 2277;
+// 256 stamps of 63 x 63, 3 components 3279 -> 2405.  The order of the sums is
+// another, so the last bits are: after 1000 iterations of 3 components the
+// amplitudes are off by 8.8e-16 against extended precision (rms; was 5.7e-16),
+// of 2 components by 4.1e-16 (3.4e-16).
+#include <type_traits>
+
 #include "tb_common.cuh"
 
 namespace {
@@ -26,17 +42,66 @@ namespace {
 constexpr int kEmThreads = 64;
 constexpr int kWarps = kEmThreads / 32;
 
+// 1 / d, as accurate as the division to its last bit or so: Newton's
+// iteration from the hardware's estimate; the division itself where the
+// estimate would be flushed.
+__device__ __forceinline__ double em_reciprocal(double d) {
+    if (!(fabs(d) > 1e-290 && fabs(d) < 1e290)) return 1.0 / d;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    r = fma(r, fma(-d, r, 1.0), r);
+    return fma(r, fma(-d, r, 1.0), r);
+}
+
+// The sums over the warp of each lane's a[0 .. N): every exchange leaves a lane
+// half of the values it had (about N shuffles instead of 5 N); at the end it
+// holds `count` sums, of the elements `first` on.
+template <int M, int N, int O>
+__device__ __forceinline__ void halve(double (&a)[M], int lane, int& first, int& count) {
+    if constexpr (O > 0) {
+        constexpr int H = (N + 1) / 2;
+        if constexpr (N > 1) {
+            const bool hi = lane & O;
+#pragma unroll
+            for (int i = 0; i < H; i++) {
+                const double up = i + H < N ? a[i + H] : 0.0;
+                const double send = hi ? a[i] : up, keep = hi ? up : a[i];
+                a[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+            }
+            first += hi ? H : 0;
+            count = hi ? count - H : min(count, H);
+        } else {
+            a[0] += __shfl_xor_sync(0xffffffffu, a[0], O);
+        }
+        halve<M, H, O / 2>(a, lane, first, count);
+    }
+}
+
+// out[e] = the sum over the warp of a[e], e < M <= 64.
+template <int M>
+__device__ __forceinline__ void warp_sums(double (&a)[M], int lane, double* out) {
+    int first = 0, count = M;
+    halve<M, M, 16>(a, lane, first, count);
+#pragma unroll
+    for (int i = 0; i < (M > 32 ? 2 : 1); i++)
+        if (i < count) out[first + i] = a[i];   // (equal values from lanes that share one)
+}
+
+// (resident CTAs: as many as registers allow without spills up to 3
+// components, 7 with a few for 4 and 5, where fewer left 1024 stamps a second
+// wave: 5 components 1748 us before, 2000 with 6, 1306 with 7)
 template <int K>
-__global__ void __launch_bounds__(kEmThreads, 8)
+__global__ void __launch_bounds__(kEmThreads, K <= 3 ? 8 : K <= 5 ? 7 : 4)
 em_fit_kernel(const double* __restrict__ img, int n, int ny, int nx,
               const int32_t* __restrict__ xy0, double* __restrict__ amp,
               double* __restrict__ mean, double* __restrict__ var, double alpha, int steps,
               int32_t* __restrict__ status) {
     constexpr int kM = 6 * K;   // moments per image
-    __shared__ double w_s[K], mu_s[K][2], v_s[K][4];
-    __shared__ double iv_s[K][4], sc_s[K];
-    __shared__ double red[kWarps][kM];
-    __shared__ int bad;
+    // per warp: the current mixture, and what the E step reads of it (all
+    // exponents in log2 units)
+    __shared__ double par[kWarps][K][8];   // mean x, y, c00, c01, c11, scale
+    __shared__ double red[2][kWarps][kM];
+    __shared__ double exp_tab[tb::kExpTab];
     const int s = blockIdx.x;
     if (s >= n) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -46,106 +111,160 @@ em_fit_kernel(const double* __restrict__ img, int n, int ny, int nx,
     double* V = var + (int64_t)s * K * 4;
     const int x0 = xy0 ? xy0[2 * s] : -(nx / 2);
     const int y0 = xy0 ? xy0[2 * s + 1] : -(ny / 2);
-    const int npix = nx * ny;
-    const int ix0 = tid % nx, iy0 = tid / nx;                       // this thread's first pixel
-    const int step_x = kEmThreads % nx, step_y = kEmThreads / nx;   // and its stride
-    const double tpd = 4.0 * TB_PI * TB_PI;   // (2 pi)^D, D = 2
-    if (tid < K) {
-        w_s[tid] = A[tid];
-        mu_s[tid][0] = Mu[2 * tid];
-        mu_s[tid][1] = Mu[2 * tid + 1];
-#pragma unroll
-        for (int d = 0; d < 4; d++) v_s[tid][d] = V[4 * tid + d];
-    }
-    if (tid == 0) bad = 0;
-    __syncthreads();
-    for (int step = 0; step < steps; step++) {
-        if (tid < K) {
-            const double* Vk = v_s[tid];
-            const double det = Vk[0] * Vk[3] - Vk[1] * Vk[2];
-            if (det <= 0.0) bad = 1;
-            iv_s[tid][0] = Vk[3] / det;
-            iv_s[tid][1] = -Vk[1] / det;
-            iv_s[tid][2] = -Vk[2] / det;
-            iv_s[tid][3] = Vk[0] / det;
-            sc_s[tid] = w_s[tid] / sqrt(tpd * det);
+    // The columns are cut into `groups` runs of `rows` pixels, taken by the
+    // threads in turn: the cut that keeps the threads busiest, a run's start
+    // counted as two pixels.
+    int groups = 1, rows = ny;
+    {
+        int best = 0x7fffffff;
+        for (int g = 1; g <= max(8, kEmThreads / nx) && g <= ny; g++) {
+            const int r = (ny + g - 1) / g;
+            const int cost = (nx * g + kEmThreads - 1) / kEmThreads * (r + 2);
+            if (cost < best) { best = cost; groups = g; rows = r; }
         }
-        __syncthreads();
-        if (bad) break;   // the same value in every thread
+    }
+    const int step_x = kEmThreads % nx, step_g = kEmThreads / nx;
+    const double tpd = 4.0 * TB_PI * TB_PI;   // (2 pi)^D, D = 2
+    tb::exp2_tab_init(exp_tab);
+    // component `lane` of this warp's copy: the exponents' coefficients and the
+    // scale from its mixture; whether its determinant is positive.  `tame`: its
+    // exponent is <= 0 (but for rounding) and finite at every pixel, as the
+    // table-driven exponential needs it.
+    bool tame = true;
+    auto prepare = [&](double w, double mx, double my, double v00, double v01, double v10,
+                       double v11) -> bool {
+        const double det = v00 * v11 - v01 * v10;
+        double* p = par[warp][lane];
+        p[0] = mx;
+        p[1] = my;
+        const double q = -0.5 * TB_LOG2E / det;
+        p[2] = v11 * q;
+        p[3] = -(v01 + v10) * q;
+        p[4] = v00 * q;
+        p[5] = w / sqrt(tpd * det);
+        const double off = v01 + v10;
+        tame = p[2] < 0.0 && p[4] < 0.0 && 4.0 * v00 * v11 > off * off && p[2] > -1e100 &&
+               p[4] > -1e100 && fabs(mx) < 1e50 && fabs(my) < 1e50;
+        return !(det <= 0.0);
+    };
+    bool ok = true;
+    double fw = 0.0, fmx = 0.0, fmy = 0.0, f00 = 0.0, f01 = 0.0, f10 = 0.0, f11 = 0.0;
+    if (lane < K) {
+        fw = A[lane];
+        fmx = Mu[2 * lane];
+        fmy = Mu[2 * lane + 1];
+        f00 = V[4 * lane];
+        f01 = V[4 * lane + 1];
+        f10 = V[4 * lane + 2];
+        f11 = V[4 * lane + 3];
+        ok = prepare(fw, fmx, fmy, f00, f01, f10, f11) || steps <= 0;
+    }
+    __syncthreads();   // the table
+    int bad = 0;
+    for (int step = 0; step < steps; step++) {
+        if (!__all_sync(0xffffffffu, ok)) {   // the same in every warp
+            bad = 1;
+            break;
+        }
         double acc[kM];
 #pragma unroll
         for (int v = 0; v < kM; v++) acc[v] = 0.0;
-        // pixel i = tid + kEmThreads j at (ix, iy), advanced without a division
-        int ix = ix0, iy = iy0;
-        for (int i = tid; i < npix; i += kEmThreads) {
-            const double x = (double)(x0 + ix), y = (double)(y0 + iy);
-            ix += step_x;
-            iy += step_y;
-            if (ix >= nx) {
-                ix -= nx;
-                iy++;
+        auto e_step = [&](auto table) {
+            int ix = tid % nx, run = tid / nx;
+            for (; run < groups; ix += step_x, run += step_g) {
+                if (ix >= nx) {
+                    ix -= nx;
+                    if (++run >= groups) break;
+                }
+                const int ra = run * rows, rb = min(ny, ra + rows);
+                const double x = (double)(x0 + ix);
+                double ca[K], cb[K], S0[K], Sy[K];
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    const double dx = x - par[warp][k][0];
+                    ca[k] = par[warp][k][2] * dx * dx;
+                    cb[k] = par[warp][k][3] * dx;
+                    S0[k] = Sy[k] = 0.0;
+                }
+                const double* px = im + ra * nx + ix;
+                double y = (double)(y0 + ra);
+                double dnext = ra < rb ? *px : 0.0;
+                for (int iy = ra; iy < rb; iy++, y += 1.0) {
+                    const double yy = y * y, d = dnext;
+                    px += nx;
+                    if (iy + 1 < rb) dnext = *px;
+                    double z[K];
+                    double zsum = 0.0;
+#pragma unroll
+                    for (int k = 0; k < K; k++) {
+                        const double dy = y - par[warp][k][1];
+                        const double e = fma(dy, fma(par[warp][k][4], dy, cb[k]), ca[k]);
+                        const double E = decltype(table)::value ? tb::exp2_tab(e, exp_tab) : exp2(e);
+                        z[k] = e <= -50.0 * TB_LOG2E ? 0.0 : par[warp][k][5] * E;   // dsq >= 100: 0
+                        zsum += z[k];
+                    }
+                    double dr;
+                    if (((unsigned)__double2hiint(zsum) << 1) - (323u << 21) < (1400u << 21)) {   // 1e-211 .. 1e210
+                        dr = d * em_reciprocal(zsum);
+                    } else {
+                        // a pixel whose z sum to 0 keeps them unnormalised (all 0
+                        // unless some amplitude is negative), as the reference does
+                        const double rz = zsum != 0.0 ? 1.0 / zsum : 1.0;
+#pragma unroll
+                        for (int k = 0; k < K; k++) z[k] *= rz;
+                        dr = d;
+                    }
+#pragma unroll
+                    for (int k = 0; k < K; k++) {
+                        const double wi = dr * z[k];
+                        S0[k] += wi;
+                        Sy[k] = fma(wi, y, Sy[k]);
+                        acc[6 * k + 5] = fma(wi, yy, acc[6 * k + 5]);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    const double xs = x * S0[k];
+                    acc[6 * k + 0] += S0[k];
+                    acc[6 * k + 1] += xs;
+                    acc[6 * k + 2] += Sy[k];
+                    acc[6 * k + 3] = fma(xs, x, acc[6 * k + 3]);
+                    acc[6 * k + 4] = fma(x, Sy[k], acc[6 * k + 4]);
+                }
             }
-            double z[K];
-            double zsum = 0.0;
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                const double dx = x - mu_s[k][0], dy = y - mu_s[k][1];
-                const double dsq = iv_s[k][0] * dx * dx + iv_s[k][1] * dx * dy +
-                                   iv_s[k][2] * dx * dy + iv_s[k][3] * dy * dy;
-                z[k] = dsq >= 100.0 ? 0.0 : sc_s[k] * exp(-0.5 * dsq);
-                zsum += z[k];
-            }
-            // a pixel whose z sum to 0 keeps them unnormalised (all 0 unless
-            // some amplitude is negative), as the reference does; one
-            // reciprocal per pixel instead of a division per component
-            const double rz = zsum != 0.0 ? 1.0 / zsum : 1.0;
-            const double d = im[i];
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                const double wi = d * (z[k] * rz);
-                acc[6 * k + 0] += wi;
-                acc[6 * k + 1] += wi * x;
-                acc[6 * k + 2] += wi * y;
-                acc[6 * k + 3] += wi * x * x;
-                acc[6 * k + 4] += wi * x * y;
-                acc[6 * k + 5] += wi * y * y;
-            }
-        }
-#pragma unroll
-        for (int v = 0; v < kM; v++) {
-            double a = acc[v];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-            if (lane == 0) red[warp][v] = a;
-        }
-        __syncthreads();
-        if (tid < K) {
+        };
+        if (__all_sync(0xffffffffu, tame)) e_step(std::true_type{});
+        else e_step(std::false_type{});
+        double* r = red[step & 1][warp];
+        warp_sums<kM>(acc, lane, r);
+        __syncthreads();   // (the other half of `red` is read before the next one)
+        if (lane < K) {
             double m[6];
 #pragma unroll
             for (int q = 0; q < 6; q++) {
                 double t = 0.0;
-                for (int w2 = 0; w2 < kWarps; w2++) t += red[w2][6 * tid + q];
+                for (int w2 = 0; w2 < kWarps; w2++) t += red[step & 1][w2][6 * lane + q];
                 m[q] = t;
             }
-            const double ws = m[0];
-            const double mx = m[1] / ws, my = m[2] / ws;
-            mu_s[tid][0] = mx;
-            mu_s[tid][1] = my;
-            const double den = ws + alpha;
-            v_s[tid][0] = (alpha + (m[3] - mx * m[1])) / den;
-            v_s[tid][1] = (m[4] - mx * m[2]) / den;
-            v_s[tid][2] = v_s[tid][1];
-            v_s[tid][3] = (alpha + (m[5] - my * m[2])) / den;
-            w_s[tid] = ws;
+            fw = m[0];
+            const double rw = 1.0 / fw, rden = 1.0 / (fw + alpha);
+            fmx = m[1] * rw;
+            fmy = m[2] * rw;
+            f00 = (alpha + (m[3] - fmx * m[1])) * rden;
+            f01 = f10 = (m[4] - fmx * m[2]) * rden;
+            f11 = (alpha + (m[5] - fmy * m[2])) * rden;
+            ok = prepare(fw, fmx, fmy, f00, f01, f10, f11);
         }
-        __syncthreads();
+        __syncwarp();
     }
-    if (tid < K) {
-        A[tid] = w_s[tid];
-        Mu[2 * tid] = mu_s[tid][0];
-        Mu[2 * tid + 1] = mu_s[tid][1];
-#pragma unroll
-        for (int d = 0; d < 4; d++) V[4 * tid + d] = v_s[tid][d];
+    if (warp == 0 && lane < K) {
+        A[lane] = fw;
+        Mu[2 * lane] = fmx;
+        Mu[2 * lane + 1] = fmy;
+        V[4 * lane] = f00;
+        V[4 * lane + 1] = f01;
+        V[4 * lane + 2] = f10;
+        V[4 * lane + 3] = f11;
     }
     if (tid == 0 && status) status[s] = bad;
 }

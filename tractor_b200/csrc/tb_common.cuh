@@ -12,11 +12,10 @@ namespace tb {
 
 // 2^e in FP64 for |e| < 1000 by the table-driven scheme of Tang (ACM TOMS
 // 15(2), 1989): n = rint(16 e), r = e - n / 16 exactly (|r| <= 1/32),
-// 2^e = 2^(n div 16) T[n mod 16] 2^r with T[j] = 2^(j / 16) and 2^r by its
-// Taylor series to degree 6 (remainder below (ln 2 / 32)^7 / 7! = 5e-16);
-// relative error below 1e-15.  Ten FP64 operations.  The 16 table entries
-// lie in 16 different pairs of shared-memory banks, so the lookups of a warp
-// never conflict.
+// 2^e = 2^(n div 16) T[n mod 16] 2^r with T[j] = 2^(j / 16) and a polynomial
+// of degree 6 for 2^r; relative error below 4e-16.  Ten FP64 operations.  The
+// 16 table entries lie in 16 different pairs of shared-memory banks, so the
+// lookups of a warp never conflict.
 constexpr int kExpTab = 16;
 
 __device__ __forceinline__ void exp2_tab_init(double* tab) {
@@ -26,18 +25,19 @@ __device__ __forceinline__ void exp2_tab_init(double* tab) {
 __device__ __forceinline__ double exp2_tab(double e, const double* tab) {
     const double magic = 6755399441055744.0;   // 1.5 x 2^52: rounds to an integer in the low word
     const double t = fma(e, (double)kExpTab, magic);
-    const int n = __double2loint(t);
+    const unsigned n = __double2loint(t);
     const double r = fma(t - magic, -1.0 / kExpTab, e);
-    // (ln 2)^k / k!
-    double p = 1.5403530393381610e-04;
-    p = fma(p, r, 1.3333558146428443e-03);
-    p = fma(p, r, 9.6181291076284772e-03);
-    p = fma(p, r, 5.5504108664821580e-02);
-    p = fma(p, r, 2.4022650695910072e-01);
-    p = fma(p, r, 6.9314718055994531e-01);
+    // (2^r - 1) / r interpolated at the six Chebyshev nodes of |r| <= 1/32
+    // (2^r to 1.5e-17; the Taylor sum of that degree is off by 4.5e-16 there)
+    double p = 1.5403723980749256e-04;
+    p = fma(p, r, 1.3333781576784268e-03);
+    p = fma(p, r, 9.6181291069195370e-03);
+    p = fma(p, r, 5.5504108656639302e-02);
+    p = fma(p, r, 2.4022650695910075e-01);
+    p = fma(p, r, 6.9314718055994573e-01);
     const double T = tab[n & (kExpTab - 1)];
     const double y = fma(T * r, p, T);
-    return __hiloint2double(__double2hiint(y) + ((n >> 4) << 20), __double2loint(y));
+    return __hiloint2double((int)(__double2hiint(y) + ((n & ~15u) << 16)), __double2loint(y));
 }
 
 // 2^x on the SFU (MUFU.EX2), flushing denormal results to zero.
