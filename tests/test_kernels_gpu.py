@@ -475,6 +475,52 @@ def test_normal_equations_and_solve(tb):
         o += P * P
 
 
+@pytest.mark.parametrize('sizes', [[1, 2, 7, 8, 9], [63, 64, 65, 3], [128, 129], [232, 5],
+                                   [233, 12, 320]])
+def test_solve_at_its_edges(tb, sizes):
+    """Padding to 8, several panels, the largest size factored in shared memory
+    and the first above it; dropped columns, and the column of a bad pivot.
+    The scaled matrices have condition numbers below 100, so one step of
+    refinement leaves a few hundred roundings of FP64 at most."""
+    import torch
+    from tractor_b200 import render
+    rng = np.random.default_rng(sum(sizes))
+    for damp, broken in ((0., False), (.3, False), (0., True)):
+        Ms, gs = [], []
+        for P in sizes:
+            B = rng.normal(size=(4 * P + 8, P)) / np.sqrt(4 * P + 8) + np.eye(4 * P + 8, P)
+            M = B.T @ B
+            D = 10. ** rng.uniform(-3, 3, P)
+            M *= D[:, None] * D
+            if P > 4:
+                M[3], M[:, 3] = 0., 0.
+            if broken and P > 1:
+                M[P - 1, P - 2] = M[P - 2, P - 1] = 2. * np.sqrt(M[P - 1, P - 1] * M[P - 2, P - 2])
+            Ms.append(M)
+            gs.append(rng.normal(size=P) * D)
+        ao = torch.tensor(np.cumsum([0] + [M.size for M in Ms])[:-1]).cuda()
+        ro = torch.tensor(np.cumsum([0] + sizes)[:-1]).cuda()
+        X, info, xo = render.solve_update(
+            torch.tensor(np.concatenate([M.ravel() for M in Ms])).cuda(),
+            torch.tensor(np.concatenate(gs)).cuda(), ao, ro, sizes, damp=damp)
+        X, info = X.cpu().numpy(), info.cpu().numpy()
+        for M, g, P, o, bad in zip(Ms, gs, sizes, xo, info):
+            if broken and P > 1 and M[P - 1, P - 2] != 0.:   # (not a dropped column)
+                assert bad == P
+                assert not X[o:o + P].any()
+                continue
+            assert bad == 0
+            live = np.diag(M) > 0
+            d = np.sqrt(np.diag(M)[live])
+            S = M[np.ix_(live, live)] / (d[:, None] * d) + damp ** 2 * np.eye(live.sum())
+            assert np.linalg.cond(S) < 100
+            ref = np.zeros(P)
+            ref[live] = np.linalg.solve(S, g[live] / d)
+            got = X[o:o + P].copy()
+            got[live] *= d
+            assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
 def test_chi2(tb):
     import torch
     from tractor_b200 import render

@@ -23,6 +23,7 @@
 //                normal equations by FP64 Cholesky with one refinement step,
 //                limits the step (bounds, maximum steps) and writes the next
 //                trial parameters.
+#include "ldl.cuh"
 #include "profile_eval.cuh"
 
 namespace {
@@ -415,12 +416,6 @@ __device__ __forceinline__ double frag(const T* X, int step) {
     return (double)X[(lane >> 2) * kLd + 4 * step + (lane & 3)];
 }
 
-__device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
-}
-
 // Where a unit adds its products.  kVjp: g alone, by parameter slot (P per
 // slice).  kEquations: compact slices that hold only the m sources whose masks
 // meet the unit (`mask`), seven columns each: a (7 m)^2 block of H (upper
@@ -556,7 +551,7 @@ __device__ void run_tiles(PassSmem<T>& sm, const PassUnit<T>& u, unsigned hit, i
 #pragma unroll
             for (int s = 0; s < R; s++) f[s] = frag(X + s * kXs, step);
 #pragma unroll
-            for (int q = 0; q < NB; q++) mma884(c[q], f[pair_a(q, R)], f[pair_b(q, R)]);
+            for (int q = 0; q < NB; q++) tb::mma884(c[q], f[pair_a(q, R)], f[pair_b(q, R)]);
         }
     }
     auto src = [&](int i) { return nth_bit(hit, i); };
@@ -610,7 +605,7 @@ __device__ void crowded_tile(PassSmem<T>& sm, const PassUnit<T>& u, unsigned hit
 #pragma unroll
                 for (int s = 0; s < kG3; s++) f[s] = frag(X + s * kXs, step);
 #pragma unroll
-                for (int q = 0; q < NB; q++) mma884(c[q], f[pair_a(q, kG3)], f[pair_b(q, kG3)]);
+                for (int q = 0; q < NB; q++) tb::mma884(c[q], f[pair_a(q, kG3)], f[pair_b(q, kG3)]);
             }
             flush<T, NB>(sm, c, [&](int q) { return src(pair_a(q, kG3)); },
                          [&](int q) { return src(pair_b(q, kG3)); }, u.out);
@@ -629,7 +624,7 @@ __device__ void crowded_tile(PassSmem<T>& sm, const PassUnit<T>& u, unsigned hit
             for (int step = 0; step < 8; step++) {
                 const double fb = frag(Xb, step);
 #pragma unroll
-                for (int q = 0; q < kG3; q++) mma884(c[q], frag(X + q * kXs, step), fb);
+                for (int q = 0; q < kG3; q++) tb::mma884(c[q], frag(X + q * kXs, step), fb);
             }
             flush<T, kG3>(sm, c, src, [&](int) { return sI; }, u.out);
         }
@@ -919,25 +914,9 @@ fit_assemble_kernel(const tb_fit_blob* __restrict__ blobs,
     }
 }
 
-// 1 / d by Newton's iteration r <- r + r (1 - d r) from the hardware's
-// 20-bit estimate (twice: past FP64's precision): a shorter chain than an
-// IEEE division, and the refinement step covers its last bit.  A d that is
-// not a positive normal number is rejected by the caller.
-__device__ __forceinline__ double reciprocal(double d) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    r = fma(r, fma(-d, r, 1.0), r);
-    return fma(r, fma(-d, r, 1.0), r);
-}
-
-// Factor storage: packed lower triangle by columns, padded to a multiple of
-// 8 rows (identity): element (i, j) at L[packed_col(j, n) + i], n the padded
-// size.
-__host__ __device__ constexpr int packed_col(int j, int n) { return j * (2 * n - j - 1) / 2; }
-__host__ __device__ constexpr int packed_size(int n) { return n * (n + 1) / 2; }
 constexpr int kStepMaxP = TB_FIT_MAX_SRC * TB_FIT_NPAR;
 constexpr int kStepSharedP = 128;      // largest padded size factored in shared memory
-constexpr int kStepSmem = 8 * (packed_size(kStepSharedP) + 5 * kStepSharedP);   // 71 KB
+constexpr int kStepSmem = 8 * (tb::packed_size(kStepSharedP) + 5 * kStepSharedP);   // 71 KB
 static_assert(kStepSmem >= 8 * 5 * ((kStepMaxP + 7) / 8 * 8), "the vectors always fit");
 
 // One CTA per blob.  Up to 128 parameters the factor lives in shared memory
@@ -982,7 +961,7 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
     double* ga = gbuf + b.g_off + (int64_t)ns * P;
     double* pa = params + (int64_t)b.src0 * TB_FIT_NPAR;
     double* pt = trial + (int64_t)b.src0 * TB_FIT_NPAR;
-    auto col = [&](int j) { return L + packed_col(j, n); };
+    auto col = [&](int j) { return L + tb::packed_col(j, n); };
 
     const double c2 = warp == 0 ? trial_chi2(chi2_part + b.unit0, ns) : 0.0;
     if (tid == 0) {
@@ -1058,92 +1037,7 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
         }
     }
     __syncthreads();
-    bool bad = false;
-    for (int k0 = 0; k0 < n; k0 += 4) {
-        const double *c0 = col(k0), *c1 = col(k0 + 1), *c2k = col(k0 + 2), *c3 = col(k0 + 3);
-        // the 4 x 4 diagonal block, the same in every thread
-        const double a10 = c0[k0 + 1], a20 = c0[k0 + 2], a30 = c0[k0 + 3];
-        const double d0 = c0[k0], r0 = reciprocal(d0);
-        const double d1 = c1[k0 + 1] - a10 * a10 * r0, r1 = reciprocal(d1);
-        const double a21 = c1[k0 + 2] - a20 * a10 * r0, a31 = c1[k0 + 3] - a30 * a10 * r0;
-        const double d2 = c2k[k0 + 2] - a20 * a20 * r0 - a21 * a21 * r1,
-                     r2 = reciprocal(d2);
-        const double a32 = c2k[k0 + 3] - a30 * a20 * r0 - a31 * a21 * r1;
-        const double d3 = c3[k0 + 3] - a30 * a30 * r0 - a31 * a31 * r1 - a32 * a32 * r2;
-        const double r3 = reciprocal(d3);
-        if (!(d0 > 0.0 && d1 > 0.0 && d2 > 0.0 && d3 > 0.0) || !isfinite(d0) || !isfinite(d1) ||
-            !isfinite(d2) || !isfinite(d3)) {
-            bad = true;
-            break;
-        }
-        // the panel's other rows, one per thread
-        const double l10 = a10 * r0, l20 = a20 * r0, l30 = a30 * r0;
-        const double l21 = a21 * r1, l31 = a31 * r1, l32 = a32 * r2;
-        for (int i = k0 + 4 + tid; i < n; i += kStepThreads) {
-            const double e0 = c0[i];
-            const double e1 = c1[i] - e0 * l10;
-            const double e2 = c2k[i] - e0 * l20 - e1 * l21;
-            const double e3 = c3[i] - e0 * l30 - e1 * l31 - e2 * l32;
-            col(k0 + 1)[i] = e1;
-            col(k0 + 2)[i] = e2;
-            col(k0 + 3)[i] = e3;
-        }
-        __syncthreads();   // the panel's rows are complete, the diagonal block is read
-        if (tid == 0) {
-            col(k0 + 1)[k0 + 1] = d1;
-            col(k0 + 1)[k0 + 2] = a21;
-            col(k0 + 1)[k0 + 3] = a31;
-            col(k0 + 2)[k0 + 2] = d2;
-            col(k0 + 2)[k0 + 3] = a32;
-            col(k0 + 3)[k0 + 3] = d3;
-            rdg[k0] = r0;
-            rdg[k0 + 1] = r1;
-            rdg[k0 + 2] = r2;
-            rdg[k0 + 3] = r3;
-        }
-        // trailing 8 x 8 tiles: row lane / 4, columns 2 (lane % 4) + {0, 1}
-        const int base = (k0 + 4) / 8 * 8, T = (n - base) / 8;
-        const int q = lane & 3;
-        const double rq = -(q == 0 ? r0 : q == 1 ? r1 : q == 2 ? r2 : r3);
-        const double* ck = col(k0 + q);
-        int tj = 0, ti = warp;
-        for (int e = warp; e < T * (T + 1) / 2; e += 3 * (kStepThreads / 32)) {
-            // three tiles' loads before the first product
-            double *p0[3], *p1[3], fa[3], fb[3], c[3][2];
-            bool on0[3], on1[3];
-#pragma unroll
-            for (int t = 0; t < 3; t++) {
-                on0[t] = on1[t] = e + t * (kStepThreads / 32) < T * (T + 1) / 2;
-                fa[t] = fb[t] = c[t][0] = c[t][1] = 0.0;
-                if (!on0[t]) continue;
-                while (ti >= T) {   // the lower triangle's tile columns in turn
-                    tj++;
-                    ti += tj - T;
-                }
-                const int i = base + 8 * ti + (lane >> 2), j = base + 8 * tj + 2 * q;
-                const int jb = base + 8 * tj + (lane >> 2);
-                p0[t] = col(j) + i;
-                p1[t] = col(j + 1) + i;
-                // rows and columns above the trailing part (first tile only)
-                // belong to the panel
-                on0[t] = j >= k0 + 4 && i >= j;
-                on1[t] = j + 1 >= k0 + 4 && i >= j + 1;
-                if (i >= k0 + 4) fa[t] = ck[i];
-                if (jb >= k0 + 4) fb[t] = ck[jb] * rq;
-                if (on0[t]) c[t][0] = *p0[t];
-                if (on1[t]) c[t][1] = *p1[t];
-                ti += kStepThreads / 32;
-            }
-#pragma unroll
-            for (int t = 0; t < 3; t++) mma884(c[t], fa[t], fb[t]);
-#pragma unroll
-            for (int t = 0; t < 3; t++) {
-                if (on0[t]) *p0[t] = c[t][0];
-                if (on1[t]) *p1[t] = c[t][1];
-            }
-        }
-        __syncthreads();
-    }
+    const bool bad = tb::ldl_factor<kStepThreads>(L, rdg, n) != 0;
     if (bad) {
         // not positive definite: treat as a rejected step with more damping
         if (tid == 0) {
@@ -1188,38 +1082,7 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
             }
             __syncthreads();
         }
-        if (warp == 0) {
-            // L z = y, w = D^-1 z, L^T x = w in place in y, four columns at a
-            // time: every lane solves the 4 x 4 triangle, then the lanes
-            // update the remaining rows; l_ik = c_ik / d_k
-            for (int k = 0; k < n; k += 4) {
-                const double *c0 = col(k), *c1 = col(k + 1), *c2k = col(k + 2), *c3 = col(k + 3);
-                const double z0 = y[k] * rdg[k];
-                const double z1 = (y[k + 1] - c0[k + 1] * z0) * rdg[k + 1];
-                const double z2 = (y[k + 2] - c0[k + 2] * z0 - c1[k + 2] * z1) * rdg[k + 2];
-                const double z3 = (y[k + 3] - c0[k + 3] * z0 - c1[k + 3] * z1 -
-                                   c2k[k + 3] * z2) * rdg[k + 3];
-                for (int i = k + 4 + lane; i < n; i += 32)
-                    y[i] -= (c0[i] * z0 + c1[i] * z1) + (c2k[i] * z2 + c3[i] * z3);
-                __syncwarp();   // the triangle's rows are read
-                if (lane < 4) y[k + lane] = lane == 0 ? z0 : lane == 1 ? z1 : lane == 2 ? z2 : z3;
-                __syncwarp();
-            }
-            for (int k = n - 4; k >= 0; k -= 4) {
-                const double *c0 = col(k), *c1 = col(k + 1), *c2k = col(k + 2);
-                const double x3 = y[k + 3];
-                const double x2 = y[k + 2] - c2k[k + 3] * rdg[k + 2] * x3;
-                const double x1 = y[k + 1] - (c1[k + 2] * x2 + c1[k + 3] * x3) * rdg[k + 1];
-                const double x0 = y[k] - (c0[k + 1] * x1 + c0[k + 2] * x2 + c0[k + 3] * x3) * rdg[k];
-                for (int j = lane; j < k; j += 32) {
-                    const double* cj = col(j) + k;
-                    y[j] -= ((cj[0] * x0 + cj[1] * x1) + (cj[2] * x2 + cj[3] * x3)) * rdg[j];
-                }
-                __syncwarp();
-                if (lane < 3) y[k + lane] = lane == 0 ? x0 : lane == 1 ? x1 : x2;
-                __syncwarp();
-            }
-        }
+        if (warp == 0) tb::ldl_solve(L, rdg, y, n);
         __syncthreads();
         for (int i = tid; i < P; i += kStepThreads) xs[i] += y[i];
         __syncthreads();

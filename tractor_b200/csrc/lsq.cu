@@ -13,6 +13,7 @@
 // the chi-square sum of Tractor.getLogLikelihood (tractor/engine.py:475-479).
 #include <atomic>
 
+#include "ldl.cuh"
 #include "tb_common.cuh"
 #include "tc_sm100.cuh"
 
@@ -425,23 +426,40 @@ normal_eq_tc_kernel(const float* __restrict__ A, const float* __restrict__ rhs,
     }
 }
 
-constexpr int kSolveThreads = 256;
+constexpr int kSolveSharedP = 232;   // largest padded size factored in shared memory (217 KB)
+
+constexpr int solve_pad(int P) { return (P + 7) / 8 * 8; }
+// Shared memory for problems of at most max_p parameters: four vectors, and
+// the packed factor up to kSolveSharedP.
+constexpr int solve_smem(int max_p) {
+    const int n = solve_pad(max_p);
+    return 8 * (4 * n + (n <= kSolveSharedP ? tb::packed_size(n) : 0));
+}
+static_assert(solve_smem(kSolveSharedP) <= 227 * 1024 - 1024, "fits a CTA");
+static_assert(tb::packed_size(solve_pad(kSolveSharedP + 1)) <=
+                  (kSolveSharedP + 1) * (kSolveSharedP + 1),
+              "above, a padded factor fits its slice of the workspace");
 
 // Solves (D^-1 AtA D^-1 + damp^2 I) x = D^-1 Atr with D = sqrt(diag(AtA)),
-// X = x / D.  L (P x P, lower) lives in `work`.
-__global__ void __launch_bounds__(kSolveThreads)
+// X = x / D, one CTA per problem: LDL^T in shared memory up to 232 parameters
+// (`shared_n` is the padded size the launch has room for), above in `work`,
+// and one step of refinement against the unscaled matrix.
+//
+// Bound: the chain of columns and of the triangular solves.  A column at a
+// time through L2 with three barriers each, and an eight-barrier sum for each
+// row of a solve, took 403 us for 512 problems of 63 parameters, now 75; 300
+// of 96: 764, 129; 150 of 200: 3485, 609; one of 4: 15, 7.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads)
 solve_kernel(const double* __restrict__ AtA, const double* __restrict__ Atr,
              const int64_t* ata_off, const int64_t* atr_off, const int32_t* Pv,
              const int64_t* x_off, double* X, int32_t* info, double damp, double* work,
-             int64_t work_stride) {
-    __shared__ double d[kMaxSmemP];
-    __shared__ double y[kMaxSmemP];
-    __shared__ double xs[kMaxSmemP];
-    __shared__ double red[kSolveThreads];
-    __shared__ int bad;
+             int64_t work_stride, int shared_n) {
+    extern __shared__ __align__(16) double solve_sm[];
     const int b = blockIdx.x;
     const int P = Pv[b];
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int kWarps = kThreads / 32;
     if (P <= 0) return;
     // P[b] is device data: a problem larger than the shared arrays or than
     // its slice of the workspace (work_stride = max_p^2 doubles) is refused
@@ -450,104 +468,103 @@ solve_kernel(const double* __restrict__ AtA, const double* __restrict__ Atr,
         if (tid == 0) info[b] = -1;
         return;
     }
+    const int n = solve_pad(P);   // <= the launch's
     const double* M = AtA + ata_off[b];
     const double* g = Atr + atr_off[b];
-    double* L = work + (int64_t)b * work_stride;
-    if (tid == 0) bad = 0;
-    for (int i = tid; i < P; i += kSolveThreads) {
-        const double a = M[(int64_t)i * P + i];
+    double* d = solve_sm;
+    double* y = d + n;
+    double* xs = y + n;
+    double* rdg = xs + n;
+    double* L = n <= shared_n ? rdg + n : work + (int64_t)b * work_stride;
+    for (int i = tid; i < n; i += kThreads) {
+        const double a = i < P ? M[(int64_t)i * P + i] : 0.0;
         d[i] = (a > 0.0 && isfinite(a)) ? sqrt(a) : 0.0;
     }
     __syncthreads();
     const double d2 = damp * damp;
     // Scaled matrix (lower triangle); a dropped column becomes a unit row.
-    for (int e = tid; e < P * P; e += kSolveThreads) {
-        const int i = e / P, j = e % P;
-        if (j > i) continue;
-        double v;
-        if (d[i] == 0.0 || d[j] == 0.0) v = (i == j) ? 1.0 : 0.0;
-        else v = M[(int64_t)i * P + j] / (d[i] * d[j]) + (i == j ? d2 : 0.0);
-        L[(int64_t)i * P + j] = v;
+    for (int i = warp; i < n; i += kWarps) {
+        const double di = d[i];
+        for (int j = lane; j <= i; j += 32) {
+            const double dj = d[j];
+            double v = i == j ? 1.0 : 0.0;
+            if (di != 0.0 && dj != 0.0)
+                v = M[(int64_t)i * P + j] / (di * dj) + (i == j ? d2 : 0.0);
+            L[tb::packed_col(j, n) + i] = v;
+        }
     }
     __syncthreads();
-    // Right-looking Cholesky.
-    for (int k = 0; k < P; k++) {
-        if (tid == 0) {
-            const double a = L[(int64_t)k * P + k];
-            if (!(a > 0.0) || !isfinite(a)) bad = k + 1;
-            else L[(int64_t)k * P + k] = sqrt(a);
-        }
-        __syncthreads();
-        if (bad) break;
-        const double lkk = L[(int64_t)k * P + k];
-        for (int i = k + 1 + tid; i < P; i += kSolveThreads) L[(int64_t)i * P + k] /= lkk;
-        __syncthreads();
-        const int m = P - k - 1;
-        for (int e = tid; e < m * m; e += kSolveThreads) {
-            const int i = k + 1 + e / m, j = k + 1 + e % m;
-            if (j > i) continue;
-            L[(int64_t)i * P + j] -= L[(int64_t)i * P + k] * L[(int64_t)j * P + k];
-        }
-        __syncthreads();
-    }
+    const int bad = tb::ldl_factor<kThreads>(L, rdg, n);
     if (bad) {
-        for (int i = tid; i < P; i += kSolveThreads) X[x_off[b] + i] = 0.0;
+        for (int i = tid; i < P; i += kThreads) X[x_off[b] + i] = 0.0;
         if (tid == 0) info[b] = bad;
         return;
     }
     // rhs and two solves (solution + one refinement step)
-    for (int i = tid; i < P; i += kSolveThreads) {
+    for (int i = tid; i < n; i += kThreads) {
         xs[i] = 0.0;
-        y[i] = (d[i] == 0.0) ? 0.0 : g[i] / d[i];
+        y[i] = d[i] == 0.0 ? 0.0 : g[i] / d[i];
     }
     __syncthreads();
     for (int pass = 0; pass < 2; pass++) {
         if (pass == 1) {
-            // residual r = rhs - M_scaled x, into y
-            for (int i = tid; i < P; i += kSolveThreads) {
-                double acc = (d[i] == 0.0) ? 0.0 : g[i] / d[i];
-                for (int j = 0; j < P; j++) {
-                    double mij;
-                    if (d[i] == 0.0 || d[j] == 0.0) mij = (i == j) ? 1.0 : 0.0;
-                    else mij = M[(int64_t)i * P + j] / (d[i] * d[j]) + (i == j ? d2 : 0.0);
-                    acc -= mij * xs[j];
-                }
-                y[i] = acc;
+            // residual r = rhs - M_scaled x, into y: a row per warp
+            for (int i = warp; i < P; i += kWarps) {
+                const double di = d[i];
+                double acc = 0.0;
+                if (di != 0.0)
+                    for (int j = lane; j < P; j += 32) {
+                        const double dj = d[j];
+                        if (dj == 0.0) continue;
+                        acc = fma(M[(int64_t)i * P + j] / (di * dj) + (i == j ? d2 : 0.0), xs[j],
+                                  acc);
+                    }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                if (lane == 0) y[i] = di == 0.0 ? -xs[i] : g[i] / di - acc;
             }
             __syncthreads();
         }
-        // forward: L z = y (in place in y)
-        for (int i = 0; i < P; i++) {
-            double part = 0.0;
-            for (int j = tid; j < i; j += kSolveThreads) part += L[(int64_t)i * P + j] * y[j];
-            red[tid] = part;
-            __syncthreads();
-            for (int s = kSolveThreads / 2; s > 0; s >>= 1) {
-                if (tid < s) red[tid] += red[tid + s];
-                __syncthreads();
-            }
-            if (tid == 0) y[i] = (y[i] - red[0]) / L[(int64_t)i * P + i];
-            __syncthreads();
-        }
-        // backward: L^T w = z (in place in y)
-        for (int i = P - 1; i >= 0; i--) {
-            double part = 0.0;
-            for (int j = i + 1 + tid; j < P; j += kSolveThreads) part += L[(int64_t)j * P + i] * y[j];
-            red[tid] = part;
-            __syncthreads();
-            for (int s = kSolveThreads / 2; s > 0; s >>= 1) {
-                if (tid < s) red[tid] += red[tid + s];
-                __syncthreads();
-            }
-            if (tid == 0) y[i] = (y[i] - red[0]) / L[(int64_t)i * P + i];
-            __syncthreads();
-        }
-        for (int i = tid; i < P; i += kSolveThreads) xs[i] += y[i];
+        if (warp == 0) tb::ldl_solve(L, rdg, y, n);
+        __syncthreads();
+        for (int i = tid; i < P; i += kThreads) xs[i] += y[i];
         __syncthreads();
     }
-    for (int i = tid; i < P; i += kSolveThreads)
-        X[x_off[b] + i] = (d[i] == 0.0) ? 0.0 : xs[i] / d[i];
+    for (int i = tid; i < P; i += kThreads)
+        X[x_off[b] + i] = d[i] == 0.0 ? 0.0 : xs[i] / d[i];
     if (tid == 0) info[b] = 0;
+}
+
+template <int kThreads>
+int launch_solve_threads(const double* AtA, const double* Atr, const int64_t* ata_off,
+                         const int64_t* atr_off, const int32_t* P, const int64_t* x_off, double* X,
+                         int32_t* info, double damp, int n_problems, int max_p, double* work,
+                         cudaStream_t s) {
+    const int smem = solve_smem(max_p), n = solve_pad(max_p);
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(solve_kernel<kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             smem) != cudaSuccess)
+        return TB_ERR_LAUNCH;
+    solve_kernel<kThreads><<<n_problems, kThreads, smem, s>>>(
+        AtA, Atr, ata_off, atr_off, P, x_off, X, info, damp, work, (int64_t)max_p * max_p,
+        n <= kSolveSharedP ? n : 0);
+    return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
+}
+
+// Threads by the launch: 256 shorten a problem's chain most (232 parameters:
+// 466 us, with 128 threads 697; one problem of 48: 37, 45), but two such CTAs
+// fill an SM's registers.  More problems than that take smaller CTAs where
+// their factors leave room for them: 1500 of 32 parameters 51 us with 64
+// threads, 60 with 128, 136 with 256; 512 of 63 parameters 100, 75, 111.
+constexpr int kSolveFew = 2 * 148;
+int launch_solve(const double* AtA, const double* Atr, const int64_t* ata_off,
+                 const int64_t* atr_off, const int32_t* P, const int64_t* x_off, double* X,
+                 int32_t* info, double damp, int n_problems, int max_p, double* work,
+                 cudaStream_t s) {
+    const auto f = n_problems <= kSolveFew || max_p > 96 ? launch_solve_threads<256>
+                   : max_p > 40                          ? launch_solve_threads<128>
+                                                         : launch_solve_threads<64>;
+    return f(AtA, Atr, ata_off, atr_off, P, x_off, X, info, damp, n_problems, max_p, work, s);
 }
 
 constexpr int kChiThreads = 1024;
@@ -958,9 +975,8 @@ extern "C" int tb_solve_update(const double* AtA, const double* Atr, const int64
     if (max_p > kMaxSmemP) return TB_ERR_SIZE;
     if (!AtA || !Atr || !ata_off || !atr_off || !P || !x_off || !X || !info || !work)
         return TB_ERR_ARG;
-    solve_kernel<<<n_problems, kSolveThreads, 0, (cudaStream_t)stream>>>(
-        AtA, Atr, ata_off, atr_off, P, x_off, X, info, damp, work, (int64_t)max_p * max_p);
-    return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
+    return launch_solve(AtA, Atr, ata_off, atr_off, P, x_off, X, info, damp, n_problems, max_p,
+                        work, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -999,9 +1015,8 @@ extern "C" int tb_solve_update_noalloc(const double* AtA, const double* Atr,
             return TB_ERR_LAUNCH;
         g_solve_scratch_addr[dev].store(scratch, std::memory_order_relaxed);
     }
-    solve_kernel<<<n_problems, kSolveThreads, 0, (cudaStream_t)stream>>>(
-        AtA, Atr, ata_off, atr_off, P, x_off, X, info, damp, scratch, (int64_t)max_p * max_p);
-    return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
+    return launch_solve(AtA, Atr, ata_off, atr_off, P, x_off, X, info, damp, n_problems, max_p,
+                        scratch, (cudaStream_t)stream);
 }
 
 extern "C" int tb_chi2(const float* data, const float* model, const float* inverr,
