@@ -101,17 +101,13 @@ class BlobFitter(object):
         units['t1'] = n_active[units['blob']]
         units['slice'] = units['band']
         # pass units: the (blob, band) images split into tile ranges
-        pu = []
-        for b in range(self.n_blobs):
-            q = int(parts[b])
-            cut = (np.arange(q + 1) * int(n_active[b])) // q
-            for k in range(self.n_bands):
-                for j in range(q):
-                    u = units[b * self.n_bands + k].copy()
-                    u['slice'] = k * q + j
-                    u['t0'], u['t1'] = cut[j], cut[j + 1]
-                    pu.append(u)
-        pass_units = np.array(pu, _lib.FIT_UNIT)
+        q = np.repeat(parts, n_slices)
+        slot = np.arange(len(q)) - np.repeat(np.cumsum(n_slices) - n_slices, n_slices)
+        of = np.repeat(np.arange(self.n_blobs), n_slices)
+        pass_units = units[of * self.n_bands + slot // q]
+        pass_units['slice'] = slot
+        pass_units['t0'] = (slot % q) * n_active[of] // q
+        pass_units['t1'] = (slot % q + 1) * n_active[of] // q
         # the pass takes units largest first
         cost = (pass_units['t1'] - pass_units['t0']).astype(np.float64) * \
             (1 + nsrc[pass_units['blob']])

@@ -156,17 +156,16 @@ class BlobModel(object):
         f = fitter
         P = f.blobs_np['P'].astype(np.int64)
         ns = f.blobs_np['n_slices'].astype(np.int64)
-        maxs = int(ns.max())
-        blob_of = np.repeat(np.arange(f.n_blobs), np.diff(np.concatenate(
-            [[0], np.cumsum(f.blobs_np['n_src'])])))
-        first = np.concatenate([[0], np.cumsum(f.blobs_np['n_src'])[:-1]])
-        idx = np.full((f.n_src * NPAR_FIT, maxs), int(f.gbuf.numel()), np.int64)
-        for q in range(f.n_src * NPAR_FIT):
-            s = q // NPAR_FIT
-            b = blob_of[s]
-            local = (s - first[b]) * NPAR_FIT + q % NPAR_FIT
-            for k in range(int(ns[b])):
-                idx[q, k] = int(f.blobs_np['g_off'][b]) + k * int(P[b]) + local
+        n_src = f.blobs_np['n_src'].astype(np.int64)
+        blob_of = np.repeat(np.arange(f.n_blobs), n_src)
+        local = np.arange(f.n_src) - (np.cumsum(n_src) - n_src)[blob_of]
+        # the place in gbuf of (source, parameter, slice)
+        k = np.arange(int(ns.max()))
+        idx = (f.blobs_np['g_off'].astype(np.int64)[blob_of, None, None] +
+               (local[:, None] * NPAR_FIT + np.arange(NPAR_FIT))[:, :, None] +
+               k * P[blob_of, None, None])
+        idx = np.where(k < ns[blob_of, None, None], idx, int(f.gbuf.numel()))
+        idx = idx.reshape(f.n_src * NPAR_FIT, -1)
         # slot gbuf.numel() reads a zero appended to the slices
         self._idx = torch.from_numpy(idx).to(f.dev)
 
