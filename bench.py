@@ -690,8 +690,9 @@ def _deriv_cpu_worker(args):
 def bench_derivs(args, dev, flush, clk, cpu_seconds):
     """All seven analytic derivative columns (x, y, counts, r_e, e1, e2, n)
     of 256 Sersic galaxies on 32-128 px masks (FFT 64-256): Jacobian through
-    tb_galaxy_fft_jac_prep + tb_fourier_render_deriv (one launch of 7 x 256
-    derivative items), and the fused vector-Jacobian product (TB_FFT_DOT).
+    tb_galaxy_fft_jac_prep + the Fourier render of 7 x 256 derivative items,
+    and the vector-Jacobian product (tb_galaxy_fft_vjp, one adjoint transform
+    per galaxy).
     Metric: Mpix x components / s with every column counted as a render."""
     import ctypes
     import torch
@@ -706,10 +707,19 @@ def bench_derivs(args, dev, flush, clk, cpu_seconds):
     out = torch.empty(7 * npix, dtype=torch.float32, device=dev)
     upstream = torch.randn(npix, generator=torch.Generator(device=dev).manual_seed(7),
                            device=dev, dtype=torch.float32)
-    dots = torch.zeros(7 * n, dtype=torch.float64, device=dev)
+    it_t, camp, cvar, dcoef, flg, misc = jac._work(n)
+
+    def prep():
+        jac._prep(d_src, n, _lib.MOG_STORE, npix, _lib.stream_ptr())
+
+    def columns():
+        render.fourier_render(it_t.data_ptr(), 7 * n, camp.data_ptr(), cvar.data_ptr(),
+                              r.spec.data_ptr(), out.data_ptr(), misc.data_ptr() + 16,
+                              dcoef_ptr=dcoef.data_ptr())
+
     for _ in range(max(3, args.warmup)):
-        jac._run(d_src, n, out, _lib.MOG_STORE, npix)
-        jac._run(d_src, n, upstream, _lib.FFT_DOT, 0, dots=dots)
+        prep()
+        columns()
     torch.cuda.synchronize()
     flags = jac._work(n)[4].cpu().numpy()
     assert np.all(flags == 0), 'jac prep flagged sources: %s' % np.unique(flags)
@@ -717,35 +727,25 @@ def bench_derivs(args, dev, flush, clk, cpu_seconds):
     pixcomp = float(np.sum(items['sz'].astype(np.float64) ** 2 * items['K']))   # 7 columns
     ex2 = float(np.sum(items['sz'].astype(np.float64) * (items['sz'] // 2 + 1) * items['K']))
     steps = max(5, min(args.steps, 20))
-    lib = _lib.load()
-    it_t, camp, cvar, dcoef, flg, misc = jac._work(n)
 
-    def timed(mode, o, dts):
+    def timed(first, second):
         tt, kt = [], []
         for _ in range(steps):
             flush.zero_()
             e = [torch.cuda.Event(enable_timing=True) for _ in range(3)]
             e[0].record()
-            rc = lib.tb_galaxy_fft_jac_prep(d_src.data_ptr(), n, ctypes.addressof(r.image),
-                                            ctypes.addressof(r.tables.struct), it_t.data_ptr(),
-                                            camp.data_ptr(), cvar.data_ptr(), dcoef.data_ptr(),
-                                            batch.COMP_STRIDE, mode,
-                                            npix if mode == _lib.MOG_STORE else 0,
-                                            flg.data_ptr(), _lib.stream_ptr())
-            _lib.check(rc, 'tb_galaxy_fft_jac_prep')
+            first()
             e[1].record()
-            render.fourier_render(it_t.data_ptr(), 7 * n, camp.data_ptr(), cvar.data_ptr(),
-                                  r.spec.data_ptr(), o.data_ptr(), misc.data_ptr() + 16,
-                                  dcoef_ptr=dcoef.data_ptr(),
-                                  dots_ptr=None if dts is None else dts.data_ptr())
+            second()
             e[2].record()
             e[2].synchronize()
             tt.append(e[0].elapsed_time(e[2]) / 1e3)
             kt.append(e[1].elapsed_time(e[2]) / 1e3)
         return float(np.mean(tt)), float(np.mean(kt))
 
-    jac_s, jac_k = timed(_lib.MOG_STORE, out, None)
-    vjp_s, vjp_k = timed(_lib.FFT_DOT, upstream, dots)
+    jac_s, jac_k = timed(prep, columns)
+    jac.vjp(d_src, n, upstream)   # its workspace
+    vjp_s, _ = timed(lambda: None, lambda: jac.vjp(d_src, n, upstream))
     # end to end: records in from pinned memory, the Jacobian out
     h_out = torch.empty(7 * npix, dtype=torch.float32).pin_memory()
     e2e = []
@@ -753,7 +753,8 @@ def bench_derivs(args, dev, flush, clk, cpu_seconds):
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
         d_src.copy_(h_src, non_blocking=True)
-        jac._run(d_src, n, out, _lib.MOG_STORE, npix)
+        prep()
+        columns()
         h_out.copy_(out, non_blocking=True)
         e1.record()
         e1.synchronize()
@@ -771,8 +772,8 @@ def bench_derivs(args, dev, flush, clk, cpu_seconds):
         'e2e': {'value': pixcomp / float(np.mean(e2e)) / 1e6, 'unit': 'Mpix*components/s',
                 'h2d_bytes_per_step': int(h_src.numel()),
                 'd2h_bytes_per_step': int(h_out.numel() * 4)},
-        'gpu_launches_per_step': 2 + 2 * (-(-7 * n // 256)),
-        'roofline': {'bound': 'sfu', 'kernel': 'tb_fourier_render_split (Jacobian items)',
+        'gpu_launches_per_step': 3,   # prep, sort, render (split); prep, render
+        'roofline': {'bound': 'sfu', 'kernel': 'Fourier render of the Jacobian items',
                      'achieved': ex2 / jac_k / 1e9, 'peak': peak, 'unit': 'Gex2/s',
                      'frac': ex2 / jac_k / 1e9 / peak, 'kernel_ms': jac_k * 1e3,
                      'algorithmic': '%.0f ex2 per launch' % ex2,

@@ -269,7 +269,8 @@ int tb_fourier_render_deriv(const tb_fft_item* items, int32_t n_items,
  * Lanczos-3 window keeps 3 px from the FFT box's edges rendered on packed
  * transforms, two columns or two row pairs at a time, by groups of warps (a
  * CTA per item of size 256, two items per CTA at 128, seven at 64, sixteen at
- * 32); the others as tb_fourier_render_deriv renders them.  Two launches.
+ * 32); the others as tb_fourier_render_deriv renders them.  Two launches;
+ * with comp_dcoef or dots, tb_fourier_render_deriv's one.
  * Results equal tb_fourier_render's up to FP32 rounding.  workspace: device,
  * 256-byte aligned, at least tb_fourier_workspace(n_items) bytes, not shared
  * by calls that may overlap. */

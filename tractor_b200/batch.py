@@ -115,6 +115,7 @@ class FourierGalaxyRenderer(object):
         self.image = img
         self.tables = device_profile_tables()
         self._scratch = {}
+        self._workspaces = {}
 
     def _work(self, n):
         """Device scratch for n sources: items, components, flags, counter,
@@ -127,9 +128,14 @@ class FourierGalaxyRenderer(object):
             cvar = torch.empty(n * COMP_STRIDE * 4, dtype=torch.float64, device=dev)
             flags = torch.empty(n, dtype=torch.int32, device=dev)
             misc = torch.zeros(8, dtype=torch.int32, device=dev)   # counter + status
-            ws = render.new_fourier_workspace(n, dev)
-            self._scratch[n] = (items, camp, cvar, flags, misc, ws)
+            self._scratch[n] = (items, camp, cvar, flags, misc)
         return self._scratch[n]
+
+    def _workspace(self, n):
+        """The sorted path's workspace for n sources."""
+        if n not in self._workspaces:
+            self._workspaces[n] = render.new_fourier_workspace(n, render.device())
+        return self._workspaces[n]
 
     METHODS = ('fused', 'persistent', 'split')
     # one launch in place of three: 17 against 29 us for one 32-px patch; from
@@ -146,7 +152,7 @@ class FourierGalaxyRenderer(object):
         'fused' for a few sources and 'split' for more (FUSED_MAX).  Returns
         the flags tensor (see tb_galaxy_fft_prep)."""
         lib = _lib.load()
-        items, camp, cvar, flags, misc, ws = self._work(n)
+        items, camp, cvar, flags, misc = self._work(n)
         s = _lib.stream_ptr(stream)
         method = method or getattr(self, 'method', None) or (
             'fused' if n <= self.FUSED_MAX else 'split')
@@ -165,7 +171,8 @@ class FourierGalaxyRenderer(object):
         _lib.check(rc, 'tb_galaxy_fft_prep')
         render.fourier_render(items.data_ptr(), n, camp.data_ptr(), cvar.data_ptr(),
                               self.spec.data_ptr(), out.data_ptr(), misc.data_ptr() + 16,
-                              stream=stream, method=method, workspace=ws)
+                              stream=stream, method=method,
+                              workspace=self._workspace(n) if method == 'split' else None)
         return flags
 
     def autotune(self, srcs, n, out):

@@ -409,16 +409,14 @@ __device__ void pair_size(unsigned char* smem, const tb_fft_item* __restrict__ i
 __global__ void __launch_bounds__(kPairThreads, 1)
 fourier_pair_kernel(const tb_fft_item* __restrict__ items, int n_items,
                     const double* __restrict__ amp, const double* __restrict__ var,
-                    const double* __restrict__ dcoef, const float* __restrict__ psf_spec,
-                    float* __restrict__ out, double* __restrict__ dots, PairWs* ws,
+                    const float* __restrict__ psf_spec, float* __restrict__ out, PairWs* ws,
                     const int32_t* __restrict__ lists, tb_status* st) {
     static_assert(kPairThreads == kThreads && kPairSmem >= kSmemBytes, "one block shape for both");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // (first: an item at the box's edge takes several times as long as another)
-    if (ws->count[4] != 0) {
-        render_items<true>(items, n_items, amp, var, dcoef, psf_spec, out, dots, &ws->next[4], st,
-                             lists + 4 * (int64_t)n_items, ws->count[4], smem_raw);
-    }
+    if (ws->count[4] != 0)
+        render_items<true>(items, n_items, amp, var, nullptr, psf_spec, out, nullptr,
+                           &ws->next[4], st, lists + 4 * (int64_t)n_items, ws->count[4], smem_raw);
     pair_size<256>(smem_raw, items, lists, ws->count[0], &ws->next[0], amp, var, psf_spec, out);
     pair_size<128>(smem_raw, items, lists + n_items, ws->count[1], &ws->next[1], amp, var,
                    psf_spec, out);
@@ -429,15 +427,15 @@ fourier_pair_kernel(const tb_fft_item* __restrict__ items, int n_items,
 }
 
 // Sorts the items into the lists by FFT size; those outside this path (a
-// window at the box's edge, derivative and difference items, TB_FFT_DOT, many
-// components) go to list 4.  Up to kSortItems items one CTA does it all (alone:
+// window at the box's edge, position derivatives, many components) go to
+// list 4.  Up to kSortItems items one CTA does it all (alone:
 // the counters and the status word are cleared here); more, many CTAs after
 // memsets.
 constexpr int kSortThreads = 512, kSortItems = 4096;
 
 __global__ void __launch_bounds__(kSortThreads)
 fourier_sort_kernel(const tb_fft_item* __restrict__ items, int n,
-                    const double* __restrict__ dcoef, PairWs* ws, int32_t* __restrict__ lists,
+                    PairWs* ws, int32_t* __restrict__ lists,
                     tb_status* st, bool alone) {
     if (alone) {
         if (threadIdx.x < 10) ws->count[threadIdx.x] = 0;   // count[5], next[5]
@@ -450,7 +448,7 @@ fourier_sort_kernel(const tb_fft_item* __restrict__ items, int n,
         int c = -1;
         if (i < n) {
             const tb_fft_item it = items[i];
-            if (!item_ok(it, dcoef)) tb::report(st, TB_STATUS_BAD_ITEM, i, it.sz);
+            if (!item_ok(it, nullptr)) tb::report(st, TB_STATUS_BAD_ITEM, i, it.sz);
             else
                 c = it.dmode != TB_FFT_VALUE || it.K > kPairMaxK || !split_eligible(it) ? 4
                     : it.sz == 256 ? 0 : it.sz == 128 ? 1 : it.sz == 64 ? 2 : 3;
