@@ -442,6 +442,30 @@ def test_approx3_region_on_device_matches_oracle(tb, oracle, derivs):
     assert flips <= 2, flips
 
 
+@pytest.mark.parametrize('P,R', [(1, 1), (7, 31), (31, 32), (32, 33), (33, 127), (47, 128),
+                                 (48, 129), (62, 257), (63, 1000), (63, 4097)])
+def test_normal_equations_at_their_edges(tb, P, R):
+    """Blocks, chunks and stages that are just full, just begun or empty, with
+    aligned and unaligned columns, against FP64."""
+    import torch
+    from tractor_b200 import render
+    rng = np.random.default_rng(P * 10000 + R)
+    n, ld = 5, R + (3 if P % 2 else -R % 4)
+    A = rng.normal(size=(n, P, ld)).astype(np.float32)
+    r = rng.normal(size=(n, R)).astype(np.float32)
+    i = np.arange(n, dtype=np.int64)
+    AtA, Atr, _, _ = render.normal_equations(
+        torch.from_numpy(A).cuda().reshape(-1), torch.from_numpy(r).cuda().reshape(-1),
+        i * P * ld, i * R, np.full(n, ld, np.int32), np.full(n, P, np.int32),
+        np.full(n, R, np.int32))
+    AtA, Atr = AtA.cpu().numpy().reshape(n, P, P), Atr.cpu().numpy().reshape(n, P)
+    A64, r64 = A[:, :, :R].astype(np.float64), r.astype(np.float64)
+    top = np.sqrt((A64 ** 2).sum(2).max() * max((A64 ** 2).sum(2).max(), (r64 ** 2).sum(1).max()))
+    assert np.abs(AtA - A64 @ A64.transpose(0, 2, 1)).max() <= 1e-6 * top
+    assert np.abs(Atr - (A64 @ r64[:, :, None])[:, :, 0]).max() <= 1e-6 * top
+    assert np.array_equal(AtA, AtA.transpose(0, 2, 1))
+
+
 def test_normal_equations_and_solve(tb):
     import torch
     from tractor_b200 import render

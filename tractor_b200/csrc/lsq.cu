@@ -607,29 +607,32 @@ chi2_kernel(const float* __restrict__ data, const float* __restrict__ model,
 // and lo, one 16-byte core-matrix row each in the canonical no-swizzle
 // K-major layout) and arrive on `full`; warp 8 issues the stage's 4 MMAs and
 // commits to `empty`.  Chunks of 128 rows alternate between two
-// accumulator sets (TMEM columns 0 and 128); the converters drain chunk c
-// after staging the first stage of chunk c + 1, whose MMAs wait until that
-// drain is done: TMEM loads that ran while MMAs into the other set were in
-// flight returned wrong values on B200 (two column layouts tried), so a drain
-// never overlaps an MMA.  A set holds two tiles (columns +0 and +64) that
-// take alternate K steps, so each FP32 accumulator takes 8 accumulations per
-// chunk: the tensor core's accumulation truncates, and its error grows with
-// that count.  A drain: the warps
-// holding E rows copy their 32 x 32 blocks to shared memory, a converter
-// barrier, then the warps holding S rows add S + E + E^T of their blocks on
-// or above the diagonal into compensated (Kahan) FP32 totals in shared
-// memory, and arrive on `accfree` (the set may be overwritten).  The FP64
-// results are written once at the end, AtA exactly symmetric.
+// accumulator sets (TMEM columns 0 and 128).  A set holds two tiles (columns
+// +0 and +64) that take alternate K steps, so each FP32 accumulator takes 8
+// accumulations per chunk: the tensor core's accumulation truncates, and its
+// error grows with that count.  Warps 9-12 drain a finished chunk (`accfull`):
+// they copy the accumulators to shared memory, release them (`accfree`) and
+// add S + E + E^T of the blocks on or above the diagonal to compensated
+// (Kahan) FP32 totals there.  The next chunk's MMAs wait for the release:
+// TMEM loads that ran while MMAs into the other set were in flight returned
+// wrong values on B200 (two column layouts tried).  The FP64 results are
+// written once at the end, AtA exactly symmetric.
+//
+// Bound: the converters' instructions and the hand-over of each stage (about
+// 600 ns alone, 470 with two CTAs per SM), against a third of that for the
+// reads from HBM.  With the drains done by the converters between stages (1.5
+// us each) 512 problems of 63 parameters x 16384 rows took 1180 us, now 961;
+// one such problem 464, 314; 1200 of 20 parameters 2137, 1508; 512 x 4099 rows
+// (4-byte copies) 393, 350.  Loading to registers in place of the ring was
+// slower (1266).
 // ---------------------------------------------------------------------------
 namespace tc64 {
 constexpr int kConv = 256;                 // converter threads
-constexpr int kThreads = kConv + 32;       // + the MMA warp
+constexpr int kDrain = 128;                // drain threads
+constexpr int kThreads = kConv + 32 + kDrain;
 constexpr int kKc = 32;                    // pixel rows per stage
 constexpr int kChunkSt = 4;                // stages per 128-row accumulation chunk
-#ifndef TB_NE64_RAW
-#define TB_NE64_RAW 3
-#endif
-constexpr int kRaw = TB_NE64_RAW;          // raw stages in flight
+constexpr int kRaw = 2;                    // raw stages in flight (3: the same times)
 constexpr int kKq = kKc / 4;               // quads per operand row and stage
 constexpr int kRowStep = kConv / kKq;      // operand rows between a thread's quads
 constexpr int kQpt = 64 / kRowStep;        // quads per thread and stage (64 x 32 / 4 / 256)
@@ -638,8 +641,10 @@ constexpr int kCbuf = 16512;               // kKc / 4 chunks of kLbo bytes, MMA 
 constexpr int kRawBytes = kRaw * kQpt * kConv * 16;
 constexpr int kEsLd = 65;                  // E staging row stride (floats)
 constexpr int kEsBytes = 64 * kEsLd * 4;
-constexpr int kTotBytes = 3 * 2 * 32 * 32 * 4;   // T, C of blocks (0,0), (0,1), (1,1)
-constexpr int kBarOff = kRawBytes + 2 * kCbuf + kEsBytes + kTotBytes;
+constexpr int kBlk = 32 * 32;                    // blocks (0,0), (0,1), (1,1) of S
+constexpr int kTotBytes = 3 * 2 * kBlk * 4;      // (T, C)
+constexpr int kSsBytes = 3 * kBlk * 4;           // S staging
+constexpr int kBarOff = kRawBytes + 2 * kCbuf + kEsBytes + kTotBytes + kSsBytes;
 constexpr int kSmem = kBarOff + 128;
 constexpr uint32_t kTmemCols = 256;
 constexpr uint64_t kWaitNs = 1000000000ull;
@@ -648,8 +653,8 @@ static_assert((kKc / 4 - 1) * kLbo + 2048 <= kCbuf, "MMA reads stay inside the o
 static_assert(kSmem + 1024 > 232448 / 3 && 2 * (kSmem + 1024) <= 232448, "two CTAs per SM");
 }  // namespace tc64
 
-__device__ __forceinline__ void conv_barrier() {
-    asm volatile("bar.sync 1, 256;" ::: "memory");
+__device__ __forceinline__ void drain_barrier() {
+    asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
 __global__ void __launch_bounds__(tc64::kThreads, 2)
@@ -663,13 +668,15 @@ normal_eq_tc64_kernel(const float* __restrict__ A, const float* __restrict__ rhs
     float4* raw = reinterpret_cast<float4*>(smem);
     unsigned char* cbuf = smem + kRawBytes;
     float* Es = reinterpret_cast<float*>(smem + kRawBytes + 2 * kCbuf);
-    float* tot = reinterpret_cast<float*>(smem + kRawBytes + 2 * kCbuf + kEsBytes);
+    float2* tot = reinterpret_cast<float2*>(smem + kRawBytes + 2 * kCbuf + kEsBytes);   // (T, C)
+    float* Ss = reinterpret_cast<float*>(smem + kRawBytes + 2 * kCbuf + kEsBytes + kTotBytes);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kBarOff);
     uint64_t* full = bar;          // [2] converters -> MMA warp: operand buffer written
     uint64_t* empty = bar + 2;     // [2] MMA warp -> converters: the stage's MMAs completed
-    uint64_t* accfree = bar + 4;   // [2] converters -> MMA warp: accumulator set drained
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 6);
-    int* flag = reinterpret_cast<int*>(bar + 7);   // a wait timed out
+    uint64_t* accfull = bar + 4;   // [2] MMA warp -> drain warps: a chunk's MMAs completed
+    uint64_t* accfree = bar + 6;   // [2] drain warps -> MMA warp: accumulator set read
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 8);
+    int* flag = reinterpret_cast<int*>(bar + 9);   // a wait timed out
 
     const int b = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -693,9 +700,10 @@ normal_eq_tc64_kernel(const float* __restrict__ A, const float* __restrict__ rhs
     if (warp == 0) tmem_alloc(tslot, kTmemCols);
     if (tid == 0) {
         for (int i = 0; i < 2; i++) {
-            mbar_init(&full[i], kConv);
+            mbar_init(&full[i], kConv / 32);   // (one arrival per warp)
             mbar_init(&empty[i], 1);
-            mbar_init(&accfree[i], kConv);
+            mbar_init(&accfull[i], 1);
+            mbar_init(&accfree[i], kDrain / 32);
         }
         *flag = 0;
     }
@@ -732,6 +740,7 @@ normal_eq_tc64_kernel(const float* __restrict__ A, const float* __restrict__ rhs
                     atomicExch(flag, 1);
                 }
                 commit(&empty[bi]);   // in every case: no converter waits on a stage never committed
+                if (s % kChunkSt == kChunkSt - 1 || s == nst - 1) commit(&accfull[c & 1]);
                 last = s;
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -741,10 +750,88 @@ normal_eq_tc64_kernel(const float* __restrict__ A, const float* __restrict__ rhs
         if (lane == 0 && last >= 0 && !mbar_wait(&empty[last & 1], (last >> 1) & 1, kWaitNs))
             atomicExch(flag, 1);
         __syncwarp();
-    } else {
-        // ---------------- converter warps ----------------
+    } else if (warp > 8) {
+        // ---------------- drain warps ----------------
+        // Each reads its TMEM lane quarter of a finished chunk into shared
+        // memory (rows 0-63 S, 64-127 E) and releases the accumulators; then
+        // the four add S + E + E^T of the blocks on or above the diagonal to
+        // the compensated (Kahan) totals.  After a wait has timed out the
+        // reads are left out (the values then are garbage, the outputs NaN).
         const int q = warp & 3;                       // TMEM lane quarter
         const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
+        const int r0 = (q & 1) * 32;                  // first row of S or E
+        const int w4 = warp - 9;
+        const int nch = (nst + kChunkSt - 1) / kChunkSt;
+        bool fail = false;
+        for (int c = 0; c < nch; c++) {
+            if (!fail && !__all_sync(0xffffffffu, mbar_wait(&accfull[c & 1], (c >> 1) & 1, kWaitNs)))
+                fail = true;
+            if (!fail) {
+                fence_after_sync();
+                const uint32_t d = tbase + (uint32_t)(128 * (c & 1)) + lane_sel;
+#pragma unroll
+                for (int j0 = 0; j0 < 64; j0 += 16) {
+                    if (j0 >= N || r0 >= Q || (q < 2 && j0 < r0)) continue;
+                    float v[16], v2[16];
+                    tmem_ld16(d + j0, v);
+                    tmem_ld16(d + 64 + j0, v2);
+                    if (q >= 2) {
+#pragma unroll
+                        for (int jj = 0; jj < 16; jj++)
+                            Es[(r0 + lane) * kEsLd + j0 + jj] = v[jj] + v2[jj];
+                    } else {
+                        float* S = Ss + ((j0 + r0) / 32) * kBlk + (j0 % 32) * 32 + lane;
+#pragma unroll
+                        for (int jj = 0; jj < 16; jj++) S[jj * 32] = v[jj] + v2[jj];
+                    }
+                }
+                fence_before_sync();
+            }
+            __syncwarp();
+            if (lane == 0) tb::tc::mbar_arrive(&accfree[c & 1]);
+            drain_barrier();   // the staged values are complete
+            for (int blk = 0; blk < 3; blk++) {
+                const int I = blk >> 1, J = (blk + 1) >> 1;   // (0,0), (0,1), (1,1)
+                if (I * 32 >= P || J * 32 > P) continue;
+                const int i = I * 32 + lane;
+#pragma unroll
+                for (int t = 0; t < 8; t++) {
+                    const int jj = w4 + 4 * t, j = J * 32 + jj;
+                    const int at = blk * kBlk + jj * 32 + lane;
+                    const float x = Ss[at] + (Es[i * kEsLd + j] + Es[j * kEsLd + i]);
+                    const float2 tc = c == 0 ? make_float2(0.f, 0.f) : tot[at];
+                    const float y = x - tc.y;
+                    const float tn = tc.x + y;
+                    tot[at] = make_float2(tn, (tn - tc.x) - y);
+                }
+            }
+            drain_barrier();   // the staged values are read
+        }
+        if (fail) {
+            if (lane == 0) atomicExch(flag, 1);
+        } else {
+            // FP64 results from the compensated totals (each thread its own):
+            // D[i][j], i <= j <= P
+            for (int blk = 0; blk < 3; blk++) {
+                const int I = blk >> 1, J = (blk + 1) >> 1;
+                const int i = I * 32 + lane;
+                if (i >= P) continue;
+                for (int jj = w4; jj < 32; jj += 4) {
+                    const int j = J * 32 + jj;
+                    if (j < i || j > P) continue;
+                    const float2 tc = tot[blk * kBlk + jj * 32 + lane];
+                    const double x = (double)tc.x - (double)tc.y;
+                    if (j == P) {
+                        g[i] = x;
+                    } else {
+                        M[(int64_t)j * P + i] = x;
+                        M[(int64_t)i * P + j] = x;
+                    }
+                }
+            }
+        }
+    } else {
+        // ---------------- converter warps ----------------
         const uint32_t raw_base = smem_u32(raw);
         // this thread's quads: pixel rows k .. k + 3 of operand rows
         // c0 + kRowStep m
@@ -775,64 +862,6 @@ normal_eq_tc64_kernel(const float* __restrict__ A, const float* __restrict__ rhs
             }
             cp_async_commit();
         };
-        int drains = 0;
-        // Drain of chunk `drains` (accumulator set drains & 1), last stage
-        // s_last.  Every converter thread runs every drain and its barrier in
-        // the same order, also after a wait has timed out (`skip`: the waits
-        // are left out, the values then are garbage and the outputs NaN).
-        auto drain = [&](int s_last, bool skip) -> bool {
-            const bool ok = __all_sync(
-                0xffffffffu, !skip && mbar_wait(&empty[s_last & 1], (s_last >> 1) & 1, kWaitNs));
-            const uint32_t d = tbase + (uint32_t)(128 * (drains & 1));
-            const int cb = warp >> 2;                  // 32-column block
-            if (ok) {
-                fence_after_sync();
-                // E rows (q - 2) * 32 .. + 31 of this column block -> shared memory
-                const int e0 = (q - 2) * 32;
-                if (q >= 2 && e0 < Q && cb * 32 < N) {
-                    float v[32], v2[32];
-                    tmem_ld32(d + cb * 32 + lane_sel, v);
-                    tmem_ld32(d + 64 + cb * 32 + lane_sel, v2);
-#pragma unroll
-                    for (int jj = 0; jj < 32; jj++)
-                        Es[(e0 + lane) * kEsLd + cb * 32 + jj] = v[jj] + v2[jj];
-                }
-            }
-            conv_barrier();
-            if (ok && q < 2 && cb >= q && q * 32 < P && cb * 32 <= P) {
-                // S block (I = q, J = cb) on or above the diagonal: T, C += S + E + E^T
-                float v[32], v2[32];
-                tmem_ld32(d + cb * 32 + lane_sel, v);
-                tmem_ld32(d + 64 + cb * 32 + lane_sel, v2);
-#pragma unroll
-                for (int jj = 0; jj < 32; jj++) v[jj] += v2[jj];
-                const int i = q * 32 + lane;
-                float* Tt = tot + (q + cb) * 2 * 1024;    // blocks (0,0) 0, (0,1) 1, (1,1) 2
-                float* Cc = Tt + 1024;
-#pragma unroll 8
-                for (int jj = 0; jj < 32; jj++) {
-                    const int j = cb * 32 + jj;
-                    const float x = v[jj] + (Es[i * kEsLd + j] + Es[j * kEsLd + i]);
-                    if (drains == 0) {
-                        Tt[jj * 32 + lane] = x;
-                        Cc[jj * 32 + lane] = 0.f;
-                    } else {
-                        const float t0 = Tt[jj * 32 + lane], c0v = Cc[jj * 32 + lane];
-                        const float y = x - c0v;
-                        const float t = t0 + y;
-                        Cc[jj * 32 + lane] = (t - t0) - y;
-                        Tt[jj * 32 + lane] = t;
-                    }
-                }
-            }
-            // the E block copies are read by other warps: no warp refills Es
-            // before every S warp has read it (the next drain needs the next
-            // chunk, whose stages need every converter's arrival)
-            fence_before_sync();
-            tb::tc::mbar_arrive(&accfree[drains & 1]);
-            drains++;
-            return ok;
-        };
         bool fail = false;
         for (int s = 0; s < kRaw - 1; s++) issue(s);
         for (int s = 0; s < nst; s++) {
@@ -856,35 +885,11 @@ normal_eq_tc64_kernel(const float* __restrict__ A, const float* __restrict__ rhs
                 *reinterpret_cast<float4*>(buf + soff[m] + 1024) = l;   // row 64 + c
             }
             fence_async_smem();
-            tb::tc::mbar_arrive(&full[bi]);
-            // the previous chunk's accumulators, while this chunk is multiplied
-            if (s % kChunkSt == 0 && s > 0 && !drain(s - 1, fail)) fail = true;
+            __syncwarp();
+            if (lane == 0) tb::tc::mbar_arrive(&full[bi]);
         }
         cp_async_wait<0>();
-        if (!drain(nst - 1, fail)) fail = true;
         if (fail) atomicExch(flag, 1);
-        conv_barrier();
-        // FP64 results from the compensated totals: D[i][j], i <= j <= P
-        const int cb = warp >> 2;
-        if (!fail && !*reinterpret_cast<volatile int*>(flag) && q < 2 && cb >= q && q * 32 < P &&
-            cb * 32 <= P) {
-            const int i = q * 32 + lane;
-            const float* Tt = tot + (q + cb) * 2 * 1024;
-            const float* Cc = Tt + 1024;
-            if (i < P) {
-                for (int jj = 0; jj < 32; jj++) {
-                    const int j = cb * 32 + jj;
-                    if (j < i || j > P) continue;
-                    const double x = (double)Tt[jj * 32 + lane] - (double)Cc[jj * 32 + lane];
-                    if (j == P) {
-                        g[i] = x;
-                    } else {
-                        M[(int64_t)j * P + i] = x;
-                        M[(int64_t)i * P + j] = x;
-                    }
-                }
-            }
-        }
     }
     __syncthreads();
     if (*reinterpret_cast<volatile int*>(flag)) {
