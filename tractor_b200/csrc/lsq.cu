@@ -602,10 +602,10 @@ chi2_kernel(const float* __restrict__ data, const float* __restrict__ model,
 // and the B operand its hi rows, so ONE kind::tf32 MMA of M = 128 per K = 8
 // step gives S = Hi Hi^T (D rows 0-63) and E = Lo Hi^T (D rows 64-127);
 // D = S + E + E^T, the cross terms symmetrised when the accumulators are
-// drained.  Warps 0-7 (converters) stage KC = 32 pixel rows per stage (4-
-// or 16-byte cp.async into their own slots of a raw ring, split into TF32 hi
-// and lo, one 16-byte core-matrix row each in the canonical no-swizzle
-// K-major layout) and arrive on `full`; warp 8 issues the stage's 4 MMAs and
+// drained.  Warps 0-7 (converters) stage KC = 32 pixel rows per stage (loaded
+// to registers two stages ahead, 16 bytes at a time where the columns are
+// aligned, split into TF32 hi and lo, one 16-byte core-matrix row each in the
+// canonical no-swizzle K-major layout) and arrive on `full`; warp 8 issues the stage's 4 MMAs and
 // commits to `empty`.  Chunks of 128 rows alternate between two
 // accumulator sets (TMEM columns 0 and 128).  A set holds two tiles (columns
 // +0 and +64) that take alternate K steps, so each FP32 accumulator takes 8
@@ -618,13 +618,14 @@ chi2_kernel(const float* __restrict__ data, const float* __restrict__ model,
 // wrong values on B200 (two column layouts tried).  The FP64 results are
 // written once at the end, AtA exactly symmetric.
 //
-// Bound: the converters' instructions and the hand-over of each stage (about
-// 600 ns alone, 470 with two CTAs per SM), against a third of that for the
-// reads from HBM.  With the drains done by the converters between stages (1.5
-// us each) 512 problems of 63 parameters x 16384 rows took 1180 us, now 961;
-// one such problem 464, 314; 1200 of 20 parameters 2137, 1508; 512 x 4099 rows
-// (4-byte copies) 393, 350.  Loading to registers in place of the ring was
-// slower (1266).
+// Bound: the shared-memory traffic of the operands (82 % of L1's throughput
+// when the loads also went through it) and the hand-over of each stage; the
+// reads from HBM take 331 of the 830 us below.  512 problems of 63 parameters
+// x 16384 rows: 1180 us with the drains done by the converters between stages
+// (1.5 us each), 961 with drain warps, 830 with the loads kept in registers
+// in place of a cp.async ring in shared memory; one such problem 464, 314,
+// 297; 1200 of 20 parameters 2137, 1508, 1403; 512 x 4099 rows (4-byte loads)
+// 393, 350, 249.  A third operand buffer and more stages ahead change nothing.
 // ---------------------------------------------------------------------------
 namespace tc64 {
 constexpr int kConv = 256;                 // converter threads
@@ -632,19 +633,18 @@ constexpr int kDrain = 128;                // drain threads
 constexpr int kThreads = kConv + 32 + kDrain;
 constexpr int kKc = 32;                    // pixel rows per stage
 constexpr int kChunkSt = 4;                // stages per 128-row accumulation chunk
-constexpr int kRaw = 2;                    // raw stages in flight (3: the same times)
+constexpr int kAhead = 2;                  // stages loaded ahead, in registers
 constexpr int kKq = kKc / 4;               // quads per operand row and stage
 constexpr int kRowStep = kConv / kKq;      // operand rows between a thread's quads
 constexpr int kQpt = 64 / kRowStep;        // quads per thread and stage (64 x 32 / 4 / 256)
 constexpr int kLbo = 128 / 8 * 128 + 16;   // bytes between K chunks (128 stacked rows)
 constexpr int kCbuf = 16512;               // kKc / 4 chunks of kLbo bytes, MMA over-read included
-constexpr int kRawBytes = kRaw * kQpt * kConv * 16;
 constexpr int kEsLd = 65;                  // E staging row stride (floats)
 constexpr int kEsBytes = 64 * kEsLd * 4;
 constexpr int kBlk = 32 * 32;                    // blocks (0,0), (0,1), (1,1) of S
 constexpr int kTotBytes = 3 * 2 * kBlk * 4;      // (T, C)
 constexpr int kSsBytes = 3 * kBlk * 4;           // S staging
-constexpr int kBarOff = kRawBytes + 2 * kCbuf + kEsBytes + kTotBytes + kSsBytes;
+constexpr int kBarOff = 2 * kCbuf + kEsBytes + kTotBytes + kSsBytes;
 constexpr int kSmem = kBarOff + 128;
 constexpr uint32_t kTmemCols = 256;
 constexpr uint64_t kWaitNs = 1000000000ull;
@@ -665,11 +665,10 @@ normal_eq_tc64_kernel(const float* __restrict__ A, const float* __restrict__ rhs
     using namespace tb::tc;
     using namespace tc64;
     extern __shared__ __align__(128) unsigned char smem[];
-    float4* raw = reinterpret_cast<float4*>(smem);
-    unsigned char* cbuf = smem + kRawBytes;
-    float* Es = reinterpret_cast<float*>(smem + kRawBytes + 2 * kCbuf);
-    float2* tot = reinterpret_cast<float2*>(smem + kRawBytes + 2 * kCbuf + kEsBytes);   // (T, C)
-    float* Ss = reinterpret_cast<float*>(smem + kRawBytes + 2 * kCbuf + kEsBytes + kTotBytes);
+    unsigned char* cbuf = smem;
+    float* Es = reinterpret_cast<float*>(smem + 2 * kCbuf);
+    float2* tot = reinterpret_cast<float2*>(smem + 2 * kCbuf + kEsBytes);   // (T, C)
+    float* Ss = reinterpret_cast<float*>(smem + 2 * kCbuf + kEsBytes + kTotBytes);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kBarOff);
     uint64_t* full = bar;          // [2] converters -> MMA warp: operand buffer written
     uint64_t* empty = bar + 2;     // [2] MMA warp -> converters: the stage's MMAs completed
@@ -832,7 +831,6 @@ normal_eq_tc64_kernel(const float* __restrict__ A, const float* __restrict__ rhs
         }
     } else {
         // ---------------- converter warps ----------------
-        const uint32_t raw_base = smem_u32(raw);
         // this thread's quads: pixel rows k .. k + 3 of operand rows
         // c0 + kRowStep m
         const int k = 4 * (tid % kKq), c0 = tid / kKq;
@@ -844,51 +842,56 @@ normal_eq_tc64_kernel(const float* __restrict__ A, const float* __restrict__ rhs
             src[m] = c < Q ? (c < P ? Ab + (int64_t)c * ld : rb) + k : nullptr;
             soff[m] = (k >> 2) * kLbo + (c >> 3) * 128 + (c & 7) * 16;
         }
-        auto issue = [&](int s) {
-            const int slot = s % kRaw;
-            const int row = s * kKc + k;
-            const int nv = s < nst ? min(max(R - row, 0), 4) : 0;
+        // stage s of this thread's quads, 0 beyond the last row
+        auto load = [&](int s, float4 (&v)[kQpt]) {
+            const int nv = s < nst ? R - (s * kKc + k) : 0;
 #pragma unroll
             for (int m = 0; m < kQpt; m++) {
-                if (src[m] == nullptr || s >= nst) continue;
-                const uint32_t dst = raw_base + 16 * ((slot * kQpt + m) * kConv + tid);
+                v[m] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (src[m] == nullptr || nv <= 0) continue;
                 const float* p = src[m] + (int64_t)s * kKc;
-                if (vec) {
-                    cp_async16(dst, nv > 0 ? p : Ab, 4 * nv);
+                if (vec && nv >= 4) {
+                    v[m] = __ldg(reinterpret_cast<const float4*>(p));
                 } else {
-#pragma unroll
-                    for (int j = 0; j < 4; j++) cp_async4(dst + 4 * j, j < nv ? p + j : Ab, j < nv);
+                    v[m].x = __ldg(p);
+                    if (nv > 1) v[m].y = __ldg(p + 1);
+                    if (nv > 2) v[m].z = __ldg(p + 2);
+                    if (nv > 3) v[m].w = __ldg(p + 3);
                 }
             }
-            cp_async_commit();
         };
         bool fail = false;
-        for (int s = 0; s < kRaw - 1; s++) issue(s);
-        for (int s = 0; s < nst; s++) {
-            issue(s + kRaw - 1);
-            cp_async_wait<kRaw - 1>();    // this thread's copies of stage s have landed
-            const int bi = s & 1;
-            unsigned char* buf = cbuf + bi * kCbuf;
-            // operand buffer bi is free once the MMAs of stage s - 2 have completed
-            if (s >= 2 && !fail && !mbar_wait(&empty[bi], ((s >> 1) - 1) & 1, kWaitNs)) fail = true;
-            const int slot = s % kRaw;
+        float4 ahead[kAhead][kQpt];
 #pragma unroll
-            for (int m = 0; m < kQpt; m++) {
-                if (src[m] == nullptr) continue;
-                const float4 v = raw[(slot * kQpt + m) * kConv + tid];
-                float4 h, l;
-                split_tf32(v.x, h.x, l.x);
-                split_tf32(v.y, h.y, l.y);
-                split_tf32(v.z, h.z, l.z);
-                split_tf32(v.w, h.w, l.w);
-                *reinterpret_cast<float4*>(buf + soff[m]) = h;          // row c
-                *reinterpret_cast<float4*>(buf + soff[m] + 1024) = l;   // row 64 + c
+        for (int s = 0; s < kAhead; s++) load(s, ahead[s]);
+        for (int s0 = 0; s0 < nst; s0 += kAhead) {
+#pragma unroll
+            for (int t = 0; t < kAhead; t++) {   // (the registers are known at compile time)
+                const int s = s0 + t;
+                if (s >= nst) break;
+                const int bi = s & 1;
+                unsigned char* buf = cbuf + bi * kCbuf;
+                // operand buffer bi is free once the MMAs of stage s - 2 have completed
+                if (s >= 2 && !fail && !mbar_wait(&empty[bi], ((s >> 1) - 1) & 1, kWaitNs))
+                    fail = true;
+#pragma unroll
+                for (int m = 0; m < kQpt; m++) {
+                    if (src[m] == nullptr) continue;
+                    const float4 v = ahead[t][m];
+                    float4 h, l;
+                    split_tf32(v.x, h.x, l.x);
+                    split_tf32(v.y, h.y, l.y);
+                    split_tf32(v.z, h.z, l.z);
+                    split_tf32(v.w, h.w, l.w);
+                    *reinterpret_cast<float4*>(buf + soff[m]) = h;          // row c
+                    *reinterpret_cast<float4*>(buf + soff[m] + 1024) = l;   // row 64 + c
+                }
+                load(s + kAhead, ahead[t]);
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) tb::tc::mbar_arrive(&full[bi]);
             }
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) tb::tc::mbar_arrive(&full[bi]);
         }
-        cp_async_wait<0>();
         if (fail) atomicExch(flag, 1);
     }
     __syncthreads();
