@@ -1507,7 +1507,8 @@ def main():
             e1.record(stream)
             R.fourier_render(items_t.data_ptr(), n, camp.data_ptr(), cvar.data_ptr(),
                              renderer.spec.data_ptr(), out.data_ptr(), misc.data_ptr() + 16,
-                             method=method)
+                             method=method,
+                             workspace=renderer._workspace(n) if method == 'split' else None)
         e2.record(stream)
     torch.cuda.synchronize()
     gpu_launches = ((0 if method == 'fused' else 1) + launches_per_render) * args.steps
