@@ -398,3 +398,29 @@ def test_c5_blobs_reach_the_fp64_optimum(tb, oracle):
     assert len(inner) >= 110 and len(other) <= 5, (len(inner), other)
     assert inner[0][0] < 1e-3, inner[:5]
     assert not other or other[0][0] < 0.1, other
+
+
+def test_blob_without_sources_keeps_to_its_own_slices(tb, oracle):
+    """A blob table entry with n_src = 0 (P = 0, slices of no elements) through
+    the passes of both precisions and the step: nothing outside its slices is
+    written (the word before them is its neighbour's accepted gradient), its
+    chi^2 is its weighted data's, and it stops at once."""
+    import torch
+    w, datas, inverrs = _small_blobs(oracle, 3, n_blobs=2)
+    f = _fitter(w, datas, inverrs)
+    f.blobs_np['n_src'][1] = f.blobs_np['P'][1] = 0
+    f.d_blobs.copy_(torch.from_numpy(f.blobs_np.view(np.uint8).copy()))
+    f.reset(w['start'])
+    ns, g0, u0 = (int(f.blobs_np[k][1]) for k in ('n_slices', 'g_off', 'unit0'))
+    chi2 = float(((datas[1].astype(np.float64) * inverrs[1]) ** 2).sum())
+    for refine in (False, True):
+        f.gbuf.fill_(-7.)
+        f._prep()
+        f._refine_pass() if refine else f._pass(0)
+        got = f.gbuf.cpu().numpy()
+        assert got[g0 - 1] == -7. and np.all(got[g0:] == -7.), refine
+        assert abs(float(f.chi2_part[u0:u0 + ns].sum()) - chi2) <= 1e-5 * chi2
+    f.reset(w['start'])
+    f._iteration(1e-3, 100)
+    st = f.states()
+    assert st['status'][1] == 1 and abs(st['chi2'][1] - chi2) <= 1e-5 * chi2

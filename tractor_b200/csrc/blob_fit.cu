@@ -662,7 +662,8 @@ fit_pass_kernel(const tb_fit_unit* __restrict__ units, const int32_t* __restrict
         if (mode == kEquations && state[u.blob].status != 0) continue;   // converged or stopped
         const int P = b.P;
         const int nsrc = b.n_src;
-        // checks, and the unit's sources into shared memory (lane = source)
+        // checks, and the unit's sources into shared memory (lane = source);
+        // a blob without sources is taken as any other (its slices hold nothing)
         if (warp == 0) {
             const bool unit_bad = nsrc < 0 || nsrc > TB_FIT_MAX_SRC || P != nsrc * TB_FIT_NPAR ||
                                   u.psf_K < 1 || u.psf_K > TB_FIT_MAX_PSF || u.band < 0 ||
@@ -793,7 +794,7 @@ fit_pass_kernel(const tb_fit_unit* __restrict__ units, const int32_t* __restrict
             for (int w2 = 0; w2 < kWarps; w2++) s += sm.red[w2];
             if (mode == kConstant) chi2_const[b.unit0 + u.slice] = s;
             else chi2_part[b.unit0 + u.slice] = s + (chi2_const ? chi2_const[b.unit0 + u.slice] : 0.0);
-            if (mode == kEquations)
+            if (mode == kEquations && P > 0)
                 pu.out.g[P - 1] = __longlong_as_double((long long)u.band << 32 | pu.out.mask);
         }
     }
