@@ -318,3 +318,30 @@ def test_mog_blob_adjoint_matches_fp64_central_differences(tb, oracle):
                     (i, j, got[i, j], fd, scale)
         # parameters a source does not have get zero gradient
     assert np.all(got[3, 5:] == 0)
+
+
+def test_blob_adjoint_of_a_bad_source_is_not_a_stale_one(tb):
+    """The gradient slices of a blob with a non-finite source: cleared, as those
+    of every other unit, and not what an earlier fit or gradient left there;
+    the launch reports the unit, the other blob's gradient is unchanged."""
+    import torch
+    from tractor_b200 import fit, grad
+    w = fit.blob_workload(2, np.random.default_rng(62), side_range=(44, 52), mean_src=2,
+                          max_src=2, flux_range=(500., 3000.))
+    npix = int(fit.pix_offsets(w['sides'], 3)[-1])
+    zeros = torch.zeros(npix, dtype=torch.float32, device='cuda')
+    f = fit.BlobFitter(w['blob_src'], w['sides'], w['psf'], w['sources'], w['truth'], zeros,
+                       torch.ones_like(zeros))
+    bm = grad.BlobModel(f)
+    G = torch.randn(npix, generator=torch.Generator(device='cuda').manual_seed(4), device='cuda')
+    theta = torch.tensor(w['truth'], dtype=torch.float64, device='cuda')
+    good = bm.vjp(theta, G)
+    s1 = int(w['blob_src'][1])
+    assert torch.all(good[s1:, 2] != 0)
+    theta[s1, 0] = float('nan')
+    with pytest.raises(RuntimeError):
+        bm.vjp(theta, G)
+    ext = torch.cat([f.gbuf, torch.zeros(1, dtype=torch.float64, device='cuda')])
+    got = ext[bm._idx].sum(dim=1).view(-1, 9)
+    assert torch.all(got[s1:] == 0)
+    assert torch.equal(got[:s1], good[:s1])

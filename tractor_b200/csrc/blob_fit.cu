@@ -694,12 +694,16 @@ fit_pass_kernel(const tb_fit_unit* __restrict__ units, const int32_t* __restrict
             }
             const bool bad = unit_bad || __any_sync(0xffffffffu, src_bad);
             if (lane == 0) {
-                sm.skip = bad;
+                sm.skip = unit_bad ? 1 : bad ? -1 : 0;   // -1: its slice is its own
                 if (bad) tb::report(st, TB_STATUS_BAD_ITEM, ui, nsrc);
             }
         }
         __syncthreads();
         if (sm.skip) {
+            // (a gradient is summed over every slice, whatever the status says)
+            if (mode == kVjp && sm.skip < 0)
+                for (int e = tid; e < P; e += kThreads)
+                    gbuf[b.g_off + (int64_t)u.slice * P + e] = 0.0;
             if (tid == 0) {
                 if (mode == kConstant) chi2_const[b.unit0 + u.slice] = INFINITY;
                 else if (mode == kEquations) chi2_part[b.unit0 + u.slice] = INFINITY;
