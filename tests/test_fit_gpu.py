@@ -424,3 +424,29 @@ def test_blob_without_sources_keeps_to_its_own_slices(tb, oracle):
     f._iteration(1e-3, 100)
     st = f.states()
     assert st['status'][1] == 1 and abs(st['chi2'][1] - chi2) <= 1e-5 * chi2
+
+
+def test_blobs_with_an_undetermined_parameter_do_not_crawl(tb):
+    """Two of 2,000 blobs, from where the FP32 iterations left them
+    (golden/slow_blobs.npz): each holds a source whose shape is all but
+    undetermined, and its step, beyond its limit by up to 1e5, scaled the steps
+    of all the others; the FP64 iterations took 97 and more than 100 (4.9 sigma
+    from the optimum).  Within 80 they converge to less than 1e-3 sigma from
+    the FP64 optimum, as every other blob."""
+    import os
+    import torch
+    from tractor_b200 import fit, plain
+    z = np.load(os.path.join(os.path.dirname(__file__), 'golden', 'slow_blobs.npz'))
+    w = fit.blob_workload(2000, np.random.default_rng(3000))
+    data, inv = fit.render_blobs(w, w['truth'], seed=3001)
+    po = fit.pix_offsets(w['sides'], 3)
+    cut = [slice(int(po[3 * b]), int(po[3 * b + 3])) for b in z['blobs']]
+    data, inv = (torch.cat([a[c] for c in cut]) for a in (data, inv))
+    w = fit.subset_workload(w, z['blobs'])
+    f = fit.BlobFitter(w['blob_src'], w['sides'], w['psf'], w['sources'], z['start'], data, inv)
+    f.fit(params0=z['start'], max_iter=0, graph=False, refine_iter=80)
+    st = f.states()
+    assert np.all(st['status'] == 1), (st['status'], st['iters'])
+    for sigma, b, _, _, converged in plain.optimum_distance(w, data, inv, f.result(), st['status'],
+                                                            [0, 1], f.dev):
+        assert converged and sigma < 1e-3, (b, sigma)

@@ -921,11 +921,19 @@ fit_assemble_kernel(const tb_fit_blob* __restrict__ blobs,
 
 constexpr int kStepMaxP = TB_FIT_MAX_SRC * TB_FIT_NPAR;
 constexpr int kStepSharedP = 128;      // largest padded size factored in shared memory
-constexpr int kStepSmem = 8 * (tb::packed_size(kStepSharedP) + 5 * kStepSharedP);   // 71 KB
-static_assert(kStepSmem >= 8 * 5 * ((kStepMaxP + 7) / 8 * 8), "the vectors always fit");
+constexpr int kStepSmem = 8 * (tb::packed_size(kStepSharedP) + 7 * kStepSharedP);   // 73 KB
+static_assert(kStepSmem >= 8 * 7 * ((kStepMaxP + 7) / 8 * 8), "the vectors always fit");
+static_assert(3 * (kStepSmem + 2048) <= 228 * 1024, "three blobs per SM");
+
+// Where the whole step would be scaled below kLimited of it, the parameters
+// beyond their limits are held there and the others solved again, kBoxRounds
+// times at most; in iterations after kPatience.
+constexpr double kLimited = 0.5;
+constexpr int kBoxRounds = 8;
+constexpr int kPatience = 8;
 
 // One CTA per blob.  Up to 128 parameters the factor lives in shared memory
-// (71 KB, three blobs per SM), above in the blob's global area.
+// (73 KB, three blobs per SM), above in the blob's global area.
 //
 // Bound: the chain of columns.  A column at a time through L2, one barrier
 // each, took 0.6 ms for 126 parameters; four columns at a time (every thread
@@ -934,6 +942,17 @@ static_assert(kStepSmem >= 8 * 5 * ((kStepMaxP + 7) / 8 * 8), "the vectors alway
 // is two barriers per four columns and 256 multiply-adds per instruction.
 // Kernel time per step: 126 parameters 615 -> 175 us (with the assembly), 36
 // parameters 87 -> 29 us.
+//
+// The step is scaled as a whole to its limits (ConstrainedOptimizer), so one
+// all but undetermined parameter (the shape of a source a tenth of a pixel wide)
+// can cut the step of all the others to 1e-5 of it, one iteration after the
+// other: such a blob took 97 iterations, others, thousands of units of chi^2
+// from their optimum, reached the limit of 100.  A blob that is still running
+// after kPatience iterations therefore takes, where the quadratic model expects
+// more of it, the step that minimises the model within the limits (each
+// parameter beyond its limit held there, the others solved for): 26 iterations
+// for the first, 12 to 50 for the others.  Most blobs stop before, and their
+// steps are what they were.
 __global__ void __launch_bounds__(kStepThreads, 3)
 fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
                 const tb_fit_source* __restrict__ srcs, double* __restrict__ params,
@@ -942,7 +961,7 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
                 double tol, int max_iter) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double red[kStepThreads / 32], red2[kStepThreads / 32];
-    __shared__ int s_active, s_accept;
+    __shared__ int s_active, s_accept, s_slow;
     __shared__ double s_lambda, s_scale, s_pa, s_pb;
     const int bi = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -961,8 +980,10 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
     double* y = dinv + n;
     double* xs = y + n;
     double* rdg = xs + n;
+    double* gm = rdg + n;      // gradient, with the held parameters at their limits
+    double* held = gm + n;     // their steps; 0 for the others
     double* Ha = hbuf + b.h_off + (int64_t)ns * P * P;   // accepted H
-    double* L = n <= kStepSharedP ? rdg + n : Ha + (int64_t)P * P;   // factor
+    double* L = n <= kStepSharedP ? held + n : Ha + (int64_t)P * P;   // factor
     double* ga = gbuf + b.g_off + (int64_t)ns * P;
     double* pa = params + (int64_t)b.src0 * TB_FIT_NPAR;
     double* pt = trial + (int64_t)b.src0 * TB_FIT_NPAR;
@@ -996,6 +1017,7 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
         if (status == 0 && S.iters >= max_iter) status = 3;
         s_accept = acc;
         s_lambda = S.lambda;
+        s_slow = S.iters > kPatience;
         s_active = status == 0;
         S.status = status;
     }
@@ -1025,148 +1047,211 @@ fit_step_kernel(const tb_fit_blob* __restrict__ blobs, int n_blobs, int n_bands,
         if ((srcs[b.src0 + i / TB_FIT_NPAR].frozen >> (i % TB_FIT_NPAR)) & 1) d = 0.0;
         dsc[i] = d;
         dinv[i] = d == 0.0 ? 0.0 : 1.0 / d;
+        gm[i] = ga[i];
+        held[i] = 0.0;
     }
     for (int i = P + tid; i < n; i += kStepThreads) dinv[i] = dsc[i] = 0.0;
     __syncthreads();
-    // LDL^T of the scaled matrix, right-looking: column k is left as d_k
-    // (diagonal) and c_ik = d_k l_ik below it, and subtracts c_ik c_jk / d_k
-    // from the trailing columns.
-    for (int j0 = 0; j0 < n; j0 += kStepThreads / 32) {
-        const int j = j0 + warp;
-        const double dj = dinv[j];
-#pragma unroll 4
-        for (int i = j + lane; i < n; i += 32) {
-            const double h = i < P ? Ha[(int64_t)j * P + i] : 0.0;   // (j <= i)
-            const bool live = dinv[i] != 0.0 && dj != 0.0;
-            col(j)[i] = live ? h * dinv[i] * dj + (i == j ? lam : 0.0) : (i == j ? 1.0 : 0.0);
-        }
-    }
-    __syncthreads();
-    const bool bad = tb::ldl_factor<kStepThreads>(L, rdg, n) != 0;
-    if (bad) {
-        // not positive definite: treat as a rejected step with more damping
-        if (tid == 0) {
-            S.lambda *= 10.0;
-            if (!(S.lambda < 1e12)) S.status = 2;
-        }
-        for (int e = tid; e < P; e += kStepThreads) pt[e] = pa[e];
-        return;
-    }
-    for (int i = tid; i < n; i += kStepThreads) {
-        xs[i] = 0.0;
-        y[i] = i < P ? ga[i] * dinv[i] : 0.0;
-    }
-    __syncthreads();
-    // solution and one refinement step
-    for (int pass = 0; pass < 2; pass++) {
-        if (pass == 1) {
-            // residual, four rows of a warp at a time (Ha is symmetric)
-            for (int i0 = 4 * warp; i0 < P; i0 += 4 * (kStepThreads / 32)) {
-                double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    // take(i, sum_j H_ij value(j)) for every row i by one thread each, four rows
+    // of a warp at a time (Ha is symmetric); elements of columns whose value is
+    // 0 are not used
+    auto rows_of_H = [&](auto value, auto take) {
+        for (int i0 = 4 * warp; i0 < P; i0 += 4 * (kStepThreads / 32)) {
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 2
-                for (int j = lane; j < P; j += 32) {
-                    const bool live = dinv[j] != 0.0;
-                    const double xj = dinv[j] * xs[j];
-#pragma unroll
-                    for (int t = 0; t < 4; t++) {
-                        const double h = i0 + t < P ? Ha[(int64_t)(i0 + t) * P + j] : 0.0;
-                        acc[t] = fma(live ? h : 0.0, xj, acc[t]);
-                    }
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                    for (int t = 0; t < 4; t++) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], o);
+            for (int j = lane; j < P; j += 32) {
+                const double vj = value(j);
 #pragma unroll
                 for (int t = 0; t < 4; t++) {
-                    const int i = i0 + t;
-                    if (lane == t && i < P)
-                        y[i] = dinv[i] != 0.0 ? ga[i] * dinv[i] - (acc[t] * dinv[i] + lam * xs[i])
-                                              : -xs[i];
+                    const double h = i0 + t < P ? Ha[(int64_t)(i0 + t) * P + j] : 0.0;
+                    acc[t] = fma(vj != 0.0 ? h : 0.0, vj, acc[t]);
                 }
             }
-            __syncthreads();
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int t = 0; t < 4; t++) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], o);
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+                if (lane == t && i0 + t < P) take(i0 + t, acc[t]);
         }
-        if (warp == 0) tb::ldl_solve(L, rdg, y, n);
-        __syncthreads();
-        for (int i = tid; i < P; i += kStepThreads) xs[i] += y[i];
-        __syncthreads();
-    }
-    // Predicted log-likelihood gain of this damped step,
-    // 1/2 (x . D^-1 g + lambda x . x); the blob has converged when it is below
-    // tol while the damping is moderate (optimize_loop stops on the gain of
-    // the last step, dchisq; the prediction is immune to FP32 noise in chi^2).
-    {
-        // a = x^T y0, b = x^T x: the gain predicted for the step is
-        // (a + lambda b) / 2, for the step scaled by s it is
-        // s a - s^2 (a - lambda b) / 2
-        double pa_ = 0.0, pb_ = 0.0;
+    };
+    // the parameters a multiple of the step y away
+    auto write_trial = [&](double scale) {
         for (int i = tid; i < P; i += kStepThreads) {
-            const double y0 = dsc[i] == 0.0 ? 0.0 : ga[i] / dsc[i];
-            pa_ += xs[i] * y0;
-            pb_ += xs[i] * xs[i];
+            double v = pa[i] + scale * y[i];
+            if (i % TB_FIT_NPAR == TB_FIT_NPAR - 1 &&
+                srcs[b.src0 + i / TB_FIT_NPAR].profile == TB_PROFILE_SERSIC)
+                v = fmin(fmax(v, TB_FIT_SERSIC_MIN), TB_FIT_SERSIC_MAX);
+            pt[i] = v;
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            pa_ += __shfl_xor_sync(0xffffffffu, pa_, o);
-            pb_ += __shfl_xor_sync(0xffffffffu, pb_, o);
-        }
-        if (lane == 0) {
-            red[warp] = pa_;
-            red2[warp] = pb_;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double ta = 0.0, tb2 = 0.0;
-            for (int w2 = 0; w2 < kStepThreads / 32; w2++) {
-                ta += red[w2];
-                tb2 += red2[w2];
+    };
+    double scaled_gain = 0.0;
+    for (int round = 0;; round++) {
+        // LDL^T of the scaled matrix, right-looking: column k is left as d_k
+        // (diagonal) and c_ik = d_k l_ik below it, and subtracts c_ik c_jk / d_k
+        // from the trailing columns.
+        for (int j0 = 0; j0 < n; j0 += kStepThreads / 32) {
+            const int j = j0 + warp;
+            const double dj = dinv[j];
+#pragma unroll 4
+            for (int i = j + lane; i < n; i += 32) {
+                const double h = i < P ? Ha[(int64_t)j * P + i] : 0.0;   // (j <= i)
+                const bool live = dinv[i] != 0.0 && dj != 0.0;
+                col(j)[i] = live ? h * dinv[i] * dj + (i == j ? lam : 0.0) : (i == j ? 1.0 : 0.0);
             }
-            s_pa = ta;
-            s_pb = tb2;
-            const double t = ta + lam * tb2;
-            S.pred = 0.5 * t;
-            s_active = !(0.5 * t < tol && lam <= 1.0);
-            if (!s_active) S.status = 1;
         }
         __syncthreads();
-        if (!s_active) {
+        const bool bad = tb::ldl_factor<kStepThreads>(L, rdg, n) != 0;
+        if (bad) {
+            if (round > 0) return;   // the scaled step stands
+            // not positive definite: treat as a rejected step with more damping
+            if (tid == 0) {
+                S.lambda *= 10.0;
+                if (!(S.lambda < 1e12)) S.status = 2;
+            }
             for (int e = tid; e < P; e += kStepThreads) pt[e] = pa[e];
             return;
         }
-    }
-    // step = x / D, limited by maximum steps and the Sersic-index bounds
-    // (ConstrainedOptimizer scales the whole step, constrained_optimizer.py)
-    double lim = 1.0;
-    for (int i = tid; i < P; i += kStepThreads) {
-        const double dlt = dsc[i] == 0.0 ? 0.0 : xs[i] / dsc[i];
-        y[i] = dlt;
-        const int off = i % TB_FIT_NPAR;
-        const double ms = max_step(off);
-        if (ms > 0.0 && fabs(dlt) > ms) lim = fmin(lim, ms / fabs(dlt));
-        if (off == TB_FIT_NPAR - 1 && srcs[b.src0 + i / TB_FIT_NPAR].profile == TB_PROFILE_SERSIC) {
-            const double nv = pa[i] + dlt;
-            if (nv > TB_FIT_SERSIC_MAX && dlt > 0.0) lim = fmin(lim, (TB_FIT_SERSIC_MAX - pa[i]) / dlt);
-            if (nv < TB_FIT_SERSIC_MIN && dlt < 0.0) lim = fmin(lim, (TB_FIT_SERSIC_MIN - pa[i]) / dlt);
+        for (int i = tid; i < n; i += kStepThreads) {
+            xs[i] = 0.0;
+            y[i] = i < P ? gm[i] * dinv[i] : 0.0;
         }
-    }
-    for (int o = 16; o > 0; o >>= 1) lim = fmin(lim, __shfl_xor_sync(0xffffffffu, lim, o));
-    if (lane == 0) red[warp] = lim;
-    __syncthreads();
-    if (tid == 0) {
-        double l = 1.0;
-        for (int w2 = 0; w2 < kStepThreads / 32; w2++) l = fmin(l, red[w2]);
-        s_scale = fmax(l, 0.0);
-        // the gain predicted for the trial as scaled (the next call's gain
-        // ratio divides by it)
-        S.pred = s_scale * s_pa - 0.5 * s_scale * s_scale * (s_pa - lam * s_pb);
-    }
-    __syncthreads();
-    for (int i = tid; i < P; i += kStepThreads) {
-        double v = pa[i] + s_scale * y[i];
-        if (i % TB_FIT_NPAR == TB_FIT_NPAR - 1 &&
-            srcs[b.src0 + i / TB_FIT_NPAR].profile == TB_PROFILE_SERSIC)
-            v = fmin(fmax(v, TB_FIT_SERSIC_MIN), TB_FIT_SERSIC_MAX);
-        pt[i] = v;
+        __syncthreads();
+        // solution and one refinement step
+        for (int pass = 0; pass < 2; pass++) {
+            if (pass == 1) {
+                rows_of_H([&](int j) { return dinv[j] * xs[j]; }, [&](int i, double hx) {
+                    y[i] = dinv[i] != 0.0 ? gm[i] * dinv[i] - (hx * dinv[i] + lam * xs[i])
+                                          : -xs[i];
+                });
+                __syncthreads();
+            }
+            if (warp == 0) tb::ldl_solve(L, rdg, y, n);
+            __syncthreads();
+            for (int i = tid; i < P; i += kStepThreads) xs[i] += y[i];
+            __syncthreads();
+        }
+        if (round == 0) {
+            // Predicted log-likelihood gain of this damped step,
+            // 1/2 (x . D^-1 g + lambda x . x); the blob has converged when it is
+            // below tol while the damping is moderate (optimize_loop stops on the
+            // gain of the last step, dchisq; the prediction is immune to FP32
+            // noise in chi^2).
+            {
+                // a = x^T y0, b = x^T x: the gain predicted for the step is
+                // (a + lambda b) / 2, for the step scaled by s it is
+                // s a - s^2 (a - lambda b) / 2
+                double pa_ = 0.0, pb_ = 0.0;
+                for (int i = tid; i < P; i += kStepThreads) {
+                    const double y0 = dsc[i] == 0.0 ? 0.0 : ga[i] / dsc[i];
+                    pa_ += xs[i] * y0;
+                    pb_ += xs[i] * xs[i];
+                }
+                for (int o = 16; o > 0; o >>= 1) {
+                    pa_ += __shfl_xor_sync(0xffffffffu, pa_, o);
+                    pb_ += __shfl_xor_sync(0xffffffffu, pb_, o);
+                }
+                if (lane == 0) {
+                    red[warp] = pa_;
+                    red2[warp] = pb_;
+                }
+                __syncthreads();
+                if (tid == 0) {
+                    double ta = 0.0, tb2 = 0.0;
+                    for (int w2 = 0; w2 < kStepThreads / 32; w2++) {
+                        ta += red[w2];
+                        tb2 += red2[w2];
+                    }
+                    s_pa = ta;
+                    s_pb = tb2;
+                    const double t = ta + lam * tb2;
+                    S.pred = 0.5 * t;
+                    s_active = !(0.5 * t < tol && lam <= 1.0);
+                    if (!s_active) S.status = 1;
+                }
+                __syncthreads();
+                if (!s_active) {
+                    for (int e = tid; e < P; e += kStepThreads) pt[e] = pa[e];
+                    return;
+                }
+            }
+            // step = x / D, limited by maximum steps and the Sersic-index bounds
+            // (ConstrainedOptimizer scales the whole step, constrained_optimizer.py)
+            double lim = 1.0;
+            for (int i = tid; i < P; i += kStepThreads) {
+                const double dlt = dsc[i] == 0.0 ? 0.0 : xs[i] / dsc[i];
+                y[i] = dlt;
+                const int off = i % TB_FIT_NPAR;
+                const double ms = max_step(off);
+                if (ms > 0.0 && fabs(dlt) > ms) lim = fmin(lim, ms / fabs(dlt));
+                if (off == TB_FIT_NPAR - 1 &&
+                    srcs[b.src0 + i / TB_FIT_NPAR].profile == TB_PROFILE_SERSIC) {
+                    const double nv = pa[i] + dlt;
+                    if (nv > TB_FIT_SERSIC_MAX && dlt > 0.0)
+                        lim = fmin(lim, (TB_FIT_SERSIC_MAX - pa[i]) / dlt);
+                    if (nv < TB_FIT_SERSIC_MIN && dlt < 0.0)
+                        lim = fmin(lim, (TB_FIT_SERSIC_MIN - pa[i]) / dlt);
+                }
+            }
+            for (int o = 16; o > 0; o >>= 1)
+                lim = fmin(lim, __shfl_xor_sync(0xffffffffu, lim, o));
+            if (lane == 0) red[warp] = lim;
+            __syncthreads();
+            if (tid == 0) {
+                double l = 1.0;
+                for (int w2 = 0; w2 < kStepThreads / 32; w2++) l = fmin(l, red[w2]);
+                s_scale = fmax(l, 0.0);
+                // the gain predicted for the trial as scaled (the next call's gain
+                // ratio divides by it)
+                S.pred = s_scale * s_pa - 0.5 * s_scale * s_scale * (s_pa - lam * s_pb);
+            }
+            __syncthreads();
+            write_trial(s_scale);
+            if (!s_slow || !(s_scale < kLimited)) return;
+            scaled_gain = s_scale * s_pa - 0.5 * s_scale * s_scale * (s_pa - lam * s_pb);
+        }
+        // the step with the held parameters' shares, and whether more of it is
+        // beyond its limits
+        bool over = false;
+        for (int i = tid; i < P; i += kStepThreads) {
+            double dlt = held[i];
+            if (dsc[i] != 0.0) {
+                dlt = xs[i] / dsc[i];
+                const int off = i % TB_FIT_NPAR;
+                const double ms = max_step(off);
+                double lo = ms > 0.0 ? -ms : -INFINITY, hi = ms > 0.0 ? ms : INFINITY;
+                if (off == TB_FIT_NPAR - 1) {
+                    lo = fmax(lo, TB_FIT_SERSIC_MIN - pa[i]);
+                    hi = fmin(hi, TB_FIT_SERSIC_MAX - pa[i]);
+                }
+                if (dlt < lo || dlt > hi) {
+                    over = true;
+                    dlt = dlt < lo ? lo : hi;
+                    dsc[i] = dinv[i] = 0.0;
+                    held[i] = dlt;
+                }
+            }
+            y[i] = dlt;
+        }
+        if (!__syncthreads_or(over)) {
+            // (g - H y / 2) . y, into the trial if that is more than the scaled one's
+            double gain = 0.0;
+            rows_of_H([&](int j) { return y[j]; },
+                      [&](int i, double hy) { gain += y[i] * (ga[i] - 0.5 * hy); });
+            for (int o = 16; o > 0; o >>= 1) gain += __shfl_xor_sync(0xffffffffu, gain, o);
+            if (lane == 0) red[warp] = gain;
+            __syncthreads();
+            gain = 0.0;
+            for (int w2 = 0; w2 < kStepThreads / 32; w2++) gain += red[w2];
+            if (!(gain > scaled_gain)) return;
+            if (tid == 0) S.pred = gain;
+            write_trial(1.0);
+            return;
+        }
+        if (round == kBoxRounds) return;
+        rows_of_H([&](int j) { return held[j]; }, [&](int i, double hh) { gm[i] = ga[i] - hh; });
+        __syncthreads();
     }
 }
 
