@@ -545,6 +545,45 @@ def test_solve_at_its_edges(tb, sizes):
             assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
 
 
+def test_solves_of_two_sizes_from_two_threads(tb):
+    """Solves of 105 and of 232 parameters (54 KB and 217 KB of shared memory)
+    from two host threads at once, each on its own stream and buffers: every
+    launch succeeds, whatever size the other thread has just asked for.  (Both
+    matrices have a bad second pivot, so that a solve is as short as its
+    launch.)"""
+    import threading
+    import torch
+    from tractor_b200 import _lib
+    lib = _lib.load()
+    start, codes = threading.Barrier(2), {105: set(), 232: set()}
+
+    def run(P):
+        dev = torch.device('cuda')
+        M, g = torch.eye(P, dtype=torch.float64, device=dev), torch.ones(P, dtype=torch.float64,
+                                                                          device=dev)
+        M[0, 1] = M[1, 0] = 2.
+        zero = torch.zeros(1, dtype=torch.int64, device=dev)
+        dP, info = (torch.full((1,), v, dtype=torch.int32, device=dev) for v in (P, -2))
+        X, work = torch.zeros_like(g), torch.empty(P * P, dtype=torch.float64, device=dev)
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        a = (M.data_ptr(), g.data_ptr(), zero.data_ptr(), zero.data_ptr(), dP.data_ptr(),
+             zero.data_ptr(), X.data_ptr(), info.data_ptr(), 0., 1, P, work.data_ptr(),
+             s.cuda_stream)
+        start.wait()
+        for i in range(20000):
+            codes[P].add(lib.tb_solve_update(*a))
+        s.synchronize()
+        assert int(info[0]) == 2
+
+    threads = [threading.Thread(target=run, args=(P,)) for P in codes]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert codes == {105: {_lib.TB_OK}, 232: {_lib.TB_OK}}
+
+
 def test_chi2(tb):
     import torch
     from tractor_b200 import render

@@ -541,9 +541,11 @@ int launch_solve_threads(const double* AtA, const double* Atr, const int64_t* at
                          int32_t* info, double damp, int n_problems, int max_p, double* work,
                          cudaStream_t s) {
     const int smem = solve_smem(max_p), n = solve_pad(max_p);
+    // (the largest launch's size, whatever this one's is: the limit belongs to
+    // the kernel, and another host thread may be between its own two calls)
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(solve_kernel<kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) != cudaSuccess)
+                             solve_smem(kSolveSharedP)) != cudaSuccess)
         return TB_ERR_LAUNCH;
     solve_kernel<kThreads><<<n_problems, kThreads, smem, s>>>(
         AtA, Atr, ata_off, atr_off, P, x_off, X, info, damp, work, (int64_t)max_p * max_p,
