@@ -224,3 +224,36 @@ def test_sharp_and_wide_components_match_oracle(tb, oracle, tile_h, sigma):
     got = r.image(r.render(s, tile_h=tile_h), 0).numpy()
     ref = oracle.scene_model(rows, [0.8, 0.2], [sigma, 2 * sigma], H, W)
     assert _peak_err(got, ref) < 1.5e-6
+
+
+@pytest.mark.parametrize('H', [500, 1300, 4000])
+@pytest.mark.parametrize('sigma', [0.85, 0.86, 0.9, 0.97, 1.0])
+def test_far_tail_of_sharp_components(tb, sigma, H):
+    """Point sources whose PSF variance lies around the limits of the row
+    recurrence (0.72 to 1 px^2), in images of few and of many tiles (each
+    variant of the render): every pixel down to the floor (Mahalanobis^2 100,
+    2^-72 of the peak) has its value.  The exponent, up to 72, is rounded a few
+    times to 2^-24 of itself: 1e-4 of the value holds a dozen such roundings."""
+    from tractor_b200 import _lib, batch
+    rng = np.random.default_rng(24)
+    W, n = 640, 60
+    s = np.zeros(n, batch.SCENE_SRC)
+    s['profile'] = _lib.PROFILE_POINT
+    # one source per cell of 64 x 64 pixels, its rectangle inside the cell
+    cell = rng.permutation((W // 64) * (H // 64))[:n]
+    cx, cy = cell % (W // 64) * 64 + 32, cell // (W // 64) * 64 + 32
+    s['px'], s['py'] = cx + rng.uniform(-3, 3, n), cy + rng.uniform(-3, 3, n)
+    s['counts'] = 1e3
+    s['mx0'], s['my0'] = cx - 31, cy - 31
+    s['mw'] = s['mh'] = 62
+    r = batch.SceneRenderer([batch.SceneImage.circular(W, H, [sigma], [1.])])
+    got = r.image(r.render(s, tile_h=32), 0).numpy()
+    y, x = np.mgrid[:62, :62]
+    for k in range(n):
+        x0, y0 = int(s['mx0'][k]), int(s['my0'][k])
+        d2 = ((x + x0 - s['px'][k]) ** 2 + (y + y0 - s['py'][k]) ** 2) / sigma ** 2
+        ref = 1e3 / (2 * np.pi * sigma ** 2) * np.exp(-.5 * d2)
+        patch = got[y0:y0 + 62, x0:x0 + 62].astype(np.float64)
+        near, far = d2 < 99.99, d2 > 100.01
+        assert np.all(np.abs(patch - ref)[near] <= 1e-4 * ref[near]), k
+        assert np.all(patch[far] == 0)

@@ -308,7 +308,9 @@ struct __align__(16) SceneC {
 constexpr uint32_t kInner = 1u << 30;    // no pixel of the rectangle is below the floor
 constexpr uint32_t kDirect = 1u << 31;   // every pixel's exponential by itself
 
-constexpr float kMaxCurve = 1.0f;
+// Largest |qyy| of a component whose rows are chained (R rows of a thread).
+template <int R>
+constexpr float kMaxCurve = R > 2 ? 0.75f : 1.0f;
 
 // Largest exponent of a component (a dx^2 + b dx dy + c dy^2, concave) over
 // the box [x0, x1] x [y0, y1] about its centre.
@@ -332,10 +334,11 @@ __device__ __forceinline__ float max_exponent(float a, float b, float c, float x
 // five packed multiplies instead of eight ex2 and their exponents.  Three
 // steps from an anchor add about 3 ulp; with the centre split into pixel and
 // fraction the result is nearer to FP64 than eight separate ex2 from a
-// rounded centre.  The chain holds while |qyy| <= 1 (variance 0.72 px^2): a
-// first row so far out that E flushes to zero (2^-126) then has no row within
-// 2^-64 of the component's peak; sharper components take every pixel's ex2.
-// Exponents below the floor count as 0 (c_gauss_2d_grid skips Mahalanobis^2
+// rounded centre.  A first row so far out that E flushes to zero (2^-126) must
+// have no later row above the floor (2^-72.1 of the component's peak): with
+// four rows that holds up to |qyy| = 0.79 (sqrt(126) - 3 sqrt(|qyy|) >=
+// sqrt(72.1)), so components above 0.75 (variances below 0.96 px^2; with two
+// rows 1 and 0.72) take every pixel's ex2.  Exponents below the floor count as 0 (c_gauss_2d_grid skips Mahalanobis^2
 // >= 100), tested only where the component reaches it inside the rectangle.
 template <int TH, int CP, int R>
 __global__ void __launch_bounds__(16 * TH / (CP * R), (CP == 1 ? 1024 : 768) / (16 * TH / (CP * R)))
@@ -512,7 +515,7 @@ scene_render_kernel(const tb_scene_item* __restrict__ items, int n_items,
                         const float lowest = fminf(fminf(e(bx0, by0), e(bx1, by0)),
                                                    fminf(e(bx0, by1), e(bx1, by1)));
                         if (lowest > fl + 1.f) c.rect |= kInner;
-                        if (!(fabsf(qc) <= kMaxCurve) || fl < -73.f) c.rect |= kDirect;
+                        if (!(fabsf(qc) <= kMaxCurve<R>) || fl < -73.f) c.rect |= kDirect;
                     }
                 }
                 // order-preserving compaction of the kept components
