@@ -167,3 +167,70 @@ def test_fused_equals_two_launch_path(tb):
             assert np.array_equal(it1[k], it2[k]), k
     assert np.all(np.isfinite(got))
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize('n', [3, 64])
+@pytest.mark.parametrize('same_stream', [False, True])
+def test_one_renderer_on_two_streams_or_threads(tb, n, same_stream):
+    """Renders and vector-Jacobian products of one renderer that overlap, from
+    two streams of one thread or from two threads on one stream, each with its
+    own sources and sizes that share a size class: every result is that of the
+    same call alone, bit for bit."""
+    import threading
+    import torch
+    from tractor_b200 import batch, grad
+    r = batch.FourierGalaxyRenderer(batch.moffat_psf(45))
+    jac = grad.FourierJacobian(r)
+    jobs = []
+    for k, m in enumerate((n, n + 1)):
+        rng = np.random.default_rng(70 + k)
+        s = batch.sersic_sources(m, rng, mask=rng.integers(30, 150, m))
+        npix = int((s['mw'].astype(np.int64) * s['mh']).sum())
+        g = torch.randn(npix, generator=torch.Generator(device='cuda').manual_seed(k), device='cuda')
+        d = torch.from_numpy(s.view(np.uint8).copy()).cuda()
+        out = torch.zeros(npix, device='cuda')
+        r.render_device(d, m, out)
+        jobs.append((d, m, g, out.clone(), jac.vjp(d, m, g)[0].clone()))
+    torch.cuda.synchronize()
+    one = torch.cuda.Stream()
+    results = [[], []]
+
+    def run(k, stream, times):
+        d, m, g, _, _ = jobs[k]
+        for _ in range(times):
+            with torch.cuda.stream(stream):
+                out = torch.zeros_like(g)
+            r.render_device(d, m, out, stream=stream)
+            results[k].append((out, jac.vjp(d, m, g, stream=stream)[0]))
+
+    if same_stream:
+        threads = [threading.Thread(target=run, args=(k, one, 30)) for k in (0, 1)]
+        for th in threads:
+            th.start()
+        for th in threads:
+            th.join()
+    else:
+        streams = [one, torch.cuda.Stream()]
+        for _ in range(30):
+            for k in (0, 1):
+                run(k, streams[k], 1)
+    torch.cuda.synchronize()
+    for k in (0, 1):
+        assert len(results[k]) == 30
+        for out, dots in results[k]:
+            assert torch.equal(out, jobs[k][3]) and torch.equal(dots, jobs[k][4])
+
+
+def test_scratch_is_bounded(tb):
+    """Buffers kept for many sizes of call: one per power of two, thread and
+    stream."""
+    import torch
+    from tractor_b200 import _lib, batch
+    assert [_lib.size_class(n) for n in (0, 1, 2, 3, 4, 5, 64, 65)] == [1, 1, 2, 4, 4, 8, 64, 128]
+    r = batch.FourierGalaxyRenderer(batch.moffat_psf(45))
+    s = batch.sersic_sources(40, np.random.default_rng(75), mask=32)
+    d = torch.from_numpy(s.view(np.uint8).copy()).cuda()
+    out = torch.zeros(40 * 32 * 32, device='cuda')
+    for n in range(20, 41):
+        r.render_device(d, n, out)
+    assert len(r._scratch.pool) == 2

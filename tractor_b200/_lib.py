@@ -2,9 +2,11 @@
 (include/tractor_b200.h).  There is no CPU implementation behind this module:
 if the library is missing, or no CUDA device is present when a kernel is
 called, it raises."""
+import contextlib
 import ctypes
 import os
 import re
+import threading
 
 import numpy as np
 
@@ -214,6 +216,72 @@ def stream_ptr(stream=None):
     if stream is None:
         return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     return stream.cuda_stream
+
+
+def on_stream(stream):
+    """Context in which torch allocates and launches on `stream` (the current
+    one if None)."""
+    import torch
+    if stream is None:
+        return contextlib.nullcontext()
+    if not isinstance(stream, torch.cuda.Stream):
+        stream = torch.cuda.ExternalStream(stream.cuda_stream)
+    return torch.cuda.stream(stream)
+
+
+def scratch_key(stream=None):
+    """What a scratch buffer belongs to: the device, the host thread and the
+    stream of the launch.  Launches that share all three run one after the
+    other; others may overlap and need buffers of their own."""
+    import torch
+    return torch._C._cuda_getDevice(), threading.get_ident(), stream_ptr(stream)
+
+
+def size_class(n):
+    """Scratch for n elements is kept for the next power of two: at most twice
+    the largest size asked for, however many different ones, and no buffer is
+    ever replaced (a captured graph may hold its address)."""
+    return 1 << max(int(n) - 1, 0).bit_length()
+
+
+class Scratch(object):
+    """Device buffers of a class of calls that may overlap: one allocation per
+    size class, thread and stream (scratch_key), cut into parts at 256-byte
+    boundaries; the flags of a call, and its counter and status words, are kept
+    for each size by themselves.  `parts(m)`: the parts' bytes for m elements."""
+
+    def __init__(self, parts):
+        self.parts = parts
+        self.pool = {}
+        self.calls = {}
+
+    def get(self, n, stream=None):
+        """(buffer, the parts' addresses, their bytes, flags, misc, the stream's
+        address) for n elements: flags int32 (n,), misc int32 (8,), cleared
+        once."""
+        import torch
+        key = scratch_key(stream)
+        w = self.calls.get((key, n))
+        if w is None:
+            m = size_class(n)
+            dev = torch.device('cuda', key[0])
+            with on_stream(stream):
+                if (key, m) not in self.pool:
+                    sizes, at = self.parts(m), [0]
+                    for b in sizes:
+                        at.append(at[-1] + (b + 255) // 256 * 256)
+                    buf = torch.empty(at.pop(), dtype=torch.uint8, device=dev)
+                    base = buf.data_ptr()
+                    self.pool[key, m] = (buf, [base + a for a in at], sizes)
+                w = self.calls[key, n] = self.pool[key, m] + (
+                    torch.empty(n, dtype=torch.int32, device=dev),
+                    torch.zeros(8, dtype=torch.int32, device=dev), key[2])
+        return w
+
+    def view(self, w, part, nbytes, dtype):
+        """The first nbytes of a part as a tensor."""
+        at = w[1][part] - w[0].data_ptr()
+        return w[0][at:at + nbytes].view(dtype)
 
 
 def require_cuda():

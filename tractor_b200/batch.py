@@ -114,28 +114,23 @@ class FourierGalaxyRenderer(object):
         self.spec = torch.cat(specs)
         self.image = img
         self.tables = device_profile_tables()
-        self._scratch = {}
-        self._workspaces = {}
+        # items, component amplitudes and variances, the sorted path's workspace
+        self._scratch = _lib.Scratch(lambda m: (
+            m * _lib.FFT_ITEM.itemsize, m * COMP_STRIDE * 8, m * COMP_STRIDE * 32,
+            render.fourier_workspace_bytes(m)))
 
-    def _work(self, n):
-        """Device scratch for n sources: items, components, flags, counter,
-        status (reused between calls of the same size)."""
-        if n not in self._scratch:
-            dev = render.device()
-            nb = n * _lib.FFT_ITEM.itemsize
-            items = torch.empty(nb, dtype=torch.uint8, device=dev)
-            camp = torch.empty(n * COMP_STRIDE, dtype=torch.float64, device=dev)
-            cvar = torch.empty(n * COMP_STRIDE * 4, dtype=torch.float64, device=dev)
-            flags = torch.empty(n, dtype=torch.int32, device=dev)
-            misc = torch.zeros(8, dtype=torch.int32, device=dev)   # counter + status
-            self._scratch[n] = (items, camp, cvar, flags, misc)
-        return self._scratch[n]
+    def _work(self, n, stream=None):
+        """The scratch of the calls for n sources as tensors: items, component
+        amplitudes and variances, flags, counter + status."""
+        S, w = self._scratch, self._scratch.get(n, stream)
+        return (S.view(w, 0, n * _lib.FFT_ITEM.itemsize, torch.uint8),
+                S.view(w, 1, n * COMP_STRIDE * 8, torch.float64),
+                S.view(w, 2, n * COMP_STRIDE * 32, torch.float64), w[3], w[4])
 
-    def _workspace(self, n):
-        """The sorted path's workspace for n sources."""
-        if n not in self._workspaces:
-            self._workspaces[n] = render.new_fourier_workspace(n, render.device())
-        return self._workspaces[n]
+    def _workspace(self, n, stream=None):
+        """(address, bytes) of the sorted path's workspace."""
+        w = self._scratch.get(n, stream)
+        return w[1][3], w[2][3]
 
     METHODS = ('fused', 'persistent', 'split')
     # one launch in place of three: 17 against 29 us for one 32-px patch; from
@@ -152,27 +147,24 @@ class FourierGalaxyRenderer(object):
         'fused' for a few sources and 'split' for more (FUSED_MAX).  Returns
         the flags tensor (see tb_galaxy_fft_prep)."""
         lib = _lib.load()
-        items, camp, cvar, flags, misc = self._work(n)
-        s = _lib.stream_ptr(stream)
+        _, (items, camp, cvar, ws), nbytes, flags, misc, s = self._scratch.get(n, stream)
         method = method or getattr(self, 'method', None) or (
             'fused' if n <= self.FUSED_MAX else 'split')
         if method == 'fused':
             rc = lib.tb_galaxy_fft_render(srcs.data_ptr(), n, ctypes.addressof(self.image),
                                           ctypes.addressof(self.tables.struct),
-                                          self.spec.data_ptr(), out.data_ptr(), items.data_ptr(),
+                                          self.spec.data_ptr(), out.data_ptr(), items,
                                           flags.data_ptr(), misc.data_ptr(), misc.data_ptr() + 16,
                                           s)
             _lib.check(rc, 'tb_galaxy_fft_render')
             return flags
         rc = lib.tb_galaxy_fft_prep(srcs.data_ptr(), n, ctypes.addressof(self.image),
-                                    ctypes.addressof(self.tables.struct), items.data_ptr(),
-                                    camp.data_ptr(), cvar.data_ptr(), COMP_STRIDE,
-                                    flags.data_ptr(), s)
+                                    ctypes.addressof(self.tables.struct), items, camp, cvar,
+                                    COMP_STRIDE, flags.data_ptr(), s)
         _lib.check(rc, 'tb_galaxy_fft_prep')
-        render.fourier_render(items.data_ptr(), n, camp.data_ptr(), cvar.data_ptr(),
-                              self.spec.data_ptr(), out.data_ptr(), misc.data_ptr() + 16,
-                              stream=stream, method=method,
-                              workspace=self._workspace(n) if method == 'split' else None)
+        render.fourier_render(items, n, camp, cvar, self.spec.data_ptr(), out.data_ptr(),
+                              misc.data_ptr() + 16, stream=stream, method=method,
+                              workspace=(ws, nbytes[3]))
         return flags
 
     def autotune(self, srcs, n, out):
@@ -195,8 +187,8 @@ class FourierGalaxyRenderer(object):
         self.method = min(times, key=times.get)
         return times
 
-    def status(self, n):
-        return self._work(n)[4][4:8]
+    def status(self, n, stream=None):
+        return self._scratch.get(n, stream)[4][4:8]
 
     def render(self, srcs_host, out_host=None, stream=None, method=None):
         """End-to-end call with host buffers: copies the GALAXY_SRC records
@@ -210,13 +202,14 @@ class FourierGalaxyRenderer(object):
         if out_host is None:
             out_host = torch.empty(nout, dtype=torch.float32).pin_memory()
         src_pinned = torch.from_numpy(srcs_host.view(np.uint8)).pin_memory()
-        d_src = src_pinned.to(dev, non_blocking=True)
-        out = torch.empty(nout, dtype=torch.float32, device=dev)
-        flags = self.render_device(d_src, n, out, stream, method=method)
-        out_host.copy_(out, non_blocking=True)
-        flags_host = flags.to('cpu', non_blocking=True)
-        torch.cuda.current_stream().synchronize()
-        render.check_status(self.status(n).clone(), 'tb_fourier_render')
+        with _lib.on_stream(stream):
+            d_src = src_pinned.to(dev, non_blocking=True)
+            out = torch.empty(nout, dtype=torch.float32, device=dev)
+            flags = self.render_device(d_src, n, out, stream, method=method)
+            out_host.copy_(out, non_blocking=True)
+            flags_host = flags.to('cpu', non_blocking=True)
+            torch.cuda.current_stream().synchronize()
+            render.check_status(self.status(n, stream).clone(), 'tb_fourier_render')
         return out_host, flags_host.numpy()
 
 

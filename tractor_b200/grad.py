@@ -20,6 +20,7 @@ parameters are the first seven fields of a GALAXY_SRC record: px, py,
 counts, s0, s1, s2 (shape, per shape_type) and sersic_n.
 """
 import ctypes
+import functools
 
 import numpy as np
 import torch
@@ -36,66 +37,64 @@ class FourierJacobian(object):
 
     def __init__(self, renderer):
         self.r = renderer
-        self._scratch = {}
-        self._vjp_scratch = {}
+        S = batch.COMP_STRIDE
+        # items, component amplitudes, variances and coefficients, the
+        # product's workspace
+        self._scratch = _lib.Scratch(lambda m: (
+            7 * m * _lib.FFT_ITEM.itemsize, m * S * 8, m * S * 32, 4 * m * S * 32,
+            self._vjp_bytes(m)))
 
-    def _work(self, n):
-        if n not in self._scratch:
-            dev = render.device()
-            S = batch.COMP_STRIDE
-            items = torch.empty(7 * n * _lib.FFT_ITEM.itemsize, dtype=torch.uint8, device=dev)
-            camp = torch.empty(n * S, dtype=torch.float64, device=dev)
-            cvar = torch.empty(n * S * 4, dtype=torch.float64, device=dev)
-            dcoef = torch.zeros(4 * n * S * 4, dtype=torch.float64, device=dev)
-            flags = torch.empty(n, dtype=torch.int32, device=dev)
-            misc = torch.zeros(8, dtype=torch.int32, device=dev)
-            self._scratch[n] = (items, camp, cvar, dcoef, flags, misc)
-        return self._scratch[n]
+    @staticmethod
+    @functools.lru_cache(maxsize=64)
+    def _vjp_bytes(n):
+        nb = ctypes.c_int64()
+        _lib.check(_lib.load().tb_galaxy_fft_vjp_workspace(n, ctypes.byref(nb)),
+                   'tb_galaxy_fft_vjp_workspace')
+        return nb.value
 
-    def _vjp_workspace(self, n):
-        if n not in self._vjp_scratch:
-            nb = ctypes.c_int64()
-            _lib.check(_lib.load().tb_galaxy_fft_vjp_workspace(n, ctypes.byref(nb)),
-                       'tb_galaxy_fft_vjp_workspace')
-            self._vjp_scratch[n] = torch.empty(nb.value, dtype=torch.uint8,
-                                               device=render.device())
-        return self._vjp_scratch[n]
+    def _work(self, n, stream=None):
+        """The scratch of the calls for n sources as tensors: items, component
+        amplitudes, variances and coefficients, flags, counter + status."""
+        P, w = self._scratch, self._scratch.get(n, stream)
+        S = batch.COMP_STRIDE
+        return (P.view(w, 0, 7 * n * _lib.FFT_ITEM.itemsize, torch.uint8),
+                P.view(w, 1, n * S * 8, torch.float64), P.view(w, 2, n * S * 32, torch.float64),
+                P.view(w, 3, 4 * n * S * 32, torch.float64), w[3], w[4])
 
-    def _prep(self, srcs, n, mode, col_stride, s):
+    def _prep(self, srcs, n, mode, col_stride, stream):
         lib = _lib.load()
-        items, camp, cvar, dcoef, flags, misc = self._work(n)
+        _, (items, camp, cvar, dcoef, ws), nbytes, flags, misc, s = self._scratch.get(n, stream)
         rc = lib.tb_galaxy_fft_jac_prep(srcs.data_ptr(), n, ctypes.addressof(self.r.image),
-                                        ctypes.addressof(self.r.tables.struct), items.data_ptr(),
-                                        camp.data_ptr(), cvar.data_ptr(), dcoef.data_ptr(),
-                                        batch.COMP_STRIDE, mode, col_stride, flags.data_ptr(), s)
+                                        ctypes.addressof(self.r.tables.struct), items, camp, cvar,
+                                        dcoef, batch.COMP_STRIDE, mode, col_stride,
+                                        flags.data_ptr(), s)
         _lib.check(rc, 'tb_galaxy_fft_jac_prep')
-        return items, camp, cvar, dcoef, flags, misc
+        return items, camp, cvar, dcoef, flags, misc, ws, nbytes[4]
 
     def jacobian(self, srcs, n, npix, stream=None):
         """float32 (7, npix) device tensor: row j holds d(model)/d(param j)
         of every galaxy, each at its record's out_off (the layout of the
         value patches).  Also returns the prep flags."""
-        out = torch.empty(7 * npix, dtype=torch.float32, device=render.device())
-        items, camp, cvar, dcoef, flags, misc = self._prep(srcs, n, _lib.MOG_STORE, npix,
-                                                           _lib.stream_ptr(stream))
-        render.fourier_render(items.data_ptr(), 7 * n, camp.data_ptr(), cvar.data_ptr(),
-                              self.r.spec.data_ptr(), out.data_ptr(), misc.data_ptr() + 16,
-                              dcoef_ptr=dcoef.data_ptr(), stream=stream)
+        with _lib.on_stream(stream):
+            out = torch.empty(7 * npix, dtype=torch.float32, device=render.device())
+        items, camp, cvar, dcoef, flags, misc, _, _ = self._prep(srcs, n, _lib.MOG_STORE, npix,
+                                                                 stream)
+        render.fourier_render(items, 7 * n, camp, cvar, self.r.spec.data_ptr(), out.data_ptr(),
+                              misc.data_ptr() + 16, dcoef_ptr=dcoef, stream=stream)
         return out.view(7, npix), flags, misc[4:8]
 
     def vjp(self, srcs, n, grad, stream=None):
         """float64 (n, 7): sum over each galaxy's patch of grad * d(model)/
         d(param), grad laid out like the value patches (tb_galaxy_fft_vjp:
         one adjoint transform per galaxy)."""
-        s = _lib.stream_ptr(stream)
-        dots = torch.zeros(7 * n, dtype=torch.float64, device=render.device())
-        grad = grad.contiguous()
-        items, camp, cvar, dcoef, flags, misc = self._prep(srcs, n, _lib.FFT_DOT, 0, s)
-        ws = self._vjp_workspace(n)
-        rc = _lib.load().tb_galaxy_fft_vjp(items.data_ptr(), n, camp.data_ptr(), cvar.data_ptr(),
-                                           dcoef.data_ptr(), self.r.spec.data_ptr(),
-                                           grad.data_ptr(), dots.data_ptr(), ws.data_ptr(),
-                                           ws.numel(), misc.data_ptr() + 16, s)
+        with _lib.on_stream(stream):
+            dots = torch.zeros(7 * n, dtype=torch.float64, device=render.device())
+            grad = grad.contiguous()
+        items, camp, cvar, dcoef, flags, misc, ws, nbytes = self._prep(srcs, n, _lib.FFT_DOT, 0,
+                                                                       stream)
+        rc = _lib.load().tb_galaxy_fft_vjp(items, n, camp, cvar, dcoef, self.r.spec.data_ptr(),
+                                           grad.data_ptr(), dots.data_ptr(), ws, nbytes,
+                                           misc.data_ptr() + 16, _lib.stream_ptr(stream))
         _lib.check(rc, 'tb_galaxy_fft_vjp')
         return dots.view(n, 7), flags, misc[4:8]
 

@@ -7,6 +7,7 @@ outputs stay torch tensors; the Tractor-facing classes copy to numpy only
 where the reference API returns numpy arrays.
 """
 import ctypes
+import functools
 
 import threading
 
@@ -588,26 +589,24 @@ LARGE_FFT_MAX = 8192     # the reference warns above a half-size of 4096 (galaxy
 _fourier_ws = {}
 
 
-def new_fourier_workspace(n_items, dev):
-    """Device scratch of tb_fourier_render_split for n_items items."""
-    lib = _lib.load()
+@functools.lru_cache(maxsize=64)
+def fourier_workspace_bytes(n_items):
     nb = ctypes.c_int64()
-    _lib.check(lib.tb_fourier_workspace(int(n_items), ctypes.byref(nb)), 'tb_fourier_workspace')
-    return torch.empty(max(nb.value, 256), dtype=torch.uint8, device=dev)
+    _lib.check(_lib.load().tb_fourier_workspace(int(n_items), ctypes.byref(nb)),
+               'tb_fourier_workspace')
+    return nb.value
 
 
-def fourier_workspace(n_items, dev=None):
-    """The device's shared scratch of tb_fourier_render_split, for callers
-    that keep none of their own (one buffer per device, grown when needed and
-    reused: launches on one stream use it one after another)."""
+def fourier_workspace(n_items, dev=None, stream=None):
+    """The shared scratch of tb_fourier_render_split for callers that keep none
+    of their own (_lib.scratch_key, _lib.size_class)."""
     dev = dev or device()
-    lib = _lib.load()
-    nb = ctypes.c_int64()
-    _lib.check(lib.tb_fourier_workspace(int(n_items), ctypes.byref(nb)), 'tb_fourier_workspace')
-    ws = _fourier_ws.get(dev.index)
-    if ws is None or ws.numel() < nb.value:
-        ws = _fourier_ws[dev.index] = torch.empty(max(nb.value, 1 << 20), dtype=torch.uint8,
-                                                  device=dev)
+    size = max(_lib.size_class(fourier_workspace_bytes(n_items)), 1 << 20)
+    key = _lib.scratch_key(stream), size
+    ws = _fourier_ws.get(key)
+    if ws is None:
+        with _lib.on_stream(stream):
+            ws = _fourier_ws[key] = torch.empty(size, dtype=torch.uint8, device=dev)
     return ws
 
 
@@ -621,21 +620,22 @@ def fourier_render(items_ptr, n_items, amp_ptr, var_ptr, spec_ptr, out_ptr, stat
     one CTA per item -- or 'split' -- tb_fourier_render_split, the items sorted
     by FFT size and rendered by groups of warps on packed transforms.  The
     default is the device's autotuned choice (autotune_fourier), else
-    'persistent'.  `workspace`: the caller's new_fourier_workspace (the
-    device's shared one if None)."""
+    'persistent'.  `workspace`: (address, bytes) of the caller's own scratch of
+    fourier_workspace_bytes, or a tensor of them (the shared one if None)."""
     lib = _lib.load()
     if method is None:
         dev = device()
         method = fourier_method.get(dev.index, fourier_method['default'])
     s = _lib.stream_ptr(stream)
     if method == 'split':
-        ws = fourier_workspace(n_items) if workspace is None else workspace
+        ws = fourier_workspace(n_items, stream=stream) if workspace is None else workspace
+        if not isinstance(ws, tuple):
+            ws = ws.data_ptr(), ws.numel()
         rc = lib.tb_fourier_render_split(items_ptr, int(n_items), amp_ptr, var_ptr, dcoef_ptr,
-                                         spec_ptr, out_ptr, dots_ptr, ws.data_ptr(), ws.numel(),
-                                         status_ptr, s)
+                                         spec_ptr, out_ptr, dots_ptr, *ws, status_ptr, s)
         _lib.check(rc, 'tb_fourier_render_split')
         return
-    ctr = _counter(device())
+    ctr = _counter(device(), stream)
     if dcoef_ptr is None and dots_ptr is None:
         rc = lib.tb_fourier_render(items_ptr, int(n_items), amp_ptr, var_ptr, spec_ptr, out_ptr,
                                    ctr.data_ptr(), status_ptr, s)
@@ -649,12 +649,14 @@ def fourier_render(items_ptr, n_items, amp_ptr, var_ptr, spec_ptr, out_ptr, stat
 _counters = {}
 
 
-def _counter(dev):
+def _counter(dev, stream=None):
     """A device int32 work counter for the persistent kernels (zeroed by each
     launch on its stream before use)."""
-    c = _counters.get(dev.index)
+    key = _lib.scratch_key(stream)
+    c = _counters.get(key)
     if c is None:
-        c = _counters[dev.index] = torch.zeros(4, dtype=torch.int32, device=dev)
+        with _lib.on_stream(stream):
+            c = _counters[key] = torch.zeros(4, dtype=torch.int32, device=dev)
     return c
 
 
