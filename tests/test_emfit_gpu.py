@@ -161,3 +161,20 @@ def test_em_indefinite_covariance_matches_oracle(tb, oracle):
         np.testing.assert_allclose(a1, a2, rtol=1e-9, atol=1e-13)
         np.testing.assert_allclose(m1, m2, rtol=0, atol=1e-9)
         np.testing.assert_allclose(v1, v2, rtol=1e-9, atol=1e-12)
+
+
+def test_slowly_converging_fits_to_the_last_bits(tb):
+    """Amplitudes of 96 three-component fits after 1000 iterations against the
+    same iteration in extended precision (golden/em_extended.npz: the images in
+    single precision, the amplitudes in two parts).  The fixed point amplifies an
+    iteration's rounding; one pixel at a time with exp() and divisions, the
+    median error over 1,024 such stamps is 1.6e-16.  A third more is allowed."""
+    import os
+    from tractor_b200 import emfit
+    z = np.load(os.path.join(os.path.dirname(__file__), 'golden', 'em_extended.npz'))
+    im = z['images'].astype(np.float64)
+    n, K = z['amp'].shape
+    amp = emfit.em_fit_2d_batch(im, np.full((n, K), 1. / K), np.zeros((n, K, 2)),
+                                np.broadcast_to(np.eye(2) * np.arange(1, K + 1)[:, None, None],
+                                                (n, K, 2, 2)).copy(), steps=1000)[0]
+    assert np.median(np.abs((np.asarray(amp) - z['amp']) - z['amp_low'])) < 4. / 3. * 1.6e-16

@@ -28,11 +28,19 @@
 // the M step and the next iteration's parameters itself, so an iteration has
 // one block barrier.  100 iterations, 1024 stamps of 25 x 25 (against a pixel
 // stride per thread with exp(), divisions and a butterfly per moment): 1
-// component 487 -> 394 us, 3 components 1045 -> 743, 8 components 4657 -> 2277;
-// 256 stamps of 63 x 63, 3 components 3279 -> 2405.  The order of the sums is
-// another, so the last bits are: after 1000 iterations of 3 components the
-// amplitudes are off by 8.8e-16 against extended precision (rms; was 5.7e-16),
-// of 2 components by 4.1e-16 (3.4e-16).
+// component 487 -> 431 us, 3 components 1033 -> 797, 8 components 4589 -> 2661;
+// 256 stamps of 63 x 63, 3 components 3080 -> 2391.
+//
+// Rounding: EM converges slowly, so the fixed point amplifies every rounding of an
+// iteration, those shared by all pixels most.  Hence the exponents' coefficients
+// to the last bit (`prepare`), the exponential's table in two parts, and, where it
+// costs no turn, a thread's runs of columns in mirrored pairs, whose first moments
+// cancel before they are rounded together.  After 1000 iterations, against
+// extended precision, over eight sets of stamps (15 to 27 px, 1 to 3 components)
+// the geometric means of the rms errors are 4.7e-16 in the amplitudes, 6.8e-16 in
+// the means and 6.6e-15 in the variances; with one pixel at a time, exp() and
+// divisions 4.6e-16, 7.0e-16 and 7.1e-15; without those three 5.3e-16, 1.0e-15 and
+// 8.4e-15 (1024 stamps, 3 components: 7.5 in place of 7.8 ms).
 #include <type_traits>
 
 #include "tb_common.cuh"
@@ -87,11 +95,11 @@ __device__ __forceinline__ void warp_sums(double (&a)[M], int lane, double* out)
         if (i < count) out[first + i] = a[i];   // (equal values from lanes that share one)
 }
 
-// (resident CTAs: as many as registers allow without spills up to 3
-// components, 7 with a few for 4 and 5, where fewer left 1024 stamps a second
-// wave: 5 components 1748 us before, 2000 with 6, 1306 with 7)
+// (resident CTAs: 7 up to 5 components, which hold 1024 stamps in one wave: 3
+// components 7.8 ms, with 8 and fewer registers 8.5; 5 components 1306 us, with 6 a
+// second wave 2000)
 template <int K>
-__global__ void __launch_bounds__(kEmThreads, K <= 3 ? 8 : K <= 5 ? 7 : 4)
+__global__ void __launch_bounds__(kEmThreads, K <= 5 ? 7 : 4)
 em_fit_kernel(const double* __restrict__ img, int n, int ny, int nx,
               const int32_t* __restrict__ xy0, double* __restrict__ amp,
               double* __restrict__ mean, double* __restrict__ var, double alpha, int steps,
@@ -101,7 +109,7 @@ em_fit_kernel(const double* __restrict__ img, int n, int ny, int nx,
     // exponents in log2 units)
     __shared__ double par[kWarps][K][8];   // mean x, y, c00, c01, c11, scale
     __shared__ double red[2][kWarps][kM];
-    __shared__ double exp_tab[tb::kExpTab];
+    __shared__ double2 exp_tab[tb::kExpTab];
     const int s = blockIdx.x;
     if (s >= n) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -124,6 +132,11 @@ em_fit_kernel(const double* __restrict__ img, int n, int ny, int nx,
         }
     }
     const int step_x = kEmThreads % nx, step_g = kEmThreads / nx;
+    // runs q and N - 1 - q (mirrored at the image's centre) by the same thread,
+    // where that takes no more turns
+    const int N = nx * groups;
+    const bool mirror = 2 * (((N + 1) / 2 + kEmThreads - 1) / kEmThreads) <=
+                        (N + kEmThreads - 1) / kEmThreads;
     const double tpd = 4.0 * TB_PI * TB_PI;   // (2 pi)^D, D = 2
     tb::exp2_tab_init(exp_tab);
     // component `lane` of this warp's copy: the exponents' coefficients and the
@@ -137,10 +150,16 @@ em_fit_kernel(const double* __restrict__ img, int n, int ny, int nx,
         double* p = par[warp][lane];
         p[0] = mx;
         p[1] = my;
-        const double q = -0.5 * TB_LOG2E / det;
-        p[2] = v11 * q;
-        p[3] = -(v01 + v10) * q;
-        p[4] = v00 * q;
+        // q + ql = -log2(e) / (2 det): the quotient's remainder, the constant's
+        // second part and the rounding of det
+        const double b = v01 * v10, be = fma(v01, v10, -b);
+        const double dl = (fma(v00, v11, -det) - b) - be;
+        const double c = -0.5 * TB_LOG2E, q = c / det;
+        const double ql = ((fma(-q, det, c) - 0.5 * 2.0355273740931033e-17) - q * dl) *
+                          (q * -1.3862943611198906);   // (1 / c)
+        p[2] = fma(v11, q, v11 * ql);
+        p[3] = -fma(v01 + v10, q, (v01 + v10) * ql);
+        p[4] = fma(v00, q, v00 * ql);
         p[5] = w / sqrt(tpd * det);
         const double off = v01 + v10;
         tame = p[2] < 0.0 && p[4] < 0.0 && 4.0 * v00 * v11 > off * off && p[2] > -1e100 &&
@@ -170,12 +189,16 @@ em_fit_kernel(const double* __restrict__ img, int n, int ny, int nx,
 #pragma unroll
         for (int v = 0; v < kM; v++) acc[v] = 0.0;
         auto e_step = [&](auto table) {
-            int ix = tid % nx, run = tid / nx;
-            for (; run < groups; ix += step_x, run += step_g) {
-                if (ix >= nx) {
-                    ix -= nx;
-                    if (++run >= groups) break;
+            int qx = tid % nx, qr = tid / nx;
+            bool back = false;
+            while (qr < groups) {
+                if (qx >= nx) {
+                    qx -= nx;
+                    if (++qr >= groups) break;
                 }
+                const int q = qr * nx + qx;
+                if (mirror && 2 * q >= N) break;
+                const int ix = back ? nx - 1 - qx : qx, run = back ? groups - 1 - qr : qr;
                 const int ra = run * rows, rb = min(ny, ra + rows);
                 const double x = (double)(x0 + ix);
                 double ca[K], cb[K], S0[K], Sy[K];
@@ -230,6 +253,11 @@ em_fit_kernel(const double* __restrict__ img, int n, int ny, int nx,
                     acc[6 * k + 2] += Sy[k];
                     acc[6 * k + 3] = fma(xs, x, acc[6 * k + 3]);
                     acc[6 * k + 4] = fma(x, Sy[k], acc[6 * k + 4]);
+                }
+                back = mirror && !back && 2 * q + 1 < N;   // the middle run is its own mirror image
+                if (!back) {
+                    qx += step_x;
+                    qr += step_g;
                 }
             }
         };
