@@ -450,3 +450,16 @@ def test_blobs_with_an_undetermined_parameter_do_not_crawl(tb):
     for sigma, b, _, _, converged in plain.optimum_distance(w, data, inv, f.result(), st['status'],
                                                             [0, 1], f.dev):
         assert converged and sigma < 1e-3, (b, sigma)
+
+
+@pytest.mark.parametrize('unit_tiles', [1, 3, 64, 100])
+def test_unit_tiles_are_the_callers(tb, unit_tiles):
+    """A caller's unit_tiles is the size of the pass units, whatever the fitter
+    would choose: ceil(active tiles / unit_tiles) units per image."""
+    from tractor_b200 import fit
+    w = fit.blob_workload(2, np.random.default_rng(41), side_range=(300, 400))
+    data, inv = fit.render_blobs(w, w['truth'], seed=5)
+    f = fit.BlobFitter(w['blob_src'], w['sides'], w['psf'], w['sources'], w['start'], data, inv,
+                       unit_tiles=unit_tiles)
+    assert np.all(f.blobs_np['n_active'] > 64)
+    assert np.array_equal(f.blobs_np['n_slices'], 3 * -(-f.blobs_np['n_active'] // unit_tiles))

@@ -25,7 +25,7 @@ import torch
 from . import _lib, batch, render
 
 NPAR = _lib.FIT_NPAR
-UNIT_TILES = 64      # active 32 x 8 tiles per pass unit at most (larger images are split)
+UNIT_TILES = 64      # most active 32 x 8 tiles of a pass unit that the fitter chooses
 SERSIC_MIN, SERSIC_MAX = 0.29, 6.3
 
 
@@ -41,11 +41,11 @@ class BlobFitter(object):
     data, inverr: float32 device tensors, unit (blob, band) images packed in
                 blob-major, band-minor order (see `pix_offsets`);
     unit_tiles: active 32 x 8 tiles per pass unit at most (a (blob, band)
-                image with more is split into that many units, each with its
-                own partial normal-equation slice)."""
+                image with more is split into units of that many, each with its
+                own partial normal-equation slice); None: pass_unit_tiles."""
 
     def __init__(self, blob_src, sides, psf, sources, params0, data, inverr, n_bands=3,
-                 cd_inv=None, unit_tiles=UNIT_TILES):
+                 cd_inv=None, unit_tiles=None):
         lib = _lib.load()
         self.dev = render.device()
         self.n_bands = int(n_bands)
@@ -70,10 +70,11 @@ class BlobFitter(object):
         # a band's active tiles go to pass units of a few tiles, each with its
         # own partial blocks (slices), so that no unit holds one CTA for long
         # while few blobs are still running
+        if unit_tiles is None:
+            unit_tiles = pass_unit_tiles(n_active, P, self.n_bands)
         unit_tiles = int(unit_tiles)
         if unit_tiles < 1:
             raise ValueError('unit_tiles must be positive')
-        unit_tiles = min(unit_tiles, pass_unit_tiles(n_active, P, self.n_bands))
         parts = np.maximum(1, -(-n_active // unit_tiles)).astype(np.int64)
         n_slices = self.n_bands * parts
         blobs['n_slices'] = n_slices
