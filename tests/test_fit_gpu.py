@@ -463,3 +463,85 @@ def test_unit_tiles_are_the_callers(tb, unit_tiles):
                        unit_tiles=unit_tiles)
     assert np.all(f.blobs_np['n_active'] > 64)
     assert np.array_equal(f.blobs_np['n_slices'], 3 * -(-f.blobs_np['n_active'] // unit_tiles))
+
+
+@pytest.mark.parametrize('unit_tiles', [1, None])
+@pytest.mark.parametrize('n_bands', [1, 2, 3])
+@pytest.mark.parametrize('precise', [False, True])
+def test_mixed_profiles_crowd_tiles(tb, oracle, precise, n_bands, unit_tiles):
+    """Both precisions of the pass where six point, exponential, de Vaucouleurs
+    and Sersic sources share tiles in ever other sets, also in units of one tile
+    whose slices hold different sources: the assembled A^T A and A^T r against
+    FP64 central differences of the oracle's model (1e-4 of their scales in
+    FP32, 1e-6 in FP64: the differences' own error), chi^2 to 1e-5 and 1e-9;
+    parameters that a profile or a band does not have hold zeros."""
+    import torch
+    from tractor_b200 import fit, _lib
+    rng = np.random.default_rng(51)
+    W, H, n = 75, 61, 6
+    w = fit.blob_workload(1, rng, side_range=(64, 64), n_bands=n_bands)
+    prof = np.array([_lib.PROFILE_POINT, _lib.PROFILE_EXP, _lib.PROFILE_DEV, _lib.PROFILE_SERSIC,
+                     _lib.PROFILE_SERSIC, _lib.PROFILE_POINT])
+    p = np.zeros((n, 9))
+    p[:, 0], p[:, 1] = np.linspace(12., W - 14.3, n), np.linspace(H - 9.2, 11., n)
+    p[:, 2:2 + n_bands] = rng.uniform(500., 3000., (n, n_bands))
+    gal = prof != _lib.PROFILE_POINT
+    p[gal, 5], p[gal, 6:8] = rng.uniform(0., 1., gal.sum()), rng.uniform(-.3, .3, (gal.sum(), 2))
+    p[3:5, 8] = 1.3, 4.4
+    src = np.zeros(n, w['sources'].dtype)
+    src['profile'] = prof
+    hw = rng.integers(9, 18, n)
+    src['x0'], src['y0'] = p[:, 0].astype(int) - hw, p[:, 1].astype(int) - hw
+    src['w'], src['h'] = 2 * hw + 1, 2 * hw
+    data = rng.normal(2., 1., (n_bands, H, W)).astype(np.float32)
+    inv = rng.uniform(.3, 1., (n_bands, H, W)).astype(np.float32)
+    f = fit.BlobFitter(np.array([0, n]), np.array([[W, H]]), w['psf'], src, p,
+                       torch.from_numpy(data.ravel()).cuda(), torch.from_numpy(inv.ravel()).cuda(),
+                       n_bands=n_bands, unit_tiles=unit_tiles)
+    f.reset(p, 1e-9)
+    f._iteration(0., 100, precise=precise)
+
+    def model(q):
+        """The oracle's model; exp and deV sources through their own mixtures."""
+        out = np.zeros((n_bands, H, W))
+        for k in range(n_bands):
+            pamp, pmean, pvar = w['psf'][0][k]
+            for th, pr, r in zip(q, prof, src):
+                X0, Y0 = max(r['x0'], 0), max(r['y0'], 0)
+                X1, Y1 = min(r['x0'] + r['w'], W), min(r['y0'] + r['h'], H)
+                if pr == _lib.PROFILE_SERSIC:
+                    a, v = oracle.sersic_profile(th[8])
+                elif pr == _lib.PROFILE_POINT:
+                    a, v = np.ones(1), np.zeros(1)
+                else:
+                    a, v = (oracle.exp_profile if pr == _lib.PROFILE_EXP else
+                            oracle.dev_profile)()
+                T = oracle.nullwcs_cdinv() @ oracle.ellipseE_basis(
+                    *oracle.ellipseESoft_to_E(*th[5:8]))
+                M = np.zeros((2, 2)) if pr == _lib.PROFILE_POINT else T @ T.T
+                amp = (pamp[:, None] * a).ravel()
+                mean = np.repeat(pmean, len(a), 0)
+                var = (pvar[:, None] + v[None, :, None, None] * M).reshape(-1, 2, 2)
+                out[k, Y0:Y1, X0:X1] += th[2 + k] * oracle.mog_grid(X0, X1, Y0, Y1, th[0], th[1],
+                                                                    amp, mean, var)
+        return out
+
+    step = np.tile([1e-5, 1e-5, 1., 1., 1., 1e-5, 1e-5, 1e-5, 1e-5], (n, 1))
+    has = np.ones((n, 9), bool)
+    has[:, 2 + n_bands:5] = False
+    has[~gal, 5:] = False
+    has[prof != _lib.PROFILE_SERSIC, 8] = False
+    A = np.zeros((n * 9, data.size))
+    for i in np.flatnonzero(has):
+        hi, lo = p.copy(), p.copy()
+        hi.flat[i] += step.flat[i]
+        lo.flat[i] -= step.flat[i]
+        A[i] = ((model(hi) - model(lo)) / (2 * step.flat[i]) * inv).ravel()
+    r = ((data - model(p)) * inv).ravel()
+    Ho, go, c2 = A @ A.T, A @ r, float(r @ r)
+    Hg, gg = f.normal_equations(0)
+    tol, ctol = (1e-6, 1e-9) if precise else (1e-4, 1e-5)
+    d = np.sqrt(np.diag(Ho))
+    assert np.all(np.abs(Hg - Ho) <= tol * np.outer(d, d))
+    assert np.all(np.abs(gg - go) <= tol * d * np.sqrt(c2))
+    assert abs(f.states()['chi2'][0] - c2) <= ctol * c2
