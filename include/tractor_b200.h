@@ -389,6 +389,19 @@ int tb_galaxy_fft_render(const tb_galaxy_src* srcs, int32_t n, const tb_fft_imag
                          tb_fft_item* items, int32_t* flags, int32_t* work_counter,
                          tb_status* status, void* stream);
 
+/* tb_galaxy_fft_prep and tb_fourier_render_split in two launches: the galaxies
+ * are prepared and sorted by FFT size in one, rendered in the other.  Results,
+ * items, components and flags as of the two calls one after the other;
+ * workspace as tb_fourier_render_split's.  The per-source work of
+ * ProfileGalaxy._realGetUnitFluxModelPatch (tractor/galaxy.py:336-519), as
+ * tb_galaxy_fft_render. */
+int tb_galaxy_fft_render_sorted(const tb_galaxy_src* srcs, int32_t n, const tb_fft_image* image,
+                                const tb_profile_tables* tables, const float* psf_spec,
+                                float* out, tb_fft_item* items, double* comp_amp,
+                                double* comp_var, int32_t comp_stride, int32_t* flags,
+                                void* workspace, int64_t workspace_bytes, tb_status* status,
+                                void* stream);
+
 /* Jacobian items of n galaxies: items[7 i + j] for the parameters j = x, y,
  * counts, s0, s1, s2 (shape, per shape_type), Sersic n of source i, on the
  * geometry tb_galaxy_fft_prep gives its value item, with out_off =

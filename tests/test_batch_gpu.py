@@ -234,3 +234,55 @@ def test_scratch_is_bounded(tb):
     for n in range(20, 41):
         r.render_device(d, n, out)
     assert len(r._scratch.pool) == 2
+
+
+@pytest.mark.parametrize('n', [1, 40, 333])
+def test_sorted_render_equals_its_two_calls(tb, n):
+    """tb_galaxy_fft_render_sorted against tb_galaxy_fft_prep +
+    tb_fourier_render_split: the same items, flags and pixels, bit for bit, for
+    ragged patches of every FFT size and profile, windows at the FFT box's edge,
+    sources off their mask and of zero flux."""
+    import ctypes
+    import torch
+    from tractor_b200 import _lib, batch, render
+    rng = np.random.default_rng(76 + n)
+    r = batch.FourierGalaxyRenderer(batch.moffat_psf(21))
+    sides = np.round(np.exp(rng.uniform(np.log(14), np.log(253), n))).astype(int)
+    sides[::7] = 253
+    s = batch.sersic_sources(n, rng, mask=sides)
+    s['profile'] = rng.integers(0, 4, n)
+    s['counts'][5::11] = 0.
+    s['px'][6::13] += 4000.
+    d = torch.from_numpy(s.view(np.uint8).copy()).cuda()
+    npix = int((s['mw'].astype(np.int64) * s['mh']).sum())
+    outs = []
+    for two in (False, True):
+        out = torch.full((npix,), -3., device='cuda')
+        items, camp, cvar, flags, misc = r._work(n)
+        if two:
+            lib = _lib.load()
+            st = _lib.stream_ptr()
+            _lib.check(lib.tb_galaxy_fft_prep(
+                d.data_ptr(), n, ctypes.addressof(r.image), ctypes.addressof(r.tables.struct),
+                items.data_ptr(), camp.data_ptr(), cvar.data_ptr(), batch.COMP_STRIDE,
+                flags.data_ptr(), st), 'prep')
+            render.fourier_render(items.data_ptr(), n, camp.data_ptr(), cvar.data_ptr(),
+                                  r.spec.data_ptr(), out.data_ptr(), misc.data_ptr() + 16,
+                                  method='split')
+        else:
+            r.render_device(d, n, out, method='split')
+        outs.append([out] + [t.clone() for t in (items, flags, misc[4:8])])
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+
+
+def test_choice_of_method(tb):
+    """`choose`: one launch up to a galaxy per SM, the sorted path at FFT size
+    256 and for many, the persistent one for a few of the smallest per SM."""
+    from tractor_b200 import batch
+    r = batch.FourierGalaxyRenderer(batch.moffat_psf(21))
+    m = r.sms
+    for n, side, want in ((1, 32, 'fused'), (m, 100, 'fused'), (m + 1, 100, 'split'),
+                          (m + 1, 40, 'persistent'), (3 * m + 1, 40, 'split'), (1, 128, 'split'),
+                          (2000, 253, 'split')):
+        assert r.choose(n, n * side * side) == want

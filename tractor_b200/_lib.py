@@ -138,6 +138,8 @@ SIGNATURES = {
     'tb_fourier_render_deriv': (_I32, [_P, _I32, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     'tb_fourier_workspace': (_I32, [_I32, _P]),
     'tb_fourier_render_split': (_I32, [_P, _I32, _P, _P, _P, _P, _P, _P, _P, _I64, _P, _P]),
+    'tb_galaxy_fft_render_sorted': (_I32, [_P, _I32, _P, _P, _P, _P, _P, _P, _P, _I32, _P, _P,
+                                           _I64, _P, _P]),
     'tb_galaxy_fft_vjp_workspace': (_I32, [_I32, _P]),
     'tb_galaxy_fft_vjp': (_I32, [_P, _I32, _P, _P, _P, _P, _P, _P, _P, _I64, _P, _P]),
     'tb_scene_prep': (_I32, [_P, _I32, _P, _I32, _P, _P, _P, _P, _P, _P, _P, _P, _I32, _P]),

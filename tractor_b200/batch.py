@@ -3,8 +3,8 @@
 FourierGalaxyRenderer renders thousands of galaxies through the
 pixelized-PSF Fourier path of ProfileGalaxy._realGetUnitFluxModelPatch
 (tractor/galaxy.py:336-519): tb_galaxy_fft_prep turns source parameters into
-work items and component tables on the device, and tb_fourier_render_split
-renders every item (sorted by FFT size); a few galaxies take one launch,
+work items and component tables on the device, sorted by FFT size, and renders
+every item (tb_galaxy_fft_render_sorted); a few small galaxies take one launch,
 tb_galaxy_fft_render.
 """
 import ctypes
@@ -114,6 +114,7 @@ class FourierGalaxyRenderer(object):
         self.spec = torch.cat(specs)
         self.image = img
         self.tables = device_profile_tables()
+        self.sms = torch.cuda.get_device_properties(render.device()).multi_processor_count
         # items, component amplitudes and variances, the sorted path's workspace
         self._scratch = _lib.Scratch(lambda m: (
             m * _lib.FFT_ITEM.itemsize, m * COMP_STRIDE * 8, m * COMP_STRIDE * 32,
@@ -133,23 +134,37 @@ class FourierGalaxyRenderer(object):
         return w[1][3], w[2][3]
 
     METHODS = ('fused', 'persistent', 'split')
-    # one launch in place of three: 17 against 29 us for one 32-px patch; from
-    # about 30 patches of 100-200 px (77 us both) the sorted path is faster
-    FUSED_MAX = 24
+
+    def choose(self, n, pixels):
+        """The method of a call without one, by its galaxies and output pixels
+        (patches lie back to back, so pixels / n tells the FFT size): us of
+        fused / persistent / split for n = 24, 148, 256, 444 and 600:
+            24-48 px (64)   22 25 34, 22 26 36, 34 30 36, 46 37 38, 65 44 38
+            90 px (128)     31 35 38, 32 36 40, 52 49 40, 73 64 57, 108 90 67
+            128 px (256)    50 51 47, 50 52 49, 88 78 74, 127 109 101, 192 157 145
+            200 px          80 78 76, 81 80 78, 147 135 131, 218 194 189, 340 293 281
+            253 px          182 186 143, 183 188 145, 351 350 263, 527 531 393, 853 848 626
+        Up to one galaxy per SM the one launch of 'fused' is the shortest where a
+        galaxy is short itself; of the smallest, a few per SM, 'persistent'; from
+        there on, and always at FFT size 256, 'split'.  'fused' and 'persistent'
+        agree bit for bit, 'split' with them to FP32 rounding."""
+        if pixels >= n * 112 ** 2:
+            return 'split'
+        if n <= self.sms:
+            return 'fused'
+        return 'persistent' if pixels <= n * 56 ** 2 and n <= 3 * self.sms else 'split'
 
     def render_device(self, srcs, n, out, stream=None, method=None):
         """Renders n sources whose GALAXY_SRC records are in device tensor
         `srcs` (uint8 view) into float32 device tensor `out`; nothing is
         copied to or from the host.  method: 'fused' (tb_galaxy_fft_render:
         preparation and render in one persistent launch), 'persistent' or
-        'split' (tb_galaxy_fft_prep, then tb_fourier_render /
-        tb_fourier_render_split); None: the method autotune chose, else
-        'fused' for a few sources and 'split' for more (FUSED_MAX).  Returns
-        the flags tensor (see tb_galaxy_fft_prep)."""
+        'split' (tb_galaxy_fft_prep and tb_fourier_render, or
+        tb_galaxy_fft_render_sorted); None: the method autotune chose, else
+        `choose`.  Returns the flags tensor (see tb_galaxy_fft_prep)."""
         lib = _lib.load()
         _, (items, camp, cvar, ws), nbytes, flags, misc, s = self._scratch.get(n, stream)
-        method = method or getattr(self, 'method', None) or (
-            'fused' if n <= self.FUSED_MAX else 'split')
+        method = method or getattr(self, 'method', None) or self.choose(n, out.numel())
         if method == 'fused':
             rc = lib.tb_galaxy_fft_render(srcs.data_ptr(), n, ctypes.addressof(self.image),
                                           ctypes.addressof(self.tables.struct),
@@ -158,13 +173,19 @@ class FourierGalaxyRenderer(object):
                                           s)
             _lib.check(rc, 'tb_galaxy_fft_render')
             return flags
+        if method == 'split':
+            rc = lib.tb_galaxy_fft_render_sorted(
+                srcs.data_ptr(), n, ctypes.addressof(self.image),
+                ctypes.addressof(self.tables.struct), self.spec.data_ptr(), out.data_ptr(), items,
+                camp, cvar, COMP_STRIDE, flags.data_ptr(), ws, nbytes[3], misc.data_ptr() + 16, s)
+            _lib.check(rc, 'tb_galaxy_fft_render_sorted')
+            return flags
         rc = lib.tb_galaxy_fft_prep(srcs.data_ptr(), n, ctypes.addressof(self.image),
                                     ctypes.addressof(self.tables.struct), items, camp, cvar,
                                     COMP_STRIDE, flags.data_ptr(), s)
         _lib.check(rc, 'tb_galaxy_fft_prep')
         render.fourier_render(items, n, camp, cvar, self.spec.data_ptr(), out.data_ptr(),
-                              misc.data_ptr() + 16, stream=stream, method=method,
-                              workspace=(ws, nbytes[3]))
+                              misc.data_ptr() + 16, stream=stream, method=method)
         return flags
 
     def autotune(self, srcs, n, out):

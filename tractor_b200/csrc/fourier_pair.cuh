@@ -404,8 +404,26 @@ __device__ void pair_size(unsigned char* smem, const tb_fft_item* __restrict__ i
     }
 }
 
-// All items of a call: those outside this path as fourier_render_kernel
-// renders them, then the lists by size.
+// A list rendered as by fourier_render_kernel, a CTA per item.  A call, not
+// inlined: each part of the kernel then has all 128 registers (4 bytes of spills
+// in place of 168; a galaxy whose window reaches the box's edge 194 -> 143 us,
+// 256 of 128 px 76 -> 74).
+template <bool kDeriv>
+__device__ __noinline__ void whole_cta_list(const tb_fft_item* __restrict__ items, int n_items,
+                                            const double* __restrict__ amp,
+                                            const double* __restrict__ var,
+                                            const float* __restrict__ psf_spec,
+                                            float* __restrict__ out, int32_t* next, tb_status* st,
+                                            const int32_t* __restrict__ list, int count,
+                                            unsigned char* smem) {
+    render_items<kDeriv>(items, n_items, amp, var, nullptr, psf_spec, out, nullptr, next, st, list,
+                         count, smem);
+}
+
+// All items of a call: those outside this path first (an item at the box's edge
+// takes several times as long as another; kDeriv: position derivatives among
+// them), then the lists by size.
+template <bool kDeriv>
 __global__ void __launch_bounds__(kPairThreads, 1)
 fourier_pair_kernel(const tb_fft_item* __restrict__ items, int n_items,
                     const double* __restrict__ amp, const double* __restrict__ var,
@@ -413,22 +431,32 @@ fourier_pair_kernel(const tb_fft_item* __restrict__ items, int n_items,
                     const int32_t* __restrict__ lists, tb_status* st) {
     static_assert(kPairThreads == kThreads && kPairSmem >= kSmemBytes, "one block shape for both");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // (first: an item at the box's edge takes several times as long as another)
-    if (ws->count[4] != 0)
-        render_items<true>(items, n_items, amp, var, nullptr, psf_spec, out, nullptr,
-                           &ws->next[4], st, lists + 4 * (int64_t)n_items, ws->count[4], smem_raw);
-    pair_size<256>(smem_raw, items, lists, ws->count[0], &ws->next[0], amp, var, psf_spec, out);
-    pair_size<128>(smem_raw, items, lists + n_items, ws->count[1], &ws->next[1], amp, var,
-                   psf_spec, out);
-    pair_size<64>(smem_raw, items, lists + 2 * (int64_t)n_items, ws->count[2], &ws->next[2], amp,
-                  var, psf_spec, out);
-    pair_size<32>(smem_raw, items, lists + 3 * (int64_t)n_items, ws->count[3], &ws->next[3], amp,
-                  var, psf_spec, out);
+    const int4 c = *reinterpret_cast<const int4*>(ws->count);   // (one load, not one for each list)
+    const int rest = ws->count[4];
+    if (rest != 0)
+        whole_cta_list<kDeriv>(items, n_items, amp, var, psf_spec, out, &ws->next[4], st,
+                               lists + 4 * (int64_t)n_items, rest, smem_raw);
+    pair_size<256>(smem_raw, items, lists, c.x, &ws->next[0], amp, var, psf_spec, out);
+    pair_size<128>(smem_raw, items, lists + n_items, c.y, &ws->next[1], amp, var, psf_spec, out);
+    pair_size<64>(smem_raw, items, lists + 2 * (int64_t)n_items, c.z, &ws->next[2], amp, var,
+                  psf_spec, out);
+    pair_size<32>(smem_raw, items, lists + 3 * (int64_t)n_items, c.w, &ws->next[3], amp, var,
+                  psf_spec, out);
 }
 
-// Sorts the items into the lists by FFT size; those outside this path (a
-// window at the box's edge, position derivatives, many components) go to
-// list 4.  Up to kSortItems items one CTA does it all (alone:
+// The list of an item: by FFT size, or 4 outside this path (a window at the
+// box's edge, position derivatives, many components); -1 and a report for a
+// bad one.
+__device__ __forceinline__ int pair_list(const tb_fft_item& it, int i, tb_status* st) {
+    if (!item_ok(it, nullptr)) {
+        tb::report(st, TB_STATUS_BAD_ITEM, i, it.sz);
+        return -1;
+    }
+    return it.dmode != TB_FFT_VALUE || it.K > kPairMaxK || !split_eligible(it) ? 4
+           : it.sz == 256 ? 0 : it.sz == 128 ? 1 : it.sz == 64 ? 2 : 3;
+}
+
+// Sorts the items into their lists.  Up to kSortItems items one CTA does it all (alone:
 // the counters and the status word are cleared here); more, many CTAs after
 // memsets.
 constexpr int kSortThreads = 512, kSortItems = 4096;
@@ -445,14 +473,7 @@ fourier_sort_kernel(const tb_fft_item* __restrict__ items, int n,
     const int lane = threadIdx.x & 31;
     for (int i0 = blockIdx.x * kSortThreads; i0 < n; i0 += gridDim.x * kSortThreads) {
         const int i = i0 + threadIdx.x;
-        int c = -1;
-        if (i < n) {
-            const tb_fft_item it = items[i];
-            if (!item_ok(it, nullptr)) tb::report(st, TB_STATUS_BAD_ITEM, i, it.sz);
-            else
-                c = it.dmode != TB_FFT_VALUE || it.K > kPairMaxK || !split_eligible(it) ? 4
-                    : it.sz == 256 ? 0 : it.sz == 128 ? 1 : it.sz == 64 ? 2 : 3;
-        }
+        const int c = i < n ? pair_list(items[i], i, st) : -1;
         for (int q = 0; q < 5; q++) {   // one atomic per warp and list
             const unsigned m = __ballot_sync(0xffffffffu, c == q);
             if (m == 0) continue;
@@ -462,4 +483,25 @@ fourier_sort_kernel(const tb_fft_item* __restrict__ items, int n,
             if (c == q) lists[q * (int64_t)n + base + __popc(m & ((1u << lane) - 1u))] = i;
         }
     }
+}
+
+// Galaxies prepared and sorted in one launch, a warp each (the lists' counters
+// and the status word cleared before).
+constexpr int kPrepSortThreads = 128;
+
+__global__ void __launch_bounds__(kPrepSortThreads)
+galaxy_prep_sort_kernel(const tb_galaxy_src* __restrict__ srcs, int n, tb_fft_image img,
+                        tb_profile_tables Tg, tb_fft_item* __restrict__ items,
+                        double* __restrict__ camp, double* __restrict__ cvar, int stride,
+                        int32_t* __restrict__ flags, PairWs* ws, int32_t* __restrict__ lists,
+                        tb_status* st) {
+    const tb_profile_tables T = Tg;   // (read where they lie, as by tb_galaxy_fft_prep)
+    const int lane = threadIdx.x & 31;
+    const int i = blockIdx.x * (kPrepSortThreads / 32) + (threadIdx.x >> 5);
+    if (i >= n) return;   // whole warps leave together
+    tb_fft_item it;
+    tb::prep_galaxy_tables(srcs, i, img, T, lane, items, camp, cvar, stride, flags, it);
+    if (lane != 0) return;
+    const int c = pair_list(it, i, st);
+    if (c >= 0) lists[c * (int64_t)n + atomicAdd(&ws->count[c], 1)] = i;
 }

@@ -941,6 +941,19 @@ extern "C" int tb_galaxy_fft_render(const tb_galaxy_src* srcs, int32_t n,
 
 namespace {
 int64_t list_bytes(int32_t n_items) { return ((int64_t)n_items * 4 * 5 + 255) / 256 * 256; }
+
+template <bool kDeriv>
+int launch_pairs(const tb_fft_item* items, int32_t n_items, const double* comp_amp,
+                 const double* comp_var, const float* psf_spec, float* out, PairWs* ws,
+                 const int32_t* lists, tb_status* status, cudaStream_t s) {
+    if (cudaFuncSetAttribute(fourier_pair_kernel<kDeriv>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem) != cudaSuccess)
+        return TB_ERR_LAUNCH;
+    const int grid = n_items < tb::num_sms() ? n_items : tb::num_sms();
+    fourier_pair_kernel<kDeriv><<<grid, kPairThreads, kPairSmem, s>>>(
+        items, n_items, comp_amp, comp_var, psf_spec, out, ws, lists, status);
+    return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
+}
 }  // namespace
 
 extern "C" int tb_fourier_workspace(int32_t n_items, int64_t* bytes) {
@@ -971,10 +984,6 @@ extern "C" int tb_fourier_render_split(const tb_fft_item* items, int32_t n_items
     if (comp_dcoef || dots)
         return launch_fourier(items, n_items, comp_amp, comp_var, comp_dcoef, psf_spec, out, dots,
                               &ws->next[4], status, stream);
-    if (cudaFuncSetAttribute(fourier_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kPairSmem) != cudaSuccess)
-        return TB_ERR_LAUNCH;
-    const int grid = n_items < tb::num_sms() ? n_items : tb::num_sms();
     if (n_items <= kSortItems) {
         fourier_sort_kernel<<<1, kSortThreads, 0, s>>>(items, n_items, ws, lists, status, true);
     } else {
@@ -984,9 +993,37 @@ extern "C" int tb_fourier_render_split(const tb_fft_item* items, int32_t n_items
         fourier_sort_kernel<<<(n_items + kSortThreads - 1) / kSortThreads, kSortThreads, 0, s>>>(
             items, n_items, ws, lists, status, false);
     }
-    fourier_pair_kernel<<<grid, kPairThreads, kPairSmem, s>>>(
-        items, n_items, comp_amp, comp_var, psf_spec, out, ws, lists, status);
-    return cudaGetLastError() == cudaSuccess ? TB_OK : TB_ERR_LAUNCH;
+    return launch_pairs<true>(items, n_items, comp_amp, comp_var, psf_spec, out, ws, lists, status,
+                              s);
+}
+
+extern "C" int tb_galaxy_fft_render_sorted(const tb_galaxy_src* srcs, int32_t n,
+                                           const tb_fft_image* image,
+                                           const tb_profile_tables* tables, const float* psf_spec,
+                                           float* out, tb_fft_item* items, double* comp_amp,
+                                           double* comp_var, int32_t comp_stride, int32_t* flags,
+                                           void* workspace, int64_t workspace_bytes,
+                                           tb_status* status, void* stream) {
+    if (n < 0) return TB_ERR_ARG;
+    if (n == 0) return TB_OK;
+    if (!srcs || !image || !tables || !psf_spec || !out || !items || !comp_amp || !comp_var ||
+        !flags || !workspace)
+        return TB_ERR_ARG;
+    if (comp_stride < tb::kMaxComp) return TB_ERR_SIZE;
+    if ((reinterpret_cast<uintptr_t>(workspace) & 255) != 0) return TB_ERR_ARG;
+    int64_t need = 0;
+    tb_fourier_workspace(n, &need);
+    if (workspace_bytes < need) return TB_ERR_SIZE;
+    cudaStream_t s = (cudaStream_t)stream;
+    PairWs* ws = static_cast<PairWs*>(workspace);
+    int32_t* lists = reinterpret_cast<int32_t*>(static_cast<char*>(workspace) + sizeof(PairWs));
+    if (cudaMemsetAsync(ws, 0, sizeof(PairWs), s) != cudaSuccess) return TB_ERR_LAUNCH;
+    if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
+        return TB_ERR_LAUNCH;
+    constexpr int kPerBlock = kPrepSortThreads / 32;
+    galaxy_prep_sort_kernel<<<(n + kPerBlock - 1) / kPerBlock, kPrepSortThreads, 0, s>>>(
+        srcs, n, *image, *tables, items, comp_amp, comp_var, comp_stride, flags, ws, lists, status);
+    return launch_pairs<false>(items, n, comp_amp, comp_var, psf_spec, out, ws, lists, status, s);
 }
 
 extern "C" int tb_galaxy_fft_vjp_workspace(int32_t n, int64_t* bytes) {

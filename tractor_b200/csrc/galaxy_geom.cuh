@@ -101,4 +101,31 @@ __device__ inline int prep_galaxy_warp(const tb_galaxy_src& s, const tb_fft_imag
     return K;
 }
 
+// Source i prepared by one warp into the tables: its components at i * stride,
+// its item (which lane 0 returns with c0 set) and flag.
+__device__ inline void prep_galaxy_tables(const tb_galaxy_src* __restrict__ srcs, int i,
+                                          const tb_fft_image& img, const tb_profile_tables& T,
+                                          int lane, tb_fft_item* __restrict__ items,
+                                          double* __restrict__ camp, double* __restrict__ cvar,
+                                          int stride, int32_t* __restrict__ flags,
+                                          tb_fft_item& it) {
+    const tb_galaxy_src s = srcs[i];
+    double a, v, M[3];
+    int rank, flag;
+    const int K = prep_galaxy_warp(s, img, T, lane, a, v, rank, M, flag, it);
+    it.c0 = i * stride;
+    if (flag == 0 && lane < K) {
+        camp[it.c0 + rank] = a;
+        double* w = cvar + 4 * (it.c0 + rank);
+        w[0] = v * M[0];
+        w[1] = v * M[1];
+        w[2] = v * M[1];
+        w[3] = v * M[2];
+    }
+    if (lane == 0) {
+        items[i] = it;
+        flags[i] = flag;
+    }
+}
+
 }  // namespace tb

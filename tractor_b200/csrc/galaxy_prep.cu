@@ -37,27 +37,8 @@ galaxy_fft_prep_kernel(const tb_galaxy_src* __restrict__ srcs, int n, tb_fft_ima
     const int lane = threadIdx.x & 31;
     const int i = blockIdx.x * (kPrepThreads / 32) + (threadIdx.x >> 5);
     if (i >= n) return;   // whole warps leave together
-    const tb_galaxy_src s = srcs[i];
-    // profile (lane l holds component l, ranked by variance), shape -> pixel
-    // factor M = T T^T, geometry and the item
-    double a, v, M[3];
-    int rank, flag;
     tb_fft_item it;
-    const int K = tb::prep_galaxy_warp(s, img, T, lane, a, v, rank, M, flag, it);
-    const int c0 = i * stride;
-    if (flag == 0 && lane < K) {
-        camp[c0 + rank] = a;
-        double* w = cvar + 4 * (c0 + rank);
-        w[0] = v * M[0];
-        w[1] = v * M[1];
-        w[2] = v * M[1];
-        w[3] = v * M[2];
-    }
-    if (lane == 0) {
-        it.c0 = c0;
-        items[i] = it;
-        flags[i] = flag;
-    }
+    tb::prep_galaxy_tables(srcs, i, img, T, lane, items, camp, cvar, stride, flags, it);
 }
 
 
