@@ -412,11 +412,13 @@ template <bool kDeriv>
 __device__ __noinline__ void whole_cta_list(const tb_fft_item* __restrict__ items, int n_items,
                                             const double* __restrict__ amp,
                                             const double* __restrict__ var,
+                                            const double* __restrict__ dcoef,
                                             const float* __restrict__ psf_spec,
-                                            float* __restrict__ out, int32_t* next, tb_status* st,
+                                            float* __restrict__ out, double* __restrict__ dots,
+                                            int32_t* next, tb_status* st,
                                             const int32_t* __restrict__ list, int count,
                                             unsigned char* smem) {
-    render_items<kDeriv>(items, n_items, amp, var, nullptr, psf_spec, out, nullptr, next, st, list,
+    render_items<kDeriv>(items, n_items, amp, var, dcoef, psf_spec, out, dots, next, st, list,
                          count, smem);
 }
 
@@ -434,8 +436,8 @@ fourier_pair_kernel(const tb_fft_item* __restrict__ items, int n_items,
     const int4 c = *reinterpret_cast<const int4*>(ws->count);   // (one load, not one for each list)
     const int rest = ws->count[4];
     if (rest != 0)
-        whole_cta_list<kDeriv>(items, n_items, amp, var, psf_spec, out, &ws->next[4], st,
-                               lists + 4 * (int64_t)n_items, rest, smem_raw);
+        whole_cta_list<kDeriv>(items, n_items, amp, var, nullptr, psf_spec, out, nullptr,
+                               &ws->next[4], st, lists + 4 * (int64_t)n_items, rest, smem_raw);
     pair_size<256>(smem_raw, items, lists, c.x, &ws->next[0], amp, var, psf_spec, out);
     pair_size<128>(smem_raw, items, lists + n_items, c.y, &ws->next[1], amp, var, psf_spec, out);
     pair_size<64>(smem_raw, items, lists + 2 * (int64_t)n_items, c.z, &ws->next[2], amp, var,

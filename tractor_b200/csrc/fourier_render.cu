@@ -1054,7 +1054,8 @@ extern "C" int tb_galaxy_fft_vjp(const tb_fft_item* items, int32_t n, const doub
     if (cudaMemsetAsync(ws, 0, sizeof(PairWs), s) != cudaSuccess) return TB_ERR_LAUNCH;
     if (status && cudaMemsetAsync(status, 0, sizeof(tb_status), s) != cudaSuccess)
         return TB_ERR_LAUNCH;
-    const int grid = n < tb::num_sms() ? n : tb::num_sms();
+    // (a galaxy at the box's edge is seven items)
+    const int grid = 7 * (int64_t)n < tb::num_sms() ? 7 * n : tb::num_sms();
     fourier_vjp_sort_kernel<<<(n + 127) / 128, 128, 0, s>>>(items, n, comp_dcoef, ws, lists, dots,
                                                             status);
     fourier_vjp_kernel<<<grid, kPairThreads, kVjpSmem, s>>>(

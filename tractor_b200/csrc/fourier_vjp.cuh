@@ -385,8 +385,8 @@ fourier_vjp_kernel(const tb_fft_item* __restrict__ items, int n,
                    const int32_t* __restrict__ lists, tb_status* st) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (ws->count[4] != 0)
-        render_items<true>(items, 7 * n, amp, var, dcoef, psf_spec, grad, dots, &ws->next[4], st,
-                           lists + 4 * (int64_t)n, ws->count[4], smem_raw);
+        whole_cta_list<true>(items, 7 * n, amp, var, dcoef, psf_spec, grad, dots, &ws->next[4], st,
+                             lists + 4 * (int64_t)n, ws->count[4], smem_raw);
     vjp_size<256>(smem_raw, items, lists, ws->count[0], &ws->next[0], amp, var, dcoef, psf_spec,
                   grad, dots);
     vjp_size<128>(smem_raw, items, lists + n, ws->count[1], &ws->next[1], amp, var, dcoef,
