@@ -283,6 +283,6 @@ def test_choice_of_method(tb):
     r = batch.FourierGalaxyRenderer(batch.moffat_psf(21))
     m = r.sms
     for n, side, want in ((1, 32, 'fused'), (m, 100, 'fused'), (m + 1, 100, 'split'),
-                          (m + 1, 40, 'persistent'), (3 * m + 1, 40, 'split'), (1, 128, 'split'),
+                          (m + 1, 40, 'persistent'), (2 * m + 1, 40, 'split'), (1, 128, 'split'),
                           (2000, 253, 'split')):
         assert r.choose(n, n * side * side) == want

@@ -139,11 +139,11 @@ class FourierGalaxyRenderer(object):
         """The method of a call without one, by its galaxies and output pixels
         (patches lie back to back, so pixels / n tells the FFT size): us of
         fused / persistent / split for n = 24, 148, 256, 444 and 600:
-            24-48 px (64)   22 25 34, 22 26 36, 34 30 36, 46 37 38, 65 44 38
-            90 px (128)     31 35 38, 32 36 40, 52 49 40, 73 64 57, 108 90 67
-            128 px (256)    50 51 47, 50 52 49, 88 78 74, 127 109 101, 192 157 145
-            200 px          80 78 76, 81 80 78, 147 135 131, 218 194 189, 340 293 281
-            253 px          182 186 143, 183 188 145, 351 350 263, 527 531 393, 853 848 626
+            24-48 px (64)   21 24 35, 22 26 35, 34 30 33, 46 37 35, 65 46 35
+            90 px (128)     30 34 35, 31 36 35, 51 48 39, 72 65 57, 107 90 68
+            128 px (256)    50 50 47, 50 51 48, 87 78 74, 127 109 101, 192 157 146
+            200 px          80 78 76, 80 80 78, 147 136 132, 217 195 189, 339 294 283
+            253 px          182 186 143, 182 188 144, 351 351 264, 527 531 393, 854 848 628
         Up to one galaxy per SM the one launch of 'fused' is the shortest where a
         galaxy is short itself; of the smallest, a few per SM, 'persistent'; from
         there on, and always at FFT size 256, 'split'.  'fused' and 'persistent'
@@ -152,7 +152,7 @@ class FourierGalaxyRenderer(object):
             return 'split'
         if n <= self.sms:
             return 'fused'
-        return 'persistent' if pixels <= n * 56 ** 2 and n <= 3 * self.sms else 'split'
+        return 'persistent' if pixels <= n * 56 ** 2 and n <= 2 * self.sms else 'split'
 
     def render_device(self, srcs, n, out, stream=None, method=None):
         """Renders n sources whose GALAXY_SRC records are in device tensor

@@ -334,7 +334,7 @@ __device__ void vjp_source(const tb_fft_item* __restrict__ items, const VjpGroup
 
 template <int N>
 __device__ void vjp_size(unsigned char* smem, const tb_fft_item* __restrict__ items,
-                         const int32_t* __restrict__ list, int count, int32_t* next,
+                         const int32_t* __restrict__ list, int count, int total, int32_t* next,
                          const double* __restrict__ amp, const double* __restrict__ var,
                          const double* __restrict__ dcoef, const float* __restrict__ psf_spec,
                          const float* __restrict__ grad, double* __restrict__ dots) {
@@ -342,7 +342,7 @@ __device__ void vjp_size(unsigned char* smem, const tb_fft_item* __restrict__ it
     if (count == 0) return;   // the same in every thread
     const int g = threadIdx.x / Plan::Pair::kThreads;
     __syncthreads();   // the previous size's groups are done with shared memory
-    if (g >= Plan::Pair::kGroups) return;
+    if (g >= active_groups(Plan::Pair::kGroups, count, total)) return;
     unsigned char* p = smem + g * Plan::kBytes;
     auto take = [&](int bytes) {
         unsigned char* q = p;
@@ -384,17 +384,19 @@ fourier_vjp_kernel(const tb_fft_item* __restrict__ items, int n,
                    float* __restrict__ grad, double* __restrict__ dots, PairWs* ws,
                    const int32_t* __restrict__ lists, tb_status* st) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (ws->count[4] != 0)
+    const int4 c = *reinterpret_cast<const int4*>(ws->count);
+    const int rest = ws->count[4], total = c.x + c.y + c.z + c.w + rest;
+    if (rest != 0)
         whole_cta_list<true>(items, 7 * n, amp, var, dcoef, psf_spec, grad, dots, &ws->next[4], st,
-                             lists + 4 * (int64_t)n, ws->count[4], smem_raw);
-    vjp_size<256>(smem_raw, items, lists, ws->count[0], &ws->next[0], amp, var, dcoef, psf_spec,
+                             lists + 4 * (int64_t)n, rest, smem_raw);
+    vjp_size<256>(smem_raw, items, lists, c.x, total, &ws->next[0], amp, var, dcoef, psf_spec, grad,
+                  dots);
+    vjp_size<128>(smem_raw, items, lists + n, c.y, total, &ws->next[1], amp, var, dcoef, psf_spec,
                   grad, dots);
-    vjp_size<128>(smem_raw, items, lists + n, ws->count[1], &ws->next[1], amp, var, dcoef,
-                  psf_spec, grad, dots);
-    vjp_size<64>(smem_raw, items, lists + 2 * (int64_t)n, ws->count[2], &ws->next[2], amp, var,
-                 dcoef, psf_spec, grad, dots);
-    vjp_size<32>(smem_raw, items, lists + 3 * (int64_t)n, ws->count[3], &ws->next[3], amp, var,
-                 dcoef, psf_spec, grad, dots);
+    vjp_size<64>(smem_raw, items, lists + 2 * (int64_t)n, c.z, total, &ws->next[2], amp, var, dcoef,
+                 psf_spec, grad, dots);
+    vjp_size<32>(smem_raw, items, lists + 3 * (int64_t)n, c.w, total, &ws->next[3], amp, var, dcoef,
+                 psf_spec, grad, dots);
 }
 
 // Sorts the galaxies by FFT size; the seven items of one whose window does not
