@@ -28,7 +28,7 @@
 // the M step and the next iteration's parameters itself, so an iteration has
 // one block barrier.  100 iterations, 1024 stamps of 25 x 25 (against a pixel
 // stride per thread with exp(), divisions and a butterfly per moment): 1
-// component 487 -> 431 us, 3 components 1033 -> 797, 8 components 4589 -> 2661;
+// component 487 -> 410 us, 3 components 1033 -> 797, 8 components 4589 -> 2661;
 // 256 stamps of 63 x 63, 3 components 3080 -> 2391.
 //
 // Rounding: EM converges slowly, so the fixed point amplifies every rounding of an
@@ -37,8 +37,8 @@
 // costs no turn, a thread's runs of columns in mirrored pairs, whose first moments
 // cancel before they are rounded together.  After 1000 iterations, against
 // extended precision, over eight sets of stamps (15 to 27 px, 1 to 3 components)
-// the geometric means of the rms errors are 4.7e-16 in the amplitudes, 6.8e-16 in
-// the means and 6.6e-15 in the variances; with one pixel at a time, exp() and
+// the geometric means of the rms errors are 4.9e-16 in the amplitudes, 6.9e-16 in
+// the means and 6.9e-15 in the variances; with one pixel at a time, exp() and
 // divisions 4.6e-16, 7.0e-16 and 7.1e-15; without those three 5.3e-16, 1.0e-15 and
 // 8.4e-15 (1024 stamps, 3 components: 7.5 in place of 7.8 ms).
 #include <type_traits>
@@ -109,7 +109,9 @@ em_fit_kernel(const double* __restrict__ img, int n, int ny, int nx,
     // exponents in log2 units)
     __shared__ double par[kWarps][K][8];   // mean x, y, c00, c01, c11, scale
     __shared__ double red[2][kWarps][kM];
-    __shared__ double2 exp_tab[tb::kExpTab];
+    // (one component's responsibility is 1 but for rounding, whatever the exponential)
+    constexpr bool kFine = K > 1;
+    __shared__ std::conditional_t<kFine, double2, double> exp_tab[tb::kExpTab];
     const int s = blockIdx.x;
     if (s >= n) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -121,13 +123,14 @@ em_fit_kernel(const double* __restrict__ img, int n, int ny, int nx,
     const int y0 = xy0 ? xy0[2 * s + 1] : -(ny / 2);
     // The columns are cut into `groups` runs of `rows` pixels, taken by the
     // threads in turn: the cut that keeps the threads busiest, a run's start
-    // counted as two pixels.
+    // counted as half a pixel (as two, 300 iterations of 1024 stamps of 23 x 23, 3
+    // components, took 2574 us, 2490 with the rounding of before; now 2259).
     int groups = 1, rows = ny;
     {
         int best = 0x7fffffff;
         for (int g = 1; g <= max(8, kEmThreads / nx) && g <= ny; g++) {
             const int r = (ny + g - 1) / g;
-            const int cost = (nx * g + kEmThreads - 1) / kEmThreads * (r + 2);
+            const int cost = (nx * g + kEmThreads - 1) / kEmThreads * (2 * r + 1);
             if (cost < best) { best = cost; groups = g; rows = r; }
         }
     }
@@ -152,11 +155,14 @@ em_fit_kernel(const double* __restrict__ img, int n, int ny, int nx,
         p[1] = my;
         // q + ql = -log2(e) / (2 det): the quotient's remainder, the constant's
         // second part and the rounding of det
-        const double b = v01 * v10, be = fma(v01, v10, -b);
-        const double dl = (fma(v00, v11, -det) - b) - be;
         const double c = -0.5 * TB_LOG2E, q = c / det;
-        const double ql = ((fma(-q, det, c) - 0.5 * 2.0355273740931033e-17) - q * dl) *
-                          (q * -1.3862943611198906);   // (1 / c)
+        double ql = 0.0;
+        if constexpr (kFine) {
+            const double b = v01 * v10, be = fma(v01, v10, -b);
+            const double dl = (fma(v00, v11, -det) - b) - be;
+            ql = ((fma(-q, det, c) - 0.5 * 2.0355273740931033e-17) - q * dl) *
+                 (q * -1.3862943611198906);   // (1 / c)
+        }
         p[2] = fma(v11, q, v11 * ql);
         p[3] = -fma(v01 + v10, q, (v01 + v10) * ql);
         p[4] = fma(v00, q, v00 * ql);
