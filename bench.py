@@ -413,7 +413,10 @@ def bench_scene(args, dev, flush, clk, cpu_seconds):
     nsm = torch.cuda.get_device_properties(dev).multi_processor_count
     peak_clk = clk['sm_mhz'] if clk else 1965.0
     peak = SFU_EX2_PER_CLK_PER_SM * nsm * peak_clk * 1e6 / 1e9
-    achieved = pixcomp / render_s / 1e9
+    # the exponential of a component follows from four ex2 for two columns of
+    # four rows (sharp components, which take one each, are not counted)
+    ex2 = pixcomp / 2
+    achieved = ex2 / render_s / 1e9
     line = {
         'workload': SCENE_WORKLOAD,
         'metric': 'Mpix*components/s (batched scene render)',
@@ -429,8 +432,8 @@ def bench_scene(args, dev, flush, clk, cpu_seconds):
         'roofline': {'bound': 'sfu', 'kernel': 'tb_scene_render (bin + render)',
                      'achieved': achieved, 'peak': peak, 'unit': 'Gex2/s',
                      'frac': achieved / peak,
-                     'algorithmic': 'sum over sources of rectangle pixels x components = '
-                                    '%.0f ex2 per launch' % pixcomp,
+                     'algorithmic': 'sum over sources of rectangle pixels x components = %.0f, '
+                                    'half an ex2 each' % pixcomp,
                      'kernel_ms': render_s * 1e3,
                      'traffic': ncu_traffic('scene_render_c3.json')},
     }
@@ -710,7 +713,7 @@ def bench_derivs(args, dev, flush, clk, cpu_seconds):
     it_t, camp, cvar, dcoef, flg, misc = jac._work(n)
 
     def prep():
-        jac._prep(d_src, n, _lib.MOG_STORE, npix, _lib.stream_ptr())
+        jac._prep(d_src, n, _lib.MOG_STORE, npix, None)
 
     def columns():
         render.fourier_render(it_t.data_ptr(), 7 * n, camp.data_ptr(), cvar.data_ptr(),
@@ -1476,9 +1479,6 @@ def main():
     clocks = ClockSampler(gpu_id)
     clocks.start()
     time.sleep(0.3)
-    # split: the sort and the render; persistent: one launch
-    # after the prep; fused: one launch in all
-    launches_per_render = 2 if method == 'split' else 1
     ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True),
            torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
     for k in range(args.steps):
@@ -1497,6 +1497,10 @@ def main():
                                           items_t.data_ptr(), flg.data_ptr(), misc.data_ptr(),
                                           misc.data_ptr() + 16, _lib.stream_ptr())
             _lib.check(rc, 'tb_galaxy_fft_render')
+        elif method == 'split':
+            # preparation and sort, then the render, by one call
+            e1.record(stream)
+            renderer.render_device(d_src, n, out, method='split')
         else:
             rc = lib.tb_galaxy_fft_prep(d_src.data_ptr(), n,
                                         __import__('ctypes').addressof(renderer.image),
@@ -1507,11 +1511,10 @@ def main():
             e1.record(stream)
             R.fourier_render(items_t.data_ptr(), n, camp.data_ptr(), cvar.data_ptr(),
                              renderer.spec.data_ptr(), out.data_ptr(), misc.data_ptr() + 16,
-                             method=method,
-                             workspace=renderer._workspace(n) if method == 'split' else None)
+                             method=method)
         e2.record(stream)
     torch.cuda.synchronize()
-    gpu_launches = ((0 if method == 'fused' else 1) + launches_per_render) * args.steps
+    gpu_launches = (1 if method == 'fused' else 2) * args.steps
     step_ms = [a.elapsed_time(c) for a, b, c in ev]
     render_ms = [b.elapsed_time(c) for a, b, c in ev]
     t_total = sum(step_ms) / 1e3
@@ -1554,8 +1557,7 @@ def main():
         t = torch.tensor([e2e_s], device=dev)
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         e2e_s = float(t.item())
-    R.check_status(renderer.status(n).clone(), 'tb_galaxy_fft_render' if method == 'fused'
-                   else 'tb_fourier_render')
+    R.check_status(renderer.status(n).clone(), 'render (%s)' % method)
 
     job_pixcomp = pixcomp
     gather_ms = None
@@ -1595,7 +1597,8 @@ def main():
         'gpu_launches': gpu_launches,
         'fourier_method': {'chosen': method, 'ms': {k: _sig(v) for k, v in tune.items()}},
         'roofline': {'bound': 'sfu', 'kernel': {
-                         'split': 'tb_fourier_render_split (sort + render by FFT size)',
+                         'split': 'tb_galaxy_fft_render_sorted (preparation + sort by FFT '
+                                  'size, render)',
                          'persistent': 'tb_fourier_render (persistent)',
                          'fused': 'tb_galaxy_fft_render (preparation + persistent render, '
                                   'one launch)'}[method],

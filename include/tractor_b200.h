@@ -562,13 +562,14 @@ int tb_tensor_core_timeouts(uint32_t* count);
 
 /* Solves each problem's column-scaled normal equations in FP64 on the device
  * (column scaling as lsqr_optimizer.py:470-489 with scale = sqrt(diag),
- * Cholesky with a `damp`^2 ridge, one step of iterative refinement) and
+ * LDL^T with a `damp`^2 ridge, one step of iterative refinement) and
  * writes X[x_off[b] + i] = update / colscale (zero for empty columns).
  * info[b] = 0 ok, >0 the failing pivot (not positive definite; X is then
  * zero, as LsqrOptimizer returns a zero update on failure,
  * lsqr_optimizer.py:586-604), -1 if P[b] > 320 or P[b] > max_p (the
  * problem is skipped and its X left as it was).  work: caller-owned FP64
- * scratch of n_problems * max_p * max_p elements (the Cholesky factors). */
+ * scratch of n_problems * max_p * max_p elements (the factors of problems of
+ * more than 232 parameters; the others' lie in shared memory). */
 int tb_solve_update(const double* AtA, const double* Atr,
                     const int64_t* ata_off, const int64_t* atr_off,
                     const int32_t* P, const int64_t* x_off, double* X,
@@ -580,9 +581,9 @@ int tb_solve_update(const double* AtA, const double* Atr,
  * call -- code that runs under another allocator that owns the device
  * memory, or latency-bound loops where an allocation, which can
  * synchronise the device, is not acceptable -- and so cannot provide the
- * `work` buffer.  The Cholesky factors go to a file-scope scratch array of
- * TB_SOLVE_NOALLOC_MAX_DOUBLES doubles (8 MiB) that the library holds on
- * every GPU that loads it, until the process exits.  Requires
+ * `work` buffer.  Factors of more than 232 parameters go to a file-scope
+ * scratch array of TB_SOLVE_NOALLOC_MAX_DOUBLES doubles (8 MiB) that the library
+ * holds on every GPU that loads it, until the process exits.  Requires
  * n_problems * max_p * max_p <= TB_SOLVE_NOALLOC_MAX_DOUBLES, else returns
  * TB_ERR_SIZE.  The first call on a device looks up the array's device
  * address (cudaGetSymbolAddress) with that device current; make that first
@@ -638,7 +639,7 @@ typedef struct {
 } tb_fit_source;
 
 /* Buffers of blob b: hbuf + h_off holds (n_slices + 2) P x P FP64 blocks
- * (per-slice partial A^T A, accepted A^T A, Cholesky factor); gbuf + g_off
+ * (per-slice partial A^T A, accepted A^T A, LDL^T factor); gbuf + g_off
  * holds (n_slices + 1) P-vectors (per-slice A^T r, accepted).  A slice is
  * one pass unit's share: a band's image, or a range of its active tiles; the
  * passes fill the slices of A^T A and A^T r compactly, over the sources their
@@ -731,10 +732,14 @@ int tb_fit_pass(const tb_fit_unit* units, const int32_t* order, int32_t n_units,
 /* One Levenberg-Marquardt step per running blob: accept the trial
  * parameters if chi^2 fell (the first pass is always accepted; the damping
  * then follows the ratio rho of the actual to the predicted gain, lambda x
- * max(1/3, 1 - (2 rho - 1)^3)), else raise the damping x 10; solve (D^-1 H D^-1 + lambda I) x = D^-1 g, D = sqrt(diag H),
- * by FP64 Cholesky with one refinement step; scale the step to respect the
- * maximum steps (PixPos 1, log r_e 1, ee 0.1, n 0.1) and the Sersic-index
- * bounds; write params + step into `trial`.  Stops a blob when the step's
+ * max(1/3, 1 - (2 rho - 1)^3)), else raise the damping x 10; solve
+ * (D^-1 H D^-1 + lambda I) x = D^-1 g, D = sqrt(diag H), by FP64 LDL^T with one
+ * refinement step; limit the step to respect the maximum steps (PixPos 1,
+ * log r_e 1, ee 0.1, n 0.1) and the Sersic-index bounds, by scaling it as a
+ * whole or, in a blob's iterations after the 8th, where a scale below 1/2 would
+ * be needed and the model expects more of it, by holding the parameters beyond
+ * their limits there and solving for the others; write params + step into
+ * `trial`.  Stops a blob when the step's
  * predicted log-likelihood gain is below `tol` with lambda <= 1
  * (optimize_loop's dchisq, tested on the prediction). */
 int tb_fit_step(const tb_fit_blob* blobs, int32_t n_blobs, int32_t n_bands,

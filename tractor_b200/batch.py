@@ -128,11 +128,6 @@ class FourierGalaxyRenderer(object):
                 S.view(w, 1, n * COMP_STRIDE * 8, torch.float64),
                 S.view(w, 2, n * COMP_STRIDE * 32, torch.float64), w[3], w[4])
 
-    def _workspace(self, n, stream=None):
-        """(address, bytes) of the sorted path's workspace."""
-        w = self._scratch.get(n, stream)
-        return w[1][3], w[2][3]
-
     METHODS = ('fused', 'persistent', 'split')
 
     def choose(self, n, pixels):

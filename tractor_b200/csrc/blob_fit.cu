@@ -12,17 +12,17 @@
 //                with respect to (log r_e, ee1, ee2) -- FP64 central
 //                differences of the exact FP64 maps (sersic.py:288-342,
 //                ellipses.py:165-263);
-//   tb_fit_pass  one CTA per (blob, band) image, 32 x 8 pixel tiles: the
-//                model (every source's PSF-convolved mixture, as
-//                galaxy.py:307-326) and the analytic derivative columns
-//                (position, flux, shape, index), weighted by inverr; A^T A,
-//                A^T r and r^T r into the slice the CTA owns (no atomics);
+//   tb_fit_pass  persistent CTAs take units of a few 32 x 8 pixel tiles of a
+//                (blob, band) image: the model (every source's PSF-convolved
+//                mixture, as galaxy.py:307-326) and the analytic derivative
+//                columns (position, flux, shape, index), weighted by inverr;
+//                A^T A, A^T r and r^T r into the unit's own slice (no atomics);
 //   tb_fit_step  sums the slices (many CTAs per blob), then one CTA per blob:
-//                accepts or
-//                rejects the trial parameters, solves the Marquardt-damped
-//                normal equations by FP64 Cholesky with one refinement step,
-//                limits the step (bounds, maximum steps) and writes the next
-//                trial parameters.
+//                accepts or rejects the trial parameters, solves the
+//                Marquardt-damped normal equations (FP64 LDL^T, one refinement
+//                step), limits the step (bounds, maximum steps: scaled as a
+//                whole, or, for a blob slow to converge, minimised within them)
+//                and writes the next trial parameters.
 #include "ldl.cuh"
 #include "profile_eval.cuh"
 

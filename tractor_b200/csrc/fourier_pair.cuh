@@ -26,8 +26,8 @@
 // on a galaxy of size 256 and a 128 x 128 window, mostly waiting for
 // instructions; packing halves the transforms' instructions.
 // Measured, with the preparation: 256 galaxies of size 256 on 128 x 128 patches
-// 84 us fused, 77 us fourier_render_kernel, 74 us here; 2,000 on ragged 25-253
-// px patches 568, 516, 379; 2,000 on 100 x 100 (size 128) 252, 225, 146.  A
+// 87 us fused, 78 us fourier_render_kernel, 74 us here; 2,000 on ragged 25-253
+// px patches 568, 516, 346; 2,000 on 100 x 100 (size 128) 252, 225, 146.  A
 // galaxy of size 256 takes 49 K cycles (columns 33 K, rows 11 K, the rest its
 // preparation, which nothing overlaps), at 1.7 instructions per cycle: held by
 // fixed latencies at 16 warps (128 registers) and the phases' barriers.

@@ -4,7 +4,7 @@
 //    tensor cores (tcgen05 kind::tf32, three-term TF32 split, FP32 partial
 //    sums over at most 128 rows, FP64 totals) for P <= 255; above that
 //    FP32 CUDA-core products with compensated (Kahan) FP32 running sums;
-//  * FP64 column-scaled Cholesky solve with a damping ridge and one step of
+//  * FP64 column-scaled solve (LDL^T) with a damping ridge and one step of
 //    iterative refinement, one CTA per problem;
 //  * per-image chi^2 with compensated FP32 sums reduced in FP64 in a fixed
 //    order (deterministic).
@@ -615,10 +615,12 @@ chi2_kernel(const float* __restrict__ data, const float* __restrict__ model,
 // error grows with that count.  Warps 9-12 drain a finished chunk (`accfull`):
 // they copy the accumulators to shared memory, release them (`accfree`) and
 // add S + E + E^T of the blocks on or above the diagonal to compensated
-// (Kahan) FP32 totals there.  The next chunk's MMAs wait for the release:
-// TMEM loads that ran while MMAs into the other set were in flight returned
-// wrong values on B200 (two column layouts tried).  The FP64 results are
-// written once at the end, AtA exactly symmetric.
+// (Kahan) FP32 totals there.  The next chunk's MMAs wait for the release, so
+// one set would do: an earlier form, whose converter warps drained a set while
+// MMAs filled the other, gave wrong sums, and why was not found.  It is no
+// limit of the tensor memory: the MMAs of the SM's other CTA run during these
+// loads, into columns of its own, and the sums agree with FP64.  The FP64
+// results are written once at the end, AtA exactly symmetric.
 //
 // Bound: the shared-memory traffic of the operands (82 % of L1's throughput
 // when the loads also went through it) and the hand-over of each stage; the
@@ -722,8 +724,8 @@ normal_eq_tc64_kernel(const float* __restrict__ A, const float* __restrict__ rhs
             const int bi = s & 1, c = s / kChunkSt;
             if (lane == 0) {
                 ok = mbar_wait(&full[bi], (s >> 1) & 1, kWaitNs);
-                // the previous chunk has been drained: no TMEM load of a drain
-                // runs while MMAs are in flight
+                // the previous chunk has been drained (see above: none of this
+                // CTA's TMEM loads runs while its MMAs are in flight)
                 if (ok && s % kChunkSt == 0 && c >= 1)
                     ok = mbar_wait(&accfree[(c - 1) & 1], ((c - 1) >> 1) & 1, kWaitNs);
                 if (ok) {

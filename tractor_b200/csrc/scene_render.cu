@@ -11,8 +11,8 @@
 // 3. tb_scene_render: a persistent kernel takes image tiles from a global
 //    counter.  For a tile it sorts the listed items by index (catalog order),
 //    stages their components -- culled against the part of the tile inside
-//    each item's rectangle -- in shared memory, evaluates them with one SFU
-//    ex2 per pixel and component, sums each source's components into a
+//    each item's rectangle -- in shared memory, evaluates them (a few ex2 for
+//    a thread's rows, carried down its columns), sums each source's components into a
 //    per-source partial (the reference's patch), adds the partial inside the
 //    rectangle to the tile accumulator, and writes every tile pixel once.
 //    No float atomics; the result does not depend on scheduling.

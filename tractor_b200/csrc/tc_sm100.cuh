@@ -121,7 +121,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
                  : "memory");
 }
 
-// 32 consecutive TMEM columns of this warp's 32 lanes (one value per lane
+// 16 consecutive TMEM columns of this warp's 32 lanes (one value per lane
 // and column); the load is complete when the function returns.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
@@ -138,6 +138,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// The same for 32 columns.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     uint32_t r[32];
     asm volatile(

@@ -234,11 +234,11 @@ class BlobFitter(object):
         blob's steps to converge.  With `refine`, the FP32 phase also ends
         once at most a fraction `handoff` of the blobs still runs: those
         continue in the FP64 phase from where they are.  The slowest blobs
-        of a 2,000-blob fit of 192-512 px blobs need about 60 FP64
+        of a 2,000-blob fit of 192-512 px blobs need 53 to 80 FP64
         iterations (Gauss-Newton steps rejected and re-damped along an
-        ill-conditioned direction); 40 left some of them several sigma from
-        the optimum.  Returns the number of iterations launched (both
-        phases)."""
+        ill-conditioned direction); the last of some sets still gains 1e-8 in
+        log-likelihood per iteration at 100.  Returns the number of
+        iterations launched (both phases)."""
         self.reset(params0, lambda0)
         g = None
         if graph:

@@ -764,7 +764,7 @@ def solve_dense(A_colmajor, b, damp=0., stream=None):
 
 
 def solve_update(AtA, Atr, ata_off, atr_off, P, damp=0., stream=None):
-    """Column-scaled FP64 Cholesky solve + one refinement step per problem.
+    """Column-scaled FP64 solve (LDL^T) + one refinement step per problem.
     Returns (X float64 device tensor, info int32 device tensor, x_off)."""
     lib = _lib.load()
     dev = AtA.device
