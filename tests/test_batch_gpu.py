@@ -286,3 +286,30 @@ def test_choice_of_method(tb):
                           (m + 1, 40, 'persistent'), (2 * m + 1, 40, 'split'), (1, 128, 'split'),
                           (2000, 253, 'split')):
         assert r.choose(n, n * side * side) == want
+
+
+def test_captured_render_and_gradient(tb):
+    """A render and a vector-Jacobian product captured in a graph without a
+    warm-up on its stream (their scratch is then the graph's), beside calls
+    outside of it on other streams and sizes: replays give the same bits."""
+    import torch
+    from tractor_b200 import batch, grad
+    r = batch.FourierGalaxyRenderer(batch.moffat_psf(45))
+    jac = grad.FourierJacobian(r)
+    s = batch.sersic_sources(40, np.random.default_rng(78), mask=np.arange(30, 150, 3))
+    d = torch.from_numpy(s.view(np.uint8).copy()).cuda()
+    npix = int((s['mw'].astype(np.int64) * s['mh']).sum())
+    g = torch.randn(npix, generator=torch.Generator(device='cuda').manual_seed(9), device='cuda')
+    out = torch.zeros(npix, device='cuda')
+    r.render_device(d, 40, out)
+    want = out.clone(), jac.vjp(d, 40, g)[0].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        r.render_device(d, 40, out)
+        dots = jac.vjp(d, 40, g)[0]
+    for _ in range(3):
+        out.zero_()
+        dots.zero_()
+        graph.replay()
+        r.render_device(d, 17, torch.empty_like(out))
+        assert torch.equal(out, want[0]) and torch.equal(dots, want[1])
