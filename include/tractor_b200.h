@@ -736,7 +736,7 @@ int tb_fit_pass(const tb_fit_unit* units, const int32_t* order, int32_t n_units,
  * (D^-1 H D^-1 + lambda I) x = D^-1 g, D = sqrt(diag H), by FP64 LDL^T with one
  * refinement step; limit the step to respect the maximum steps (PixPos 1,
  * log r_e 1, ee 0.1, n 0.1) and the Sersic-index bounds, by scaling it as a
- * whole or, in a blob's iterations after the 8th, where a scale below 1/2 would
+ * whole or, in a blob's iterations after the 8th, where a scale below 1/5 would
  * be needed and the model expects more of it, by holding the parameters beyond
  * their limits there and solving for the others; write params + step into
  * `trial`.  Stops a blob when the step's

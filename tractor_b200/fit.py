@@ -234,7 +234,7 @@ class BlobFitter(object):
         blob's steps to converge.  With `refine`, the FP32 phase also ends
         once at most a fraction `handoff` of the blobs still runs: those
         continue in the FP64 phase from where they are.  The slowest blobs
-        of a 2,000-blob fit of 192-512 px blobs need 53 to 80 FP64
+        of a 2,000-blob fit of 192-512 px blobs need 55 to 94 FP64
         iterations (Gauss-Newton steps rejected and re-damped along an
         ill-conditioned direction); the last of some sets still gains 1e-8 in
         log-likelihood per iteration at 100.  Returns the number of
